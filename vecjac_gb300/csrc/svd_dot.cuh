@@ -58,14 +58,66 @@ template <typename T, bool CPLX> struct DotTerms {
   T pd[CPLX ? 4 : 1], dn[CPLX ? 4 : 1];
 };
 
-// The accumulation uses branch-free 2Sum: on GB300 a value moving from the FP64 unit to
-// the integer pipes (as Fast2Sum's magnitude test would need) costs several hundred
-// cycles, more than 2Sum's three extra FP64 additions.
-template <typename T>
-__device__ __forceinline__ void dot_acc(T pd, T dn, T &s, T &t, T &s_, T &t_)
+// FP64 additions and products as three-register FMAs. GB300's FP64 unit takes a warp
+// instruction every 16 clocks per SM when all three operands come from registers and every
+// 19 when it is a DADD, a DMUL or an FMA with a constant operand (measured with 4 to 16
+// warps of independent chains; the latency of 64 clocks is the same), so a + b is formed as
+// a * 1 + b and the round-down product as a * b + (-0), with the 1 and the -0 held in
+// registers. The values are those of the plain operations; only a zero product may come out
+// as -0 instead of +0, which no sum below can tell apart (a sum that starts at +0 never
+// becomes -0 in round-to-nearest).
+template <typename T> struct DotOps {
+  static __device__ __forceinline__ DotOps make() { return DotOps(); }
+  __device__ __forceinline__ T add(T a, T b) const { return a + b; }
+  __device__ __forceinline__ T sub(T a, T b) const { return a - b; }
+  __device__ __forceinline__ T mul_rd(T a, T b) const { return fp<T>::mul_rd(a, b); }
+};
+#ifdef __CUDA_ARCH__
+template <> struct DotOps<double> {
+  double one, mzero;
+  static __device__ __forceinline__ DotOps make()
+  {
+    DotOps o;
+    o.one = 1.0;
+    o.mzero = -0.0;
+    asm("" : "+d"(o.one), "+d"(o.mzero));  // registers, not constants
+    return o;
+  }
+  __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
+  __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(a, one, -b); }
+  __device__ __forceinline__ double mul_rd(double a, double b) const { return __fma_rd(a, b, mzero); }
+};
+#endif
+
+// One step of a 2Sum recurrence, (s, t) := (RN(s + b), s + b - RN(s + b)) with b = p + t.
+// FP64: Dekker's Fast2Sum on the operands ordered by their high words. Fast2Sum's error is
+// exact when the first operand's exponent is not below the second's (T. J. Dekker, "A
+// floating-point technique for extending the available precision", Numer. Math. 18, 1971),
+// which is 2Sum's error too, and the error of an addition is unique. That is 3 instead of 6
+// FP64 operations after p + t; the comparison and the four selects run on the integer pipes
+// while the FP64 unit forms s + b. Measured on one warp: 328 clocks per step against 448
+// (2Sum), and 341 against 533 with one warp on each sub-partition. (An infinite s + b leaves
+// t infinite or NaN and the dot product not finite, as with 2Sum.) FP32, where an addition
+// costs no more than a select, keeps 2Sum.
+template <typename T> __device__ __forceinline__ void sum_step(const DotOps<T> &o, T p, T &s, T &t)
 {
-  two_sum(s, pd + t, s, t);
-  two_sum(s_, dn + t_, s_, t_);
+  const T b = o.add(p, t);
+  if constexpr (sizeof(T) == 8) {
+    const T r = o.add(s, b);
+    const bool sw = ((unsigned)(fp<T>::bits(b) >> 32) << 1) > ((unsigned)(fp<T>::bits(s) >> 32) << 1);
+    const T h = sw ? b : s, l = sw ? s : b;
+    t = o.sub(l, o.sub(r, h));
+    s = r;
+  }
+  else
+    two_sum(s, b, s, t);
+}
+
+template <typename T>
+__device__ __forceinline__ void dot_acc(const DotOps<T> &o, T pd, T dn, T &s, T &t, T &s_, T &t_)
+{
+  sum_step(o, pd, s, t);
+  sum_step(o, dn, s_, t_);
 }
 
 template <typename T, bool CPLX>
@@ -78,6 +130,7 @@ __device__ void pair_dot(long long m, const T *xr, const T *xi, const T *yr, con
   constexpr int D = 4;              // elements per block (the next block's loads in flight)
   const int lane = (threadIdx.x & 31) % L;
   const int nx = -(int)ex, ny = -(int)ey;
+  const DotOps<T> o = DotOps<T>::make();
   T sr = 0, tr = 0, sr_ = 0, tr_ = 0, si = 0, ti = 0, si_ = 0, ti_ = 0;
   auto load = [&](long long i, T (&v)[NV]) {
     if (i < m) {
@@ -96,24 +149,24 @@ __device__ void pair_dot(long long m, const T *xr, const T *xi, const T *yr, con
       const T xs[4] = {xri, xii, xri, -xii}, ys[4] = {yri, yii, yii, yri};
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        d.pd[k] = F::mul_rd(xs[k], ys[k]);
+        d.pd[k] = o.mul_rd(xs[k], ys[k]);
         d.dn[k] = F::fma_(xs[k], ys[k], -d.pd[k]);
       }
     }
     else {
-      d.pd[0] = F::mul_rd(xri, yri);
+      d.pd[0] = o.mul_rd(xri, yri);
       d.dn[0] = F::fma_(xri, yri, -d.pd[0]);
     }
   };
   auto accumulate = [&](const DotTerms<T, CPLX> &c) {
     if (CPLX) {
-      dot_acc(c.pd[0], c.dn[0], sr, tr, sr_, tr_);
-      dot_acc(c.pd[1], c.dn[1], sr, tr, sr_, tr_);
-      dot_acc(c.pd[2], c.dn[2], si, ti, si_, ti_);
-      dot_acc(c.pd[3], c.dn[3], si, ti, si_, ti_);
+      dot_acc(o, c.pd[0], c.dn[0], sr, tr, sr_, tr_);
+      dot_acc(o, c.pd[1], c.dn[1], sr, tr, sr_, tr_);
+      dot_acc(o, c.pd[2], c.dn[2], si, ti, si_, ti_);
+      dot_acc(o, c.pd[3], c.dn[3], si, ti, si_, ti_);
     }
     else
-      dot_acc(c.pd[0], c.dn[0], sr, tr, sr_, tr_);
+      dot_acc(o, c.pd[0], c.dn[0], sr, tr, sr_, tr_);
   };
   auto normal_after = [&](T w, int n) {
     const int be = (int)((F::bits(w) & ~F::SIGN) >> F::MB);
@@ -200,6 +253,7 @@ __device__ void chain_dot(long long m, const T *xr, const T *xi, const T *yr, co
   constexpr int D = CPLX ? 4 : 8;   // elements per block: the next block's loads are in flight
                                     // while this block is accumulated (hides L2 latency)
   const int nx = -(int)ex, ny = -(int)ey;
+  const DotOps<T> o = DotOps<T>::make();
   T s = 0, t = 0;
   auto load = [&](long long i, T (&v)[NV]) {
     if (i < m) {
@@ -215,11 +269,11 @@ __device__ void chain_dot(long long m, const T *xr, const T *xi, const T *yr, co
   // xr yi, xi (-yr) (= (-xi) yr exactly)
   auto terms = [&](T xr_, T yr_, T xi_, T yi_, T (&v)[NT]) {
     const T a0 = xr_, b0 = (CPLX && IM) ? yi_ : yr_;
-    const T q0 = F::mul_rd(a0, b0);
+    const T q0 = o.mul_rd(a0, b0);
     v[0] = DN ? F::fma_(a0, b0, -q0) : q0;
     if (CPLX) {
       const T a1 = xi_, b1 = IM ? -yr_ : yi_;
-      const T q1 = F::mul_rd(a1, b1);
+      const T q1 = o.mul_rd(a1, b1);
       v[NT - 1] = DN ? F::fma_(a1, b1, -q1) : q1;
     }
   };
@@ -229,7 +283,7 @@ __device__ void chain_dot(long long m, const T *xr, const T *xi, const T *yr, co
     terms(scale2(w[0], nx), scale2(w[1], ny), CPLX ? scale2(w[2], nx) : (T)0, CPLX ? scale2(w[3], ny) : (T)0, v);
 #pragma unroll
     for (int k = 0; k < NT; ++k)
-      two_sum(s, v[k] + t, s, t);
+      sum_step(o, v[k], s, t);
   };
   // the power-of-two scaling of a normal value to a normal result is an integer add on the
   // exponent field (scale2's fast path)
@@ -266,7 +320,7 @@ __device__ void chain_dot(long long m, const T *xr, const T *xi, const T *yr, co
         for (int d = 0; d < D; ++d)
 #pragma unroll
           for (int k = 0; k < NT; ++k)
-            two_sum(s, v[d][k] + t, s, t);
+            sum_step(o, v[d][k], s, t);
       }
       else {
 #pragma unroll
