@@ -214,7 +214,7 @@ template <typename T> __device__ long long svd_one(const BatchArgs<T> &a, BatchS
         return sh.err;
       swt += sh.cnt;
       // ---- all transformations (src/dvjsvd.c:460-574), one pair per warp at a time ----
-      unsigned long long mG = 0ull, mV = 0ull;
+      typename F::U mx[2] = {0, 0}, mV = 0;
       for (long long k = warp; k < n_2; k += nw) {
         unsigned p, q;
         step_pair(a.strategy, (unsigned)n, st, (unsigned)k, p, q);
@@ -226,14 +226,14 @@ template <typename T> __device__ long long svd_one(const BatchArgs<T> &a, BatchS
         T *Gp = G + (long long)p * m, *Gq = G + (long long)q * m;
         pair_apply<T, false, false>(s, m, n, Gp, Gq, nullptr, nullptr, V + (long long)p * n, V + (long long)q * n,
                                     nullptr, nullptr, Gp, Gq, nullptr, nullptr, eS + p, eS + q, fS + p, fS + q,
-                                    lane, 32, mG, mV);
+                                    lane, 32, false, mx, mV);
         if (lane == 0) {
           const int c = s.code;
           sh.w1[p] = (c == 2 || c == -2) ? 1 : 0;
           sh.w1[q] = (c == 2 || c == -2 || c == 3 || c == -3) ? 1 : 0;
         }
       }
-      mG = warp_max_u64(mG);
+      const unsigned long long mG = warp_max_u64((unsigned long long)((mx[0] > mx[1]) ? mx[0] : mx[1]));
       if (lane == 0 && mG)
         atomicMax(&sh.nmg, mG);
       __syncthreads();

@@ -39,22 +39,145 @@
 
 namespace vj {
 
-// Pairs handled by one CTA: the LANES-wide dot of pair j runs on lanes [j LANES,
-// (j+1) LANES) of warp 0. GB300's FP64 unit accepts about one warp instruction every 19
-// cycles per SM whatever the number of active lanes, so the four FP64 dot products of a
-// CTA share every FP64 instruction (32 active lanes) instead of issuing four.
-template <typename T> struct ppc { static constexpr int P = 32 / svdc<T>::LANES; };
+// ---- one pivot step ----
+// A CTA owns P pairs. The dot products of a pair are NCH accumulator chains (2 for real, 4
+// for complex data: round-down products and their errors, real and imaginary parts), each of
+// LANES lanes and each a serial recurrence over the rows; a (pair, chain) group of LANES lanes
+// sits on one of the CTA's first warps, the chain warps, which do nothing but the recurrence:
+// all eight warps scale the columns and form the products of the first chunk of rows, and then
+// the other warps those of the next chunk into the second of two shared-memory buffers while
+// the chain warps accumulate this one. The recurrence is the step's floor (FP64: 330 clocks
+// per row of a lane, m / 8 rows), and products, checks and scalings in the same warp had
+// doubled it: at 1024 x 1024 real the dots took 78.7k of a step's 134k clocks.
+template <typename T, bool CPLX, int P> struct StepDims {
+  static constexpr int L = svdc<T>::LANES;
+  static constexpr int NCH = CPLX ? 4 : 2;                  // chains per pair
+  static constexpr int NT = CPLX ? 2 : 1;                   // terms per row and chain
+  static constexpr int NG = P * NCH;                        // (pair, chain) groups
+  static constexpr int NCW = (NG * L + 31) / 32;            // chain warps
+  static constexpr int K = ((sizeof(T) == 8) ? 16 : 32) / NT;  // rows per lane and chunk
+  static constexpr int RC = K * L;                          // rows per chunk
+  static constexpr int BUF = K * NT * NG * L;               // elements of one buffer
+  static constexpr size_t buf_bytes() { return 2u * (size_t)BUF * sizeof(T); }
+  static_assert(NCW <= 4, "at least half of the warps form products");
+};
 
-template <typename T, bool CPLX, bool TRACKV, bool STAGE>
+// The FP64 / FP32 2x2 of jac2.cuh (cosine and tangent form) by the four lanes of a quad, r =
+// lane % 4, base = lane - r, all 32 lanes of the warp converged: the last three divisions of
+// the formulas (c, L1, L2; also the two of the complex direction) are independent and take the
+// place of one, each on its lane. One pair's 2x2 is latency (four dependent divisions and two
+// or three roots) with nothing else to run in the CTA.
+template <typename T> __device__ unsigned rjac2_quad(T a1, T a2, T ar, int r, int base, T &c, T &at)
+{
+  using F = fp<T>;
+  const T one = (T)1;
+  const int b1 = bexp(a1), b2 = bexp(a2), br = bexp(ar);
+  int bmax = max(max(b1, b2), br);
+  const int bmin = min(min(b1, b2), br);
+  const bool fast = bmin > 0 && bmax <= F::EMAXB && bmax - bmin < fastc<T>::TOP;
+  r2out<T> g = {};
+  if (!fast) {
+    g = rjac2_gen<T, 0>(a1, a2, ar);
+    a1 = a2 = ar = one;
+    bmax = F::BIAS;
+  }
+  const int es = fastc<T>::TOP - bmax;
+  ar = addexp(ar, es);
+  a1 = addexp(a1, es);
+  a2 = addexp(a2, es);
+  const T as = vsgn(ar), ab = addexp(vabs(ar), 1);
+  T ad;
+  const angle<T> n = jac_angle<T, true>(a1, a2, ab, ad);
+  const T num = (r == 1)   ? F::fma_(n.t1, F::fma_(a2, n.t1, ab), a1)
+                : (r == 2) ? F::fma_(n.t1, F::fma_(a1, n.t1, -ab), a2)
+                           : one;
+  const T q = qdiv(num, (r == 1 || r == 2) ? n.s2 : n.s1);
+  c = __shfl_sync(0xffffffffu, q, base);
+  const T L1 = __shfl_sync(0xffffffffu, q, base + 1), L2 = __shfl_sync(0xffffffffu, q, base + 2);
+  at = vxor(n.t1, as);
+  unsigned bit = lt_fin(L1, L2) ? 1u : 0u;
+  if (!fast) {
+    c = g.c;
+    at = g.at;
+    bit = g.bit;
+  }
+  return bit;
+}
+
+template <typename T>
+__device__ unsigned cjac2_quad(T a1, T a2, T ar, T ai, int r, int base, T &c, T &cat, T &sat)
+{
+  using F = fp<T>;
+  const T one = (T)1;
+  const int b1 = bexp(a1), b2 = bexp(a2), br = bexp(ar), bi = bexp(ai);
+  int bmax = max(max(b1, b2), max(br, bi));
+  const int bmin = min(min(b1, b2), min(br, bi));
+  const bool fast = bmin > 0 && bmax <= F::EMAXB && bmax - bmin < fastc<T>::TOP;
+  c2out<T> g = {};
+  if (!fast) {
+    g = cjac2_gen<T, 0>(a1, a2, ar, ai);
+    a1 = a2 = ar = ai = one;
+    bmax = F::BIAS;
+  }
+  const int es = fastc<T>::TOP - bmax;
+  ar = addexp(ar, es);
+  ai = addexp(ai, es);
+  a1 = addexp(a1, es);
+  a2 = addexp(a2, es);
+  T ar_ = vabs(ar), ai_ = vabs(ai);
+  const T as = vsgn(ar);
+  const T am = nnmin(ar_, ai_), aM = nnmax(ar_, ai_);
+  T aa = qdiv(am, aM);
+  aa = sqrt_ge1(F::fma_(aa, aa, one)) * aM;
+  T q = qdiv((r & 1) ? ai : ar_, aa);
+  ar_ = vor(nnmin(__shfl_sync(0xffffffffu, q, base), one), as);
+  ai_ = __shfl_sync(0xffffffffu, q, base + 1);
+  const T ab = addexp(aa, 1);
+  T ad;
+  const angle<T> n = jac_angle<T, true>(a1, a2, ab, ad);
+  const T num = (r == 1)   ? F::fma_(n.t1, F::fma_(a2, n.t1, ab), a1)
+                : (r == 2) ? F::fma_(n.t1, F::fma_(a1, n.t1, -ab), a2)
+                           : one;
+  q = qdiv(num, (r == 1 || r == 2) ? n.s2 : n.s1);
+  c = __shfl_sync(0xffffffffu, q, base);
+  const T L1 = __shfl_sync(0xffffffffu, q, base + 1), L2 = __shfl_sync(0xffffffffu, q, base + 2);
+  cat = ar_ * n.t1;
+  sat = ai_ * n.t1;
+  unsigned bit = lt_fin(L1, L2) ? 1u : 0u;
+  if (!fast) {
+    c = g.c;
+    cat = g.cat;
+    sat = g.sat;
+    bit = g.bit;
+  }
+  return bit;
+}
+
+// the warp's largest value, on every lane
+__device__ __forceinline__ unsigned warp_max_bits(unsigned v) { return __reduce_max_sync(0xffffffffu, v); }
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v)
+{
+  const unsigned h = (unsigned)(v >> 32), hm = __reduce_max_sync(0xffffffffu, h);
+  const unsigned lm = __reduce_max_sync(0xffffffffu, (h == hm) ? (unsigned)v : 0u);
+  return ((unsigned long long)hm << 32) | lm;
+}
+
+template <typename T, bool CPLX, bool STAGE, int P>
 __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int last)
 {
   using F = fp<T>;
-  constexpr int P = ppc<T>::P;
-  constexpr int L = svdc<T>::LANES;
+  using U = typename F::U;
+  using D = StepDims<T, CPLX, P>;
+  constexpr int L = D::L;
   constexpr int NC = CPLX ? 4 : 2;   // staged columns per pair (real and imaginary planes)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ PairState<T> ps[P];
-  __shared__ unsigned long long red[8][2];
+  __shared__ PairPre<T> pre[P];
+  __shared__ T dsum[D::NG][2];
+  __shared__ U cmx[P][NC];           // largest |.| of the changed columns' planes
+  __shared__ U vmx;
+  __shared__ T cnrm[2 * P][CPLX ? 2 : 1];
+  __shared__ int s_col[P][2], s_n[P][2], s_live[P], s_trk[P];
   __shared__ int s_err;
   __shared__ unsigned long long bar;
   pdl_enter();
@@ -78,6 +201,18 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
       tmark = t;
     }
   };
+  if (tid < 2 * P) {
+    const int j = tid >> 1, c = tid & 1;
+    s_col[j][c] = (j < np) ? (int)r[2 * (pair0 + j) + c] : 0;
+  }
+  if (tid < P * NC)
+    cmx[tid / NC][tid % NC] = 0;
+  if (tid == 0) {
+    s_err = 0;
+    vmx = 0;
+    if (STAGE)
+      mbar_init(&bar, 1u);
+  }
   const Decision<T> d = decide(a, cur);
   if (blockIdx.x == 0 && tid == 0) {
     nxt.MGbase = (double)d.MG;
@@ -88,10 +223,9 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
     nn.nMV = 0ull;
     nn.ovf = 0;
   }
-  if (tid == 0)
-    s_err = 0;
-  auto colp = [&](int j) { return (long long)r[2 * (pair0 + j)]; };
-  auto colq = [&](int j) { return (long long)r[2 * (pair0 + j) + 1]; };
+  __syncthreads();
+  auto colp = [&](int j) { return (long long)s_col[j][0]; };
+  auto colq = [&](int j) { return (long long)s_col[j][1]; };
   // ---- 1. rescaling (rare) ----
   if (d.gres || d.ovf) {
     const int e = d.gres ? d.sNg : d.sNv;
@@ -122,18 +256,29 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
     }
   tphase(0);
   // ---- stage the columns of G in shared memory (TMA bulk copies) ----
-  // staged layout: pair j, column c (p, q, pi, qi) at sm + (j * NC + c) * m
-  T *const sm = reinterpret_cast<T *>(smem_raw);
+  // two product buffers, then (staged) pair j's column c (p, q, pi, qi) at sm + (j * NC + c) * m
+  T *const buf = reinterpret_cast<T *>(smem_raw);
+  T *const sm = buf + 2 * D::BUF;
   auto rcol = [&](int j, int c) -> T * {
     if (STAGE)
       return sm + ((long long)j * NC + c) * a.m;
     const long long col = (c & 1) ? colq(j) : colp(j);
     return (c < 2) ? (a.G + col * a.ldG) : (a.Gi + col * a.ldGi);
   };
+  if (tid < P) {
+    const int j = tid;
+    const T ep = (j < np) ? a.eS[colp(j)] : (T)0, eq = (j < np) ? a.eS[colq(j)] : (T)0;
+    const bool live = (j < np) && (eq >= -svdc<T>::RMAX) && (ep >= -svdc<T>::RMAX);
+    PairState<T> &s = ps[j];
+    s.ep = ep;
+    s.eq = eq;
+    s.fp = (j < np) ? a.fS[colp(j)] : (T)1;
+    s.fq = (j < np) ? a.fS[colq(j)] : (T)1;
+    s_live[j] = live ? 1 : 0;
+    s_n[j][0] = live ? -(int)eq : 0;  // scale exponents of x = column q and y = column p
+    s_n[j][1] = live ? -(int)ep : 0;
+  }
   if (STAGE) {
-    if (tid == 0)
-      mbar_init(&bar, 1u);
-    __syncthreads();
     if (tid == 0) {
       const unsigned colb = (unsigned)(a.m * (long long)sizeof(T));
       mbar_expect_tx(&bar, colb * (unsigned)(NC * np));
@@ -159,107 +304,149 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
   }
   __syncthreads();
   tphase(1);
-  // ---- 2. scaled dot products ----
-  // FP32: pair j on lanes [j L, (j+1) L) of warp 0. FP64: one warp per accumulator chain
-  // (warp c runs chain c of the CTA's four pairs, pair j on lanes [8j, 8j+8)), so that the
-  // FP64 work of the step is spread over two (real) or four (complex) of the SM's
-  // sub-partitions; the chains meet in shared memory.
-  int cj = -1;  // the pair this thread classifies
-  T zr = 0, zi = 0, ep = 0, fp_ = 0, eq = 0, fq = 0;
-  bool live = false;
-  if constexpr (sizeof(T) == 8) {
-    constexpr int NCH = CPLX ? 4 : 2;
-    constexpr int PPW = 4;  // pairs per chain warp
-    __shared__ T dsum[ppc<T>::P][NCH][2];
-    if (warp < NCH * (ppc<T>::P / PPW)) {
-      const int jw = lane >> 3, l8 = lane & 7;
-      const int j = (warp / NCH) * PPW + jw;
-      const bool act = (jw < PPW) && (j < np);
-      const int jj = act ? j : 0;
-      const long long p = colp(jj), q = colq(jj);
-      const T ep_ = a.eS[p], eq_ = a.eS[q];
-      const bool lv = act && (eq_ >= -svdc<T>::RMAX) && (ep_ >= -svdc<T>::RMAX);
-      const T *xr = rcol(jj, 1), *xi = CPLX ? rcol(jj, 3) : nullptr, *yr = rcol(jj, 0),
-              *yi = CPLX ? rcol(jj, 2) : nullptr;
-      T S = 0, Tt = 0;
-      const int c = warp % NCH;
-      switch (c) {
-        case 0: chain_dot<T, CPLX, 0>(a.m, xr, xi, yr, yi, eq_, ep_, lv, l8, S, Tt); break;
-        case 1: chain_dot<T, CPLX, 1>(a.m, xr, xi, yr, yi, eq_, ep_, lv, l8, S, Tt); break;
-        case 2: chain_dot<T, CPLX, 2>(a.m, xr, xi, yr, yi, eq_, ep_, lv, l8, S, Tt); break;
-        default: chain_dot<T, CPLX, 3>(a.m, xr, xi, yr, yi, eq_, ep_, lv, l8, S, Tt); break;
+  // ---- 2. scaled dot products: x = column q, y = column p ----
+  const int mi = (int)a.m;
+  const DotOps<T> ops = DotOps<T>::make();
+  // the products of chunk ck: row i of pair j, chain c, term t at ((i / L) NT + t) NG L +
+  // (j NCH + c) L + i % L
+  auto produce = [&](int ck, int t0, int nt) {
+    T *const bf = buf + (ck & 1) * D::BUF;
+    const int r0 = ck * D::RC, rows = min(D::RC, mi - r0);
+    for (int e = t0; e < D::RC * P; e += nt) {
+      const int j = e / D::RC, i = e % D::RC;
+      if (i >= rows || j >= np)
+        continue;
+      T *const o = bf + (i / L) * (D::NT * D::NG * L) + j * (D::NCH * L) + i % L;
+      if (!s_live[j]) {
+#pragma unroll
+        for (int c = 0; c < D::NCH; ++c)
+#pragma unroll
+          for (int t = 0; t < D::NT; ++t)
+            o[t * D::NG * L + c * L] = (T)0;
+        continue;
       }
-      if (act && l8 == 0) {
-        dsum[j][c][0] = S;
-        dsum[j][c][1] = Tt;
+      const int nx = s_n[j][0], ny = s_n[j][1];
+      const T x = scale2(rcol(j, 1)[r0 + i], nx), y = scale2(rcol(j, 0)[r0 + i], ny);
+      T pd = ops.mul_rd(x, y);
+      o[0] = pd;
+      o[L] = F::fma_(x, y, -pd);
+      if constexpr (CPLX) {
+        // real part: x_r y_r, x_i y_i; imaginary part: x_r y_i, -x_i y_r
+        const T xi = scale2(rcol(j, 3)[r0 + i], nx), yi = scale2(rcol(j, 2)[r0 + i], ny);
+        pd = ops.mul_rd(x, yi);
+        o[2 * L] = pd;
+        o[3 * L] = F::fma_(x, yi, -pd);
+        T *const o1 = o + D::NG * L;
+        pd = ops.mul_rd(xi, yi);
+        o1[0] = pd;
+        o1[L] = F::fma_(xi, yi, -pd);
+        pd = ops.mul_rd(-xi, y);
+        o1[2 * L] = pd;
+        o1[3 * L] = F::fma_(-xi, y, -pd);
       }
+    }
+  };
+  produce(0, tid, 256);
+  __syncthreads();
+  T cs = 0, ct = 0;  // this lane's recurrence
+  const int gl = warp * 32 + lane;
+  const int nchunks = (mi + D::RC - 1) / D::RC;
+  for (int ck = 0; ck < nchunks; ++ck) {
+    if (warp < D::NCW) {
+      const T *v = buf + (ck & 1) * D::BUF + gl % (D::NG * L);
+      constexpr int W = D::NG * L, UN = 8;
+      int left = min(D::RC, mi - ck * D::RC) / L * D::NT;  // recurrence steps of this chunk
+      for (; left >= UN; left -= UN, v += UN * W) {
+        T x[UN];
+#pragma unroll
+        for (int u = 0; u < UN; ++u)
+          x[u] = v[u * W];
+#pragma unroll
+        for (int u = 0; u < UN; ++u)
+          sum_step(ops, x[u], cs, ct);
+      }
+      for (; left > 0; --left, v += W)
+        sum_step(ops, v[0], cs, ct);
+    }
+    else {
+      if (ck == 0 && warp == 7 && lane < np) {
+        const PairState<T> &s = ps[lane];
+        pre[lane] = pair_pre(s.ep, s.fp, s.eq, s.fq, a.gst);
+      }
+      if (ck + 1 < nchunks)
+        produce(ck + 1, tid - 32 * D::NCW, 256 - 32 * D::NCW);
     }
     __syncthreads();
-    if (tid < np) {
-      cj = tid;
-      const long long p = colp(cj), q = colq(cj);
-      ep = a.eS[p]; fp_ = a.fS[p]; eq = a.eS[q]; fq = a.fS[q];
-      live = (eq >= -svdc<T>::RMAX) && (ep >= -svdc<T>::RMAX);
-      // nu = S(s_pd) + (S(t_pd) + (S(s_dn) + S(t_dn))), divided by fx fy (x = G_q)
-      const T de = fq * fp_;
-      zr = F::div(dsum[cj][0][0] + (dsum[cj][0][1] + (dsum[cj][1][0] + dsum[cj][1][1])), de);
-      if (CPLX)
-        zi = F::div(dsum[cj][NCH - 2][0] + (dsum[cj][NCH - 2][1] + (dsum[cj][NCH - 1][0] + dsum[cj][NCH - 1][1])), de);
+  }
+  if (warp < D::NCW) {
+    const T S = hsum<L>(cs), Tt = hsum<L>(ct);
+    if ((lane % L) == 0 && gl < D::NG * L) {
+      dsum[gl / L][0] = S;
+      dsum[gl / L][1] = Tt;
     }
   }
-  else if (warp == 0) {
-    const int j = lane / L;
-    const bool act = (j < np);
-    const int jj = act ? j : 0;
-    const long long p = colp(jj), q = colq(jj);
-    const T ep_ = a.eS[p], fp0 = a.fS[p], eq_ = a.eS[q], fq0 = a.fS[q];
-    const bool lv = act && (eq_ >= -svdc<T>::RMAX) && (ep_ >= -svdc<T>::RMAX);
-    T zr_ = 0, zi_ = 0;
-    pair_dot<T, CPLX>(a.m, rcol(jj, 1), CPLX ? rcol(jj, 3) : nullptr, rcol(jj, 0), CPLX ? rcol(jj, 2) : nullptr, eq_,
-                      ep_, fq0, fp0, lv, zr_, zi_);
-    if (act && (lane % L) == 0) {
-      cj = j;
-      ep = ep_; fp_ = fp0; eq = eq_; fq = fq0;
-      live = lv;
-      zr = zr_;
-      zi = zi_;
-    }
-  }
+  __syncthreads();
   tphase(2);
-  if (cj >= 0) {
-    const int j = cj;
-    const long long p = colp(j), q = colq(j);
-    {
-      PairState<T> &s = ps[j];
-      s.ep = ep; s.fp = fp_; s.eq = eq; s.fq = fq;
-      if (!live) {
-        zr = 0;
-        zi = 0;
-      }
+  // ---- 3. convergence, 2x2, classification: one quad of warp 0 per pair ----
+  if (warp == 0) {
+    const int q4 = lane & 3, base = lane & ~3;
+    const int j = min(lane >> 2, np - 1);
+    const bool own = (q4 == 0) && (lane >> 2) < np;
+    PairState<T> &s = ps[j];
+    const T ep = s.ep, fp_ = s.fp, eq = s.eq, fq = s.fq;
+    // nu = S(s_pd) + (S(t_pd) + (S(s_dn) + S(t_dn))), divided by fx fy
+    const T de = fq * fp_;
+    const T(*ds)[2] = dsum + j * D::NCH + ((CPLX && (q4 & 1)) ? 2 : 0);
+    const T z = F::div(ds[0][0] + (ds[0][1] + (ds[1][0] + ds[1][1])), de);
+    T zr = __shfl_sync(0xffffffffu, z, base), zi = CPLX ? __shfl_sync(0xffffffffu, z, base + 1) : (T)0;
+    if (!s_live[j]) {
+      zr = 0;
+      zi = 0;
+    }
+    long long code = 0;
+    if (CPLX) {
+      if (!visfinite(zr))
+        code = a.e_dot;
+      if (!visfinite(zi))
+        code = (a.e_doti < code) ? a.e_doti : code;
+    }
+    else if (!visfinite(zr))
+      code = a.e_dot;
+    const T ab = CPLX ? vhypot(zr, zi) : vabs(zr);
+    const bool trans = (code == 0) && (a.tol <= ab);
+    T cc = 1, at = 0, sat = 0;
+    unsigned perm = 0u;
+    const PairPre<T> pp = pre[j];
+    if (__any_sync(0xffffffffu, trans)) {
+      // (a pair that is not transformed passes ones and is ignored)
+      const T w11 = trans ? pp.w11 : (T)1, w22 = trans ? pp.w22 : (T)1, w21r = trans ? scalef(zr, pp.dd) : (T)1;
+      if constexpr (CPLX)
+        perm = cjac2_quad<T>(w11, w22, w21r, trans ? scalef(zi, pp.dd) : (T)1, q4, base, cc, at, sat);
+      else
+        perm = rjac2_quad<T>(w11, w22, w21r, q4, base, cc, at);
+    }
+    if (own) {
       s.a21r = zr;
       s.a21i = zi;
       s.skip = 0;
-      long long code = 0;
-      if (CPLX) {
-        if (!visfinite(zr))
-          code = a.e_dot;
-        if (!visfinite(zi))
-          code = (a.e_doti < code) ? a.e_doti : code;
-      }
-      else if (!visfinite(zr))
-        code = a.e_dot;
+      s.code = 1;
       if (code) {
         atomicMin((long long *)&g->err, code);
         s.skip = 1;
       }
-      else {
-        // ---- 3. convergence, shear test, prescale, 2x2, classification ----
-        if (pair_classify<T, CPLX>(ep, fp_, eq, fq, zr, zi, a.tol, a.gst, s))
-          atomicAdd(&g->swt, 1ull);
-        if (s.code == -1) {
-          a.eS[p] = eq; a.eS[q] = ep;
-          a.fS[p] = fq; a.fS[q] = fp_;
-        }
+      else if (trans) {
+        s.c = cc;
+        s.cat = at;
+        s.sat = sat;
+        s.code = pair_code(pp, perm);
+        atomicAdd(&g->swt, 1ull);
+      }
+      else if (efcmp(ep, fp_, eq, fq) < 0) {
+        s.code = -1;
+        a.eS[colp(j)] = eq;
+        a.eS[colq(j)] = ep;
+        a.fS[colp(j)] = fq;
+        a.fS[colq(j)] = fp_;
       }
     }
   }
@@ -267,60 +454,87 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
   tphase(3);
   // ---- 4. apply: the CTA's pairs concurrently, blockDim/P threads each; G is read from
   // the staged copy ----
-  unsigned long long mG = 0ull, mV = 0ull;
-  unsigned chmask = 0u;  // bit 2j: column p of pair j changed, bit 2j+1: column q
-  for (int j = 0; j < np; ++j) {
-    const int cj = ps[j].code;
-    if (!ps[j].skip)
-      chmask |= ((cj == 3 || cj == -3) ? 2u : ((cj == 2 || cj == -2) ? 3u : 0u)) << (2 * j);
-  }
-  const int TPP = (int)blockDim.x / P;
-  const int j = tid / TPP;
-  const int ltid = tid - j * TPP;
-  if (j < np && !ps[j].skip) {
-    const long long p = colp(j), q = colq(j);
-    T *Gip = CPLX ? (a.Gi + p * a.ldGi) : nullptr, *Giq = CPLX ? (a.Gi + q * a.ldGi) : nullptr;
-    T *Vip = CPLX ? (a.Vi + p * a.ldVi) : nullptr, *Viq = CPLX ? (a.Vi + q * a.ldVi) : nullptr;
-    pair_apply<T, CPLX, TRACKV>(ps[j], a.m, a.n, a.G + p * a.ldG, a.G + q * a.ldG, Gip, Giq, a.V + p * a.ldV,
-                                a.V + q * a.ldV, Vip, Viq, rcol(j, 0), rcol(j, 1), CPLX ? rcol(j, 2) : nullptr,
-                                CPLX ? rcol(j, 3) : nullptr, a.eS + p, a.eS + q, a.fS + p, a.fS + q, ltid, TPP, mG,
-                                mV);
-  }
-  tphase(4);
-  // block max of |G| and |V| updates
-  mG = warp_max_u64(mG);
-  mV = warp_max_u64(mV);
-  if (lane == 0) {
-    red[warp][0] = mG;
-    red[warp][1] = mV;
+  constexpr int TPP = 256 / P;
+  {
+    const int j = tid / TPP;
+    const int ltid = tid - j * TPP;
+    U mx[CPLX ? 4 : 2] = {};
+    U mV = 0;
+    if (j < np && !ps[j].skip) {
+      const long long p = colp(j), q = colq(j);
+      T *Gip = CPLX ? (a.Gi + p * a.ldGi) : nullptr, *Giq = CPLX ? (a.Gi + q * a.ldGi) : nullptr;
+      T *Vip = CPLX ? (a.Vi + p * a.ldVi) : nullptr, *Viq = CPLX ? (a.Vi + q * a.ldVi) : nullptr;
+      const bool trk = pair_apply<T, CPLX, STAGE>(
+          ps[j], a.m, a.n, a.G + p * a.ldG, a.G + q * a.ldG, Gip, Giq, a.V + p * a.ldV, a.V + q * a.ldV, Vip, Viq,
+          rcol(j, 0), rcol(j, 1), CPLX ? rcol(j, 2) : nullptr, CPLX ? rcol(j, 3) : nullptr, a.eS + p, a.eS + q,
+          a.fS + p, a.fS + q, ltid, TPP, a.trackv != 0, mx, mV);
+      if (ltid == 0)
+        s_trk[j] = trk ? 1 : 0;
+    }
+    // largest |.| per changed plane and of V's update
+#pragma unroll
+    for (int c = 0; c < NC; ++c) {
+      const U w = warp_max_bits(mx[c]);
+      if (lane == 0 && w)
+        atomicMax(&cmx[j][c], w);
+    }
+    if (a.trackv) {
+      const U w = warp_max_bits(mV);
+      if (lane == 0 && w)
+        atomicMax(&vmx, w);
+    }
   }
   __syncthreads();
+  tphase(4);
   if (tid == 0) {
-    unsigned long long bg = 0ull, bv = 0ull;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-      bg = (red[w][0] > bg) ? red[w][0] : bg;
-      bv = (red[w][1] > bv) ? red[w][1] : bv;
-    }
-    const T tG = bitst<T>(bg), tV = bitst<T>(bv);
+    U bg = 0;
+    for (int j = 0; j < np; ++j)
+#pragma unroll
+      for (int c = 0; c < NC; ++c)
+        bg = (cmx[j][c] > bg) ? cmx[j][c] : bg;
+    const U bv = vmx;
+    const T tG = F::val(bg), tV = F::val(bv);
     if (!visfinite(tG))
       atomicMin((long long *)&g->err, a.e_appg);
     else if (!visfinite(tV))
       atomicMin((long long *)&g->err, a.e_appv);
     else {
       if (bg)
-        atomicMax(&nxt.nMG, bg);
+        atomicMax(&nxt.nMG, (unsigned long long)bg);
       if (bv)
-        atomicMax(&nxt.nMV, bv);
+        atomicMax(&nxt.nMV, (unsigned long long)bv);
     }
   }
-  // ---- 5. norms of the changed columns (warp w: pair w/2, column p or q), for the next step ----
+  // ---- 5. norms of the changed columns for the next step: one warp per column and plane ----
   // (not after the last step of the last allowed sweep: the reference returns there with
   // the norms of those columns not yet recomputed)
-  if (!last && warp < 2 * np && ((chmask >> warp) & 1u)) {
-    const int j = warp >> 1, c = warp & 1;
-    const long long col = c ? colq(j) : colp(j);
-    const T nv = col_norm_at<T, CPLX>(a, col, rcol(j, c), CPLX ? rcol(j, 2 + c) : nullptr);
-    if ((lane == 0) && !(nv <= svdc<T>::RMAX))
+  if (last)
+    return;
+  auto changed = [&](int j, int c) {
+    const int code = ps[j].code;
+    return !ps[j].skip && (code == 2 || code == -2 || (c && (code == 3 || code == -3)));
+  };
+  constexpr int NPL = CPLX ? 2 : 1;
+  for (int u = warp; u < 2 * np * NPL; u += 8) {
+    const int pl = u % NPL, j = u / (2 * NPL), c = (u / NPL) & 1;
+    if (changed(j, c)) {
+      const T *x = rcol(j, 2 * pl + c);
+      const T nv = s_trk[j] ? warp_nrm2_scaled<T>(x, a.m, (unsigned long long)cmx[j][2 * pl + c]) : warp_nrm2<T>(x, a.m);
+      if (lane == 0)
+        cnrm[2 * j + c][pl] = nv;
+    }
+  }
+  __syncthreads();
+  if (tid < 2 * np && changed(tid >> 1, tid & 1)) {
+    const int j = tid >> 1, c = tid & 1;
+    T nv = cnrm[tid][0];
+    if (CPLX)
+      nv = vhypot(nv, cnrm[tid][CPLX ? 1 : 0]);
+    T e, f;
+    ef_split(nv, e, f);
+    a.eS[s_col[j][c]] = e;
+    a.fS[s_col[j][c]] = f;
+    if (!(nv <= svdc<T>::RMAX))
       atomicOr(&nxt.ovf, 1);
   }
   tphase(5);
@@ -617,6 +831,40 @@ static inline bool is_al(const void *p)
   return !((uintptr_t)p & 63u);
 }
 
+// most pairs a CTA takes: what leaves half of its warps free to form products
+template <typename T, bool CPLX> struct StepPairs {
+  static constexpr int MAX = (CPLX && sizeof(T) == 4) ? 2 : 4;
+};
+// the step kernel for about P pairs per CTA and m rows (columns staged in shared memory when
+// they and the product buffers fit in 192 KiB), with its dynamic shared memory allowed
+template <typename T> struct StepLaunch {
+  void (*k)(SvdArgs<T>, int, int, int);
+  size_t smem;
+  int pairs;  // per CTA
+};
+template <typename T, bool CPLX, int P> static size_t step_smem(long long m)
+{
+  return StepDims<T, CPLX, P>::buf_bytes() + (size_t)m * sizeof(T) * (CPLX ? 4u : 2u) * P;
+}
+template <typename T, bool CPLX> static StepLaunch<T> step_launch(long long m, int P)
+{
+  constexpr int PMAX = StepPairs<T, CPLX>::MAX;
+  constexpr size_t LIM = 192 * 1024;
+  StepLaunch<T> r;
+  if (P == 1 && step_smem<T, CPLX, 1>(m) <= LIM)
+    r = {k_step<T, CPLX, true, 1>, step_smem<T, CPLX, 1>(m), 1};
+  else if (P <= 2 && step_smem<T, CPLX, 2>(m) <= LIM)
+    r = {k_step<T, CPLX, true, 2>, step_smem<T, CPLX, 2>(m), 2};
+  else if (step_smem<T, CPLX, PMAX>(m) <= LIM)
+    r = {k_step<T, CPLX, true, PMAX>, step_smem<T, CPLX, PMAX>(m), PMAX};
+  else
+    r = {k_step<T, CPLX, false, PMAX>, StepDims<T, CPLX, PMAX>::buf_bytes(), PMAX};
+  if (r.smem > 40 * 1024 &&
+      cudaFuncSetAttribute(r.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r.smem) != cudaSuccess)
+    r.k = nullptr;
+  return r;
+}
+
 template <typename T, bool CPLX>
 static vj_fint svd_dev(vj_fnat m_, vj_fnat n_, T *G, vj_fnat ldG, T *Gi, vj_fnat ldGi, T *V, vj_fnat ldV, T *Vi,
                        vj_fnat ldVi, T *eS, T *fS, const unsigned *js, unsigned stp, unsigned swp, int preset,
@@ -742,6 +990,7 @@ static vj_fint svd_dev(vj_fnat m_, vj_fnat n_, T *G, vj_fnat ldG, T *Gi, vj_fnat
     return VJ_ERR_CUDA;
   SvdArgs<T> a;
   a.trace = host::trace_enabled() ? 1 : 0;
+  a.trackv = preset ? 1 : 0;
   a.m = m; a.n = n; a.ldG = (long long)ldG; a.ldGi = (long long)ldGi; a.ldV = (long long)ldV;
   a.ldVi = (long long)ldVi;
   a.G = G; a.Gi = Gi; a.V = V; a.Vi = Vi; a.eS = eS; a.fS = fS; a.js = js; a.g = dg;
@@ -759,15 +1008,13 @@ static vj_fint svd_dev(vj_fnat m_, vj_fnat n_, T *G, vj_fnat ldG, T *Gi, vj_fnat
     k_norms<T, CPLX><<<(unsigned)((n + 7) / 8), blk, 0, s>>>(a);
   if (cudaGetLastError() != cudaSuccess)
     return VJ_ERR_CUDA;
-  // stage each pair's columns of G in shared memory when they fit (160 KiB per CTA)
-  constexpr int P = ppc<T>::P;
-  const size_t smem = (size_t)m * sizeof(T) * (CPLX ? 4u : 2u) * P;
-  const bool stage = (smem <= (size_t)160 * 1024);
-  const unsigned grid = (unsigned)((n_2 + P - 1) / P);
-  if (stage && smem > 48 * 1024) {
-    cudaFuncSetAttribute(k_step<T, CPLX, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(k_step<T, CPLX, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  }
+  // Pairs per CTA: as few as leave every CTA of a step its own SM, so that a small matrix
+  // spreads its rotations and norms over the GPU; otherwise the most.
+  const long long sms = host::sm_count();
+  const StepLaunch<T> sl = step_launch<T, CPLX>(m, (n_2 <= sms) ? 1 : (n_2 <= 2 * sms) ? 2 : StepPairs<T, CPLX>::MAX);
+  if (!sl.k)
+    return VJ_ERR_CUDA;
+  const unsigned grid = (unsigned)((n_2 + sl.pairs - 1) / sl.pairs);
   unsigned sw = 0;
   long long gstep = 0;
   // preset == 2 (the mixed path's finishing call, whose columns are orthogonal already):
@@ -821,13 +1068,7 @@ static vj_fint svd_dev(vj_fnat m_, vj_fnat n_, T *G, vj_fnat ldG, T *Gi, vj_fnat
       const int last = ((sw + 1u == swp) && (st + 1u == stp)) ? 1 : 0;
       const int g3 = (int)(gstep % 3);
       const int ist = (int)st;
-      cudaError_t e;
-      if (stage)
-        e = preset ? host::launch_pdl(k_step<T, CPLX, true, true>, dim3(grid), blk, smem, s, a, ist, g3, last)
-                   : host::launch_pdl(k_step<T, CPLX, false, true>, dim3(grid), blk, smem, s, a, ist, g3, last);
-      else
-        e = preset ? host::launch_pdl(k_step<T, CPLX, true, false>, dim3(grid), blk, 0, s, a, ist, g3, last)
-                   : host::launch_pdl(k_step<T, CPLX, false, false>, dim3(grid), blk, 0, s, a, ist, g3, last);
+      const cudaError_t e = host::launch_pdl(sl.k, dim3(grid), blk, sl.smem, s, a, ist, g3, last);
       if (e != cudaSuccess)
         return VJ_ERR_CUDA;
     }

@@ -38,6 +38,7 @@ struct SvdGlobal {
 
 template <typename T> struct SvdArgs {
   int trace;                    // record per-phase cycles (VJ_TRACE=1)
+  int trackv;                   // V is a preset matrix: its largest entry is tracked
   long long m, n, ldG, ldGi, ldV, ldVi;
   T *G, *Gi, *V, *Vi, *eS, *fS;
   const unsigned *js;
@@ -260,10 +261,54 @@ template <typename T> __device__ void scale_cols(T *A, long long ld, long long r
   }
 }
 
-template <typename T> __device__ __forceinline__ void amax(unsigned long long &m, T v)
+template <typename T> __device__ __forceinline__ void amax(typename fp<T>::U &m, T v)
 {
-  const unsigned long long b = absbits(v);
+  const typename fp<T>::U b = fp<T>::bits(v) & ~fp<T>::SIGN;
   m = (b > m) ? b : m;
+}
+
+// What the classification of a pair takes from the columns' norms alone: the order of the
+// norms, the shear test and the Gram prescale (src/dvjsvd.c:349-405).
+template <typename T> struct PairPre {
+  T w11, w22, dd;  // scaled squared-norm ratios and the prescale exponent (<= 0)
+  int ngs, cgs;    // p shorter than q; a shear instead of a rotation
+};
+
+template <typename T> __device__ __forceinline__ PairPre<T> pair_pre(T ep, T fp_, T eq, T fq, T gst)
+{
+  using F = fp<T>;
+  PairPre<T> r;
+  const T e1 = ep, e2 = eq, f1 = fp_, f2 = fq;
+  const bool ngs = eflt(e1, e2, f1, f2);
+  T maf = ngs ? f1 : f2, mae = ngs ? e1 : e2;
+  const T Maf = ngs ? f2 : f1, Mae = ngs ? e2 : e1;
+  maf = gst * maf;
+  mae = mae + getexp(maf);
+  maf = getmant(maf);
+  r.ngs = ngs ? 1 : 0;
+  r.cgs = eflt(mae, Mae, maf, Maf) ? 1 : 0;
+  T f12 = F::div(f1, f2), e12 = e1 - e2, f21 = F::div(f2, f1), e21 = e2 - e1;
+  e12 = e12 + getexp(f12);
+  f12 = getmant(f12);
+  e21 = e21 + getexp(f21);
+  f21 = getmant(f21);
+  const bool c12 = efle(e12, e21, f12, f21);
+  const T E = c12 ? e21 : e12;
+  const T dd = vmin(svdc<T>::MAX_FIN_EXP - E, (T)0);
+  e12 = e12 + dd;
+  e21 = e21 + dd;
+  r.w11 = scalef(f12, e12);
+  r.w22 = scalef(f21, e21);
+  r.dd = dd;
+  return r;
+}
+
+// the code of a transformed pair: 3/-3 shear, 2/-2 rotation (src/dvjsvd.c:422-459)
+template <typename T> __device__ __forceinline__ int pair_code(const PairPre<T> &r, unsigned perm)
+{
+  if (r.cgs)
+    return r.ngs ? -3 : 3;
+  return perm ? -2 : 2;
 }
 
 // Convergence test, shear test, Gram prescale, 2x2 EVD and classification of one pair
@@ -273,48 +318,21 @@ template <typename T> __device__ __forceinline__ void amax(unsigned long long &m
 template <typename T, bool CPLX>
 __device__ bool pair_classify(T ep, T fp_, T eq, T fq, T zr, T zi, T tol, T gst, PairState<T> &s)
 {
-  using F = fp<T>;
   const T ab = CPLX ? vhypot(zr, zi) : vabs(zr);
   const bool trans = (tol <= ab);
   if (trans) {
-    const T e1 = ep, e2 = eq, f1 = fp_, f2 = fq;
-    const bool ngs = eflt(e1, e2, f1, f2);
-    T maf = ngs ? f1 : f2, mae = ngs ? e1 : e2;
-    const T Maf = ngs ? f2 : f1, Mae = ngs ? e2 : e1;
-    maf = gst * maf;
-    mae = mae + getexp(maf);
-    maf = getmant(maf);
-    const bool cgs = eflt(mae, Mae, maf, Maf);
-    T f12 = F::div(f1, f2), e12 = e1 - e2, f21 = F::div(f2, f1), e21 = e2 - e1;
-    e12 = e12 + getexp(f12);
-    f12 = getmant(f12);
-    e21 = e21 + getexp(f21);
-    f21 = getmant(f21);
-    const bool c12 = efle(e12, e21, f12, f21);
-    const T E = c12 ? e21 : e12;
-    const T dd = vmin(svdc<T>::MAX_FIN_EXP - E, (T)0);
-    e12 = e12 + dd;
-    e21 = e21 + dd;
-    const T w11 = scalef(f12, e12), w22 = scalef(f21, e21), w21r = scalef(zr, dd);
+    const PairPre<T> r = pair_pre(ep, fp_, eq, fq, gst);
+    const T w21r = scalef(zr, r.dd);
     unsigned perm;
     T cc, at, sat = 0, l1, l2;
-    if (CPLX) {
-      const T w21i = scalef(zi, dd);
-      perm = cjac2<T, 0>(w11, w22, w21r, w21i, cc, at, sat, l1, l2);
-    }
+    if (CPLX)
+      perm = cjac2<T, 0>(r.w11, r.w22, w21r, scalef(zi, r.dd), cc, at, sat, l1, l2);
     else
-      perm = rjac2<T, 0>(w11, w22, w21r, cc, at, l1, l2);
+      perm = rjac2<T, 0>(r.w11, r.w22, w21r, cc, at, l1, l2);
     s.c = cc;
     s.cat = at;
     s.sat = sat;
-    if (!ngs && cgs)
-      s.code = 3;
-    else if (ngs && cgs)
-      s.code = -3;
-    else if (perm)
-      s.code = -2;
-    else
-      s.code = 2;
+    s.code = pair_code(r, perm);
   }
   else if (efcmp(ep, fp_, eq, fq) < 0)
     s.code = -1;
@@ -323,33 +341,169 @@ __device__ bool pair_classify(T ep, T fp_, T eq, T fq, T zr, T zi, T tol, T gst,
   return trans;
 }
 
+// exchange two columns
+template <typename T> __device__ __forceinline__ void swap_cols(T *x, T *y, long long rows, int ltid, int TPP)
+{
+#pragma unroll 4
+  for (long long i = ltid; i < rows; i += TPP) {
+    const T t = x[i];
+    x[i] = y[i];
+    y[i] = t;
+  }
+}
+
+// Rows of a column pair rotated, UR of a thread's rows loaded before any is stored: a store
+// may alias a later load as far as the compiler knows, so a row-by-row loop would wait for
+// one memory round trip per row. Reads (rx, ry), writes (x, y) and, when STG, the staged copy
+// as well; mx and my collect max |.| of what x and y receive when track is set. The products by the
+// cosine are three-register FMAs (svd_dot.cuh, DotOps).
+template <typename T, bool STG, int UR>
+__device__ __forceinline__ void rot_real(int rows, const T *rx, const T *ry, T *x, T *y, T *sx, T *sy, T at, T c,
+                                         bool perm, int ltid, int TPP, bool track, typename fp<T>::U &mx,
+                                         typename fp<T>::U &my)
+{
+  using F = fp<T>;
+  const DotOps<T> o = DotOps<T>::make();
+  const bool cone = (c == (T)1);
+  // the permuted form writes (y - t x) c to x and (x + t y) c to y: the same two products
+  // with the destinations exchanged
+  T *const dx = perm ? y : x, *const dy = perm ? x : y, *const dsx = perm ? sy : sx, *const dsy = perm ? sx : sy;
+  typename F::U mu = 0, mw = 0;
+  for (int i0 = ltid; i0 < rows; i0 += UR * TPP) {
+    T u[UR], w[UR];
+#pragma unroll
+    for (int k = 0; k < UR; ++k) {
+      const int i = i0 + k * TPP;
+      u[k] = (i < rows) ? rx[i] : (T)0;
+      w[k] = (i < rows) ? ry[i] : (T)0;
+    }
+#pragma unroll
+    for (int k = 0; k < UR; ++k) {
+      const T a = F::fma_(w[k], at, u[k]), b = F::fma_(-u[k], at, w[k]);
+      u[k] = cone ? a : o.mul(a, c);
+      w[k] = cone ? b : o.mul(b, c);
+    }
+#pragma unroll
+    for (int k = 0; k < UR; ++k) {
+      const int i = i0 + k * TPP;
+      if (i < rows) {
+        dx[i] = u[k];
+        dy[i] = w[k];
+        if (STG) {
+          dsx[i] = u[k];
+          dsy[i] = w[k];
+        }
+        if (track) {
+          amax(mu, u[k]);
+          amax(mw, w[k]);
+        }
+      }
+    }
+  }
+  if (track) {
+    mx = perm ? mw : mu;
+    my = perm ? mu : mw;
+  }
+}
+
+template <typename T, bool STG, int UR>
+__device__ __forceinline__ void rot_cplx(int rows, const T *rxr, const T *rxi, const T *ryr, const T *ryi, T *xr,
+                                         T *xi, T *yr, T *yi, T *sxr, T *sxi, T *syr, T *syi, T cta, T sta, T c,
+                                         bool perm, int ltid, int TPP, bool track, typename fp<T>::U *m4)
+{
+  using F = fp<T>;
+  const DotOps<T> o = DotOps<T>::make();
+  const bool cone = (c == (T)1);
+  const T cna = -cta;
+  T *const dar = perm ? yr : xr, *const dai = perm ? yi : xi, *const dbr = perm ? xr : yr, *const dbi = perm ? xi : yi;
+  T *const sar = perm ? syr : sxr, *const sai = perm ? syi : sxi, *const sbr = perm ? sxr : syr,
+           *const sbi = perm ? sxi : syi;
+  typename F::U mar = 0, mai = 0, mbr = 0, mbi = 0;
+  for (int i0 = ltid; i0 < rows; i0 += UR * TPP) {
+    T ar[UR], ai[UR], br[UR], bi[UR];
+#pragma unroll
+    for (int k = 0; k < UR; ++k) {
+      const int i = i0 + k * TPP;
+      const bool in = (i < rows);
+      ar[k] = in ? rxr[i] : (T)0;
+      ai[k] = in ? rxi[i] : (T)0;
+      br[k] = in ? ryr[i] : (T)0;
+      bi[k] = in ? ryi[i] : (T)0;
+    }
+#pragma unroll
+    for (int k = 0; k < UR; ++k) {
+      const T x_r = ar[k], x_i = ai[k], y_r = br[k], y_i = bi[k];
+      T u = F::fma_(y_r, cta, F::fma_(-y_i, sta, x_r)), v = F::fma_(y_r, sta, F::fma_(y_i, cta, x_i));
+      ar[k] = cone ? u : o.mul(u, c);
+      ai[k] = cone ? v : o.mul(v, c);
+      u = F::fma_(x_r, cna, F::fma_(-x_i, sta, y_r));
+      v = F::fma_(x_r, sta, F::fma_(x_i, cna, y_i));
+      br[k] = cone ? u : o.mul(u, c);
+      bi[k] = cone ? v : o.mul(v, c);
+    }
+#pragma unroll
+    for (int k = 0; k < UR; ++k) {
+      const int i = i0 + k * TPP;
+      if (i < rows) {
+        dar[i] = ar[k];
+        dai[i] = ai[k];
+        dbr[i] = br[k];
+        dbi[i] = bi[k];
+        if (STG) {
+          sar[i] = ar[k];
+          sai[i] = ai[k];
+          sbr[i] = br[k];
+          sbi[i] = bi[k];
+        }
+        if (track) {
+          amax(mar, ar[k]);
+          amax(mai, ai[k]);
+          amax(mbr, br[k]);
+          amax(mbi, bi[k]);
+        }
+      }
+    }
+  }
+  if (track) {
+    m4[0] = perm ? mbr : mar;
+    m4[1] = perm ? mar : mbr;
+    m4[2] = perm ? mbi : mai;
+    m4[3] = perm ? mai : mbi;
+  }
+}
+
 // The transformation of one classified pair applied by a group of TPP threads (ltid =
 // this thread's index in the group): rotation (src/djrot.c, src/djrotf.c, src/zjrot.c,
 // src/zjrotf.c), shear (src/dgsscl.c, src/zgsscl.c) or swap, to the columns of G (read from
-// rp/rq[/rpi/rqi], which may be a staged copy, written to both) and of V. mG and mV collect
-// max |.| of the updated G and (with TRACKV) V columns.
-template <typename T, bool CPLX, bool TRACKV>
-__device__ void pair_apply(const PairState<T> &s, long long m, long long nv, T *Gp, T *Gq, T *Gip, T *Giq, T *Vp,
+// rp/rq[/rpi/rqi], which is a staged copy when STG, written to both; the columns themselves
+// otherwise) and of V. mx collects this thread's max |.| of the rows that the transformed
+// columns p and q of G receive (their imaginary planes in mx[2], mx[3]) and mV, with trackv,
+// that of V. Returns whether mx holds the maxima of the changed columns: false for a
+// rotation by nothing or by a plain exchange, whose columns count as changed without being
+// tracked.
+template <typename T, bool CPLX, bool STG>
+__device__ bool pair_apply(const PairState<T> &s, long long m, long long nv, T *Gp, T *Gq, T *Gip, T *Giq, T *Vp,
                            T *Vq, T *Vip, T *Viq, T *rp, T *rq, T *rpi, T *rqi, T *eSp, T *eSq, T *fSp, T *fSq,
-                           int ltid, int TPP, unsigned long long &mG, unsigned long long &mV)
+                           int ltid, int TPP, bool trackv, typename fp<T>::U (&mx)[CPLX ? 4 : 2],
+                           typename fp<T>::U &mV)
 {
   using F = fp<T>;
+  using U = typename F::U;
   const int code = s.code;
   if (code == 1) {
     // the pair is in order and orthogonal: nothing to apply
   }
   else if (code == -1) {
+    // (the staged copy is not read again: a swapped pair's norms are exchanged, not recomputed)
     #pragma unroll 4
     for (long long i = ltid; i < m; i += TPP) {
       const T x = rp[i], y = rq[i];
       Gp[i] = y; Gq[i] = x;
       if (CPLX) { const T xi = rpi[i], yi = rqi[i]; Gip[i] = yi; Giq[i] = xi; }
     }
-    #pragma unroll 4
-    for (long long i = ltid; i < nv; i += TPP) {
-      T t = Vp[i]; Vp[i] = Vq[i]; Vq[i] = t;
-      if (CPLX) { t = Vip[i]; Vip[i] = Viq[i]; Viq[i] = t; }
-    }
+    swap_cols(Vp, Vq, nv, ltid, TPP);
+    if (CPLX)
+      swap_cols(Vip, Viq, nv, ltid, TPP);
   }
   else if (code == 3 || code == -3) {
     // Gram-Schmidt-like shear (src/dgsscl.c:5-85, src/zgsscl.c)
@@ -369,16 +523,16 @@ __device__ void pair_apply(const PairState<T> &s, long long m, long long nv, T *
           const T xi = F::fma_(tfr, xii_, F::fma_(tfi, xri_, yii_));
           const T ur = scale2(xr, py), ui = scale2(xi, py);
           Gq[i] = ur; Giq[i] = ui;
-          rq[i] = ur; rqi[i] = ui;
-          amax(mG, ur); amax(mG, ui);
+          if (STG) { rq[i] = ur; rqi[i] = ui; }
+          amax(mx[1], ur); amax(mx[CPLX ? 3 : 1], ui);
         }
         else {
           const T xi = scale2(rp[i], nx);
           const T yi = scale2(rq[i], ny);
           const T u = scale2(F::fma_(tfr, xi, yi), py);
           Gq[i] = u;
-          rq[i] = u;
-          amax(mG, u);
+          if (STG) rq[i] = u;
+          amax(mx[1], u);
         }
       }
     }
@@ -391,31 +545,29 @@ __device__ void pair_apply(const PairState<T> &s, long long m, long long nv, T *
         if (CPLX) {
           const T yri = rq[i], yii = rqi[i], xri = rp[i], xii = rpi[i];
           Gp[i] = yri; Gip[i] = yii;
-          rp[i] = yri; rpi[i] = yii;
+          if (STG) { rp[i] = yri; rpi[i] = yii; }
           const T yri_ = scale2(yri, ny), yii_ = scale2(yii, ny);
           const T xri_ = scale2(xri, nx), xii_ = scale2(xii, nx);
           const T vr = F::fma_(tfr, yri_, F::fma_(-tfi, yii_, xri_));
           const T vi = F::fma_(tfr, yii_, F::fma_(tfi, yri_, xii_));
           const T ur = scale2(vr, px), ui = scale2(vi, px);
           Gq[i] = ur; Giq[i] = ui;
-          rq[i] = ur; rqi[i] = ui;
-          amax(mG, ur); amax(mG, ui);
+          if (STG) { rq[i] = ur; rqi[i] = ui; }
+          amax(mx[1], ur); amax(mx[CPLX ? 3 : 1], ui);
         }
         else {
           const T xi = rp[i], yi = rq[i];
           Gp[i] = yi;
-          rp[i] = yi;
+          if (STG) rp[i] = yi;
           const T u = scale2(F::fma_(tfr, scale2(yi, ny), scale2(xi, nx)), px);
           Gq[i] = u;
-          rq[i] = u;
-          amax(mG, u);
+          if (STG) rq[i] = u;
+          amax(mx[1], u);
         }
       }
-      #pragma unroll 4
-      for (long long i = ltid; i < nv; i += TPP) {
-        T t = Vp[i]; Vp[i] = Vq[i]; Vq[i] = t;
-        if (CPLX) { t = Vip[i]; Vip[i] = Viq[i]; Viq[i] = t; }
-      }
+      swap_cols(Vp, Vq, nv, ltid, TPP);
+      if (CPLX)
+        swap_cols(Vip, Viq, nv, ltid, TPP);
       if (ltid == 0) {
         *eSp = s.eq; *eSq = s.ep;
         *fSp = s.fq; *fSq = s.fp;
@@ -428,78 +580,56 @@ __device__ void pair_apply(const PairState<T> &s, long long m, long long nv, T *
     const T c = s.c, at = s.cat, sat = s.sat;
     // the reference marks both columns as changed after any rotation (src/dvjsvd.c:573)
     const bool real_rot = (!CPLX) || (sat == (T)0);
-    const bool cone = (c == (T)1);
     if (real_rot && at == (T)0) {
       // c == 1: identity (or a swap when permuting); c != 1 "never happens" (-4 / -10)
-      if (cone && perm) {
+      if (c == (T)1 && perm) {
         #pragma unroll 4
         for (long long i = ltid; i < m; i += TPP) {
           const T x = rp[i], y = rq[i];
-          Gp[i] = y; Gq[i] = x; rp[i] = y; rq[i] = x;
-          if (CPLX) { const T xi = rpi[i], yi = rqi[i]; Gip[i] = yi; Giq[i] = xi; rpi[i] = yi; rqi[i] = xi; }
-        }
-        #pragma unroll 4
-        for (long long i = ltid; i < nv; i += TPP) {
-          T t = Vp[i]; Vp[i] = Vq[i]; Vq[i] = t;
-          if (CPLX) { t = Vip[i]; Vip[i] = Viq[i]; Viq[i] = t; }
-        }
-      }
-    }
-    else if (real_rot) {
-      // the permuted form writes (y - t x) c to x and (x + t y) c to y: the same two
-      // products with the destinations exchanged
-      for (int pl = 0; pl < (CPLX ? 2 : 1); ++pl) {
-        T *X = pl ? Gip : Gp, *Y = pl ? Giq : Gq, *RX = pl ? rpi : rp, *RY = pl ? rqi : rq;
-        T *DX = perm ? Y : X, *DY = perm ? X : Y, *RDX = perm ? RY : RX, *RDY = perm ? RX : RY;
-        #pragma unroll 4
-        for (long long i = ltid; i < m; i += TPP) {
-          const T x = RX[i], y = RY[i];
-          T u = F::fma_(y, at, x);
-          T w = F::fma_(-x, at, y);
-          if (!cone) { u = u * c; w = w * c; }
-          DX[i] = u; DY[i] = w;
-          RDX[i] = u; RDY[i] = w;
-          amax(mG, u); amax(mG, w);
-        }
-        T *XV = pl ? Vip : Vp, *YV = pl ? Viq : Vq;
-        T *DXV = perm ? YV : XV, *DYV = perm ? XV : YV;
-        #pragma unroll 4
-        for (long long i = ltid; i < nv; i += TPP) {
-          const T x = XV[i], y = YV[i];
-          T u = F::fma_(y, at, x);
-          T w = F::fma_(-x, at, y);
-          if (!cone) { u = u * c; w = w * c; }
-          DXV[i] = u; DYV[i] = w;
-          if (TRACKV) { amax(mV, u); amax(mV, w); }
-        }
-      }
-    }
-    else {
-      const T cta = at, sta = sat, cna = -at;
-      for (int mat = 0; mat < 2; ++mat) {
-        T *Xr = mat ? Vp : Gp, *Xi = mat ? Vip : Gip, *Yr = mat ? Vq : Gq, *Yi = mat ? Viq : Giq;
-        const T *Rxr = mat ? Vp : rp, *Rxi = mat ? Vip : rpi, *Ryr = mat ? Vq : rq, *Ryi = mat ? Viq : rqi;
-        const long long rows = mat ? nv : m;
-        unsigned long long &mm = mat ? mV : mG;
-        #pragma unroll 4
-        for (long long i = ltid; i < rows; i += TPP) {
-          const T x_r = Rxr[i], x_i = Rxi[i], y_r = Ryr[i], y_i = Ryi[i];
-          T ar = F::fma_(y_r, cta, F::fma_(-y_i, sta, x_r));
-          T ai = F::fma_(y_r, sta, F::fma_(y_i, cta, x_i));
-          T br = F::fma_(x_r, cna, F::fma_(-x_i, sta, y_r));
-          T bi = F::fma_(x_r, sta, F::fma_(x_i, cna, y_i));
-          if (!cone) { ar = ar * c; ai = ai * c; br = br * c; bi = bi * c; }
-          if (perm) { Yr[i] = ar; Yi[i] = ai; Xr[i] = br; Xi[i] = bi; }
-          else { Xr[i] = ar; Xi[i] = ai; Yr[i] = br; Yi[i] = bi; }
-          if (!mat) {
-            if (perm) { rq[i] = ar; rqi[i] = ai; rp[i] = br; rpi[i] = bi; }
-            else { rp[i] = ar; rpi[i] = ai; rq[i] = br; rqi[i] = bi; }
+          Gp[i] = y; Gq[i] = x;
+          if (STG) { rp[i] = y; rq[i] = x; }
+          if (CPLX) {
+            const T xi = rpi[i], yi = rqi[i];
+            Gip[i] = yi; Giq[i] = xi;
+            if (STG) { rpi[i] = yi; rqi[i] = xi; }
           }
-          if (!mat || TRACKV) { amax(mm, ar); amax(mm, ai); amax(mm, br); amax(mm, bi); }
         }
+        swap_cols(Vp, Vq, nv, ltid, TPP);
+        if (CPLX)
+          swap_cols(Vip, Viq, nv, ltid, TPP);
+      }
+      return false;
+    }
+    U v0 = 0, v1 = 0;
+    if (real_rot) {
+      rot_real<T, STG, 4>((int)m, rp, rq, Gp, Gq, rp, rq, at, c, perm, ltid, TPP, true, mx[0], mx[1]);
+      rot_real<T, false, 4>((int)nv, Vp, Vq, Vp, Vq, nullptr, nullptr, at, c, perm, ltid, TPP, trackv, v0, v1);
+      if (trackv)
+        mV = (v0 > v1) ? v0 : v1;
+      if (CPLX) {
+        rot_real<T, STG, 4>((int)m, rpi, rqi, Gip, Giq, rpi, rqi, at, c, perm, ltid, TPP, true, mx[CPLX ? 2 : 0],
+                                  mx[CPLX ? 3 : 1]);
+        rot_real<T, false, 4>((int)nv, Vip, Viq, Vip, Viq, nullptr, nullptr, at, c, perm, ltid, TPP, trackv, v0, v1);
+        if (trackv) {
+          v0 = (v0 > v1) ? v0 : v1;
+          mV = (v0 > mV) ? v0 : mV;
+        }
+      }
+    }
+    else if constexpr (CPLX) {
+      U v4[4] = {0, 0, 0, 0};
+      rot_cplx<T, STG, 2>((int)m, rp, rpi, rq, rqi, Gp, Gip, Gq, Giq, rp, rpi, rq, rqi, at, sat, c, perm, ltid,
+                                TPP, true, mx);
+      rot_cplx<T, false, 2>((int)nv, Vp, Vip, Vq, Viq, Vp, Vip, Vq, Viq, nullptr, nullptr, nullptr, nullptr,
+                                    at, sat, c, perm, ltid, TPP, trackv, v4);
+      if (trackv) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          mV = (v4[k] > mV) ? v4[k] : mV;
       }
     }
   }
+  return true;
 }
 
 }  // namespace vj

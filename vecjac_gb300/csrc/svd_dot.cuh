@@ -63,13 +63,14 @@ template <typename T, bool CPLX> struct DotTerms {
 // 19 when it is a DADD, a DMUL or an FMA with a constant operand (measured with 4 to 16
 // warps of independent chains; the latency of 64 clocks is the same), so a + b is formed as
 // a * 1 + b and the round-down product as a * b + (-0), with the 1 and the -0 held in
-// registers. The values are those of the plain operations; only a zero product may come out
-// as -0 instead of +0, which no sum below can tell apart (a sum that starts at +0 never
+// registers. The values are those of the plain operations; only a zero round-down product
+// may come out as -0 instead of +0, which no sum below can tell apart (a sum that starts at +0 never
 // becomes -0 in round-to-nearest).
 template <typename T> struct DotOps {
   static __device__ __forceinline__ DotOps make() { return DotOps(); }
   __device__ __forceinline__ T add(T a, T b) const { return a + b; }
   __device__ __forceinline__ T sub(T a, T b) const { return a - b; }
+  __device__ __forceinline__ T mul(T a, T b) const { return a * b; }
   __device__ __forceinline__ T mul_rd(T a, T b) const { return fp<T>::mul_rd(a, b); }
 };
 #ifdef __CUDA_ARCH__
@@ -85,6 +86,7 @@ template <> struct DotOps<double> {
   }
   __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
   __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(a, one, -b); }
+  __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, mzero); }
   __device__ __forceinline__ double mul_rd(double a, double b) const { return __fma_rd(a, b, mzero); }
 };
 #endif

@@ -25,33 +25,68 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
   return v;
 }
 
-// The project's column norm (two-pass power-of-two scaling, 32 lanes, halving tree) for
-// one warp; every lane returns the same value.
-template <typename T> __device__ T warp_nrm2(const T *x, long long m)
+// The second pass of the project's column norm: the sum of squares of x scaled by the power of
+// two of its largest magnitude (mx: that magnitude's bits), for one warp; every lane returns
+// the same value. Blocks of four elements per lane that scale to normal values (all of a
+// column but its smallest entries) run as straight-line code, so that their loads and
+// exponent adds overlap the accumulator's FMAs.
+template <typename T> __device__ T warp_nrm2_scaled(const T *x, long long m, unsigned long long mx)
 {
+  using F = fp<T>;
   const int lane = threadIdx.x & 31;
-  unsigned long long mx = 0ull;
-  for (long long i = lane; i < m; i += 32) {
-    const unsigned long long a = absbits(x[i]);
-    mx = (a > mx) ? a : mx;
-  }
-  mx = warp_max_u64(mx);
   const T a = bitst<T>(mx);
   if (!visfinite(a))
-    return visnan(a) ? fp<T>::qnan() : a;
+    return visnan(a) ? F::qnan() : a;
   if (mx == 0ull)
     return (T)0;
-  const int k = ilogb_(a);
+  const int k = ilogb_(a), mm = (int)m;
   T acc = (T)0;
-  for (long long i = lane; i < m; i += 32) {
+  int i = lane;
+  for (; i + 96 < mm; i += 128) {
+    T y[4];
+    bool fast = true;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      y[u] = x[i + 32 * u];
+      const int be = (int)((F::bits(y[u]) & ~F::SIGN) >> F::MB);
+      fast = fast && (be > 0) && (be - k > 0);  // (|x| <= 2^(k+1): no overflow)
+    }
+    if (fast) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        y[u] = F::val(F::bits(y[u]) + ((typename F::U)(long long)(-k) << F::MB));
+    }
+    else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        y[u] = scale2(y[u], -k);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      acc = F::fma_(y[u], y[u], acc);
+  }
+  for (; i < mm; i += 32) {
     const T y = scale2(x[i], -k);
-    acc = fp<T>::fma_(y, y, acc);
+    acc = F::fma_(y, y, acc);
   }
 #pragma unroll
   for (int w = 16; w >= 1; w >>= 1)
     acc = acc + __shfl_down_sync(0xffffffffu, acc, w);
   acc = __shfl_sync(0xffffffffu, acc, 0);
-  return scale2(fp<T>::sqrt_(acc), k);
+  return scale2(F::sqrt_(acc), k);
+}
+
+// The project's column norm (two-pass power-of-two scaling, 32 lanes, halving tree) for
+// one warp; every lane returns the same value.
+template <typename T> __device__ T warp_nrm2(const T *x, long long m)
+{
+  const int lane = threadIdx.x & 31;
+  typename fp<T>::U mx = 0;
+  for (long long i = lane; i < m; i += 32) {
+    const typename fp<T>::U a = fp<T>::bits(x[i]) & ~fp<T>::SIGN;
+    mx = (a > mx) ? a : mx;
+  }
+  return warp_nrm2_scaled(x, m, warp_max_u64((unsigned long long)mx));
 }
 
 }  // namespace vj
