@@ -224,7 +224,7 @@ template <typename T> __device__ long long svd_one(const BatchArgs<T> &a, BatchS
           fS[p] = s.fq; fS[q] = s.fp;
         }
         T *Gp = G + (long long)p * m, *Gq = G + (long long)q * m;
-        pair_apply<T, false, false>(s, m, n, Gp, Gq, nullptr, nullptr, V + (long long)p * n, V + (long long)q * n,
+        pair_apply<T, false, false, 4>(s, m, n, Gp, Gq, nullptr, nullptr, V + (long long)p * n, V + (long long)q * n,
                                     nullptr, nullptr, Gp, Gq, nullptr, nullptr, eS + p, eS + q, fS + p, fS + q,
                                     lane, 32, false, mx, mV);
         if (lane == 0) {

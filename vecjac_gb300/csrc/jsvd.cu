@@ -55,11 +55,12 @@ template <typename T, bool CPLX, int P> struct StepDims {
   static constexpr int NT = CPLX ? 2 : 1;                   // terms per row and chain
   static constexpr int NG = P * NCH;                        // (pair, chain) groups
   static constexpr int NCW = (NG * L + 31) / 32;            // chain warps
-  static constexpr int K = ((sizeof(T) == 8) ? 16 : 32) / NT;  // rows per lane and chunk
+  static constexpr int K = ((sizeof(T) == 8) ? 16 : 64) / NT;  // rows per lane and chunk
   static constexpr int RC = K * L;                          // rows per chunk
   static constexpr int BUF = K * NT * NG * L;               // elements of one buffer
   static constexpr size_t buf_bytes() { return 2u * (size_t)BUF * sizeof(T); }
-  static_assert(NCW <= 4, "at least half of the warps form products");
+  static constexpr int NPT = (NCW == 4) ? 128 : 64 * (4 - NCW);  // producing threads
+  static_assert(NCW <= 4, "at least two warps form products");
 };
 
 // The FP64 / FP32 2x2 of jac2.cuh (cosine and tangent form) by the four lanes of a quad, r =
@@ -180,27 +181,12 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
   __shared__ int s_col[P][2], s_n[P][2], s_live[P], s_trk[P];
   __shared__ int s_err;
   __shared__ unsigned long long bar;
-  pdl_enter();
-  SvdGlobal *const g = a.g;
-  if (*(volatile long long *)&g->err)
-    return;
-  const Ctl &cur = g->ctl[g3];
-  Ctl &nxt = g->ctl[(g3 + 1) % 3];
-  Ctl &nn = g->ctl[(g3 + 2) % 3];
+  // before the previous step is waited for: the pivot table, which no step writes
   const unsigned *r = a.js + (size_t)st * (size_t)a.n;
   const long long n_2 = a.n >> 1;
   const long long pair0 = (long long)blockIdx.x * P;
   const int np = (int)((n_2 - pair0 < P) ? (n_2 - pair0) : P);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool tr = a.trace && blockIdx.x == 0 && tid == 0;
-  long long tmark = tr ? clock64() : 0;
-  auto tphase = [&](int ph) {
-    if (tr) {
-      const long long t = clock64();
-      atomicAdd(&g->phase[ph], (unsigned long long)(t - tmark));
-      tmark = t;
-    }
-  };
   if (tid < 2 * P) {
     const int j = tid >> 1, c = tid & 1;
     s_col[j][c] = (j < np) ? (int)r[2 * (pair0 + j) + c] : 0;
@@ -213,6 +199,23 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
     if (STAGE)
       mbar_init(&bar, 1u);
   }
+  __syncthreads();
+  pdl_enter();
+  SvdGlobal *const g = a.g;
+  if (*(volatile long long *)&g->err)
+    return;
+  const Ctl &cur = g->ctl[g3];
+  Ctl &nxt = g->ctl[(g3 + 1) % 3];
+  Ctl &nn = g->ctl[(g3 + 2) % 3];
+  const bool tr = a.trace && blockIdx.x == 0 && tid == 0;
+  long long tmark = tr ? clock64() : 0;
+  auto tphase = [&](int ph) {
+    if (tr) {
+      const long long t = clock64();
+      atomicAdd(&g->phase[ph], (unsigned long long)(t - tmark));
+      tmark = t;
+    }
+  };
   const Decision<T> d = decide(a, cur);
   if (blockIdx.x == 0 && tid == 0) {
     nxt.MGbase = (double)d.MG;
@@ -223,7 +226,6 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
     nn.nMV = 0ull;
     nn.ovf = 0;
   }
-  __syncthreads();
   auto colp = [&](int j) { return (long long)s_col[j][0]; };
   auto colq = [&](int j) { return (long long)s_col[j][1]; };
   // ---- 1. rescaling (rare) ----
@@ -265,8 +267,8 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
     const long long col = (c & 1) ? colq(j) : colp(j);
     return (c < 2) ? (a.G + col * a.ldG) : (a.Gi + col * a.ldGi);
   };
-  if (tid < P) {
-    const int j = tid;
+  if (tid >= 32 && tid < 32 + P) {  // (not the warp that issues the copies)
+    const int j = tid - 32;
     const T ep = (j < np) ? a.eS[colp(j)] : (T)0, eq = (j < np) ? a.eS[colq(j)] : (T)0;
     const bool live = (j < np) && (eq >= -svdc<T>::RMAX) && (ep >= -svdc<T>::RMAX);
     PairState<T> &s = ps[j];
@@ -351,19 +353,35 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
   T cs = 0, ct = 0;  // this lane's recurrence
   const int gl = warp * 32 + lane;
   const int nchunks = (mi + D::RC - 1) / D::RC;
+  // this thread's index among the producers: the warps of the sub-partitions without a chain
+  // warp where there are any (warp w runs on sub-partition w mod 4)
+  const int wp = warp & 3, skip = D::NCW & 3;
+  const int pt = (D::NCW == 4) ? tid - 128 : (wp < skip) ? -1 : ((warp >> 2) * (4 - skip) + wp - skip) * 32 + lane;
   for (int ck = 0; ck < nchunks; ++ck) {
     if (warp < D::NCW) {
       const T *v = buf + (ck & 1) * D::BUF + gl % (D::NG * L);
       constexpr int W = D::NG * L, UN = 8;
       int left = min(D::RC, mi - ck * D::RC) / L * D::NT;  // recurrence steps of this chunk
-      for (; left >= UN; left -= UN, v += UN * W) {
-        T x[UN];
+      T x[UN];
+      if (left >= UN) {
 #pragma unroll
         for (int u = 0; u < UN; ++u)
           x[u] = v[u * W];
+      }
+      for (; left >= UN; left -= UN) {
+        v += UN * W;
+        T y[UN];
+        if (left >= 2 * UN) {
+#pragma unroll
+          for (int u = 0; u < UN; ++u)
+            y[u] = v[u * W];
+        }
 #pragma unroll
         for (int u = 0; u < UN; ++u)
           sum_step(ops, x[u], cs, ct);
+#pragma unroll
+        for (int u = 0; u < UN; ++u)
+          x[u] = y[u];
       }
       for (; left > 0; --left, v += W)
         sum_step(ops, v[0], cs, ct);
@@ -373,8 +391,8 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
         const PairState<T> &s = ps[lane];
         pre[lane] = pair_pre(s.ep, s.fp, s.eq, s.fq, a.gst);
       }
-      if (ck + 1 < nchunks)
-        produce(ck + 1, tid - 32 * D::NCW, 256 - 32 * D::NCW);
+      if (ck + 1 < nchunks && pt >= 0)
+        produce(ck + 1, pt, D::NPT);
     }
     __syncthreads();
   }
@@ -464,7 +482,7 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
       const long long p = colp(j), q = colq(j);
       T *Gip = CPLX ? (a.Gi + p * a.ldGi) : nullptr, *Giq = CPLX ? (a.Gi + q * a.ldGi) : nullptr;
       T *Vip = CPLX ? (a.Vi + p * a.ldVi) : nullptr, *Viq = CPLX ? (a.Vi + q * a.ldVi) : nullptr;
-      const bool trk = pair_apply<T, CPLX, STAGE>(
+      const bool trk = pair_apply<T, CPLX, STAGE, (P == 4) ? 8 : 4>(
           ps[j], a.m, a.n, a.G + p * a.ldG, a.G + q * a.ldG, Gip, Giq, a.V + p * a.ldV, a.V + q * a.ldV, Vip, Viq,
           rcol(j, 0), rcol(j, 1), CPLX ? rcol(j, 2) : nullptr, CPLX ? rcol(j, 3) : nullptr, a.eS + p, a.eS + q,
           a.fS + p, a.fS + q, ltid, TPP, a.trackv != 0, mx, mV);

@@ -352,9 +352,9 @@ template <typename T> __device__ __forceinline__ void swap_cols(T *x, T *y, long
   }
 }
 
-// Rows of a column pair rotated, UR of a thread's rows loaded before any is stored: a store
-// may alias a later load as far as the compiler knows, so a row-by-row loop would wait for
-// one memory round trip per row. Reads (rx, ry), writes (x, y) and, when STG, the staged copy
+// Rows of a column pair rotated, UR of a thread's rows at a time with the next UR loaded before
+// these are stored: a store may alias a later load as far as the compiler knows, so a
+// row-by-row loop would wait for one memory round trip per row. Reads (rx, ry), writes (x, y) and, when STG, the staged copy
 // as well; mx and my collect max |.| of what x and y receive when track is set. The products by the
 // cosine are three-register FMAs (svd_dot.cuh, DotOps).
 template <typename T, bool STG, int UR>
@@ -369,35 +369,64 @@ __device__ __forceinline__ void rot_real(int rows, const T *rx, const T *ry, T *
   // with the destinations exchanged
   T *const dx = perm ? y : x, *const dy = perm ? x : y, *const dsx = perm ? sy : sx, *const dsy = perm ? sx : sy;
   typename F::U mu = 0, mw = 0;
-  for (int i0 = ltid; i0 < rows; i0 += UR * TPP) {
-    T u[UR], w[UR];
-#pragma unroll
-    for (int k = 0; k < UR; ++k) {
-      const int i = i0 + k * TPP;
-      u[k] = (i < rows) ? rx[i] : (T)0;
-      w[k] = (i < rows) ? ry[i] : (T)0;
-    }
-#pragma unroll
-    for (int k = 0; k < UR; ++k) {
-      const T a = F::fma_(w[k], at, u[k]), b = F::fma_(-u[k], at, w[k]);
-      u[k] = cone ? a : o.mul(a, c);
-      w[k] = cone ? b : o.mul(b, c);
-    }
+  T nu[UR], nw[UR];
+  auto load = [&](int i0) {
 #pragma unroll
     for (int k = 0; k < UR; ++k) {
       const int i = i0 + k * TPP;
       if (i < rows) {
-        dx[i] = u[k];
-        dy[i] = w[k];
-        if (STG) {
-          dsx[i] = u[k];
-          dsy[i] = w[k];
-        }
-        if (track) {
-          amax(mu, u[k]);
-          amax(mw, w[k]);
-        }
+        nu[k] = rx[i];
+        nw[k] = ry[i];
       }
+    }
+  };
+  load(ltid);
+  for (int i0 = ltid; i0 < rows; i0 += UR * TPP) {
+    T u[UR], w[UR];
+#pragma unroll
+    for (int k = 0; k < UR; ++k) {
+      u[k] = nu[k];
+      w[k] = nw[k];
+    }
+    load(i0 + UR * TPP);
+    auto rotate = [&](int k) {
+      const T x = u[k];
+      u[k] = F::fma_(w[k], at, x);
+      w[k] = F::fma_(-x, at, w[k]);
+      if (!cone) {
+        u[k] = o.mul(u[k], c);
+        w[k] = o.mul(w[k], c);
+      }
+    };
+    auto store = [&](int k) {
+      const int i = i0 + k * TPP;
+      dx[i] = u[k];
+      dy[i] = w[k];
+      if (STG) {
+        dsx[i] = u[k];
+        dsy[i] = w[k];
+      }
+      if (track) {
+        amax(mu, u[k]);
+        amax(mw, w[k]);
+      }
+    };
+    // (all of a batch's FMAs before the first use of their results)
+    if (i0 + (UR - 1) * TPP < rows) {
+#pragma unroll
+      for (int k = 0; k < UR; ++k)
+        rotate(k);
+#pragma unroll
+      for (int k = 0; k < UR; ++k)
+        store(k);
+    }
+    else {
+#pragma unroll
+      for (int k = 0; k < UR - 1; ++k)
+        if (i0 + k * TPP < rows) {
+          rotate(k);
+          store(k);
+        }
     }
   }
   if (track) {
@@ -419,49 +448,77 @@ __device__ __forceinline__ void rot_cplx(int rows, const T *rxr, const T *rxi, c
   T *const sar = perm ? syr : sxr, *const sai = perm ? syi : sxi, *const sbr = perm ? sxr : syr,
            *const sbi = perm ? sxi : syi;
   typename F::U mar = 0, mai = 0, mbr = 0, mbi = 0;
-  for (int i0 = ltid; i0 < rows; i0 += UR * TPP) {
-    T ar[UR], ai[UR], br[UR], bi[UR];
-#pragma unroll
-    for (int k = 0; k < UR; ++k) {
-      const int i = i0 + k * TPP;
-      const bool in = (i < rows);
-      ar[k] = in ? rxr[i] : (T)0;
-      ai[k] = in ? rxi[i] : (T)0;
-      br[k] = in ? ryr[i] : (T)0;
-      bi[k] = in ? ryi[i] : (T)0;
-    }
-#pragma unroll
-    for (int k = 0; k < UR; ++k) {
-      const T x_r = ar[k], x_i = ai[k], y_r = br[k], y_i = bi[k];
-      T u = F::fma_(y_r, cta, F::fma_(-y_i, sta, x_r)), v = F::fma_(y_r, sta, F::fma_(y_i, cta, x_i));
-      ar[k] = cone ? u : o.mul(u, c);
-      ai[k] = cone ? v : o.mul(v, c);
-      u = F::fma_(x_r, cna, F::fma_(-x_i, sta, y_r));
-      v = F::fma_(x_r, sta, F::fma_(x_i, cna, y_i));
-      br[k] = cone ? u : o.mul(u, c);
-      bi[k] = cone ? v : o.mul(v, c);
-    }
+  T nxr[UR], nxi[UR], nyr[UR], nyi[UR];
+  auto load = [&](int i0) {
 #pragma unroll
     for (int k = 0; k < UR; ++k) {
       const int i = i0 + k * TPP;
       if (i < rows) {
-        dar[i] = ar[k];
-        dai[i] = ai[k];
-        dbr[i] = br[k];
-        dbi[i] = bi[k];
-        if (STG) {
-          sar[i] = ar[k];
-          sai[i] = ai[k];
-          sbr[i] = br[k];
-          sbi[i] = bi[k];
-        }
-        if (track) {
-          amax(mar, ar[k]);
-          amax(mai, ai[k]);
-          amax(mbr, br[k]);
-          amax(mbi, bi[k]);
-        }
+        nxr[k] = rxr[i];
+        nxi[k] = rxi[i];
+        nyr[k] = ryr[i];
+        nyi[k] = ryi[i];
       }
+    }
+  };
+  load(ltid);
+  for (int i0 = ltid; i0 < rows; i0 += UR * TPP) {
+    T xr_[UR], xi_[UR], yr_[UR], yi_[UR];
+#pragma unroll
+    for (int k = 0; k < UR; ++k) {
+      xr_[k] = nxr[k];
+      xi_[k] = nxi[k];
+      yr_[k] = nyr[k];
+      yi_[k] = nyi[k];
+    }
+    load(i0 + UR * TPP);
+    auto rotate = [&](int k) {
+      const T x_r = xr_[k], x_i = xi_[k], y_r = yr_[k], y_i = yi_[k];
+      xr_[k] = F::fma_(y_r, cta, F::fma_(-y_i, sta, x_r));
+      xi_[k] = F::fma_(y_r, sta, F::fma_(y_i, cta, x_i));
+      yr_[k] = F::fma_(x_r, cna, F::fma_(-x_i, sta, y_r));
+      yi_[k] = F::fma_(x_r, sta, F::fma_(x_i, cna, y_i));
+      if (!cone) {
+        xr_[k] = o.mul(xr_[k], c);
+        xi_[k] = o.mul(xi_[k], c);
+        yr_[k] = o.mul(yr_[k], c);
+        yi_[k] = o.mul(yi_[k], c);
+      }
+    };
+    auto store = [&](int k) {
+      const int i = i0 + k * TPP;
+      dar[i] = xr_[k];
+      dai[i] = xi_[k];
+      dbr[i] = yr_[k];
+      dbi[i] = yi_[k];
+      if (STG) {
+        sar[i] = xr_[k];
+        sai[i] = xi_[k];
+        sbr[i] = yr_[k];
+        sbi[i] = yi_[k];
+      }
+      if (track) {
+        amax(mar, xr_[k]);
+        amax(mai, xi_[k]);
+        amax(mbr, yr_[k]);
+        amax(mbi, yi_[k]);
+      }
+    };
+    if (i0 + (UR - 1) * TPP < rows) {
+#pragma unroll
+      for (int k = 0; k < UR; ++k)
+        rotate(k);
+#pragma unroll
+      for (int k = 0; k < UR; ++k)
+        store(k);
+    }
+    else {
+#pragma unroll
+      for (int k = 0; k < UR - 1; ++k)
+        if (i0 + k * TPP < rows) {
+          rotate(k);
+          store(k);
+        }
     }
   }
   if (track) {
@@ -480,8 +537,8 @@ __device__ __forceinline__ void rot_cplx(int rows, const T *rxr, const T *rxi, c
 // columns p and q of G receive (their imaginary planes in mx[2], mx[3]) and mV, with trackv,
 // that of V. Returns whether mx holds the maxima of the changed columns: false for a
 // rotation by nothing or by a plain exchange, whose columns count as changed without being
-// tracked.
-template <typename T, bool CPLX, bool STG>
+// tracked. UR: rows per thread in flight (rot_real; half of it for complex columns).
+template <typename T, bool CPLX, bool STG, int UR>
 __device__ bool pair_apply(const PairState<T> &s, long long m, long long nv, T *Gp, T *Gq, T *Gip, T *Giq, T *Vp,
                            T *Vq, T *Vip, T *Viq, T *rp, T *rq, T *rpi, T *rqi, T *eSp, T *eSq, T *fSp, T *fSq,
                            int ltid, int TPP, bool trackv, typename fp<T>::U (&mx)[CPLX ? 4 : 2],
@@ -602,14 +659,14 @@ __device__ bool pair_apply(const PairState<T> &s, long long m, long long nv, T *
     }
     U v0 = 0, v1 = 0;
     if (real_rot) {
-      rot_real<T, STG, 4>((int)m, rp, rq, Gp, Gq, rp, rq, at, c, perm, ltid, TPP, true, mx[0], mx[1]);
-      rot_real<T, false, 4>((int)nv, Vp, Vq, Vp, Vq, nullptr, nullptr, at, c, perm, ltid, TPP, trackv, v0, v1);
+      rot_real<T, STG, UR>((int)m, rp, rq, Gp, Gq, rp, rq, at, c, perm, ltid, TPP, true, mx[0], mx[1]);
+      rot_real<T, false, UR>((int)nv, Vp, Vq, Vp, Vq, nullptr, nullptr, at, c, perm, ltid, TPP, trackv, v0, v1);
       if (trackv)
         mV = (v0 > v1) ? v0 : v1;
       if (CPLX) {
-        rot_real<T, STG, 4>((int)m, rpi, rqi, Gip, Giq, rpi, rqi, at, c, perm, ltid, TPP, true, mx[CPLX ? 2 : 0],
+        rot_real<T, STG, UR>((int)m, rpi, rqi, Gip, Giq, rpi, rqi, at, c, perm, ltid, TPP, true, mx[CPLX ? 2 : 0],
                                   mx[CPLX ? 3 : 1]);
-        rot_real<T, false, 4>((int)nv, Vip, Viq, Vip, Viq, nullptr, nullptr, at, c, perm, ltid, TPP, trackv, v0, v1);
+        rot_real<T, false, UR>((int)nv, Vip, Viq, Vip, Viq, nullptr, nullptr, at, c, perm, ltid, TPP, trackv, v0, v1);
         if (trackv) {
           v0 = (v0 > v1) ? v0 : v1;
           mV = (v0 > mV) ? v0 : mV;
@@ -618,9 +675,9 @@ __device__ bool pair_apply(const PairState<T> &s, long long m, long long nv, T *
     }
     else if constexpr (CPLX) {
       U v4[4] = {0, 0, 0, 0};
-      rot_cplx<T, STG, 2>((int)m, rp, rpi, rq, rqi, Gp, Gip, Gq, Giq, rp, rpi, rq, rqi, at, sat, c, perm, ltid,
+      rot_cplx<T, STG, UR / 2>((int)m, rp, rpi, rq, rqi, Gp, Gip, Gq, Giq, rp, rpi, rq, rqi, at, sat, c, perm, ltid,
                                 TPP, true, mx);
-      rot_cplx<T, false, 2>((int)nv, Vp, Vip, Vq, Viq, Vp, Vip, Vq, Viq, nullptr, nullptr, nullptr, nullptr,
+      rot_cplx<T, false, UR / 2>((int)nv, Vp, Vip, Vq, Viq, Vp, Vip, Vq, Viq, nullptr, nullptr, nullptr, nullptr,
                                     at, sat, c, perm, ltid, TPP, trackv, v4);
       if (trackv) {
 #pragma unroll
