@@ -1,54 +1,154 @@
 // Batched one-sided Jacobi SVD: thousands of independent matrices of uneven size in one
 // persistent launch (real FP64 and FP32; every matrix with dvjsvd_'s / svjsvd_'s result).
 //
-// One CTA owns one matrix at a time and runs the reference driver on it literally
-// (src/dvjsvd.c:78-638): setup and global prescale, then sweeps of pivot steps, each step
-// being "norms of the changed columns (with the overflow retry) -> all scaled dot products
-// -> error check -> classification -> all transformations -> max |G|, max |V| update", with
-// __syncthreads between the phases. Matrices are handed out by an atomic work queue in the
-// order the caller gives (largest first balances the tail); a matrix stops at its own
-// convergence (its own sweep count, its own info entry), so uneven convergence does not
-// hold the batch back. Pivot pairs are computed on the fly from the strategy's closed
-// form (pjs.cuh), so no tables are stored. Matrix sizes: m >= n, n <= 512, and the
-// reference's divisibility rules (the host wrapper pads with zero rows/columns).
+// A matrix is worked on by one CTA, or, when it is so large that its CTA would finish after
+// the rest of the batch, by a cluster of BATCH_CS CTAs (svd_one's team, batch_core.cuh). Each
+// team runs the reference driver on its matrix (src/dvjsvd.c:78-638) with one barrier per
+// pivot step. Matrices are handed out by atomic work queues in the order the caller gives
+// (largest first balances the tail); a matrix stops at its own convergence (its own sweep
+// count, its own info entry), so uneven convergence does not hold the batch back. Pivot pairs
+// are computed on the fly from the strategy's closed form (pjs.cuh), so no tables are stored.
+// Matrix sizes: m >= n, n <= 512, and the reference's divisibility rules (the host wrapper
+// pads with zero rows/columns).
 #include <cuda_runtime.h>
 
 #include "batch_core.cuh"
 
 namespace vj {
 
+// CTAs per cluster, and the cost of a large matrix in shares of a CTA (k_plan): 300 FP32
+// matrices of up to 512 rows take 717 ms by single CTAs and 171 ms in clusters of 4 (119 ms in
+// clusters of 8), 1500 FP64 ones of up to 128 rows 129, 117 and 145 ms, and from half a share
+// 128 ms in clusters of 4: a cluster larger than its matrix leaves CTAs idle.
+constexpr int BATCH_CS = 4;
+constexpr double BATCH_SHARE = 1.0;
+
+// a matrix's work, up to its number of sweeps
+__device__ __forceinline__ double batch_cost(long long m, long long n)
+{
+  return (n > 0 && m > 0) ? (double)n * (double)n * (double)(m + n) : 0.0;
+}
+
+// The queues' heads and the size from which a matrix is large: its cost above `share` times
+// what each of `slots` CTAs would have of the whole batch's, and enough groups of pairs for
+// more than the `warps` warps of one CTA. One CTA of 1024 threads.
+template <typename T>
+__global__ void __launch_bounds__(1024) k_plan(BatchArgs<T> a, int slots, int warps, double share)
+{
+  __shared__ double sum[32];
+  __shared__ unsigned end;
+  const int tid = threadIdx.x;
+  double c = 0;
+  for (long long i = tid; i < a.count; i += blockDim.x)
+    c += batch_cost(a.m[i], a.n[i]);
+  for (int o = 16; o >= 1; o >>= 1)
+    c += __shfl_xor_sync(0xffffffffu, c, o);
+  if ((tid & 31) == 0)
+    sum[tid >> 5] = c;
+  if (tid == 0)
+    end = 0u;
+  __syncthreads();
+  c = 0;
+  for (int w = 0; w < 32; ++w)
+    c += sum[w];
+  const double nmin = 2.0 * (32 / svdc<T>::LANES) * warps;  // columns that one CTA's warps take at once
+  const double limit = fmax(share * c / slots, 2.0 * nmin * nmin * nmin);
+  for (long long i = tid; i < a.count; i += blockDim.x) {
+    const int b = a.order ? a.order[i] : (int)i;
+    if (batch_cost(a.m[b], a.n[b]) > limit)
+      atomicMax(&end, (unsigned)(i + 1));
+  }
+  __syncthreads();
+  if (tid == 0) {
+    a.plan->next_large = 0u;
+    a.plan->next = 0u;
+    a.plan->end_large = end;
+    a.plan->limit = limit;
+  }
+}
+
+// (one copy of the driver for the two places that call it)
+template <typename T>
+__device__ __noinline__ void svd_matrix(const BatchArgs<T> &a, BatchShared<T> &sh, int b, Team tm, BatchShared<T> *s0)
+{
+  const long long r = svd_one<T>(a, sh, a.m[b], a.n[b], a.G + a.offG[b], a.V + a.offV[b], a.eS + a.offS[b],
+                                 a.fS + a.offS[b], tm, s0);
+  if (threadIdx.x == 0 && tm.rank == 0)
+    a.info[b] = r;
+}
+
 // MINB: the register bound for MINB resident CTAs of 256 threads per SM (more, smaller
 // CTAs when the caller launches fewer threads per CTA). The best bound depends on the
-// batch (the autotuner of vecjac_gb300/batch.py searches it with the CTA size): on the
-// 20,000-matrix FP32 batch 4 CTAs of 256 threads (64 registers) gave 1434 matrices/s,
-// 3 (80 registers) 1221, 2 (128) 937.
+// batch (the autotuner of vecjac_gb300/batch.py searches it with the CTA size).
 template <typename T, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_batch(BatchArgs<T> a)
 {
   __shared__ BatchShared<T> sh;
-  __shared__ long long s_b;
+  __shared__ long long s_b[2];
+  unsigned rank, size;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+  BatchPlan *const plan = a.plan;
+  const double limit = plan->limit;
+  const unsigned end = plan->end_large;
+  auto large = [&](int b) { return batch_cost(a.m[b], a.n[b]) > limit; };
+  // the large matrices, by whole clusters
+  if (end && size > 1u) {
+    const Team tm{(int)rank, (int)size};
+    // rank 0's shared words as seen from this CTA
+    BatchShared<T> *const s0 = team_peer(tm, &sh, 0);
+    volatile long long *const b0 = team_peer(tm, s_b, 0);
+    for (int it = 0;; it ^= 1) {
+      if (rank == 0 && threadIdx.x == 0) {
+        long long got = -1;
+        for (;;) {
+          const unsigned i = atomicAdd(&plan->next_large, 1u);
+          if (i >= end)
+            break;
+          const int b = a.order ? a.order[i] : (int)i;
+          if (large(b)) {
+            got = b;
+            break;
+          }
+        }
+        s_b[it] = got;
+      }
+      team_sync(tm);
+      const long long b = b0[it];
+      if (b < 0)
+        break;
+      svd_matrix<T>(a, sh, (int)b, tm, s0);
+    }
+    team_sync(tm);  // no CTA's shared words are read by another from here on
+  }
+  // the others, by single CTAs
+  const bool split = end && size > 1u;
   for (;;) {
-    if (threadIdx.x == 0)
-      s_b = (long long)atomicAdd(a.queue, 1u);
     __syncthreads();
-    const long long bi = s_b;
+    if (threadIdx.x == 0) {
+      long long got = -1;
+      for (;;) {
+        const long long i = (long long)atomicAdd(&plan->next, 1u);
+        if (i >= a.count)
+          break;
+        const int b = a.order ? a.order[i] : (int)i;
+        if (!split || i >= (long long)end || !large(b)) {
+          got = b;
+          break;
+        }
+      }
+      s_b[0] = got;
+    }
     __syncthreads();
-    if (bi >= a.count)
+    const long long b = s_b[0];
+    if (b < 0)
       return;
-    const int b = a.order ? a.order[bi] : (int)bi;
-    const long long r = svd_one<T>(a, sh, a.m[b], a.n[b], a.G + a.offG[b], a.V + a.offV[b], a.eS + a.offS[b],
-                                   a.fS + a.offS[b]);
-    if (threadIdx.x == 0)
-      a.info[b] = r;
-    __syncthreads();
+    svd_matrix<T>(a, sh, (int)b, Team{0, 1}, &sh);
   }
 }
 
-// default register bound: FP32 4 CTAs of 256 threads per SM, FP64 2 (118 registers; a
-// bound of 3 spills)
+// default register bound: FP32 4 CTAs of 256 threads per SM, FP64 2
 template <typename T> constexpr int batch_occ_default() { return sizeof(T) == 4 ? 4 : 2; }
-
-template <typename T, int MINB> static void *batch_kernel() { return reinterpret_cast<void *>(k_batch<T, MINB>); }
 
 template <typename T>
 static vj_fint batch_dev(vj_fint count, const long long *m, const long long *n, T *G, const long long *offG, T *V,
@@ -66,30 +166,40 @@ static vj_fint batch_dev(vj_fint count, const long long *m, const long long *n, 
   if (occ < 2 || occ > 6)
     occ = batch_occ_default<T>();
   cudaStream_t s = (cudaStream_t)stream;
-  unsigned *queue = host::batch_queue();
-  if (!queue)
+  BatchPlan *plan = static_cast<BatchPlan *>(host::batch_plan());
+  if (!plan)
     return VJ_ERR_NOMEM;
-  if (cudaMemsetAsync(queue, 0, sizeof(unsigned), s) != cudaSuccess)
-    return VJ_ERR_CUDA;
   BatchArgs<T> a;
   a.count = count;
   a.m = m; a.n = n; a.offG = offG; a.offV = offV; a.offS = offS; a.order = order;
-  a.G = G; a.V = V; a.eS = eS; a.fS = fS; a.info = info; a.queue = queue;
+  a.G = G; a.V = V; a.eS = eS; a.fS = fS; a.info = info; a.plan = plan;
   a.strategy = (int)strategy;
   a.swp = swp;
-  void *k = (occ == 2)   ? batch_kernel<T, 2>()
-            : (occ == 3) ? batch_kernel<T, 3>()
-            : (occ == 4) ? batch_kernel<T, 4>()
-            : (occ == 5) ? batch_kernel<T, 5>()
-                         : batch_kernel<T, 6>();
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, block, 0) != cudaSuccess || per_sm < 1)
-    per_sm = 1;
-  long long grid = (long long)host::sm_count() * per_sm;
-  if (grid > count)
-    grid = count;
-  void *args[] = {&a};
-  if (cudaLaunchKernel(k, dim3((unsigned)grid), dim3((unsigned)block), args, 0, s) != cudaSuccess)
+  void (*k)(BatchArgs<T>) = (occ == 2)   ? k_batch<T, 2>
+                            : (occ == 3) ? k_batch<T, 3>
+                            : (occ == 4) ? k_batch<T, 4>
+                            : (occ == 5) ? k_batch<T, 5>
+                                         : k_batch<T, 6>;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = BATCH_CS;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cfg.gridDim = dim3(BATCH_CS);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = s;
+  int clusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) != cudaSuccess || clusters < 1) {
+    cudaGetLastError();
+    clusters = 1;
+  }
+  const int slots = clusters * BATCH_CS;
+  k_plan<T><<<1, 1024, 0, s>>>(a, slots, block / 32, BATCH_SHARE);
+  // a cluster per matrix at most: every matrix may be large
+  cfg.gridDim = dim3((unsigned)(((long long)clusters < count ? (long long)clusters : (long long)count) * BATCH_CS));
+  if (cudaLaunchKernelEx(&cfg, k, a) != cudaSuccess)
     return VJ_ERR_CUDA;
   return (cudaGetLastError() == cudaSuccess) ? 0 : VJ_ERR_CUDA;
 }

@@ -1,7 +1,16 @@
-// The batched SVD's per-matrix driver (svd_one): one CTA runs the reference's algorithm
-// on one matrix (src/dvjsvd.c:78-638) with __syncthreads between the phases; and the
+// The batched SVD's per-matrix driver (svd_one): a team of CTAs (one, or the CTAs of a
+// cluster) runs the reference's algorithm on one matrix (src/dvjsvd.c:78-638); and the
 // batch's argument and shared-memory layouts. Kept apart from the kernel and its launcher
 // (batch.cu) so that a host harness can run it with an emulated CTA.
+//
+// A step goes through the team's pairs in four phases: the dot products (LANES lanes per
+// pair), the classification (a thread per pair: the 2x2 with its divisions costs a warp the
+// same for one lane as for 32, so it is done by as few warps as hold the pairs), the rotation
+// of a pair and the sums of squares of its new columns (a warp per pair), and the tails of
+// the norms (a thread per pair). What the reference decides between the steps (rescaling, the
+// retry after a norm overflow, errors) is decided by every thread from the same few words at
+// the start of the next step, as in the one-launch-per-step kernel (jsvd.cu); a step has three
+// barriers of a CTA and one of the team.
 #pragma once
 #include "pjs.cuh"
 #include "svd_core.cuh"
@@ -10,54 +19,115 @@ namespace vj {
 
 constexpr int BATCH_MAXN = 512;
 
+// what the steps of one launch share about the batch (batch.cu, k_plan)
+struct BatchPlan {
+  unsigned next_large, next;  // work-queue heads: matrices for whole clusters, for single CTAs
+  unsigned end_large;         // one past the last large matrix in the caller's order
+  double limit;               // a matrix of a larger cost (batch_cost) is large
+};
+
 template <typename T> struct BatchArgs {
   long long count;
   const long long *m, *n, *offG, *offV, *offS;
   const int *order;
   T *G, *V, *eS, *fS;
   long long *info;
-  unsigned *queue;
+  BatchPlan *plan;
   int strategy;
   unsigned swp;
 };
 
-template <typename T> struct BatchShared {
-  PairState<T> ps[BATCH_MAXN / 2];
-  unsigned char w1[BATCH_MAXN];
-  unsigned long long nmg, nmv, cnt;
-  long long err;
-  int flag;
+// what a step leaves for the next (three slots in turn: read, written, being cleared)
+// (32-bit words: another CTA's shared memory takes 32-bit atomics)
+struct BatchCtl {
+  unsigned nmg;   // largest |.| of the transformed columns: the high word of its bits
+  int ovf, edot;  // a norm overflowed; a dot product was not finite
 };
 
-// max |a_ij| (NaN counts as inf, as VMINPD(|x|, inf) maps it) of an rows x cols block
-template <typename T> __device__ T cta_normx(const T *A, long long ld, long long rows, long long cols,
-                                             unsigned long long *red)
+template <typename T> struct BatchShared {
+  BatchCtl ctl[3];
+  unsigned swt[3];        // transformed pairs per sweep (slots in turn)
+  unsigned long long mx;  // max |g_ij| over this CTA's columns (T bits)
+  // this CTA's pairs of the step: scaled dot product (then the rotation's tangent), cosine,
+  // class; the new columns' sums of squares and largest magnitudes
+  T z[BATCH_MAXN / 2], c[BATCH_MAXN / 2], acc[BATCH_MAXN / 2][2];
+  typename fp<T>::U cmx[BATCH_MAXN / 2][2];
+  int code[BATCH_MAXN / 2];
+};
+
+// The CTAs that work on one matrix: this CTA's rank among them; their shared words are rank
+// 0's (s0 of svd_one).
+struct Team {
+  int rank, size;
+};
+
+__device__ __forceinline__ void warp_sync()
 {
-  const unsigned long long inf = absbits(fp<T>::inf());
-  unsigned long long mx = 0ull;
-  for (long long j = 0; j < cols; ++j)
-    for (long long i = threadIdx.x; i < rows; i += blockDim.x) {
-      unsigned long long b = absbits(A[j * ld + i]);
-      b = (b > inf) ? inf : b;
-      mx = (b > mx) ? b : mx;
-    }
-  mx = warp_max_u64(mx);
-  if ((threadIdx.x & 31) == 0)
-    atomicMax(red, mx);
-  __syncthreads();
-  const T r = bitst<T>(*red);
-  __syncthreads();
-  return r;
+#ifdef __CUDA_ARCH__
+  __syncwarp();
+#else
+  __syncthreads();  // (a host harness's CTA is one warp)
+#endif
 }
 
-template <typename T> __device__ void cta_scale(T *A, long long ld, long long rows, long long cols, int e)
+// barrier of the team's threads; orders their memory accesses
+__device__ __forceinline__ void team_sync(const Team &tm)
 {
-  if (!e)
+#ifdef __CUDA_ARCH__
+  if (tm.size > 1) {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     return;
-  for (long long j = 0; j < cols; ++j)
-    for (long long i = threadIdx.x; i < rows; i += blockDim.x)
-      A[j * ld + i] = scale2(A[j * ld + i], e);
+  }
+#else
+  (void)tm;
+#endif
   __syncthreads();
+}
+
+// the address of this CTA's shared word p in the team's CTA r
+template <typename P> __device__ __forceinline__ P *team_peer(const Team &tm, P *p, int r)
+{
+#ifdef __CUDA_ARCH__
+  if (tm.size > 1) {
+    unsigned long long d;
+    asm("mapa.u64 %0, %1, %2;" : "=l"(d) : "l"((unsigned long long)p), "r"(r));
+    return reinterpret_cast<P *>(d);
+  }
+#endif
+  (void)tm;
+  (void)r;
+  return p;
+}
+
+// max and sum into a shared word of this CTA or of another of the cluster (as explicit
+// operations on the cluster's shared memory: a generic atomic of an address that may be
+// shared was seen to miss the other CTA's word)
+__device__ __forceinline__ void team_max(unsigned *p, unsigned v)
+{
+#ifdef __CUDA_ARCH__
+  asm volatile("red.relaxed.cluster.shared::cluster.max.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
+#else
+  *p = (v > *p) ? v : *p;  // (a host harness's lanes take turns)
+#endif
+}
+__device__ __forceinline__ void team_add(unsigned *p, unsigned v)
+{
+#ifdef __CUDA_ARCH__
+  asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(smem_u32(p)), "r"(v) : "memory");
+#else
+  *p += v;
+#endif
+}
+
+// the high word of a magnitude's bits, all that MG is needed for (its exponent, and whether
+// it is finite), and a value with that high word
+template <typename T> __device__ __forceinline__ unsigned hi_word(typename fp<T>::U b)
+{
+  return (sizeof(T) == 8) ? (unsigned)((unsigned long long)b >> 32) : (unsigned)b;
+}
+template <typename T> __device__ __forceinline__ T from_hi(unsigned h)
+{
+  return (sizeof(T) == 8) ? bitst<T>((unsigned long long)h << 32) : bitst<T>((unsigned long long)h);
 }
 
 __device__ __forceinline__ void step_pair(int strategy, unsigned n, unsigned st, unsigned k, unsigned &p,
@@ -69,199 +139,516 @@ __device__ __forceinline__ void step_pair(int strategy, unsigned n, unsigned st,
     pair_mod(n, st, k, p, q);
 }
 
-// the whole SVD of one matrix by this CTA; returns the sweep count or an error code
-template <typename T> __device__ long long svd_one(const BatchArgs<T> &a, BatchShared<T> &sh, long long m,
-                                                   long long n, T *G, T *V, T *eS, T *fS)
+// A by 2^e, a column per warp
+template <typename T>
+__device__ void team_scale(T *A, long long rows, long long cols, int e, int gw, int GW)
+{
+  if (!e)
+    return;
+  for (long long j = gw; j < cols; j += GW)
+    for (long long i = threadIdx.x & 31; i < rows; i += 32)
+      A[j * rows + i] = scale2(A[j * rows + i], e);
+}
+
+#ifdef __CUDA_ARCH__
+// the larger of m and |x|, a NaN if either is one
+__device__ __forceinline__ float max_nan(float m, float x)
+{
+  float r;
+  asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(m), "f"(fabsf(x)));
+  return r;
+}
+// rot_real (svd_core.cuh) for FP32 columns at 8-byte boundaries and one warp: two rows per
+// load and packed FMAs; m is a multiple of 16. UR loads of two rows in flight.
+struct RotF32 {
+  F32x2 t, tn, c;
+  const unsigned long long *rx, *ry;
+  unsigned long long *dx, *dy;
+  float mu, mw;
+};
+template <bool TRACK, int UR> __device__ __forceinline__ void rot_f32_rows(RotF32 &r, int i, bool cone)
+{
+  F32x2 u[UR], w[UR];
+#pragma unroll
+  for (int k = 0; k < UR; ++k) {
+    u[k].v = r.rx[i + 32 * k];
+    w[k].v = r.ry[i + 32 * k];
+  }
+#pragma unroll
+  for (int k = 0; k < UR; ++k) {
+    F32x2 a = f2_fma(w[k], r.t, u[k]), b = f2_fma(u[k], r.tn, w[k]);
+    if (!cone) {
+      a = f2_mul(a, r.c);
+      b = f2_mul(b, r.c);
+    }
+    r.dx[i + 32 * k] = a.v;
+    r.dy[i + 32 * k] = b.v;
+    if (TRACK) {
+      float a0, a1, b0, b1;
+      f2_get(a, a0, a1);
+      f2_get(b, b0, b1);
+      r.mu = max_nan(max_nan(r.mu, a0), a1);
+      r.mw = max_nan(max_nan(r.mw, b0), b1);
+    }
+  }
+}
+template <bool TRACK>
+__device__ __forceinline__ void rot_f32(int m, float *x, float *y, float at, float c, bool perm, unsigned &mx,
+                                        unsigned &my)
+{
+  const bool cone = (c == 1.0f);
+  RotF32 r;
+  r.t = f2_make(at, at);
+  r.tn = f2_make(-at, -at);
+  r.c = f2_make(c, c);
+  r.rx = reinterpret_cast<const unsigned long long *>(x);
+  r.ry = reinterpret_cast<const unsigned long long *>(y);
+  r.dx = reinterpret_cast<unsigned long long *>(perm ? y : x);
+  r.dy = reinterpret_cast<unsigned long long *>(perm ? x : y);
+  r.mu = r.mw = 0.0f;
+  const int h = m >> 1;
+  int i = (int)(threadIdx.x & 31u);
+  for (; i + 96 < h; i += 128)
+    rot_f32_rows<TRACK, 4>(r, i, cone);
+  if (i + 32 < h) {
+    rot_f32_rows<TRACK, 2>(r, i, cone);
+    i += 64;
+  }
+  if (i < h)
+    rot_f32_rows<TRACK, 1>(r, i, cone);
+  if (TRACK) {
+    mx = fp<float>::bits(perm ? r.mw : r.mu);
+    my = fp<float>::bits(perm ? r.mu : r.mw);
+  }
+}
+#endif
+
+// The sums of squares of two columns, each scaled by 2^-k with k the exponent of its largest
+// magnitude (mx, my: that magnitude's bits; zero or not finite: the sum is not used), in the
+// project's norm order (svd_norm.cuh) for one warp, on its lane 0.
+template <typename T>
+__device__ void pair_sumsq(int m, const T *x, const T *y, typename fp<T>::U mx, typename fp<T>::U my, T &ax, T &ay)
 {
   using F = fp<T>;
+  const int lane = (int)(threadIdx.x & 31u);
+  const T vx = F::val(mx), vy = F::val(my);
+  const int kx = (mx && visfinite(vx)) ? -ilogb_(vx) : 0, ky = (my && visfinite(vy)) ? -ilogb_(vy) : 0;
+  ax = ay = (T)0;
+  if (sizeof(T) == 4 && kx >= 1 - F::BIAS && kx <= F::BIAS && ky >= 1 - F::BIAS && ky <= F::BIAS) {
+    // (the product by a normal power of two is scale2's value)
+    const T px = pow2<T>(kx), py = pow2<T>(ky);
+#pragma unroll 4
+    for (int i = lane; i < m; i += 32) {
+      const T a = x[i] * px, b = y[i] * py;
+      ax = F::fma_(a, a, ax);
+      ay = F::fma_(b, b, ay);
+    }
+  }
+  else {
+    int i = lane;
+    for (; i + 96 < m; i += 128) {
+      T a[4], b[4];
+      bool fast = true;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        a[u] = x[i + 32 * u];
+        b[u] = y[i + 32 * u];
+        const int ba = (int)((F::bits(a[u]) & ~F::SIGN) >> F::MB), bb = (int)((F::bits(b[u]) & ~F::SIGN) >> F::MB);
+        fast = fast && (ba > 0) && (ba + kx > 0) && (bb > 0) && (bb + ky > 0) && (ba + kx <= F::EMAXB) &&
+               (bb + ky <= F::EMAXB);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        a[u] = fast ? F::val(F::bits(a[u]) + ((typename F::U)(long long)kx << F::MB)) : scale2(a[u], kx);
+        b[u] = fast ? F::val(F::bits(b[u]) + ((typename F::U)(long long)ky << F::MB)) : scale2(b[u], ky);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        ax = F::fma_(a[u], a[u], ax);
+        ay = F::fma_(b[u], b[u], ay);
+      }
+    }
+    for (; i < m; i += 32) {
+      const T a = scale2(x[i], kx), b = scale2(y[i], ky);
+      ax = F::fma_(a, a, ax);
+      ay = F::fma_(b, b, ay);
+    }
+  }
+#pragma unroll
+  for (int w = 16; w >= 1; w >>= 1) {
+    ax = ax + __shfl_down_sync(0xffffffffu, ax, w);
+    ay = ay + __shfl_down_sync(0xffffffffu, ay, w);
+  }
+}
+
+// the norm from its scaled sum of squares; the same as warp_nrm2's
+template <typename T> __device__ __forceinline__ T finish_nrm(T acc, typename fp<T>::U mx)
+{
+  const T a = fp<T>::val(mx);
+  if (!visfinite(a))
+    return visnan(a) ? fp<T>::qnan() : a;
+  if (mx == 0)
+    return (T)0;
+  return scale2(sqrt_ge1(acc), ilogb_(a));  // (the largest magnitude scales to [1, 2): acc >= 1)
+}
+
+// What a step needs seldom or once per round is kept out of line: inlined, its registers would
+// be taken from the loops over the rows (FP32 at 64 registers: 1256 bytes of spills).
+// a pair's class and rotation
+template <typename T> struct PairClass {
+  T c, cat;
+  int code, trans;
+};
+template <typename T> __device__ __noinline__ PairClass<T> classify_pair(T ep, T fp_, T eq, T fq, T zr, T tol, T gst)
+{
+  PairState<T> s;
+  s.c = (T)1;
+  s.cat = (T)0;
+  const bool t = pair_classify<T, false>(ep, fp_, eq, fq, zr, (T)0, tol, gst, s);
+  return PairClass<T>{s.c, s.cat, s.code, t ? 1 : 0};
+}
+// everything but a rotation: shears, swaps and rotations by nothing (pair_apply); mx: the
+// changed columns' largest |.|, or false
+template <typename T>
+__device__ __noinline__ bool apply_other(const PairState<T> &b, int m, int n, T *Gp, T *Gq, T *Vp, T *Vq, T *eSp, T *eSq,
+                                         T *fSp, T *fSq, typename fp<T>::U (&mx)[2])
+{
+  typename fp<T>::U mV = 0;
+  return pair_apply<T, false, false, 4>(b, m, n, Gp, Gq, nullptr, nullptr, Vp, Vq, nullptr, nullptr, Gp, Gq, nullptr,
+                                        nullptr, eSp, eSq, fSp, fSq, (int)(threadIdx.x & 31u), 32, false, mx, mV);
+}
+// the columns' largest |.| (of this lane's rows)
+template <typename T> __device__ __noinline__ void cols_max(int m, const T *x, const T *y, typename fp<T>::U (&mx)[2])
+{
+  for (int i = (int)(threadIdx.x & 31u); i < m; i += 32) {
+    amax(mx[0], x[i]);
+    amax(mx[1], y[i]);
+  }
+}
+// norm of column c into eS, fS; *ovf set when it overflows
+template <typename T> __device__ __noinline__ void one_norm(int m, const T *x, T *eS, T *fS, int *ovf)
+{
+  const T d = warp_nrm2(x, m);
+  if ((threadIdx.x & 31u) == 0) {
+    T e, f;
+    ef_split(d, e, f);
+    *eS = e;
+    *fS = f;
+    if (!(d <= svdc<T>::RMAX))
+      *(volatile int *)ovf = 1;
+  }
+}
+// a norm from its sum of squares into eS, fS; whether it overflows
+template <typename T> __device__ __noinline__ bool put_norm(T acc, typename fp<T>::U mx, T *eS, T *fS)
+{
+  const T d = finish_nrm<T>(acc, mx);
+  T e, f;
+  ef_split(d, e, f);
+  *eS = e;
+  *fS = f;
+  return !(d <= svdc<T>::RMAX);
+}
+
+// the whole SVD of one matrix by this team; returns the sweep count or an error code
+template <typename T>
+__device__ long long svd_one(const BatchArgs<T> &a, BatchShared<T> &sh, long long m_, long long n_, T *G, T *V, T *eS,
+                             T *fS, Team tm = Team{0, 1}, BatchShared<T> *s0 = nullptr)
+{
+  using F = fp<T>;
+  using U = typename F::U;
   constexpr int L = svdc<T>::LANES;
-  constexpr int PW = 32 / L;
+  constexpr int PW = 32 / L;  // pairs whose dot products a warp forms at once
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-  const long long n_2 = n >> 1;
-  if (!n)
+  const int gw = tm.rank * nw + warp, GW = tm.size * nw;  // this warp among the team's
+  if (!s0)
+    s0 = &sh;
+  if (!n_)
     return 0;
-  if (m < n || (m % L))
+  if (m_ < n_ || (m_ % L) || m_ > 0x7fffffffLL)
     return -1;
-  if ((n & 1) || (n_2 % L) || n > BATCH_MAXN)
+  if ((n_ & 1) || ((n_ >> 1) % L) || n_ > BATCH_MAXN)
     return -2;
-  const long long E_MG = -80, E_DOT = -320, E_APPG = -580, E_APPV = -588;
-  if (tid == 0)
-    sh.nmg = 0ull;
-  __syncthreads();
-  T MG = cta_normx(G, m, m, n, &sh.nmg);
-  if (!(MG <= svdc<T>::RMAX))
-    return E_MG;
-  // V := I, eS = -inf, fS = 1
-  for (long long j = 0; j < n; ++j)
-    for (long long i = tid; i < n; i += blockDim.x)
-      V[j * n + i] = (i == j) ? (T)1 : (T)0;
-  for (long long j = tid; j < n; j += blockDim.x) {
-    eS[j] = vneg(F::inf());
-    fS[j] = (T)1;
+  const int m = (int)m_, n = (int)n_, n_2 = n >> 1;
+  // column c of G (a column's rows are an int, the matrix's elements need not be)
+  auto col = [&](int c) { return G + (size_t)c * (size_t)m; };
+  const long long E_MG = -80, E_DOT = -320, E_APPG = -580;
+  if (tid == 0) {
+    for (int k = 0; k < 3; ++k) {
+      sh.ctl[k] = BatchCtl{};
+      sh.swt[k] = 0u;
+    }
+    sh.mx = 0ull;
   }
   __syncthreads();
+  {
+    // max |g_ij| (a NaN counts as inf, as VMINPD(|x|, inf) maps it); V := I, eS = -inf, fS = 1
+    const U inf = F::bits(F::inf());
+    U mx = 0;
+    for (int j = gw; j < n; j += GW) {
+      const T *x = col(j);
+      for (int i = lane; i < m; i += 32) {
+        U b = F::bits(x[i]) & ~F::SIGN;
+        b = (b > inf) ? inf : b;
+        mx = (b > mx) ? b : mx;
+      }
+      for (int i = lane; i < n; i += 32)
+        V[j * n + i] = (i == j) ? (T)1 : (T)0;
+      if (lane == 0) {
+        eS[j] = vneg(F::inf());
+        fS[j] = (T)1;
+      }
+    }
+    mx = warp_max_bits(mx);
+    if (lane == 0 && mx)
+      atomicMax(&sh.mx, (unsigned long long)mx);
+  }
+  team_sync(tm);
+  T MG = (T)0;
+  {
+    unsigned long long mx = 0ull;
+    for (int r = 0; r < tm.size; ++r) {
+      const unsigned long long v = *(volatile unsigned long long *)team_peer(tm, &sh.mx, r);
+      mx = (v > mx) ? v : mx;
+    }
+    MG = bitst<T>(mx);
+  }
+  if (tm.size > 1)
+    team_sync(tm);  // (a CTA may leave and reuse its words only when all have read them)
+  if (!(MG <= svdc<T>::RMAX))
+    return E_MG;
   if (MG == (T)0)
     return 0;
   // global prescale (src/dvjsvd.c:120-137)
   const int ROT = svdc<T>::ROT_R;
   const T M_m = F::div(svdc<T>::RMAX, (T)((unsigned long long)m << 1u));
   const int NRM = ilogb_(M_m);
-  int eM = ilogb_(MG);
-  int sN = NRM - eM - 1;
+  int sN = NRM - ilogb_(MG) - 1;
   if (sN) {
-    cta_scale(G, m, m, n, sN);
+    team_scale(G, m, n, sN, gw, GW);
     MG = scale2(MG, sN);
   }
-  int sT = sN, sV = 0;
-  T MV = (T)1;
+  int sT = sN;
   const T tol = F::sqrt_((T)m) * scale2(svdc<T>::EPS, -1);
   const T gst = scale2(tol, (int)svdc<T>::MAX_FIN_EXP);
-  for (long long c = tid; c < n; c += blockDim.x)
-    sh.w1[c] = a.swp ? 1 : 0;
-  __syncthreads();
+  // norms of all columns, a column per warp (the columns that this warp has just scaled)
+  auto all_norms = [&](int *ovf) {
+    for (int c = gw; c < n; c += GW)
+      one_norm<T>(m, col(c), eS + c, fS + c, ovf);
+  };
   const unsigned stp = (a.strategy == 2) ? (unsigned)(n - 1) : (unsigned)n;
-  unsigned sw = 0;
-  while (sw < a.swp) {
-    unsigned long long swt = 0ull;
-    for (unsigned st = 0; st < stp; ++st) {
-      // ---- rescaling of G and V (src/dvjsvd.c:199-233) ----
-      eM = ilogb_(MG);
-      int sR = ROT - eM;
-      sN = NRM - eM - 1;
-      if (sR < 0) {
-        cta_scale(G, m, m, n, sN);
-        MG = scale2(MG, sN);
-        sT += sN;
-        for (long long c = tid; c < n; c += blockDim.x)
-          sh.w1[c] = 1;
-        __syncthreads();
+  const unsigned swp = a.swp;
+  if (swp) {
+    warp_sync();
+    all_norms(&s0->ctl[0].ovf);
+  }
+  team_sync(tm);
+  // (FP32 columns are rotated two rows per load where they start at 8-byte boundaries)
+  const bool al8 = !(((uintptr_t)G | (uintptr_t)V) & 7u);
+  (void)al8;
+  // this CTA's groups of PW pairs (dealt out to the team's CTAs in turn) and its pairs
+  const int litems = (n_2 / PW - tm.rank + tm.size - 1) / tm.size, lpairs = litems * PW;
+  unsigned sw = 0, g = 0;
+  while (sw < swp) {
+    unsigned cnt = 0;  // this lane's transformed pairs of the sweep
+    for (unsigned st = 0; st < stp; ++st, ++g) {
+      // ---- between the steps (src/dvjsvd.c:199-233, :276-295), decided by every thread alike ----
+      const BatchCtl *cur = &s0->ctl[g % 3u];
+      BatchCtl *nxt = &s0->ctl[(g + 1u) % 3u];
+      const T nMG = from_hi<T>(*(volatile const unsigned *)&cur->nmg);
+      const int ovf = *(volatile const int *)&cur->ovf, edot = *(volatile const int *)&cur->edot;
+      if (tm.rank == 0 && tid == 0) {
+        BatchCtl *clr = &s0->ctl[(g + 2u) % 3u];
+        clr->nmg = 0u;
+        clr->ovf = 0;
+        clr->edot = 0;
       }
-      eM = ilogb_(MV);
-      sR = ROT - eM;
-      sN = sR;
-      if (sR < 0) {
-        cta_scale(V, n, n, n, sN);
-        MV = scale2(MV, sR);
-        sV += sR;
+      if (edot || !visfinite(nMG)) {
+        if (tm.size > 1)
+          team_sync(tm);
+        return edot ? E_DOT : E_APPG;
       }
-      // ---- norms of the changed columns, overflow-aware (src/dvjsvd.c:236-296) ----
-      for (int tries = 0;; ++tries) {
-        if (tid == 0)
-          sh.flag = 0;
-        __syncthreads();
-        for (long long c = warp; c < n; c += nw)
-          if (sh.w1[c]) {
-            const T d = warp_nrm2(G + c * m, m);
-            if (lane == 0) {
-              T e, f;
-              ef_split(d, e, f);
-              eS[c] = e;
-              fS[c] = f;
-              if (!(d <= svdc<T>::RMAX))
-                sh.flag = 1;
-            }
-          }
-        __syncthreads();
-        if (!sh.flag)
-          break;
-        if (tries >= 3)
-          return (long long)VJ_ERR_ARG;
-        cta_scale(G, m, m, n, sN);
-        MG = scale2(MG, sN);
-        sT += sN;
-        for (long long c = tid; c < n; c += blockDim.x)
-          sh.w1[c] = 1;
-        __syncthreads();
-      }
-      // ---- all scaled dot products and the classification (src/dvjsvd.c:297-459) ----
-      if (tid == 0) {
-        sh.err = 0;
-        sh.cnt = 0ull;
-        sh.nmg = 0ull;
-        sh.nmv = 0ull;
-      }
-      __syncthreads();
-      for (long long base = (long long)warp * PW; base < n_2; base += (long long)nw * PW) {
-        const int j = lane / L;
-        const long long k = base + j;
-        const bool act = (k < n_2);
-        unsigned p = 0, q = 0;
-        step_pair(a.strategy, (unsigned)n, st, (unsigned)(act ? k : base), p, q);
-        const T ep = eS[p], fp_ = fS[p], eq = eS[q], fq = fS[q];
-        T zr = 0, zi = 0;
-        const bool live = act && (eq >= -svdc<T>::RMAX) && (ep >= -svdc<T>::RMAX);
-        pair_dot<T, false>(m, G + (long long)q * m, nullptr, G + (long long)p * m, nullptr, eq, ep, fq, fp_, live,
-                           zr, zi);
-        if (act && (lane % L) == 0) {
-          PairState<T> &s = sh.ps[k];
-          s.ep = ep; s.fp = fp_; s.eq = eq; s.fq = fq;
-          if (!live)
-            zr = 0;
-          s.a21r = zr;
-          s.a21i = 0;
-          s.skip = 0;
-          if (!visfinite(zr)) {
-            atomicMin(&sh.err, E_DOT);
-            s.skip = 1;
-            s.code = 1;
-          }
-          else if (pair_classify<T, false>(ep, fp_, eq, fq, zr, (T)0, tol, gst, s))
-            atomicAdd(&sh.cnt, 1ull);
-        }
-      }
-      __syncthreads();
-      if (sh.err)
-        return sh.err;
-      swt += sh.cnt;
-      // ---- all transformations (src/dvjsvd.c:460-574), one pair per warp at a time ----
-      typename F::U mx[2] = {0, 0}, mV = 0;
-      for (long long k = warp; k < n_2; k += nw) {
-        unsigned p, q;
-        step_pair(a.strategy, (unsigned)n, st, (unsigned)k, p, q);
-        const PairState<T> &s = sh.ps[k];
-        if (s.code == -1 && lane == 0) {
-          eS[p] = s.eq; eS[q] = s.ep;
-          fS[p] = s.fq; fS[q] = s.fp;
-        }
-        T *Gp = G + (long long)p * m, *Gq = G + (long long)q * m;
-        pair_apply<T, false, false, 4>(s, m, n, Gp, Gq, nullptr, nullptr, V + (long long)p * n, V + (long long)q * n,
-                                    nullptr, nullptr, Gp, Gq, nullptr, nullptr, eS + p, eS + q, fS + p, fS + q,
-                                    lane, 32, false, mx, mV);
-        if (lane == 0) {
-          const int c = s.code;
-          sh.w1[p] = (c == 2 || c == -2) ? 1 : 0;
-          sh.w1[q] = (c == 2 || c == -2 || c == 3 || c == -3) ? 1 : 0;
-        }
-      }
-      const unsigned long long mG = warp_max_u64((unsigned long long)((mx[0] > mx[1]) ? mx[0] : mx[1]));
-      if (lane == 0 && mG)
-        atomicMax(&sh.nmg, mG);
-      __syncthreads();
-      const T nMG = bitst<T>(sh.nmg);
-      if (!visfinite(nMG))
-        return E_APPG;
       MG = fmax(MG, nMG);
-      (void)mV;
-      (void)E_APPV;
+      const int eM = ilogb_(MG);
+      const bool gres = (ROT - eM < 0);
+      if (gres || ovf) {
+        // G's own rescaling, or (the reference's retry) by the exponent that the V block has
+        // set, ROT - 0; then every norm anew
+        const int e = gres ? (NRM - eM - 1) : ROT;
+        team_sync(tm);  // every thread has read the slot
+        if (tm.rank == 0 && tid == 0)
+          s0->ctl[g % 3u].ovf = 0;
+        team_sync(tm);
+        team_scale(G, m, n, e, gw, GW);
+        MG = scale2(MG, e);
+        sT += e;
+        warp_sync();
+        all_norms(&s0->ctl[g % 3u].ovf);
+        team_sync(tm);
+        const int again = *(volatile const int *)&s0->ctl[g % 3u].ovf;
+        if (tm.size > 1)
+          team_sync(tm);
+        if (again)
+          return (long long)VJ_ERR_ARG;
+      }
+      const bool last = (sw + 1u == swp) && (st + 1u == stp);
+      // the global pair and the columns of this CTA's pair lp (items of PW pairs are dealt out
+      // to the team's CTAs in turn)
+      auto pair_of = [&](int lp, unsigned &p, unsigned &q) {
+        step_pair(a.strategy, (unsigned)n, st, (unsigned)(((lp / PW) * tm.size + tm.rank) * PW + lp % PW), p, q);
+      };
+      // ---- scaled dot products (src/dvjsvd.c:297-348), PW pairs per warp ----
+      for (int li = warp; li < litems; li += nw) {
+        const int lp = li * PW + lane / L;
+        unsigned p, q;
+        pair_of(lp, p, q);
+        const T ep = eS[p], eq = eS[q];
+        const bool live = (eq >= -svdc<T>::RMAX) && (ep >= -svdc<T>::RMAX);
+        T zr, zi;
+        pair_nu<T, false>(m, col(q), nullptr, col(p), nullptr, live ? eq : (T)0, live ? ep : (T)0, live, zr, zi);
+        if (lane % L == 0)
+          sh.z[lp] = live ? zr : (T)0;
+      }
+      __syncthreads();
+      // ---- convergence test, 2x2, classification, a pair per thread (src/dvjsvd.c:349-459) ----
+      for (int lp = tid; lp < lpairs; lp += (int)blockDim.x) {
+        unsigned p, q;
+        pair_of(lp, p, q);
+        const T ep = eS[p], fp_ = fS[p], eq = eS[q], fq = fS[q];
+        const T z = qdiv(sh.z[lp], fq * fp_);
+        PairClass<T> s{(T)1, (T)0, 1, 0};
+        if (!visfinite(z))
+          *(volatile int *)&nxt->edot = 1;
+        else {
+          s = classify_pair<T>(ep, fp_, eq, fq, z, tol, gst);
+          cnt += (unsigned)s.trans;
+        }
+        if (s.code == -1) {
+          eS[p] = eq; eS[q] = ep;
+          fS[p] = fq; fS[q] = fp_;
+        }
+        // (a shear needs the dot product itself and the old norms)
+        const bool shear = (s.code == 3 || s.code == -3);
+        sh.z[lp] = shear ? z : s.cat;
+        sh.c[lp] = s.c;
+        sh.code[lp] = s.code;
+      }
+      __syncthreads();
+      // ---- transformations (src/dvjsvd.c:460-574) and the new columns' sums of squares
+      // (:236-275), a pair per warp ----
+      U mG = 0;
+      for (int lp = warp; lp < lpairs; lp += nw) {
+        const int code = sh.code[lp];
+        if (code == 1)
+          continue;
+        unsigned p, q;
+        pair_of(lp, p, q);
+        T *Gp = col(p), *Gq = col(q), *Vp = V + p * n, *Vq = V + q * n;
+        const T at = sh.z[lp], cc = sh.c[lp];
+        U mx[2] = {0, 0};
+        bool trk = true;
+        if ((code == 2 || code == -2) && at != (T)0) {
+          U d0, d1;
+          bool done = false;
+#ifdef __CUDA_ARCH__
+          if constexpr (sizeof(T) == 4)
+            if (al8) {
+              rot_f32<true>(m, Gp, Gq, at, cc, code == -2, mx[0], mx[1]);
+              rot_f32<false>(n, Vp, Vq, at, cc, code == -2, d0, d1);
+              done = true;
+            }
+#endif
+          if (!done) {
+            rot_real<T, false, 4>(m, Gp, Gq, Gp, Gq, nullptr, nullptr, at, cc, code == -2, lane, 32, true, mx[0], mx[1]);
+            rot_real<T, false, 4>(n, Vp, Vq, Vp, Vq, nullptr, nullptr, at, cc, code == -2, lane, 32, false, d0, d1);
+          }
+        }
+        else {
+          PairState<T> b;
+          b.code = code;
+          b.skip = 0;
+          b.c = cc;
+          b.cat = b.a21r = at;
+          b.sat = b.a21i = (T)0;
+          b.ep = eS[p];
+          b.eq = eS[q];
+          b.fp = fS[p];
+          b.fq = fS[q];
+          warp_sync();  // (a permuting shear exchanges the norms)
+          trk = apply_other<T>(b, m, n, Gp, Gq, Vp, Vq, eS + p, eS + q, fS + p, fS + q, mx);
+        }
+        if (code == -1)
+          continue;
+        mx[0] = warp_max_bits(mx[0]);
+        mx[1] = warp_max_bits(mx[1]);
+        mG = (mx[0] > mG) ? mx[0] : mG;
+        mG = (mx[1] > mG) ? mx[1] : mG;
+        if (last)
+          continue;
+        warp_sync();  // the columns as written by the other lanes
+        if (!trk) {
+          cols_max<T>(m, Gp, Gq, mx);
+          mx[0] = warp_max_bits(mx[0]);
+          mx[1] = warp_max_bits(mx[1]);
+        }
+        T ax, ay;
+        pair_sumsq<T>(m, Gp, Gq, mx[0], mx[1], ax, ay);
+        if (lane == 0) {
+          sh.acc[lp][0] = ax;
+          sh.acc[lp][1] = ay;
+          sh.cmx[lp][0] = mx[0];
+          sh.cmx[lp][1] = mx[1];
+        }
+      }
+      if (lane == 0 && mG)
+        team_max(&nxt->nmg, hi_word<T>(mG));
+      __syncthreads();
+      // ---- the norms' tails, a pair per thread ----
+      if (!last)
+        for (int lp = tid; lp < lpairs; lp += (int)blockDim.x) {
+          const int code = sh.code[lp];
+          if (code == 1 || code == -1)
+            continue;
+          unsigned p, q;
+          pair_of(lp, p, q);
+          bool o = false;
+          if (code == 2 || code == -2)
+            o = put_norm<T>(sh.acc[lp][0], sh.cmx[lp][0], eS + p, fS + p);
+          if (put_norm<T>(sh.acc[lp][1], sh.cmx[lp][1], eS + q, fS + q) || o)
+            *(volatile int *)&nxt->ovf = 1;
+        }
+      if (st + 1u == stp && cnt)
+        team_add(&s0->swt[sw % 3u], cnt);
+      team_sync(tm);
+    }
+    const unsigned swt = *(volatile unsigned *)&s0->swt[sw % 3u];
+    if (tm.rank == 0 && tid == 0)
+      s0->swt[(sw + 1u) % 3u] = 0u;
+    // the last step's errors
+    const BatchCtl *cur = &s0->ctl[g % 3u];
+    const T nMG = from_hi<T>(*(volatile const unsigned *)&cur->nmg);
+    const int edot = *(volatile const int *)&cur->edot;
+    if (edot || !visfinite(nMG)) {
+      if (tm.size > 1)
+        team_sync(tm);
+      return edot ? E_DOT : E_APPG;
     }
     if (!swt)
       break;
     ++sw;
   }
-  if (sw < a.swp) {
-    // U = G diag(1/f) 2^-e and eS -= sT (src/dvjsvd.c:604-631); V is not rescaled (sV == 0)
-    for (long long j = 0; j < n; ++j) {
-      const T f = fS[j], sc = vneg(eS[j]);
-      for (long long i = tid; i < m; i += blockDim.x)
-        G[j * m + i] = scalef(F::div(G[j * m + i], f), sc);
+  if (sw < swp) {
+    // U = G diag(1/f) 2^-e and eS -= sT (src/dvjsvd.c:604-631); V was never rescaled
+    for (int j = gw; j < n; j += GW) {
+      const T f = fS[j], e = eS[j], sc = vneg(e);
+      T *x = col(j);
+      for (int i = lane; i < m; i += 32)
+        x[i] = scalef(qdiv(x[i], f), sc);
+      warp_sync();
+      if (lane == 0)
+        eS[j] = e - (T)sT;
     }
-    __syncthreads();
-    for (long long j = tid; j < n; j += blockDim.x)
-      eS[j] = eS[j] - (T)sT;
-    if (sV)
-      cta_scale(V, n, n, n, -sV);
   }
-  __syncthreads();
+  team_sync(tm);
   return (long long)sw;
 }
 

@@ -96,11 +96,19 @@ Staging &staging()
   return s[device_slot()];
 }
 
-unsigned *batch_queue()
+void *batch_plan()
 {
+  // a slot per launch, in turn: launches on several streams or threads do not share one
+  // unless BATCH_SLOTS later ones have been made while the first is still running
+  constexpr unsigned BATCH_SLOTS = 1024, BYTES = 64;
+  static std::mutex mu;
   static Staging q[MAX_DEVICES];
-  Staging &b = q[device_slot()];
-  return b.reserve(256) ? reinterpret_cast<unsigned *>(b.ptr) : nullptr;
+  static unsigned next[MAX_DEVICES] = {};
+  const int dev = device_slot();
+  std::lock_guard<std::mutex> lk(mu);
+  if (!q[dev].reserve((size_t)BATCH_SLOTS * BYTES))
+    return nullptr;
+  return q[dev].ptr + (size_t)(next[dev]++ % BATCH_SLOTS) * BYTES;
 }
 
 Staging &staging2()

@@ -154,15 +154,6 @@ __device__ unsigned cjac2_quad(T a1, T a2, T ar, T ai, int r, int base, T &c, T 
   return bit;
 }
 
-// the warp's largest value, on every lane
-__device__ __forceinline__ unsigned warp_max_bits(unsigned v) { return __reduce_max_sync(0xffffffffu, v); }
-__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v)
-{
-  const unsigned h = (unsigned)(v >> 32), hm = __reduce_max_sync(0xffffffffu, h);
-  const unsigned lm = __reduce_max_sync(0xffffffffu, (h == hm) ? (unsigned)v : 0u);
-  return ((unsigned long long)hm << 32) | lm;
-}
-
 template <typename T, bool CPLX, bool STAGE, int P>
 __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int last)
 {

@@ -25,6 +25,19 @@ __device__ __forceinline__ unsigned long long warp_max_u64(unsigned long long v)
   return v;
 }
 
+// the warp's largest value, on every lane
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ unsigned warp_max_bits(unsigned v) { return __reduce_max_sync(0xffffffffu, v); }
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v)
+{
+  const unsigned h = (unsigned)(v >> 32), hm = __reduce_max_sync(0xffffffffu, h);
+  const unsigned lm = __reduce_max_sync(0xffffffffu, (h == hm) ? (unsigned)v : 0u);
+  return ((unsigned long long)hm << 32) | lm;
+}
+#else
+template <typename U> __device__ U warp_max_bits(U v) { return (U)warp_max_u64((unsigned long long)v); }
+#endif
+
 // The second pass of the project's column norm: the sum of squares of x scaled by the power of
 // two of its largest magnitude (mx: that magnitude's bits), for one warp; every lane returns
 // the same value. Blocks of four elements per lane that scale to normal values (all of a

@@ -52,8 +52,9 @@ Staging &staging2();
 // scratch of the mixed-precision SVD (its inner SVD calls use staging2)
 Staging &staging3();
 
-// the work-queue counter of the batched SVD (device memory, allocated on first use)
-unsigned *batch_queue();
+// 64 bytes of device memory for one launch of the batched SVD: its work queues and what its
+// CTAs need to know of the batch (allocated on first use)
+void *batch_plan();
 
 // two non-blocking streams owned by the library
 bool streams2(cudaStream_t s[2]);
