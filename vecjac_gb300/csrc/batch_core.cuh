@@ -24,6 +24,7 @@ struct BatchPlan {
   unsigned next_large, next;  // work-queue heads: matrices for whole clusters, for single CTAs
   unsigned end_large;         // one past the last large matrix in the caller's order
   double limit;               // a matrix of a larger cost (batch_cost) is large
+  unsigned on_sm[256];        // CTAs of each SM that have come to take single matrices
 };
 
 template <typename T> struct BatchArgs {
@@ -35,6 +36,7 @@ template <typename T> struct BatchArgs {
   BatchPlan *plan;
   int strategy;
   unsigned swp;
+  int sms;  // SMs of the device
 };
 
 // what a step leaves for the next (three slots in turn: read, written, being cleared)
@@ -245,33 +247,40 @@ __device__ void pair_sumsq(int m, const T *x, const T *y, typename fp<T>::U mx, 
     }
   }
   else {
-    int i = lane;
-    for (; i + 96 < m; i += 128) {
-      T a[4], b[4];
+    // four rows of a lane at a time, rows past the end as zeros (which add nothing)
+    auto scaled = [](T v, int k, bool &fast) {
+      const int e = (int)((F::bits(v) & ~F::SIGN) >> F::MB);
+      if ((F::bits(v) & ~F::SIGN) != 0)
+        fast = fast && (e > 0) && (e + k > 0) && (e + k <= F::EMAXB);
+      return (e == 0) ? (T)0 : F::val(F::bits(v) + ((typename F::U)(long long)k << F::MB));
+    };
+    for (int i = lane; i < m; i += 128) {
+      T a[4], b[4], sa[4], sb[4];
       bool fast = true;
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        a[u] = x[i + 32 * u];
-        b[u] = y[i + 32 * u];
-        const int ba = (int)((F::bits(a[u]) & ~F::SIGN) >> F::MB), bb = (int)((F::bits(b[u]) & ~F::SIGN) >> F::MB);
-        fast = fast && (ba > 0) && (ba + kx > 0) && (bb > 0) && (bb + ky > 0) && (ba + kx <= F::EMAXB) &&
-               (bb + ky <= F::EMAXB);
+        const bool in = i + 32 * u < m;
+        a[u] = in ? x[i + 32 * u] : (T)0;
+        b[u] = in ? y[i + 32 * u] : (T)0;
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        a[u] = fast ? F::val(F::bits(a[u]) + ((typename F::U)(long long)kx << F::MB)) : scale2(a[u], kx);
-        b[u] = fast ? F::val(F::bits(b[u]) + ((typename F::U)(long long)ky << F::MB)) : scale2(b[u], ky);
+        sa[u] = scaled(a[u], kx, fast);
+        sb[u] = scaled(b[u], ky, fast);
+      }
+      if (!fast) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          sa[u] = scale2(a[u], kx);
+          sb[u] = scale2(b[u], ky);
+        }
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        ax = F::fma_(a[u], a[u], ax);
-        ay = F::fma_(b[u], b[u], ay);
-      }
-    }
-    for (; i < m; i += 32) {
-      const T a = scale2(x[i], kx), b = scale2(y[i], ky);
-      ax = F::fma_(a, a, ax);
-      ay = F::fma_(b, b, ay);
+      for (int u = 0; u < 4; ++u)
+        if (u == 0 || i + 32 * u < m) {
+          ax = F::fma_(sa[u], sa[u], ax);
+          ay = F::fma_(sb[u], sb[u], ay);
+        }
     }
   }
 #pragma unroll

@@ -96,19 +96,20 @@ Staging &staging()
   return s[device_slot()];
 }
 
-void *batch_plan()
+void *batch_plan(size_t bytes)
 {
   // a slot per launch, in turn: launches on several streams or threads do not share one
   // unless BATCH_SLOTS later ones have been made while the first is still running
-  constexpr unsigned BATCH_SLOTS = 1024, BYTES = 64;
+  constexpr unsigned BATCH_SLOTS = 1024;
+  bytes = (bytes + 255) & ~(size_t)255;
   static std::mutex mu;
   static Staging q[MAX_DEVICES];
   static unsigned next[MAX_DEVICES] = {};
   const int dev = device_slot();
   std::lock_guard<std::mutex> lk(mu);
-  if (!q[dev].reserve((size_t)BATCH_SLOTS * BYTES))
+  if (!q[dev].reserve((size_t)BATCH_SLOTS * bytes))
     return nullptr;
-  return q[dev].ptr + (size_t)(next[dev]++ % BATCH_SLOTS) * BYTES;
+  return q[dev].ptr + (size_t)(next[dev]++ % BATCH_SLOTS) * bytes;
 }
 
 Staging &staging2()

@@ -423,10 +423,12 @@ __device__ __forceinline__ void rot_real(int rows, const T *rx, const T *ry, T *
     else {
 #pragma unroll
       for (int k = 0; k < UR - 1; ++k)
-        if (i0 + k * TPP < rows) {
+        if (i0 + k * TPP < rows)
           rotate(k);
+#pragma unroll
+      for (int k = 0; k < UR - 1; ++k)
+        if (i0 + k * TPP < rows)
           store(k);
-        }
     }
   }
   if (track) {
@@ -515,10 +517,12 @@ __device__ __forceinline__ void rot_cplx(int rows, const T *rxr, const T *rxi, c
     else {
 #pragma unroll
       for (int k = 0; k < UR - 1; ++k)
-        if (i0 + k * TPP < rows) {
+        if (i0 + k * TPP < rows)
           rotate(k);
+#pragma unroll
+      for (int k = 0; k < UR - 1; ++k)
+        if (i0 + k * TPP < rows)
           store(k);
-        }
     }
   }
   if (track) {

@@ -52,9 +52,9 @@ Staging &staging2();
 // scratch of the mixed-precision SVD (its inner SVD calls use staging2)
 Staging &staging3();
 
-// 64 bytes of device memory for one launch of the batched SVD: its work queues and what its
-// CTAs need to know of the batch (allocated on first use)
-void *batch_plan();
+// device memory for one launch of the batched SVD (always the same size): its work queues and
+// what its CTAs need to know of the batch (allocated on first use)
+void *batch_plan(size_t bytes);
 
 // two non-blocking streams owned by the library
 bool streams2(cudaStream_t s[2]);
