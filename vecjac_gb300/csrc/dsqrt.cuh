@@ -43,8 +43,9 @@ __device__ __forceinline__ float rsqrt_approx(float x)
 #endif
 }
 
-// sqrt(x) rounded to nearest for 1 <= x < 2^1024
-__device__ __forceinline__ double dsqrt_pos(double x)
+// sqrt(x) rounded to nearest for 1 <= x < 2^1024 (the product and the constant in registers:
+// FpOps, vj_fp.cuh)
+__device__ __forceinline__ double dsqrt_pos(double x, const FpOps<double> &o = FpOps<double>::make())
 {
   using U = unsigned long long;
   const U ux = fp<double>::bits(x);
@@ -58,8 +59,8 @@ __device__ __forceinline__ double dsqrt_pos(double x)
   // y0 = 1/sqrt(x) estimate, and y0 / 2, as doubles (exact assembly from the FP32 fields)
   const double y0 = fp<double>::val(((U)(ey - k + 1023) << 52) | frac);
   const double h0 = fp<double>::val(((U)(ey - k + 1022) << 52) | frac);
-  const double g0 = x * y0;
-  const double r = fp<double>::fma_(-g0, h0, 0.5);
+  const double g0 = o.mul(x, y0);
+  const double r = fp<double>::fma_(-g0, h0, o.half);
   const double g1 = fp<double>::fma_(g0, r, g0);
   const double d1 = fp<double>::fma_(-g1, g1, x);
   const double g2 = fp<double>::fma_(d1, h0, g1);

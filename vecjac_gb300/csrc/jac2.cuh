@@ -111,11 +111,12 @@ template <typename T, bool FAST = false>
 __device__ __forceinline__ angle<T> jac_angle(T a1, T a2, T ab, T &ad_out)
 {
   using F = fp<T>;
-  const T one = (T)1;
-  const T ad = a1 - a2;
+  const FpOps<T> o = FpOps<T>::make();
+  const T one = o.one;
+  const T ad = o.sub(a1, a2);
   ad_out = ad;
   const T t2 = vor(clamp_t2(qdiv(ab, vabs(ad))), vsgn(ad));
-  const T t1 = qdiv(t2, one + (FAST ? sqrt_ge1(F::fma_(t2, t2, one)) : F::sqrt_(F::fma_(t2, t2, one))));
+  const T t1 = qdiv(t2, o.add(FAST ? sqrt_ge1(F::fma_(t2, t2, one)) : F::sqrt_(F::fma_(t2, t2, one)), one));
   const T s2 = F::fma_(t1, t1, one);
   return angle<T>{t1, s2, FAST ? sqrt_ge1(s2) : F::sqrt_(s2)};
 }
@@ -228,6 +229,7 @@ __device__ __forceinline__ unsigned cjac2_body(T a1, T a2, T ar, T ai, T &c, T &
 {
   using F = fp<T>;
   const T one = (T)1, zero = (T)0;
+  const FpOps<T> o = FpOps<T>::make();
   T L1, L2, t1, s1, s2, ar_, ai_;
   bool fin = false;
   (void)bmax;
@@ -246,7 +248,7 @@ __device__ __forceinline__ unsigned cjac2_body(T a1, T a2, T ar, T ai, T &c, T &
     const T am = nnmin(ar_, ai_);
     const T aM = nnmax(ar_, ai_);
     T aa = qdiv(am, aM);
-    aa = sqrt_ge1(F::fma_(aa, aa, one)) * aM;
+    aa = o.mul(sqrt_ge1(F::fma_(aa, aa, o.one)), aM);
     ar_ = vor(nnmin(qdiv(ar_, aa), one), as);
     ai_ = qdiv(ai, aa);
     const T ab = addexp(aa, 1);
@@ -314,19 +316,19 @@ __device__ __forceinline__ unsigned cjac2_body(T a1, T a2, T ar, T ai, T &c, T &
   }
   // ai_ is NaN only for inputs with an inf or NaN: keep the x86 NaN rules there
   if (KIND == 2) {
-    ar_ = ar_ * t1;
+    ar_ = o.mul(ar_, t1);
     c = s1;
-    ai_ = xmul(ai_, t1);
+    ai_ = fin ? o.mul(ai_, t1) : xmul(ai_, t1);
   }
   else if (KIND == 1) {
     c = qdiv(one, s1);
-    ar_ = qdiv(ar_ * t1, s1);
-    ai_ = xdiv(xmul(ai_, t1), s1);
+    ar_ = qdiv(o.mul(ar_, t1), s1);
+    ai_ = fin ? qdiv(o.mul(ai_, t1), s1) : xdiv(xmul(ai_, t1), s1);
   }
   else {
     c = qdiv(one, s1);
-    ar_ = ar_ * t1;
-    ai_ = xmul(ai_, t1);
+    ar_ = o.mul(ar_, t1);
+    ai_ = fin ? o.mul(ai_, t1) : xmul(ai_, t1);
   }
   cat = ar_;
   sat = ai_;

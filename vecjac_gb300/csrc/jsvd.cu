@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
   tphase(1);
   // ---- 2. scaled dot products: x = column q, y = column p ----
   const int mi = (int)a.m;
-  const DotOps<T> ops = DotOps<T>::make();
+  const FpOps<T> ops = FpOps<T>::make();
   // the products of chunk ck: row i of pair j, chain c, term t at ((i / L) NT + t) NG L +
   // (j NCH + c) L + i % L
   auto produce = [&](int ck, int t0, int nt) {

@@ -356,14 +356,14 @@ template <typename T> __device__ __forceinline__ void swap_cols(T *x, T *y, long
 // these are stored: a store may alias a later load as far as the compiler knows, so a
 // row-by-row loop would wait for one memory round trip per row. Reads (rx, ry), writes (x, y) and, when STG, the staged copy
 // as well; mx and my collect max |.| of what x and y receive when track is set. The products by the
-// cosine are three-register FMAs (svd_dot.cuh, DotOps).
+// cosine are three-register FMAs (vj_fp.cuh, FpOps).
 template <typename T, bool STG, int UR>
 __device__ __forceinline__ void rot_real(int rows, const T *rx, const T *ry, T *x, T *y, T *sx, T *sy, T at, T c,
                                          bool perm, int ltid, int TPP, bool track, typename fp<T>::U &mx,
                                          typename fp<T>::U &my)
 {
   using F = fp<T>;
-  const DotOps<T> o = DotOps<T>::make();
+  const FpOps<T> o = FpOps<T>::make();
   const bool cone = (c == (T)1);
   // the permuted form writes (y - t x) c to x and (x + t y) c to y: the same two products
   // with the destinations exchanged
@@ -443,7 +443,7 @@ __device__ __forceinline__ void rot_cplx(int rows, const T *rxr, const T *rxi, c
                                          bool perm, int ltid, int TPP, bool track, typename fp<T>::U *m4)
 {
   using F = fp<T>;
-  const DotOps<T> o = DotOps<T>::make();
+  const FpOps<T> o = FpOps<T>::make();
   const bool cone = (c == (T)1);
   const T cna = -cta;
   T *const dar = perm ? yr : xr, *const dai = perm ? yi : xi, *const dbr = perm ? xr : yr, *const dbi = perm ? xi : yi;

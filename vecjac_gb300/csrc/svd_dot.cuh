@@ -58,41 +58,6 @@ template <typename T, bool CPLX> struct DotTerms {
   T pd[CPLX ? 4 : 1], dn[CPLX ? 4 : 1];
 };
 
-// FP64 additions and products as three-register FMAs. GB300's FP64 unit takes a warp
-// instruction every 16 clocks per SM when all three operands come from registers and every
-// 19 when it is a DADD, a DMUL or an FMA with a constant operand (measured with 4 to 16
-// warps of independent chains; the latency of 64 clocks is the same), so a + b is formed as
-// a * 1 + b and the round-down product as a * b + (-0), with the 1 and the -0 held in
-// registers. The values are those of the plain operations; only a zero round-down product
-// may come out as -0 instead of +0, which no sum below can tell apart (a sum that starts at +0 never
-// becomes -0 in round-to-nearest).
-template <typename T> struct DotOps {
-  static __device__ __forceinline__ DotOps make() { return DotOps(); }
-  __device__ __forceinline__ T add(T a, T b) const { return a + b; }
-  __device__ __forceinline__ T sub(T a, T b) const { return a - b; }
-  __device__ __forceinline__ T mul(T a, T b) const { return a * b; }
-  __device__ __forceinline__ T mul_rd(T a, T b) const { return fp<T>::mul_rd(a, b); }
-};
-#ifdef __CUDA_ARCH__
-template <> struct DotOps<double> {
-  double one, mzero;
-  static __device__ __forceinline__ DotOps make()
-  {
-    // (gridDim.z is 1 in every launch, which the assembler cannot know: it folds known
-    // constants back into the two-operand forms)
-    const int z = (int)gridDim.z - 1;
-    DotOps o;
-    o.one = __hiloint2double(0x3ff00000 + z, z);
-    o.mzero = __hiloint2double((int)0x80000000u + z, z);
-    return o;
-  }
-  __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
-  __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(a, one, -b); }
-  __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, mzero); }
-  __device__ __forceinline__ double mul_rd(double a, double b) const { return __fma_rd(a, b, mzero); }
-};
-#endif
-
 // One step of a 2Sum recurrence, (s, t) := (RN(s + b), s + b - RN(s + b)) with b = p + t.
 // FP64: Dekker's Fast2Sum on the operands ordered by their high words. Fast2Sum's error is
 // exact when the first operand's exponent is not below the second's (T. J. Dekker, "A
@@ -115,7 +80,7 @@ __device__ __forceinline__ bool hi_larger(double b, double s)
   return ((unsigned)(fp<double>::bits(b) >> 32) << 1) > ((unsigned)(fp<double>::bits(s) >> 32) << 1);
 #endif
 }
-template <typename T> __device__ __forceinline__ void sum_step(const DotOps<T> &o, T p, T &s, T &t)
+template <typename T> __device__ __forceinline__ void sum_step(const FpOps<T> &o, T p, T &s, T &t)
 {
   const T b = o.add(p, t);
   if constexpr (sizeof(T) == 8) {
@@ -130,7 +95,7 @@ template <typename T> __device__ __forceinline__ void sum_step(const DotOps<T> &
 }
 
 template <typename T>
-__device__ __forceinline__ void dot_acc(const DotOps<T> &o, T pd, T dn, T &s, T &t, T &s_, T &t_)
+__device__ __forceinline__ void dot_acc(const FpOps<T> &o, T pd, T dn, T &s, T &t, T &s_, T &t_)
 {
   sum_step(o, pd, s, t);
   sum_step(o, dn, s_, t_);
@@ -252,7 +217,7 @@ __device__ void pair_nu(long long m, const T *xr, const T *xi, const T *yr, cons
   constexpr int D = 4;              // elements per block (the next block's loads in flight)
   const int lane = (threadIdx.x & 31) % L;
   const int nx = -(int)ex, ny = -(int)ey;
-  const DotOps<T> o = DotOps<T>::make();
+  const FpOps<T> o = FpOps<T>::make();
   T sr = 0, tr = 0, sr_ = 0, tr_ = 0, si = 0, ti = 0, si_ = 0, ti_ = 0;
   auto load = [&](long long i, T (&v)[NV]) {
     if (i < m) {
@@ -392,7 +357,7 @@ __device__ void chain_dot(long long m, const T *xr, const T *xi, const T *yr, co
   constexpr int D = CPLX ? 4 : 8;   // elements per block: the next block's loads are in flight
                                     // while this block is accumulated (hides L2 latency)
   const int nx = -(int)ex, ny = -(int)ey;
-  const DotOps<T> o = DotOps<T>::make();
+  const FpOps<T> o = FpOps<T>::make();
   T s = 0, t = 0;
   auto load = [&](long long i, T (&v)[NV]) {
     if (i < m) {

@@ -212,4 +212,41 @@ template <typename T> __device__ __forceinline__ T getmant(T x)
   return getmant_fin(x);
 }
 
+// FP64 additions and products as three-register FMAs. GB300's FP64 unit takes a warp
+// instruction every 16 clocks per SM when all three operands come from registers and every
+// 19 when it is a DADD, a DMUL or an FMA with a constant operand (measured with 4 to 16
+// warps of independent chains; the latency of 64 clocks is the same), so a + b is formed as
+// a * 1 + b and the round-down product as a * b + (-0), with the 1 and the -0 held in
+// registers. The values are those of the plain operations; only a zero round-down product
+// may come out as -0 instead of +0, which the dot products' sums cannot tell apart (a sum that starts
+// at +0 never becomes -0 in round-to-nearest).
+template <typename T> struct FpOps {
+  T one = (T)1, half = (T)0.5;
+  static __device__ __forceinline__ FpOps make() { return FpOps(); }
+  __device__ __forceinline__ T add(T a, T b) const { return a + b; }
+  __device__ __forceinline__ T sub(T a, T b) const { return a - b; }
+  __device__ __forceinline__ T mul(T a, T b) const { return a * b; }
+  __device__ __forceinline__ T mul_rd(T a, T b) const { return fp<T>::mul_rd(a, b); }
+};
+#ifdef __CUDA_ARCH__
+template <> struct FpOps<double> {
+  double one, mzero, half;
+  static __device__ __forceinline__ FpOps make()
+  {
+    // (gridDim.z is 1 in every launch, which the assembler cannot know: it folds known
+    // constants back into the two-operand forms)
+    const int z = (int)gridDim.z - 1;
+    FpOps o;
+    o.one = __hiloint2double(0x3ff00000 + z, z);
+    o.mzero = __hiloint2double((int)0x80000000u + z, z);
+    o.half = __hiloint2double(0x3fe00000 + z, z);
+    return o;
+  }
+  __device__ __forceinline__ double add(double a, double b) const { return __fma_rn(a, one, b); }
+  __device__ __forceinline__ double sub(double a, double b) const { return __fma_rn(a, one, -b); }
+  __device__ __forceinline__ double mul(double a, double b) const { return __fma_rn(a, b, mzero); }
+  __device__ __forceinline__ double mul_rd(double a, double b) const { return __fma_rd(a, b, mzero); }
+};
+#endif
+
 }  // namespace vj
