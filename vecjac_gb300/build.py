@@ -3,8 +3,7 @@
 Every translation unit under csrc/ is compiled in parallel with
 ``-gencode arch=compute_103a,code=sm_103a -lineinfo --fmad=false`` (no implicit
 multiply-add contraction: the kernels reproduce the reference's rounding op by op)
-and linked against the CUDA runtime and cuBLAS (the plain FP64 GEMMs of the mixed-precision
-SVD) -- PyTorch is not a dependency of the library.
+and linked against the CUDA runtime -- PyTorch is not a dependency of the library.
 """
 import concurrent.futures as cf
 import glob
@@ -67,7 +66,7 @@ def build(verbose=False, extra=(), lp64=False, out_dir=None):
         objs = list(ex.map(lambda s: _compile(s, extra, out), srcs))
     if os.path.exists(lib) and os.path.getmtime(lib) >= max(os.path.getmtime(o) for o in objs):
         return lib
-    cmd = [nvcc()] + ARCH + ["-shared", "-o", lib] + objs + ["-lcudart", "-lcublas", "-lcusolver"]
+    cmd = [nvcc()] + ARCH + ["-shared", "-o", lib] + objs + ["-lcudart"]
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("link failed:\n%s\n%s" % (" ".join(cmd), r.stderr))

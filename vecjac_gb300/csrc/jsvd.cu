@@ -562,8 +562,10 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
 // normal range) goes to list (up to cap entries; *nlist counts them all), for k_confirm
 // to decide exactly. The first step's rescaling decision is checked as in k_confirm. About
 // 9 FP64 operations per complex element instead of the 76 of the reference's four
-// compensated chains.
-template <bool CPLX>
+// compensated chains. Without COSINES the caller has bounded every pair's cosine by the same
+// limit already (the mixed SVD, from a Gram matrix with a rigorous error bound), and only the
+// order of the columns and the first step's rescaling are left to check.
+template <bool CPLX, bool COSINES>
 __global__ void __launch_bounds__(256) k_certify(SvdArgs<double> a, unsigned stp, unsigned *flag, unsigned *list,
                                                  unsigned cap, unsigned *nlist)
 {
@@ -593,8 +595,8 @@ __global__ void __launch_bounds__(256) k_certify(SvdArgs<double> a, unsigned stp
     }
     // 2^-e_q as a normal double, and |y| = f_p 2^e_p as a finite double, or no certificate
     const bool ok = (eq >= -1021.0) && (eq <= 1021.0) && (ep >= -1021.0) && (ep <= 1021.0);
-    bool cert = false;
-    if (ok) {
+    bool cert = !COSINES;
+    if (COSINES && ok) {
       const double sx = ldexp(1.0, -(int)eq);
       const T *xr = a.G + q * a.ldG, *yr = a.G + p * a.ldG;
       const T *xi = CPLX ? (a.Gi + q * a.ldGi) : nullptr, *yi = CPLX ? (a.Gi + p * a.ldGi) : nullptr;
@@ -877,7 +879,7 @@ template <typename T, bool CPLX> static StepLaunch<T> step_launch(long long m, i
 template <typename T, bool CPLX>
 static vj_fint svd_dev(vj_fnat m_, vj_fnat n_, T *G, vj_fnat ldG, T *Gi, vj_fnat ldGi, T *V, vj_fnat ldV, T *Vi,
                        vj_fnat ldVi, T *eS, T *fS, const unsigned *js, unsigned stp, unsigned swp, int preset,
-                       cudaStream_t s, unsigned char *scratch = nullptr)
+                       cudaStream_t s, unsigned char *scratch = nullptr, bool certified = false)
 {
   constexpr int L = svdc<T>::LANES;
   const host::NearestRounding rn;
@@ -1044,7 +1046,10 @@ static vj_fint svd_dev(vj_fnat m_, vj_fnat n_, T *G, vj_fnat ldG, T *Gi, vj_fnat
       unsigned *list = reinterpret_cast<unsigned *>(lst.ptr);
       if (cudaMemsetAsync(dmx, 0, 8, s) != cudaSuccess)
         return VJ_ERR_CUDA;
-      k_certify<CPLX><<<(unsigned)(host::sm_count() * 4), blk, 0, s>>>(a, stp, flag, list, cap, nl);
+      if (certified)  // the caller has bounded every cosine below the certificate's limit
+        k_certify<CPLX, false><<<(unsigned)(host::sm_count() * 4), blk, 0, s>>>(a, stp, flag, list, cap, nl);
+      else
+        k_certify<CPLX, true><<<(unsigned)(host::sm_count() * 4), blk, 0, s>>>(a, stp, flag, list, cap, nl);
       if (cudaGetLastError() != cudaSuccess)
         return VJ_ERR_CUDA;
       unsigned hf[2] = {1u, 0u};
@@ -1219,22 +1224,16 @@ namespace vj {
 template <typename T, bool CPLX>
 vj_fint svd_dev_entry(vj_fnat m, vj_fnat n, T *G, vj_fnat ldG, T *Gi, vj_fnat ldGi, T *V, vj_fnat ldV, T *Vi,
                       vj_fnat ldVi, T *eS, T *fS, const unsigned *js, unsigned stp, unsigned swp, int preset,
-                      cudaStream_t s)
+                      bool certified, cudaStream_t s)
 {
-  return svd_dev<T, CPLX>(m, n, G, ldG, Gi, ldGi, V, ldV, Vi, ldVi, eS, fS, js, stp, swp, preset, s);
+  return svd_dev<T, CPLX>(m, n, G, ldG, Gi, ldGi, V, ldV, Vi, ldVi, eS, fS, js, stp, swp, preset, s, nullptr, certified);
 }
 template vj_fint svd_dev_entry<double, false>(vj_fnat, vj_fnat, double *, vj_fnat, double *, vj_fnat, double *,
                                               vj_fnat, double *, vj_fnat, double *, double *, const unsigned *,
-                                              unsigned, unsigned, int, cudaStream_t);
+                                              unsigned, unsigned, int, bool, cudaStream_t);
 template vj_fint svd_dev_entry<double, true>(vj_fnat, vj_fnat, double *, vj_fnat, double *, vj_fnat, double *,
                                              vj_fnat, double *, vj_fnat, double *, double *, const unsigned *,
-                                             unsigned, unsigned, int, cudaStream_t);
-template vj_fint svd_dev_entry<float, false>(vj_fnat, vj_fnat, float *, vj_fnat, float *, vj_fnat, float *,
-                                             vj_fnat, float *, vj_fnat, float *, float *, const unsigned *,
-                                             unsigned, unsigned, int, cudaStream_t);
-template vj_fint svd_dev_entry<float, true>(vj_fnat, vj_fnat, float *, vj_fnat, float *, vj_fnat, float *,
-                                            vj_fnat, float *, vj_fnat, float *, float *, const unsigned *,
-                                            unsigned, unsigned, int, cudaStream_t);
+                                             unsigned, unsigned, int, bool, cudaStream_t);
 }  // namespace vj
 
 extern "C" {

@@ -32,10 +32,9 @@
 #include <algorithm>
 #include <vector>
 
-#include <cublas_v2.h>
 #include <cuda_runtime.h>
-#include <cusolverDn.h>
 
+#include "fp64tc.cuh"
 #include "presweep.cuh"
 #include "svd_core.cuh"
 #include "vj_fp.cuh"
@@ -54,7 +53,7 @@ long long block_sweep(bool cplx, int m, int n, float *Gr, float *Gi, long long l
 template <typename T, bool CPLX>
 vj_fint svd_dev_entry(vj_fnat m, vj_fnat n, T *G, vj_fnat ldG, T *Gi, vj_fnat ldGi, T *V, vj_fnat ldV, T *Vi,
                       vj_fnat ldVi, T *eS, T *fS, const unsigned *js, unsigned stp, unsigned swp, int preset,
-                      cudaStream_t s);
+                      bool certified, cudaStream_t s);
 
 __global__ void k_to_f32(const double *A, long long ld, long long rows, long long cols, int e, float *B)
 {
@@ -557,29 +556,6 @@ __global__ void k_gather_cols(int rows, int n, const double *A, long long lda, c
       B[(size_t)j * rows + i] = A[(size_t)perm[j] * lda + i];
 }
 
-// library handles, one per device (created with that device current)
-static cublasHandle_t cublas()
-{
-  static std::mutex mu;
-  static cublasHandle_t hs[host::MAX_DEVICES] = {};
-  std::lock_guard<std::mutex> lk(mu);
-  cublasHandle_t &h = hs[host::device_slot()];
-  if (!h && cublasCreate(&h) != CUBLAS_STATUS_SUCCESS)
-    h = nullptr;
-  return h;
-}
-
-static cusolverDnHandle_t cusolver()
-{
-  static std::mutex mu;
-  static cusolverDnHandle_t hs[host::MAX_DEVICES] = {};
-  std::lock_guard<std::mutex> lk(mu);
-  cusolverDnHandle_t &h = hs[host::device_slot()];
-  if (!h && cusolverDnCreate(&h) != CUSOLVER_STATUS_SUCCESS)
-    h = nullptr;
-  return h;
-}
-
 // squared 2-norms of the columns of planar FP32 G (one CTA per column): the order key of
 // the orthonormalisation below
 template <bool CPLX>
@@ -609,142 +585,216 @@ __global__ void __launch_bounds__(256) k_colnorm2_f32(int m, const float *Gr, co
   }
 }
 
-// planar (re, im) n x n <-> interleaved complex n x n (both with leading dimension n)
-__global__ void k_to_interleaved(const double *re, const double *im, long long nn, double2 *z)
-{
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += (long long)gridDim.x * blockDim.x)
-    z[i] = make_double2(re[i], im[i]);
-}
-__global__ void k_from_interleaved(const double2 *z, long long nn, double *re, double *im)
-{
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nn; i += (long long)gridDim.x * blockDim.x) {
-    re[i] = z[i].x;
-    im[i] = z[i].y;
-  }
-}
-
-// split-plane complex matrix: real and imaginary planes with their leading dimensions
-struct Planes {
+// planar complex n x n matrix in FP64 (im null: real data), leading dimension n
+struct Mat {
   double *re, *im;
-  int ldr, ldi;
 };
 
-// C = op(A) B on split planes (op(A) = A or A^H; complex: four real products)
-static bool zgemm(cublasHandle_t h, bool cplx, bool conjA, int m, int n, int k, Planes A, Planes B, Planes Cm)
+// T[:, j] = W[:, perm[j]] widened to FP64
+__global__ void k_widen_cols(int n, const float *W, const int *perm, double *T)
 {
-  const cublasOperation_t op = conjA ? CUBLAS_OP_T : CUBLAS_OP_N;
-  auto g = [&](const double *X, int ldx, const double *Y, int ldy, double a, double b, double *Z, int ldz) {
-    return cublasDgemm(h, op, CUBLAS_OP_N, m, n, k, &a, X, ldx, Y, ldy, &b, Z, ldz) == CUBLAS_STATUS_SUCCESS;
-  };
-  if (!cplx)
-    return g(A.re, A.ldr, B.re, B.ldr, 1.0, 0.0, Cm.re, Cm.ldr);
-  // real part: Ar Br - Ai Bi, or Ar^T Br + Ai^T Bi for A^H
-  const double sgn = conjA ? 1.0 : -1.0;
-  bool ok = g(A.re, A.ldr, B.re, B.ldr, 1.0, 0.0, Cm.re, Cm.ldr) && g(A.im, A.ldi, B.im, B.ldi, sgn, 1.0, Cm.re, Cm.ldr);
-  // imaginary part: Ar Bi + Ai Br, or Ar^T Bi - Ai^T Br for A^H
-  ok = ok && g(A.re, A.ldr, B.im, B.ldi, 1.0, 0.0, Cm.im, Cm.ldi) && g(A.im, A.ldi, B.re, B.ldr, -sgn, 1.0, Cm.im, Cm.ldi);
-  return ok;
+  for (int j = blockIdx.y; j < n; j += gridDim.y)
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+      T[(size_t)j * n + i] = (double)W[(size_t)perm[j] * n + i];
 }
 
-// T(r, c) = T(c, r) for r < c (fill the upper triangle of an n x n matrix from the lower)
-__global__ void k_sym_lower(double *Tm, int n)
-{
-  for (int c = blockIdx.y; c < n; c += gridDim.y)
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < c; r += gridDim.x * blockDim.x)
-      Tm[(size_t)c * n + r] = Tm[(size_t)r * n + c];
-}
+// what an all-pairs kernel finds
+struct PairStats {
+  unsigned long long cosmax, cosbound;  // largest |cos| and largest upper bound of one (bits of doubles)
+  double f2;                            // squared Frobenius norm of the rotation generator
+  unsigned over, skipped;               // pairs above the tolerance; of those, not in the generator
+};
 
-// D(r, c) = M(r, c) - M(c, r) (n x n)
-__global__ void k_antisym(const double *M, int n, double *D)
+// Kernels on the lower triangle of an n x n Hermitian matrix and its mirror, 32 x 32 tiles:
+// thread (x, y) takes rows i = 32 blockIdx.x + x of columns j = 32 blockIdx.y + y + 8 k; f(i, j,
+// diagonal) returns the mirror's value, which goes through shared memory and is stored by
+// put(j, i, value) with its row j along the threads.
+template <typename F, typename P> __device__ void lower_tiles(int n, F f, P put)
 {
-  for (int c = blockIdx.y; c < n; c += gridDim.y)
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
-      D[(size_t)c * n + r] = M[(size_t)c * n + r] - M[(size_t)r * n + c];
-}
-
-// 3M combination: Cr holds P1 = Ar Br, Ci holds P3 = (Ar + Ai)(Br + Bi), P2 = Ai Bi:
-// Cr = P1 - P2, Ci = P3 - P1 - P2 (rows x cols, leading dimensions ldr / ldi / rows)
-__global__ void k_combine3m(int rows, int cols, double *Cr, long long ldr, double *Ci, long long ldi, const double *P2)
-{
-  for (int c = blockIdx.y; c < cols; c += gridDim.y)
-    for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
-      const double p1 = Cr[(size_t)c * ldr + r], p2 = P2[(size_t)c * rows + r], p3 = Ci[(size_t)c * ldi + r];
-      Cr[(size_t)c * ldr + r] = p1 - p2;
-      Ci[(size_t)c * ldi + r] = (p3 - p1) - p2;
-    }
-}
-
-// T = X^H X for an n x n split-plane X (leading dimension n): the real part by two
-// symmetric rank-k updates (half a product each), the imaginary part from one product
-// M = Xr^T Xi as M - M^T. tmp: n x n doubles.
-static bool gram(cublasHandle_t h, bool cplx, int n, Planes X, Planes Tm, double *tmp, cudaStream_t s)
-{
-  const double one = 1.0, zero = 0.0;
-  if (cublasDsyrk(h, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, n, n, &one, X.re, X.ldr, &zero, Tm.re, n) !=
-      CUBLAS_STATUS_SUCCESS)
-    return false;
-  if (cplx) {
-    if (cublasDsyrk(h, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, n, n, &one, X.im, X.ldi, &one, Tm.re, n) !=
-            CUBLAS_STATUS_SUCCESS ||
-        cublasDgemm(h, CUBLAS_OP_T, CUBLAS_OP_N, n, n, n, &one, X.re, X.ldr, X.im, X.ldi, &zero, tmp, n) !=
-            CUBLAS_STATUS_SUCCESS)
-      return false;
-    k_antisym<<<grid2(n, n), 256, 0, s>>>(tmp, n, Tm.im);
+  __shared__ double2 t[32][33];
+  const int bi = blockIdx.x, bj = blockIdx.y;
+  if (bj > bi)
+    return;
+  for (int k = threadIdx.y; k < 32; k += 8) {
+    const int i = bi * 32 + threadIdx.x, j = bj * 32 + k;
+    if (i < n && j < n && i >= j)
+      t[k][threadIdx.x] = f(i, j);
   }
-  k_sym_lower<<<grid2(n, n), 256, 0, s>>>(Tm.re, n);
-  return cudaGetLastError() == cudaSuccess;
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += 8) {
+    const int j = bj * 32 + threadIdx.x, i = bi * 32 + k;
+    if (i < n && j < n && i > j)
+      put(j, i, t[threadIdx.x][k]);
+  }
 }
 
-// C = A B for complex split planes with three real products (Gauss / 3M): P1 = Ar Br,
-// P2 = Ai Bi, P3 = (Ar + Ai)(Br + Bi). Used for products of near-unitary n x n matrices
-// (rotation accumulators), where its slightly larger error bound is harmless. tmp: room
-// for m k + k n + m n doubles. Real data: one product.
-static bool zgemm3m(cublasHandle_t h, bool cplx, int m, int n, int k, Planes A, Planes B, Planes Cm, double *tmp,
-                    cudaStream_t s)
+// M = -(strict upper triangle + half of the diagonal of E), E = H - I from H's lower triangle; the
+// largest |E_ij| into st->cosmax
+__global__ void __launch_bounds__(256) k_neg_upper(int n, Mat H, Mat M, PairStats *st)
 {
-  const double one = 1.0, zero = 0.0;
-  if (!cplx)
-    return cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, &one, A.re, A.ldr, B.re, B.ldr, &zero, Cm.re, Cm.ldr) ==
-           CUBLAS_STATUS_SUCCESS;
-  double *As = tmp, *Bs = As + (size_t)m * k, *P2 = Bs + (size_t)k * n;
-  bool ok = cublasDgeam(h, CUBLAS_OP_N, CUBLAS_OP_N, m, k, &one, A.re, A.ldr, &one, A.im, A.ldi, As, m) ==
-                CUBLAS_STATUS_SUCCESS &&
-            cublasDgeam(h, CUBLAS_OP_N, CUBLAS_OP_N, k, n, &one, B.re, B.ldr, &one, B.im, B.ldi, Bs, k) ==
-                CUBLAS_STATUS_SUCCESS &&
-            cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, &one, A.re, A.ldr, B.re, B.ldr, &zero, Cm.re, Cm.ldr) ==
-                CUBLAS_STATUS_SUCCESS &&
-            cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, &one, A.im, A.ldi, B.im, B.ldi, &zero, P2, m) ==
-                CUBLAS_STATUS_SUCCESS &&
-            cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, &one, As, m, Bs, k, &zero, Cm.im, Cm.ldi) ==
-                CUBLAS_STATUS_SUCCESS;
-  if (!ok)
-    return false;
-  k_combine3m<<<grid2(m, n), 256, 0, s>>>(m, n, Cm.re, Cm.ldr, Cm.im, Cm.ldi, P2);
-  return cudaGetLastError() == cudaSuccess;
+  double mx = 0;
+  lower_tiles(
+      n,
+      [&](int i, int j) {
+        const size_t o = (size_t)j * n + i;
+        const double re = H.re[o] - ((i == j) ? 1.0 : 0.0), im = (H.im && i != j) ? H.im[o] : 0.0;
+        // (a NaN must not pass for a small value)
+        const double a = fabs(re) + fabs(im);
+        mx = (a <= 1e300) ? fmax(mx, a) : 1e300;
+        M.re[o] = (i == j) ? -0.5 * re : 0.0;
+        if (M.im)
+          M.im[o] = 0.0;
+        return make_double2(-re, im);
+      },
+      [&](int j, int i, double2 v) {
+        M.re[(size_t)i * n + j] = v.x;
+        if (M.im)
+          M.im[(size_t)i * n + j] = v.y;
+      });
+  atomicMax(&st->cosmax, (unsigned long long)__double_as_longlong(mx));
 }
 
-// C = A B for complex split planes by 3M as above, with A's imaginary plane overwritten by
-// Ar + Ai (A is a scratch copy) so that the temporaries are only P2 (m n) and Br + Bi (k n):
-// tmp holds m n + k n doubles. For G := G Q (m x n by n x n): three products instead of four.
-static bool zgemm3m_overwrite(cublasHandle_t h, int m, int n, int k, Planes A, Planes B, Planes Cm, double *tmp,
-                              cudaStream_t s)
+// The generator K of the rotation exp(K) that makes the columns of G orthogonal to first order,
+// from the lower triangle of the Gram matrix H of the columns times 2^-e_j: K_ij = h_ij / (h_jj -
+// h_ii) in the columns' true lengths, stored as K~_ij = 2^(e_i - e_j) K_ij (the factor of column i
+// of length about 1 in column j of length about 1: never much larger than the cosine, however the
+// lengths differ). Pairs with |cos| below `tol` / 4 are left alone; pairs with |K_ij| > 2^-7 (nearly
+// equal lengths) too, and counted. hb: bound of the error of a Gram entry.
+__global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, Mat Kt, double tol, double hb, PairStats *st)
 {
-  const double one = 1.0, zero = 0.0;
-  double *P2 = tmp, *Bs = tmp + (size_t)m * n;
-  bool ok = cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, &one, A.im, A.ldi, B.im, B.ldi, &zero, P2, m) ==
-                CUBLAS_STATUS_SUCCESS &&
-            cublasDgeam(h, CUBLAS_OP_N, CUBLAS_OP_N, k, n, &one, B.re, B.ldr, &one, B.im, B.ldi, Bs, k) ==
-                CUBLAS_STATUS_SUCCESS &&
-            cublasDgeam(h, CUBLAS_OP_N, CUBLAS_OP_N, m, k, &one, A.re, A.ldr, &one, A.im, A.ldi, A.im, A.ldi) ==
-                CUBLAS_STATUS_SUCCESS &&
-            cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, &one, A.re, A.ldr, B.re, B.ldr, &zero, Cm.re, Cm.ldr) ==
-                CUBLAS_STATUS_SUCCESS &&
-            cublasDgemm(h, CUBLAS_OP_N, CUBLAS_OP_N, m, n, k, &one, A.im, A.ldi, Bs, k, &zero, Cm.im, Cm.ldi) ==
-                CUBLAS_STATUS_SUCCESS;
-  if (!ok)
-    return false;
-  k_combine3m<<<grid2(m, n), 256, 0, s>>>(m, n, Cm.re, Cm.ldr, Cm.im, Cm.ldi, P2);
-  return cudaGetLastError() == cudaSuccess;
+  double cm = 0, cb = 0, f2 = 0;
+  unsigned over = 0, skipped = 0;
+  lower_tiles(
+      n,
+      [&](int i, int j) {
+        const size_t o = (size_t)j * n + i;
+        double2 kij = make_double2(0, 0), kji = kij;
+        if (i != j) {
+          const double hr = H.re[o], him = H.im ? H.im[o] : 0.0;
+          const double hi = H.re[(size_t)i * n + i], hj = H.re[(size_t)j * n + j];
+          if (hi > 0 && hj > 0) {
+            const double a = H.im ? hypot(hr, him) : fabs(hr), s = rsqrt(hi) * rsqrt(hj);
+            const double c = a * s;
+            cm = (c <= 2.0) ? fmax(cm, c) : 2.0;  // (a NaN counts as large)
+            cb = (c <= 2.0) ? fmax(cb, (a * (1.0 + 1e-14) + hb) * s * (1.0 + 1e-14)) : 2.0;
+            over += (c > tol) ? 1u : 0u;
+            if (c > 0.25 * tol) {
+              // d = e_j - e_i: denominators h_jj 4^d - h_ii and h_jj - h_ii 4^-d
+              const int d = max(-500, min(500, e[j] - e[i]));
+              const double di = scalbn(hj, 2 * d) - hi, dj = hj - scalbn(hi, -2 * d);
+              // |K_ij| = a 2^d / |di|
+              const double k = scalbn(a, d);
+              if (k <= 0.0078125 * fabs(di)) {
+                kij = make_double2(hr / di, him / di);
+                kji = make_double2(-hr / dj, him / dj);
+                const double q = k / fabs(di);
+                f2 += 2.0 * q * q;
+              }
+              else if (c > tol)
+                ++skipped;
+            }
+          }
+        }
+        Kt.re[o] = kij.x;
+        if (Kt.im)
+          Kt.im[o] = kij.y;
+        return kji;
+      },
+      [&](int j, int i, double2 v) {
+        Kt.re[(size_t)i * n + j] = v.x;
+        if (Kt.im)
+          Kt.im[(size_t)i * n + j] = v.y;
+      });
+  for (int o = 16; o >= 1; o >>= 1) {
+    cm = fmax(cm, __shfl_xor_sync(0xffffffffu, cm, o));
+    cb = fmax(cb, __shfl_xor_sync(0xffffffffu, cb, o));
+    f2 += __shfl_xor_sync(0xffffffffu, f2, o);
+    over += __shfl_xor_sync(0xffffffffu, over, o);
+    skipped += __shfl_xor_sync(0xffffffffu, skipped, o);
+  }
+  if (threadIdx.x == 0 && blockIdx.y <= blockIdx.x) {
+    atomicMax(&st->cosmax, (unsigned long long)__double_as_longlong(cm));
+    atomicMax(&st->cosbound, (unsigned long long)__double_as_longlong(cb));
+    if (f2 > 0)
+      atomicAdd(&st->f2, f2);
+    if (over)
+      atomicAdd(&st->over, over);
+    if (skipped)
+      atomicAdd(&st->skipped, skipped);
+  }
+}
+
+// y = a x + b y (y := a x when b is 0), n elements
+__global__ void k_lincomb(long long n, double a, const double *x, double b, double *y)
+{
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
+    y[i] = (b == 0.0) ? a * x[i] : fma(a, x[i], b * y[i]);
+}
+
+// From the odd and even parts O~, E~ of exp(K) - I in scaled form (E may be empty): O~ := O~ + E~ (for
+// the columns of G), and N = exp(K) - I in true form (for V), whose two entries of a pair both
+// come from the scaled entry that is divided by the ratio of the lengths, by the parts' symmetry
+// (O^H = -O, E^H = E): the other one would be multiplied by it, errors included.
+__global__ void __launch_bounds__(256) k_exp_parts(int n, Mat O, Mat E, const int *e, Mat N)
+{
+  __shared__ double2 so[32][33], se[32][33];
+  const int bi = blockIdx.x, bj = blockIdx.y;
+  if (bj > bi)
+    return;
+  auto get = [&](const Mat &M, size_t o) {
+    return M.re ? make_double2(M.re[o], M.im ? M.im[o] : 0.0) : make_double2(0.0, 0.0);
+  };
+  // the tile's mirror: entries (j, i), rows j along the threads
+  for (int k = threadIdx.y; k < 32; k += 8) {
+    const int j = bj * 32 + threadIdx.x, i = bi * 32 + k;
+    if (i < n && j < n && i > j) {
+      const size_t o = (size_t)i * n + j;
+      so[threadIdx.x][k] = get(O, o);
+      se[threadIdx.x][k] = get(E, o);
+    }
+  }
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += 8) {
+    const int i = bi * 32 + threadIdx.x, j = bj * 32 + k;
+    if (i < n && j < n && i >= j) {
+      const size_t o = (size_t)j * n + i;
+      const double2 a = get(O, o), b = get(E, o);
+      double2 x = make_double2(a.x + b.x, a.y + b.y), y = make_double2(0, 0);
+      O.re[o] = x.x;
+      if (O.im)
+        O.im[o] = x.y;
+      if (i != j) {
+        const double2 c = so[k][threadIdx.x], f = se[k][threadIdx.x];
+        so[k][threadIdx.x] = make_double2(c.x + f.x, c.y + f.y);
+        const int d = max(-2000, min(2000, e[j] - e[i]));
+        if (d <= 0) {
+          y = make_double2(scalbn(b.x - a.x, d), scalbn(a.y - b.y, d));  // (j, i) from (i, j)
+          x = make_double2(scalbn(x.x, d), scalbn(x.y, d));
+        }
+        else {
+          x = make_double2(scalbn(f.x - c.x, -d), scalbn(c.y - f.y, -d));
+          y = make_double2(scalbn(c.x + f.x, -d), scalbn(c.y + f.y, -d));
+        }
+        se[k][threadIdx.x] = y;
+      }
+      N.re[o] = x.x;
+      if (N.im)
+        N.im[o] = x.y;
+    }
+  }
+  __syncthreads();
+  for (int k = threadIdx.y; k < 32; k += 8) {
+    const int j = bj * 32 + threadIdx.x, i = bi * 32 + k;
+    if (i < n && j < n && i > j) {
+      const size_t o = (size_t)i * n + j;
+      O.re[o] = so[threadIdx.x][k].x;
+      N.re[o] = se[threadIdx.x][k].x;
+      if (O.im) {
+        O.im[o] = so[threadIdx.x][k].y;
+        N.im[o] = se[threadIdx.x][k].y;
+      }
+    }
+  }
 }
 
 static bool copy2d(double *dst, long long ldd, const double *src, long long lds, long long rows, long long cols,
@@ -777,19 +827,8 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     stages = 2;
   if (!host::gpu_ready())
     return VJ_ERR_NO_GPU;
-  cublasHandle_t h = cublas();
-  if (!h)
-    return VJ_ERR_CUDA;
-  if (cublasSetStream(h, s) != CUBLAS_STATUS_SUCCESS)
-    return VJ_ERR_CUDA;
   const int P = CPLX ? 2 : 1;
   const size_t mn = (size_t)m * n, nn = (size_t)n * n;
-  // scratch: G32 (P m n), W32 (P n n) floats; Gp, X, T, Y (P n n each) doubles; counters
-  const size_t f32b = ((P * (mn + nn) * 4) + 255) & ~(size_t)255;
-  // Gp: the copy of G for G W (P m n doubles), earlier the temporaries of the 3M products
-  // (3 n n doubles)
-  const size_t gpn = ((size_t)P * mn > 3 * nn) ? (size_t)P * mn : 3 * nn;
-  const size_t f64b = (gpn + P * 3 * nn) * 8;
   // FP32 stages: block sweeps on the tensor cores where the shape has whole blocks and at
   // least 16 block pairs per step (fewer pairs leave most SMs idle in the pair
   // eigenproblems: at 1024 x 1024 real the column-pair sweeps take 109 ms against 176 ms,
@@ -805,23 +844,96 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   const char *ei = getenv("VJ_BLOCK_INNER");
   const int inner = (ei && atoi(ei) >= 1 && atoi(ei) <= 8) ? atoi(ei) : 1;
   const size_t blkb = blk ? ((block_sweep_scratch(CPLX, m, n, inner) + 255) & ~(size_t)255) : 0;
-  host::Staging &stg = host::staging3();
-  if (!stg.reserve(f32b + f64b + 256 + blkb))
-    return VJ_ERR_NOMEM;
-  unsigned char *bscr = reinterpret_cast<unsigned char *>(stg.ptr) + f32b + f64b + 256;
-  float *G32 = reinterpret_cast<float *>(stg.ptr);
-  float *W32 = G32 + P * mn;
-  double *Gp = reinterpret_cast<double *>(stg.ptr + f32b);
-  double *X = Gp + gpn;
-  double *T = X + P * nn;
-  double *Y = T + P * nn;
-  unsigned long long *cell = reinterpret_cast<unsigned long long *>(Y + P * nn);
-  unsigned *cnt = reinterpret_cast<unsigned *>(cell + 1);
+  // scratch: the FP32 copy of G and W (P m n and P n n floats); five P n n matrices of doubles; two
+  // digit operands of the FP64 products (fp64tc.cuh), the first as large as G's columns or rows
+  // take, the second as an n x n matrix takes, with their exponents; counters; the block sweeps'
+  // own. The columns' gather before the finishing sweeps goes through the digits' room.
   const int ni = (int)n, mi = (int)m;
-  const Planes Gpl{G, Gi, (int)ldG, (int)(CPLX ? ldGi : ldG)};
-  const Planes Vpl{V, Vi, (int)ldV, (int)(CPLX ? ldVi : ldV)};
-  const Planes Xp{X, X + nn, ni, ni}, Tp{T, T + nn, ni, ni}, Yp{Y, Y + nn, ni, ni};
-  const Planes Gpp{Gp, Gp + mn, mi, mi};
+  oz::Source sc{G, Gi, (long long)ldG, (long long)(CPLX ? ldGi : ldG), ni, mi, nullptr, 0, oz::COLS};
+  oz::Source sr{G, Gi, (long long)ldG, (long long)(CPLX ? ldGi : ldG), mi, ni, nullptr, 0, oz::ROWS};
+  const oz::Operand oc = oz::shape(sc, CPLX), orw = oz::shape(sr, CPLX);
+  const oz::Operand on = oz::shape(oz::Source{G, Gi, 0, 0, ni, ni, nullptr, 0, oz::PROD}, CPLX);
+  auto up = [](size_t x) { return (x + 1023) & ~(size_t)1023; };
+  const size_t f32b = up(P * (mn + nn) * 4), f64b = up(5 * P * nn * 8);
+  const size_t d1b = up(std::max({(size_t)oc.bytes(), (size_t)orw.bytes(), (size_t)on.bytes(), mn * 8}));
+  const size_t d2b = up(std::max((size_t)on.bytes(), nn * 8));
+  const size_t e1b = up((size_t)(2 * std::max(oc.np, orw.np)) * 4), e2b = up((size_t)(2 * on.np) * 4);
+  const size_t ekb = up((size_t)n * 4), vecb = up((size_t)n * 16);
+  host::Staging &stg = host::staging3();
+  if (!stg.reserve(f32b + f64b + d1b + d2b + e1b + e2b + ekb + vecb + 1024 + blkb))
+    return VJ_ERR_NOMEM;
+  unsigned char *at = reinterpret_cast<unsigned char *>(stg.ptr);
+  auto take = [&](size_t bytes) {
+    unsigned char *r = at;
+    at += bytes;
+    return r;
+  };
+  float *G32 = reinterpret_cast<float *>(take(f32b));
+  float *W32 = G32 + P * mn;
+  double *f64 = reinterpret_cast<double *>(take(f64b));
+  unsigned char *d1 = take(d1b), *d2 = take(d2b);
+  int *e1 = reinterpret_cast<int *>(take(e1b)), *e2 = reinterpret_cast<int *>(take(e2b));
+  int *ek = reinterpret_cast<int *>(take(ekb));  // exponents of G's columns
+  double *vec = reinterpret_cast<double *>(take(vecb));
+  unsigned char *cells = take(1024);
+  unsigned char *bscr = at;
+  unsigned long long *cell = reinterpret_cast<unsigned long long *>(cells);
+  unsigned *cnt = reinterpret_cast<unsigned *>(cell + 1);
+  unsigned *gerr = cnt + 4;
+  PairStats *st = reinterpret_cast<PairStats *>(cells + 256);
+  Mat M[5];
+  for (int k = 0; k < 5; ++k)
+    M[k] = Mat{f64 + (size_t)k * P * nn, CPLX ? f64 + (size_t)k * P * nn + nn : nullptr};
+  double *const Y = M[4].re;
+  const dim3 tiles((unsigned)((n + 31) / 32), (unsigned)((n + 31) / 32)), tblk(32, 8);
+  if (cudaMemsetAsync(gerr, 0, 4, s) != cudaSuccess)
+    return VJ_ERR_CUDA;
+  // X's columns (for X^H X), rows (for X Y) or an n x n matrix as the right factor, cut into digits
+  auto cut = [&](const oz::Source &src, unsigned char *d, int *e, oz::Operand &o) {
+    o = oz::shape(src, CPLX);
+    o.d = d;
+    o.e = e;
+    return oz::split(src, o, s) == cudaSuccess;
+  };
+  auto cut_cols = [&](const double *re, const double *im, long long ldr, long long ldi, int rows, oz::Operand &o) {
+    return cut(oz::Source{re, im, ldr, ldi, ni, rows, nullptr, 0, oz::COLS}, d1, e1, o);
+  };
+  auto cut_rows = [&](const double *re, const double *im, long long ldr, long long ldi, int rows, const int *x,
+                      oz::Operand &o) {
+    return cut(oz::Source{re, im, ldr, ldi, rows, ni, x, -1, oz::ROWS}, d1, e1, o);
+  };
+  auto cut_prod = [&](const Mat &X, const int *x, oz::Operand &o) {
+    return cut(oz::Source{X.re, X.im, n, n, ni, ni, x, 1, oz::PROD}, d2, e2, o);
+  };
+  // H's lower triangle = X^H X of columns cut into o
+  auto gram = [&](const oz::Operand &o, const Mat &H, int scaled, int nd) {
+    oz::Operand a = o;
+    a.halves = 1;
+    return oz::gemm(a, o, oz::Result{H.re, H.im, n, n, ni, ni, nullptr, scaled, 0, 1}, nd, gerr, s) == cudaSuccess;
+  };
+  // X (+)= A B for an n x n X
+  auto mult = [&](const oz::Operand &A, const oz::Operand &B, const Mat &X, int add) {
+    return oz::gemm(A, B, oz::Result{X.re, X.im, n, n, ni, ni, nullptr, 1, add, 0}, 7, gerr, s) == cudaSuccess;
+  };
+  // V (+)= A B, G (+)= A B (G's columns times 2^ej)
+  auto mult_v = [&](const oz::Operand &A, const oz::Operand &B, int add) {
+    return oz::gemm(A, B, oz::Result{V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, ni, nullptr, 1, add, 0},
+                    7, gerr, s) == cudaSuccess;
+  };
+  auto mult_g = [&](const oz::Operand &A, const oz::Operand &B, const int *ej, int add) {
+    return oz::gemm(A, B, oz::Result{G, Gi, sc.ldr, sc.ldi, mi, ni, ej, 1, add, 0}, 7, gerr, s) == cudaSuccess;
+  };
+  PairStats hst;
+  auto read_stats = [&]() {
+    return cudaGetLastError() == cudaSuccess &&
+           cudaMemcpyAsync(&hst, st, sizeof(hst), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
+           cudaStreamSynchronize(s) == cudaSuccess;
+  };
+  auto asdbl = [](unsigned long long b) {
+    double v;
+    memcpy(&v, &b, 8);
+    return v;
+  };
   // sqrt(m)/2 units of FP32 roundoff (the reference's FP32 tolerance), at least 8 units
   const float tol = fmaxf(0.5f * sqrtf((float)m), 8.f) * 5.9604645e-8f;
   const unsigned maxsw = swp < 60u ? swp : 60u;
@@ -901,23 +1013,21 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     }
     if (!sw)
       break;  // already orthogonal to the FP32 level: later stages would change nothing
-    // 3. W (FP64) made unitary by one Cholesky QR, Q = W R^-1 with R^H R = W^H W (a Gram
-    //    product, cuSOLVER's Cholesky factorisation, a triangular solve): W^H W is within
-    //    1e-4 of I after the FP32 stage, so one pass is unitary to FP64 accuracy, at about
-    //    half the cost of the two Newton-Schulz steps that the same accuracy needs. W's
-    //    columns go in ascending order of the norms of the FP32 G's columns first: R^-1 is
-    //    upper triangular, so the correction mixes into each column of G Q only columns of
-    //    smaller norm. (The first FP64 sweep below still meets scaled inner products of up
-    //    to ~5e-3 at 4096 x 2048 complex with sigma down to 1e-8, and 2e-5 at 4096 x 2048 real
-    //    with sigma down to 1e-6: the FP32 rounding of W's own entries couples large columns
-    //    of G into small ones, which no orthonormalisation of W undoes; the descending order
-    //    measured worse, 1e-2 and 1.5e-4, and one FP64 sweep more at 4096 x 2048 complex.)
-    for (int pl = 0; pl < P; ++pl)
-      k_to_f64<<<(unsigned)((nn + 255) / 256 < 4096 ? (nn + 255) / 256 : 4096), 256, 0, s>>>(
-          W32 + pl * nn, (long long)nn, X + pl * nn);
+    // 3. W (FP64) made unitary, with its columns in ascending order of the norms of the FP32 G's
+    //    columns: W^H W = I + E with E of the order of FP32 rounding, and the factor R of its
+    //    Cholesky factorisation R^H R is I + U to first order, U the strict upper triangle of E
+    //    and half its diagonal; W := W (I - U), repeated while the second-order terms left
+    //    (about E^2) exceed FP64 rounding. Two rounds of a Gram product and a correction, all
+    //    on the tensor cores, in place of a factorisation and a triangular solve on the FP64
+    //    unit. The correction is upper triangular, so it mixes into each column of G Q only
+    //    columns of smaller norm. (The first refinement below still meets scaled inner products
+    //    of up to ~5e-3 at 4096 x 2048 complex with sigma down to 1e-8: the FP32 rounding of W's
+    //    own entries couples large columns of G into small ones, which no orthonormalisation of
+    //    W undoes; the descending order measured worse.)
+    const Mat &T = M[0];
     {
-      double *nrm = Y;  // n entries of scratch, free until the Gram product below
-      int *perm = reinterpret_cast<int *>(Y + n);
+      double *nrm = vec;
+      int *perm = reinterpret_cast<int *>(vec + n);
       k_colnorm2_f32<CPLX><<<(unsigned)n, 256, 0, s>>>(mi, G32, CPLX ? G32 + mn : nullptr, nrm);
       std::vector<double> hn((size_t)n);
       std::vector<int> hp((size_t)n);
@@ -929,82 +1039,43 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
       std::stable_sort(hp.begin(), hp.end(), [&](int x, int y) { return hn[(size_t)x] < hn[(size_t)y]; });
       if (cudaMemcpyAsync(perm, hp.data(), (size_t)n * 4, cudaMemcpyHostToDevice, s) != cudaSuccess)
         return VJ_ERR_CUDA;
-      // T := W with its columns permuted (the copy reads the host vector: wait for it)
-      for (int pl = 0; pl < P; ++pl)
-        k_gather_cols<<<grid2(n, n), 256, 0, s>>>(ni, ni, X + pl * nn, n, perm, T + pl * nn);
+      k_widen_cols<<<grid2(n, n), 256, 0, s>>>(ni, W32, perm, T.re);
+      if (CPLX)
+        k_widen_cols<<<grid2(n, n), 256, 0, s>>>(ni, W32 + nn, perm, T.im);
+      // (the copy reads the host vector: wait for it)
       if (cudaStreamSynchronize(s) != cudaSuccess)
         return VJ_ERR_CUDA;
     }
-    if (!gram(h, CPLX, ni, Tp, Yp, Gp, s))
-      return VJ_ERR_CUDA;
-    {
-      cusolverDnHandle_t hs = cusolver();
-      if (!hs || cusolverDnSetStream(hs, s) != CUSOLVER_STATUS_SUCCESS)
+    oz::Operand oa, ob;
+    for (int round = 0;; ++round) {
+      if (!cut_cols(T.re, T.im, n, n, ni, oa) || !gram(oa, M[1], 1, 7) ||
+          cudaMemsetAsync(st, 0, sizeof(PairStats), s) != cudaSuccess)
         return VJ_ERR_CUDA;
-      int *info = reinterpret_cast<int *>(cell);
-      static host::Staging wsps[host::MAX_DEVICES];  // the factorisation's workspace, per device
-      host::Staging &wsp = wsps[host::device_slot()];
-      const double one = 1.0;
-      int lw = 0, hinfo = 0;
-      if (!CPLX) {
-        // R overwrites the upper triangle of Y; T := T R^-1
-        if (cusolverDnDpotrf_bufferSize(hs, CUBLAS_FILL_MODE_UPPER, ni, Y, ni, &lw) != CUSOLVER_STATUS_SUCCESS ||
-            !wsp.reserve((size_t)(lw > 0 ? lw : 1) * 8) ||
-            cusolverDnDpotrf(hs, CUBLAS_FILL_MODE_UPPER, ni, Y, ni, reinterpret_cast<double *>(wsp.ptr), lw, info) !=
-                CUSOLVER_STATUS_SUCCESS ||
-            cublasDtrsm(h, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT, ni, ni, &one,
-                        Y, ni, T, ni) != CUBLAS_STATUS_SUCCESS)
-          return VJ_ERR_CUDA;
-      }
-      else {
-        // interleaved copies for the complex factorisation: Z = W^H W (in Gp), Xz = W (in Y)
-        cuDoubleComplex *Z = reinterpret_cast<cuDoubleComplex *>(Gp);
-        cuDoubleComplex *Xz = reinterpret_cast<cuDoubleComplex *>(Y);
-        const unsigned g1 = (unsigned)((nn + 255) / 256 < 4096 ? (nn + 255) / 256 : 4096);
-        k_to_interleaved<<<g1, 256, 0, s>>>(Y, Y + nn, (long long)nn, reinterpret_cast<double2 *>(Z));
-        k_to_interleaved<<<g1, 256, 0, s>>>(T, T + nn, (long long)nn, reinterpret_cast<double2 *>(Xz));
-        const cuDoubleComplex zone = make_cuDoubleComplex(1.0, 0.0);
-        if (cusolverDnZpotrf_bufferSize(hs, CUBLAS_FILL_MODE_UPPER, ni, Z, ni, &lw) != CUSOLVER_STATUS_SUCCESS ||
-            !wsp.reserve((size_t)(lw > 0 ? lw : 1) * 16) ||
-            cusolverDnZpotrf(hs, CUBLAS_FILL_MODE_UPPER, ni, Z, ni, reinterpret_cast<cuDoubleComplex *>(wsp.ptr), lw,
-                             info) != CUSOLVER_STATUS_SUCCESS ||
-            cublasZtrsm(h, CUBLAS_SIDE_RIGHT, CUBLAS_FILL_MODE_UPPER, CUBLAS_OP_N, CUBLAS_DIAG_NON_UNIT, ni, ni, &zone,
-                        Z, ni, Xz, ni) != CUBLAS_STATUS_SUCCESS)
-          return VJ_ERR_CUDA;
-        k_from_interleaved<<<g1, 256, 0, s>>>(reinterpret_cast<const double2 *>(Xz), (long long)nn, T, T + nn);
-      }
-      if (cudaMemcpyAsync(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-          cudaStreamSynchronize(s) != cudaSuccess)
+      k_neg_upper<<<tiles, tblk, 0, s>>>(ni, M[1], M[2], st);
+      if (!read_stats())
         return VJ_ERR_CUDA;
-      if (hinfo != 0)
-        return VJ_ERR_CUDA;  // W^H W not positive definite: W was not near unitary
-      // Q (in T) becomes the stage's transformation X
-      for (int pl = 0; pl < P; ++pl)
-        if (!copy2d(X + pl * nn, n, T + pl * nn, n, n, n, s))
-          return VJ_ERR_CUDA;
+      const double emax = asdbl(hst.cosmax);
       if (trace)
-        std::fprintf(stderr, "mixed SVD stage %u: Cholesky QR of W\n", stage);
+        std::fprintf(stderr, "mixed SVD stage %u: largest entry of W^H W - I %.2e\n", stage, emax);
+      if (!(emax < 0.03) || round == 6)
+        return VJ_ERR_CUDA;  // W was not near unitary
+      if (!cut_rows(T.re, T.im, n, n, ni, nullptr, oa) || !cut_prod(M[2], nullptr, ob) || !mult(oa, ob, T, 1))
+        return VJ_ERR_CUDA;
+      if (emax * emax * std::sqrt((double)n) < 2e-17)
+        break;
     }
-    // 4. V <- V W (V_0 = I, so the first stage that rotates sets V = W), G <- G W
+    // 4. V <- V W (V_0 = I, so the first stage that rotates sets V = W), G <- G W; G's columns
+    //    enter the product with their lengths' powers of two moved to the rows of W, so that the
+    //    digits resolve every column of the result to its own length
     if (total32 == sw) {
-      if (!copy2d(V, ldV, X, n, n, n, s) || (CPLX && !copy2d(Vi, ldVi, X + nn, n, n, n, s)))
+      if (!copy2d(V, ldV, T.re, n, n, n, s) || (CPLX && !copy2d(Vi, ldVi, T.im, n, n, n, s)))
         return VJ_ERR_CUDA;
     }
-    else {
-      if (!copy2d(T, n, V, ldV, n, n, s) || (CPLX && !copy2d(T + nn, n, Vi, ldVi, n, n, s)))
-        return VJ_ERR_CUDA;
-      if (!zgemm3m(h, CPLX, ni, ni, ni, Tp, Xp, Vpl, Gp, s))
-        return VJ_ERR_CUDA;
-    }
-    if (!copy2d(Gp, m, G, ldG, m, n, s) || (CPLX && !copy2d(Gp + mn, m, Gi, ldGi, m, n, s)))
+    else if (!cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, nullptr, oa) ||
+             !cut_prod(T, nullptr, ob) || !mult_v(oa, ob, 0))
       return VJ_ERR_CUDA;
-    // complex G := G Q by 3M when its temporaries fit in the free T and Y scratch
-    // (m n + n n <= 4 n n doubles), else by four real products
-    if (CPLX && m <= 3 * n) {
-      if (!zgemm3m_overwrite(h, mi, ni, ni, Gpp, Xp, Gpl, T, s))
-        return VJ_ERR_CUDA;
-    }
-    else if (!zgemm(h, CPLX, false, mi, ni, ni, Gpp, Xp, Gpl))
+    if (oz::row_exponents(sc, ek, s) != cudaSuccess || !cut_rows(G, Gi, sc.ldr, sc.ldi, mi, ek, oa) ||
+        !cut_prod(T, ek, ob) || !mult_g(oa, ob, nullptr, 0))
       return VJ_ERR_CUDA;
     {
       if (cudaStreamSynchronize(s) != cudaSuccess)
@@ -1022,45 +1093,118 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     if (CPLX)
       k_eye_p<double><<<grid2(n, n), 256, 0, s>>>(Vi, (long long)ldVi, n, 0);
   }
-  // 5. FP64 sweeps with plain dot products on G and V themselves until no pair reaches half
-  //    the reference's tolerance sqrt(m) eps / 2 (at most 20 sweeps): they take the columns from
-  //    FP32 to FP64 orthogonality at a fraction of a reference sweep's cost (4 FP64
-  //    operations per complex element of G for the inner product with tracked norms and 8
-  //    for the rotation in the short form of Rot, instead of 68), so the reference's sweeps below
-  //    have at most the last rotations to do and the convergence to confirm.
+  // 5. G's columns from FP32 to FP64 orthogonality, to half the reference's tolerance sqrt(m) eps / 2
+  //    (pairs the reference would still rotate are rotated here), by refinements on the tensor
+  //    cores: the Gram matrix of the columns to FP64 accuracy, the generator K of the rotation
+  //    that makes them orthogonal to first order, N = exp(K) - I by its series, and G := G + G N,
+  //    V := V + V N. What is left is of second order, so two refinements and the Gram matrix that
+  //    confirms them replace the plain-dot FP64 sweeps (4096 x 2048 complex: 689 ms of sweeps).
+  //    Pairs of nearly equal norms, whose rotation is not small, are left out of K; they, and
+  //    whatever a refinement cannot improve, go to those sweeps, which run until no pair is left.
+  bool certified = false;
   if (total32) {
-    // half the reference's tolerance: the plain dot product's rounding (a few eps) stays
-    // well below it, and pairs the reference would still rotate are rotated here
-    const double tol64 = 0.5 * std::sqrt((double)m) * 1.1102230246251565e-16;
+    const double u = 1.1102230246251565e-16;
+    const double tol64 = 0.5 * std::sqrt((double)m) * u;
+    // the finishing check's limit (jsvd.cu, k_certify)
+    const double lim = 0.9 * std::sqrt((double)m) * u - 16.0 * u;
     const unsigned maxsw64 = swp < 20u ? swp : 20u;
     unsigned sw64 = 0;
+    bool sweeps = true;
+    double before = 1e300;
+    for (unsigned it = 0; it < 8u && swp; ++it) {
+      oz::Operand oa, ob;
+      const Mat &H = M[0], &K = M[1], &P3 = M[2], &Q = M[3], &E = M[4];
+      if (!cut_cols(G, Gi, sc.ldr, sc.ldi, mi, oa) || !gram(oa, H, 0, 8) ||
+          cudaMemcpyAsync(ek, e1, (size_t)n * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
+          cudaMemsetAsync(st, 0, sizeof(PairStats), s) != cudaSuccess)
+        return VJ_ERR_CUDA;
+      // digit pairs left out of the Gram entries: below 2^-62.8 per element of K
+      const double hb = (double)((long long)P * m) * 1.25e-19;
+      k_generator<<<tiles, tblk, 0, s>>>(ni, H, ek, K, tol64, hb, st);
+      if (!read_stats())
+        return VJ_ERR_CUDA;
+      const double cmax = asdbl(hst.cosmax), f = std::sqrt(hst.f2);
+      if (trace)
+        std::fprintf(stderr, "mixed SVD refinement %u: %u pairs above the tolerance, max |cos| %.3e, |K| %.2e, %u left out, "
+                     "%.1f ms since the phase began\n", it, hst.over, cmax, f, hst.skipped,
+                     std::chrono::duration<double, std::milli>(now() - t0).count());
+      if (!hst.over && cmax <= tol64) {
+        sweeps = false;
+        certified = (asdbl(hst.cosbound) <= lim);
+        break;
+      }
+      // (K's series below is to sixth order: |K|^7 / 7! <= 2.5e-15 in the Frobenius norm, below the
+      // rounding of V's n^2 entries)
+      if (!(f <= 0.0277) || hst.over == hst.skipped || !(cmax <= 0.25 * before))
+        break;
+      before = cmax;
+      const int terms = (f < 1e-8) ? 1 : (f < 6e-6) ? 2 : (f < 1.8e-4) ? 3 : (f < 1.4e-3) ? 4 : (f < 5.7e-3) ? 5 : 6;
+      const long long np = (long long)(P * nn);
+      const unsigned gl = (unsigned)((np + 255) / 256 < 4096 ? (np + 255) / 256 : 4096);
+      Mat Ev{nullptr, nullptr};
+      bool ok = true;
+      if (terms >= 2) {
+        // K^2 (in H's place)
+        ok = cut_rows(K.re, K.im, n, n, ni, nullptr, oa) && cut_prod(K, nullptr, ob) && mult(oa, ob, H, 0);
+        k_lincomb<<<gl, 256, 0, s>>>(np, 0.5, H.re, 0.0, E.re);
+        Ev = E;
+      }
+      if (ok && terms >= 3) {
+        // K^3; the odd part K + K^3 / 6 takes K's place
+        ok = cut_prod(H, nullptr, ob) && mult(oa, ob, P3, 0);
+        k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 6.0, P3.re, 1.0, K.re);
+      }
+      if (ok && terms >= 4) {
+        ok = cut_rows(H.re, H.im, n, n, ni, nullptr, oa) && mult(oa, ob, Q, 0);  // K^4
+        k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 24.0, Q.re, 1.0, E.re);
+      }
+      if (ok && terms >= 5) {
+        ok = cut_prod(P3, nullptr, ob) && mult(oa, ob, Q, 0);  // K^5
+        k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 120.0, Q.re, 1.0, K.re);
+      }
+      if (ok && terms >= 6) {
+        ok = cut_rows(P3.re, P3.im, n, n, ni, nullptr, oa) && mult(oa, ob, Q, 0);  // K^6
+        k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 720.0, Q.re, 1.0, E.re);
+      }
+      if (!ok)
+        return VJ_ERR_CUDA;
+      k_exp_parts<<<tiles, tblk, 0, s>>>(ni, K, Ev, ek, Q);
+      if (!cut_rows(G, Gi, sc.ldr, sc.ldi, mi, ek, oa) || !cut_prod(K, nullptr, ob) || !mult_g(oa, ob, ek, 1) ||
+          !cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, nullptr, oa) || !cut_prod(Q, nullptr, ob) ||
+          !mult_v(oa, ob, 1))
+        return VJ_ERR_CUDA;
+      ++sw64;
+    }
+    unsigned herr = 0;
+    if (cudaMemcpyAsync(&herr, gerr, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess || herr)
+      return VJ_ERR_CUDA;
     // A sweep whose rotated pairs all had |cos| <= 1e-11 leaves off-diagonal terms of the
     // order of their squares (times n / relative gap), far below the tolerance: its
     // confirming sweep is skipped, the reference's sweep below confirms.
-    for (; sw64 < maxsw64; ++sw64) {
+    for (unsigned sw = 0; sweeps && sw < maxsw64; ++sw) {
       float mu = 0.f;
-      // (column scales and tracked norms in Y, free scratch until the sort below)
       const long long hc = presweep<double, CPLX>(mi, ni, G, (long long)ldG, Gi, (long long)(CPLX ? ldGi : ldG), V,
                                                   (long long)ldV, Vi, (long long)(CPLX ? ldVi : ldV), js, stp, tol64,
-                                                  cnt, s, &mu, Y, Y + n);
+                                                  cnt, s, &mu, vec, vec + n);
       if (hc < 0)
         return VJ_ERR_CUDA;
       if (trace)
         std::fprintf(stderr, "mixed SVD FP64 sweep %u: %lld rotations, max |cos| %.3e, %.1f ms since the phase began\n",
-                     sw64, hc, (double)mu, std::chrono::duration<double, std::milli>(now() - t0).count());
+                     sw, hc, (double)mu, std::chrono::duration<double, std::milli>(now() - t0).count());
       if (!hc)
         break;
-      if (mu <= 1e-11f) {
-        ++sw64;
+      ++sw64;
+      if (mu <= 1e-11f)
         break;
-      }
     }
     if (presweeps)
       presweeps[1] = sw64;
     // columns in descending order of their norms, the order the reference's sweeps keep
     // (src/dvjsvd.c:367-370): its sweeps then have no pair to reorder
-    double *nrm = T;  // n entries of scratch
-    int *perm = reinterpret_cast<int *>(T + n);
+    double *nrm = vec;
+    int *perm = reinterpret_cast<int *>(vec + n);
+    double *Gp = reinterpret_cast<double *>(d1);
     k_colnorm2<CPLX><<<(unsigned)n, 256, 0, s>>>(mi, G, (long long)ldG, Gi, (long long)(CPLX ? ldGi : ldG), nrm);
     std::vector<double> hn((size_t)n);
     std::vector<int> hp((size_t)n);
@@ -1096,14 +1240,14 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     t0 = t1;
   }
   // 6. FP64 finishing sweeps (the reference's algorithm) with V preset
-  const vj_fint r = svd_dev_entry<double, CPLX>(m_, n_, G, ldG, Gi, ldGi, V, ldV, Vi, ldVi, eS, fS, js, stp, swp, 2, s);
+  const vj_fint r = svd_dev_entry<double, CPLX>(m_, n_, G, ldG, Gi, ldGi, V, ldV, Vi, ldVi, eS, fS, js, stp, swp, 2, certified, s);
   const double msfin = std::chrono::duration<double, std::milli>(now() - t0).count();
   // FP32 launches: 5 per block step (Gram, its reduction, the pair eigenproblems, R, the
   // rotation; n/b - 1 steps per block sweep), else 1 per pivot step
   const double steps32 = blk ? (double)total32 * (double)(n / (CPLX ? 32 : 64) - 1) * 5.0 : (double)total32 * stp;
   host::mixed_phases_set(ms32, msgemm, ms64, msfin, steps32, blk ? 1.0 : 0.0);
   if (trace)
-    std::fprintf(stderr, "mixed SVD phases (ms): FP32 sweeps %.1f, Newton-Schulz + GEMMs %.1f, plain FP64 sweeps + sort %.1f, "
+    std::fprintf(stderr, "mixed SVD phases (ms): FP32 sweeps %.1f, orthonormalisation + products %.1f, FP64 refinement + sort %.1f, "
                  "finishing %.1f\n", ms32, msgemm, ms64, msfin);
   return r;
 }
