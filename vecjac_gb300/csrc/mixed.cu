@@ -912,16 +912,22 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     return oz::gemm(a, o, oz::Result{H.re, H.im, n, n, ni, ni, nullptr, scaled, 0, 1}, nd, gerr, s) == cudaSuccess;
   };
   // X (+)= A B for an n x n X
-  auto mult = [&](const oz::Operand &A, const oz::Operand &B, const Mat &X, int add) {
-    return oz::gemm(A, B, oz::Result{X.re, X.im, n, n, ni, ni, nullptr, 1, add, 0}, 7, gerr, s) == cudaSuccess;
+  auto mult = [&](const oz::Operand &A, const oz::Operand &B, const Mat &X, int add, int nd) {
+    return oz::gemm(A, B, oz::Result{X.re, X.im, n, n, ni, ni, nullptr, 1, add, 0}, nd, gerr, s) == cudaSuccess;
   };
   // V (+)= A B, G (+)= A B (G's columns times 2^ej)
-  auto mult_v = [&](const oz::Operand &A, const oz::Operand &B, int add) {
+  auto mult_v = [&](const oz::Operand &A, const oz::Operand &B, int add, int nd) {
     return oz::gemm(A, B, oz::Result{V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, ni, nullptr, 1, add, 0},
-                    7, gerr, s) == cudaSuccess;
+                    nd, gerr, s) == cudaSuccess;
   };
-  auto mult_g = [&](const oz::Operand &A, const oz::Operand &B, const int *ej, int add) {
-    return oz::gemm(A, B, oz::Result{G, Gi, sc.ldr, sc.ldi, mi, ni, ej, 1, add, 0}, 7, gerr, s) == cudaSuccess;
+  auto mult_g = [&](const oz::Operand &A, const oz::Operand &B, const int *ej, int add, int nd) {
+    return oz::gemm(A, B, oz::Result{G, Gi, sc.ldr, sc.ldi, mi, ni, ej, 1, add, 0}, nd, gerr, s) == cudaSuccess;
+  };
+  // digits that a correction of relative size x needs: what nd digits leave out, about 2^(5 - 8 nd)
+  // of a product of rows of length 1, stays below 2^-57
+  auto digits = [](double x) {
+    const int nd = (int)std::ceil((62.0 + std::log2(std::max(x, 1e-20))) / 8.0);
+    return nd < 3 ? 3 : nd > 8 ? 8 : nd;
   };
   PairStats hst;
   auto read_stats = [&]() {
@@ -1047,22 +1053,28 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
         return VJ_ERR_CUDA;
     }
     oz::Operand oa, ob;
+    // (the Gram matrices before the last need no more digits than their own second-order terms
+    // justify: 4 give E to 1e-9, 6 to 1e-13)
+    int nd = 4;
     for (int round = 0;; ++round) {
-      if (!cut_cols(T.re, T.im, n, n, ni, oa) || !gram(oa, M[1], 1, 7) ||
+      if (!cut_cols(T.re, T.im, n, n, ni, oa) || !gram(oa, M[1], 1, nd) ||
           cudaMemsetAsync(st, 0, sizeof(PairStats), s) != cudaSuccess)
         return VJ_ERR_CUDA;
       k_neg_upper<<<tiles, tblk, 0, s>>>(ni, M[1], M[2], st);
       if (!read_stats())
         return VJ_ERR_CUDA;
-      const double emax = asdbl(hst.cosmax);
+      const double emax = asdbl(hst.cosmax), rn_ = std::sqrt((double)n);
       if (trace)
         std::fprintf(stderr, "mixed SVD stage %u: largest entry of W^H W - I %.2e\n", stage, emax);
-      if (!(emax < 0.03) || round == 6)
+      if (!(emax < 0.03) || round == 8)
         return VJ_ERR_CUDA;  // W was not near unitary
-      if (!cut_rows(T.re, T.im, n, n, ni, nullptr, oa) || !cut_prod(M[2], nullptr, ob) || !mult(oa, ob, T, 1))
+      if (!cut_rows(T.re, T.im, n, n, ni, nullptr, oa) || !cut_prod(M[2], nullptr, ob) ||
+          !mult(oa, ob, T, 1, digits(emax)))
         return VJ_ERR_CUDA;
-      if (emax * emax * std::sqrt((double)n) < 2e-17)
+      const double next = std::max(emax * emax * rn_, nd == 4 ? 1e-9 : nd == 6 ? 1e-13 : 0.0);
+      if (nd == 8 && next < 2e-17)
         break;
+      nd = (next * next * rn_ < 2e-17) ? 8 : 6;
     }
     // 4. V <- V W (V_0 = I, so the first stage that rotates sets V = W), G <- G W; G's columns
     //    enter the product with their lengths' powers of two moved to the rows of W, so that the
@@ -1072,10 +1084,10 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
         return VJ_ERR_CUDA;
     }
     else if (!cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, nullptr, oa) ||
-             !cut_prod(T, nullptr, ob) || !mult_v(oa, ob, 0))
+             !cut_prod(T, nullptr, ob) || !mult_v(oa, ob, 0, 8))
       return VJ_ERR_CUDA;
     if (oz::row_exponents(sc, ek, s) != cudaSuccess || !cut_rows(G, Gi, sc.ldr, sc.ldi, mi, ek, oa) ||
-        !cut_prod(T, ek, ob) || !mult_g(oa, ob, nullptr, 0))
+        !cut_prod(T, ek, ob) || !mult_g(oa, ob, nullptr, 0, 8))
       return VJ_ERR_CUDA;
     {
       if (cudaStreamSynchronize(s) != cudaSuccess)
@@ -1114,12 +1126,14 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     for (unsigned it = 0; it < 8u && swp; ++it) {
       oz::Operand oa, ob;
       const Mat &H = M[0], &K = M[1], &P3 = M[2], &Q = M[3], &E = M[4];
-      if (!cut_cols(G, Gi, sc.ldr, sc.ldi, mi, oa) || !gram(oa, H, 0, 8) ||
+      // (5 digits give the first cosines, of the order of FP32 rounding, to about 1e-11)
+      const int nd = it ? 8 : 5;
+      if (!cut_cols(G, Gi, sc.ldr, sc.ldi, mi, oa) || !gram(oa, H, 0, nd) ||
           cudaMemcpyAsync(ek, e1, (size_t)n * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
           cudaMemsetAsync(st, 0, sizeof(PairStats), s) != cudaSuccess)
         return VJ_ERR_CUDA;
-      // digit pairs left out of the Gram entries: below 2^-62.8 per element of K
-      const double hb = (double)((long long)P * m) * 1.25e-19;
+      // digit pairs left out of the Gram entries: with 8 digits below 2^-62.8 per element of K
+      const double hb = (nd == 8) ? (double)((long long)P * m) * 1.25e-19 : 1e300;
       k_generator<<<tiles, tblk, 0, s>>>(ni, H, ek, K, tol64, hb, st);
       if (!read_stats())
         return VJ_ERR_CUDA;
@@ -1128,50 +1142,51 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
         std::fprintf(stderr, "mixed SVD refinement %u: %u pairs above the tolerance, max |cos| %.3e, |K| %.2e, %u left out, "
                      "%.1f ms since the phase began\n", it, hst.over, cmax, f, hst.skipped,
                      std::chrono::duration<double, std::milli>(now() - t0).count());
-      if (!hst.over && cmax <= tol64) {
+      if (nd == 8 && !hst.over && cmax <= tol64) {
         sweeps = false;
         certified = (asdbl(hst.cosbound) <= lim);
         break;
       }
       // (K's series below is to sixth order: |K|^7 / 7! <= 2.5e-15 in the Frobenius norm, below the
       // rounding of V's n^2 entries)
-      if (!(f <= 0.0277) || hst.over == hst.skipped || !(cmax <= 0.25 * before))
+      if (!(f <= 0.0277) || (hst.over && hst.over == hst.skipped) || !(cmax <= 0.25 * before))
         break;
       before = cmax;
       const int terms = (f < 1e-8) ? 1 : (f < 6e-6) ? 2 : (f < 1.8e-4) ? 3 : (f < 1.4e-3) ? 4 : (f < 5.7e-3) ? 5 : 6;
       const long long np = (long long)(P * nn);
       const unsigned gl = (unsigned)((np + 255) / 256 < 4096 ? (np + 255) / 256 : 4096);
+      const int nk = digits(f * f), ng = digits(8.0 * cmax), nv = digits(f);  // for the powers of K, G N, V N
       Mat Ev{nullptr, nullptr};
       bool ok = true;
       if (terms >= 2) {
         // K^2 (in H's place)
-        ok = cut_rows(K.re, K.im, n, n, ni, nullptr, oa) && cut_prod(K, nullptr, ob) && mult(oa, ob, H, 0);
+        ok = cut_rows(K.re, K.im, n, n, ni, nullptr, oa) && cut_prod(K, nullptr, ob) && mult(oa, ob, H, 0, nk);
         k_lincomb<<<gl, 256, 0, s>>>(np, 0.5, H.re, 0.0, E.re);
         Ev = E;
       }
       if (ok && terms >= 3) {
         // K^3; the odd part K + K^3 / 6 takes K's place
-        ok = cut_prod(H, nullptr, ob) && mult(oa, ob, P3, 0);
+        ok = cut_prod(H, nullptr, ob) && mult(oa, ob, P3, 0, nk);
         k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 6.0, P3.re, 1.0, K.re);
       }
       if (ok && terms >= 4) {
-        ok = cut_rows(H.re, H.im, n, n, ni, nullptr, oa) && mult(oa, ob, Q, 0);  // K^4
+        ok = cut_rows(H.re, H.im, n, n, ni, nullptr, oa) && mult(oa, ob, Q, 0, nk);  // K^4
         k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 24.0, Q.re, 1.0, E.re);
       }
       if (ok && terms >= 5) {
-        ok = cut_prod(P3, nullptr, ob) && mult(oa, ob, Q, 0);  // K^5
+        ok = cut_prod(P3, nullptr, ob) && mult(oa, ob, Q, 0, nk);  // K^5
         k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 120.0, Q.re, 1.0, K.re);
       }
       if (ok && terms >= 6) {
-        ok = cut_rows(P3.re, P3.im, n, n, ni, nullptr, oa) && mult(oa, ob, Q, 0);  // K^6
+        ok = cut_rows(P3.re, P3.im, n, n, ni, nullptr, oa) && mult(oa, ob, Q, 0, nk);  // K^6
         k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 720.0, Q.re, 1.0, E.re);
       }
       if (!ok)
         return VJ_ERR_CUDA;
       k_exp_parts<<<tiles, tblk, 0, s>>>(ni, K, Ev, ek, Q);
-      if (!cut_rows(G, Gi, sc.ldr, sc.ldi, mi, ek, oa) || !cut_prod(K, nullptr, ob) || !mult_g(oa, ob, ek, 1) ||
+      if (!cut_rows(G, Gi, sc.ldr, sc.ldi, mi, ek, oa) || !cut_prod(K, nullptr, ob) || !mult_g(oa, ob, ek, 1, ng) ||
           !cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, nullptr, oa) || !cut_prod(Q, nullptr, ob) ||
-          !mult_v(oa, ob, 1))
+          !mult_v(oa, ob, 1, nv))
         return VJ_ERR_CUDA;
       ++sw64;
     }
