@@ -189,8 +189,10 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, unsigne
 // 2^n x for a normal or zero x and any n (exact while the result is normal)
 __device__ __forceinline__ double scaled(double x, int n) { return scalbn(x, n); }
 
-__global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Result C, int nd, int kb0, int nkb,
-                                                     unsigned *err)
+// ND: digits used, a template so that the issue of the MMAs is straight-line code with constant
+// descriptor offsets (computed in loops, the issuing thread took three times the MMAs' own time)
+template <int ND>
+__global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Result C, int kb0, int nkb, unsigned *err)
 {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *const smem = smem_raw + ((1024u - (tc::saddr(smem_raw) & 1023u)) & 1023u);
@@ -227,13 +229,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
     const int st = kb & 1;
     const uint32_t s0 = tc::saddr(smem) + st * STAGE;
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(tc::saddr(&full[st])),
-                 "r"((unsigned)(nd * 3 * PLANE))
+                 "r"((unsigned)(ND * 3 * PLANE))
                  : "memory");
-    for (int d = 0; d < nd; ++d) {
+#pragma unroll
+    for (int d = 0; d < ND; ++d) {
       bulk_load(s0 + d * APLANE, a0 + kb * blk + d * PLANE, PLANE, &full[st]);
       bulk_load(s0 + d * APLANE + PLANE, a1 + kb * blk + d * PLANE, PLANE, &full[st]);
     }
-    bulk_load(s0 + DIGITS * APLANE, b0 + kb * blk, (unsigned)(nd * PLANE), &full[st]);
+    bulk_load(s0 + DIGITS * APLANE, b0 + kb * blk, (unsigned)(ND * PLANE), &full[st]);
   };
   long long hi[32], lo[32];  // this thread's row, 32 columns: weights 0-3 and 4-7
 #pragma unroll
@@ -260,13 +263,17 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
           break;
         tc::fence_after();
         const uint32_t s0 = tc::saddr(smem) + st * STAGE;
+        // (a descriptor's address field counts 16 bytes: offsets are added to it)
+        const uint64_t da = tc::sdesc(s0, LBO, SBO), db = tc::sdesc(s0 + DIGITS * APLANE, LBO, SBO);
+        const uint32_t more = (kb > g * GROUP) ? 1u : 0u;
+#pragma unroll
         for (int kk = 0; kk < KB / 16; ++kk)
-          for (int w = 0; w < nd; ++w)
-            for (int s = 0; s <= w; ++s) {
-              const uint64_t da = tc::sdesc(s0 + s * APLANE + kk * 2 * LBO, LBO, SBO);
-              const uint64_t db = tc::sdesc(s0 + DIGITS * APLANE + (w - s) * PLANE + kk * 2 * LBO, LBO, SBO);
-              tc::mma_bf16(tmem + w * ROWB, da, db, IDESC, (kb > g * GROUP || kk > 0 || s > 0) ? 1u : 0u);
-            }
+#pragma unroll
+          for (int w = 0; w < ND; ++w)
+#pragma unroll
+            for (int s = 0; s <= w; ++s)
+              tc::mma_bf16(tmem + w * ROWB, da + (uint64_t)((s * APLANE + kk * 2 * LBO) >> 4),
+                           db + (uint64_t)(((w - s) * PLANE + kk * 2 * LBO) >> 4), IDESC, (kk > 0 || s > 0) ? 1u : more);
         tc::commit(&freed[st]);
         // the other stage's next block, once its MMAs are done
         if (kb >= 1 && kb + 1 < nkb) {
@@ -289,17 +296,16 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
     tc::fence_after();
     const uint32_t t0 = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)((warp >> 2) * 32);
 #pragma unroll
-    for (int d = 0; d < DIGITS; ++d)
-      if (d < nd) {
-        uint32_t v[32];
-        tc::tmem_ld32(t0 + d * ROWB, v);
+    for (int d = 0; d < ND; ++d) {
+      uint32_t v[32];
+      tc::tmem_ld32(t0 + d * ROWB, v);
 #pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const int x = __float2int_rn(__uint_as_float(v[c]));
-          long long &to = (d < 4) ? hi[c] : lo[c];
-          to += (long long)x * (1 << (8 * (3 - (d & 3))));
-        }
+      for (int c = 0; c < 32; ++c) {
+        const int x = __float2int_rn(__uint_as_float(v[c]));
+        long long &to = (d < 4) ? hi[c] : lo[c];
+        to += (long long)x * (1 << (8 * (3 - (d & 3))));
       }
+    }
     tc::fence_before();
     __syncthreads();
     tc::fence_after();
@@ -375,7 +381,13 @@ cudaError_t split(const Source &s, const Operand &o, cudaStream_t st)
 
 cudaError_t gemm(const Operand &A, const Operand &B, const Result &C, int nd, unsigned *err, cudaStream_t st)
 {
-  const cudaError_t e = cudaFuncSetAttribute(k_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
+  void (*const k)(Operand, Operand, Result, int, int, unsigned *) = (nd <= 3)   ? k_gemm<3>
+                                                                    : (nd == 4) ? k_gemm<4>
+                                                                    : (nd == 5) ? k_gemm<5>
+                                                                    : (nd == 6) ? k_gemm<6>
+                                                                    : (nd == 7) ? k_gemm<7>
+                                                                                : k_gemm<8>;
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
   if (e != cudaSuccess)
     return e;
   const dim3 grid((unsigned)(B.np / ROWB * B.halves), (unsigned)((C.rows + 127) / 128));
@@ -383,7 +395,7 @@ cudaError_t gemm(const Operand &A, const Operand &B, const Result &C, int nd, un
   const int nkb = A.kp / KB * A.parts, most = (1 << 22) / KB;
   Result c = C;
   for (int kb = 0; kb < nkb; kb += most) {
-    k_gemm<<<grid, THREADS, SMEM, st>>>(A, B, c, nd, kb, nkb - kb < most ? nkb - kb : most, err);
+    k<<<grid, THREADS, SMEM, st>>>(A, B, c, kb, nkb - kb < most ? nkb - kb : most, err);
     c.add = 1;
   }
   return cudaGetLastError();

@@ -59,7 +59,7 @@ struct Result {
   const int *ej;
   int scaled, add, lower;
 };
-// C (+)= A B^T over the operands' K (A one half), with digits 0..nd-1 of each (nd <= 8); err is set
+// C (+)= A B^T over the operands' K (A one half), with digits 0..nd-1 of each (3 <= nd <= 8); err is set
 // nonzero when a wait inside the kernel gave up
 cudaError_t gemm(const Operand &A, const Operand &B, const Result &C, int nd, unsigned *err, cudaStream_t st);
 

@@ -519,6 +519,18 @@ static long long presweep(int m, int n, T *Gr, long long ldr, T *Gi, long long l
   return (long long)hc[0];
 }
 
+// the plain Hestenes rotation of npairs disjoint pairs (2 npairs column indices at pairs)
+template <bool CPLX>
+static bool rotate_pairs(int m, int n, double *Gr, long long ldr, double *Gi, long long ldi, double *Vr, long long lvr,
+                         double *Vi, long long lvi, const unsigned *pairs, int npairs, double tol, unsigned *cnt,
+                         cudaStream_t s)
+{
+  double *none = nullptr;
+  return cudaMemsetAsync(cnt, 0, 8, s) == cudaSuccess &&
+         host::launch_pdl(k_presweep<double, CPLX>, dim3((unsigned)npairs), dim3(256), 0, s, m, n, Gr, ldr, Gi, ldi, Vr,
+                          lvr, Vi, lvi, pairs, 0, tol, cnt, none, none) == cudaSuccess;
+}
+
 // squared 2-norms of the columns of planar G (one CTA per column)
 template <bool CPLX>
 __global__ void __launch_bounds__(256) k_colnorm2(int m, const double *Gr, long long ldr, const double *Gi,
@@ -602,8 +614,17 @@ __global__ void k_widen_cols(int n, const float *W, const int *perm, double *T)
 struct PairStats {
   unsigned long long cosmax, cosbound;  // largest |cos| and largest upper bound of one (bits of doubles)
   double f2;                            // squared Frobenius norm of the rotation generator
+  unsigned long long rowmax;            // its largest row sum (bits of a double)
   unsigned over, skipped;               // pairs above the tolerance; of those, not in the generator
+  unsigned listed;                      // the latter again, as they are listed
 };
+// v into *p when larger (bits of non-negative doubles); the plain read spares most of the atomics
+__device__ __forceinline__ void stat_max(unsigned long long *p, double v)
+{
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  if (b > *(volatile unsigned long long *)p)
+    atomicMax(p, b);
+}
 
 // Kernels on the lower triangle of an n x n Hermitian matrix and its mirror, 32 x 32 tiles:
 // thread (x, y) takes rows i = 32 blockIdx.x + x of columns j = 32 blockIdx.y + y + 8 k; f(i, j,
@@ -651,16 +672,21 @@ __global__ void __launch_bounds__(256) k_neg_upper(int n, Mat H, Mat M, PairStat
         if (M.im)
           M.im[(size_t)i * n + j] = v.y;
       });
-  atomicMax(&st->cosmax, (unsigned long long)__double_as_longlong(mx));
+  for (int o = 16; o >= 1; o >>= 1)
+    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (threadIdx.x == 0)
+    stat_max(&st->cosmax, mx);
 }
 
 // The generator K of the rotation exp(K) that makes the columns of G orthogonal to first order,
 // from the lower triangle of the Gram matrix H of the columns times 2^-e_j: K_ij = h_ij / (h_jj -
 // h_ii) in the columns' true lengths, stored as K~_ij = 2^(e_i - e_j) K_ij (the factor of column i
 // of length about 1 in column j of length about 1: never much larger than the cosine, however the
-// lengths differ). Pairs with |cos| below `tol` / 4 are left alone; pairs with |K_ij| > 2^-7 (nearly
-// equal lengths) too, and counted. hb: bound of the error of a Gram entry.
-__global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, Mat Kt, double tol, double hb, PairStats *st)
+// lengths differ). Pairs with |cos| below `tol` / 4 are left alone; pairs with |K_ij| > 2^-6 (nearly
+// equal lengths) too: they are counted, and the first `cap` of them go to list. rows: the row sums of
+// |K_ij|. hb: bound of the error of a Gram entry.
+__global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, Mat Kt, double tol, double hb,
+                                                   PairStats *st, double *rows, uint2 *list, unsigned cap)
 {
   double cm = 0, cb = 0, f2 = 0;
   unsigned over = 0, skipped = 0;
@@ -684,14 +710,22 @@ __global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, M
               const double di = scalbn(hj, 2 * d) - hi, dj = hj - scalbn(hi, -2 * d);
               // |K_ij| = a 2^d / |di|
               const double k = scalbn(a, d);
-              if (k <= 0.0078125 * fabs(di)) {
+              if (k <= 0.015625 * fabs(di)) {
                 kij = make_double2(hr / di, him / di);
                 kji = make_double2(-hr / dj, him / dj);
                 const double q = k / fabs(di);
                 f2 += 2.0 * q * q;
+                if (q > 1e-7) {  // (n smaller ones add at most 1e-7 n to a row sum)
+                  atomicAdd(rows + i, q);
+                  atomicAdd(rows + j, q);
+                }
               }
-              else if (c > tol)
+              else if (c > tol) {
                 ++skipped;
+                const unsigned at = atomicAdd(&st->listed, 1u);
+                if (at < cap)
+                  list[at] = make_uint2((unsigned)j, (unsigned)i);
+              }
             }
           }
         }
@@ -713,8 +747,8 @@ __global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, M
     skipped += __shfl_xor_sync(0xffffffffu, skipped, o);
   }
   if (threadIdx.x == 0 && blockIdx.y <= blockIdx.x) {
-    atomicMax(&st->cosmax, (unsigned long long)__double_as_longlong(cm));
-    atomicMax(&st->cosbound, (unsigned long long)__double_as_longlong(cb));
+    stat_max(&st->cosmax, cm);
+    stat_max(&st->cosbound, cb);
     if (f2 > 0)
       atomicAdd(&st->f2, f2);
     if (over)
@@ -722,6 +756,18 @@ __global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, M
     if (skipped)
       atomicAdd(&st->skipped, skipped);
   }
+}
+
+// the largest row sum of k_generator's rows
+__global__ void __launch_bounds__(1024) k_rowmax(int n, const double *rows, PairStats *st)
+{
+  double m = 0;
+  for (int i = threadIdx.x; i < n; i += 1024)
+    m = fmax(m, rows[i]);
+  for (int o = 16; o >= 1; o >>= 1)
+    m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if ((threadIdx.x & 31) == 0)
+    stat_max(&st->rowmax, m);
 }
 
 // y = a x + b y (y := a x when b is 0), n elements
@@ -1111,8 +1157,9 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   //    that makes them orthogonal to first order, N = exp(K) - I by its series, and G := G + G N,
   //    V := V + V N. What is left is of second order, so two refinements and the Gram matrix that
   //    confirms them replace the plain-dot FP64 sweeps (4096 x 2048 complex: 689 ms of sweeps).
-  //    Pairs of nearly equal norms, whose rotation is not small, are left out of K; they, and
-  //    whatever a refinement cannot improve, go to those sweeps, which run until no pair is left.
+  //    Pairs of nearly equal norms, whose rotation is not small, are rotated one by one before;
+  //    whatever that and a refinement cannot improve goes to the sweeps, which run until no pair
+  //    is left.
   bool certified = false;
   if (total32) {
     const double u = 1.1102230246251565e-16;
@@ -1123,66 +1170,103 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     unsigned sw64 = 0;
     bool sweeps = true;
     double before = 1e300;
-    for (unsigned it = 0; it < 8u && swp; ++it) {
-      oz::Operand oa, ob;
-      const Mat &H = M[0], &K = M[1], &P3 = M[2], &Q = M[3], &E = M[4];
-      // (5 digits give the first cosines, of the order of FP32 rounding, to about 1e-11)
-      const int nd = it ? 8 : 5;
-      if (!cut_cols(G, Gi, sc.ldr, sc.ldi, mi, oa) || !gram(oa, H, 0, nd) ||
-          cudaMemcpyAsync(ek, e1, (size_t)n * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
-          cudaMemsetAsync(st, 0, sizeof(PairStats), s) != cudaSuccess)
-        return VJ_ERR_CUDA;
+    constexpr unsigned CAP = 8192;  // pairs of nearly equal norms that are rotated one by one
+    uint2 *const list = reinterpret_cast<uint2 *>(d2);  // (free between the products)
+    double *const rows = vec;
+    const Mat &H = M[0], &K = M[1], &S = M[2], &Q = M[3], &E = M[4];
+    // the Gram matrix with nd digits, the generator and what it finds; columns' exponents in ek
+    auto survey = [&](int nd) {
+      oz::Operand oa;
       // digit pairs left out of the Gram entries: with 8 digits below 2^-62.8 per element of K
       const double hb = (nd == 8) ? (double)((long long)P * m) * 1.25e-19 : 1e300;
-      k_generator<<<tiles, tblk, 0, s>>>(ni, H, ek, K, tol64, hb, st);
-      if (!read_stats())
+      if (!cut_cols(G, Gi, sc.ldr, sc.ldi, mi, oa) || !gram(oa, H, 0, nd) ||
+          cudaMemcpyAsync(ek, e1, (size_t)n * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
+          cudaMemsetAsync(st, 0, sizeof(PairStats), s) != cudaSuccess ||
+          cudaMemsetAsync(rows, 0, (size_t)n * 8, s) != cudaSuccess)
+        return false;
+      k_generator<<<tiles, tblk, 0, s>>>(ni, H, ek, K, tol64, hb, st, rows, list, CAP);
+      k_rowmax<<<1, 1024, 0, s>>>(ni, rows, st);
+      return read_stats();
+    };
+    for (unsigned it = 0; it < 12u && swp; ++it) {
+      oz::Operand oa, ob;
+      // (5 digits give the first cosines, of the order of FP32 rounding, to about 1e-11)
+      const int nd = it ? 8 : 5;
+      if (!survey(nd))
         return VJ_ERR_CUDA;
-      const double cmax = asdbl(hst.cosmax), f = std::sqrt(hst.f2);
+      const double cmax = asdbl(hst.cosmax), f = std::min(std::sqrt(hst.f2), asdbl(hst.rowmax) + 1e-7 * (double)n);
       if (trace)
-        std::fprintf(stderr, "mixed SVD refinement %u: %u pairs above the tolerance, max |cos| %.3e, |K| %.2e, %u left out, "
-                     "%.1f ms since the phase began\n", it, hst.over, cmax, f, hst.skipped,
+        std::fprintf(stderr, "mixed SVD refinement %u: %u pairs above the tolerance, max |cos| %.3e, |K| <= %.2e, %u left "
+                     "out, %.1f ms since the phase began\n", it, hst.over, cmax, f, hst.skipped,
                      std::chrono::duration<double, std::milli>(now() - t0).count());
       if (nd == 8 && !hst.over && cmax <= tol64) {
         sweeps = false;
         certified = (asdbl(hst.cosbound) <= lim);
         break;
       }
-      // (K's series below is to sixth order: |K|^7 / 7! <= 2.5e-15 in the Frobenius norm, below the
-      // rounding of V's n^2 entries)
-      if (!(f <= 0.0277) || (hst.over && hst.over == hst.skipped) || !(cmax <= 0.25 * before))
+      if (hst.skipped) {
+        // pairs of nearly equal norms: rotate disjoint ones of them by their angles and look again
+        // (many of them are clusters, where the sweeps do better)
+        std::vector<uint2> hl(hst.skipped < CAP ? hst.skipped : CAP);
+        std::vector<unsigned> hp;
+        std::vector<char> used((size_t)n, 0);
+        if (hst.skipped > (unsigned)(n / 2) || hst.skipped > CAP || it == 11u ||
+            cudaMemcpyAsync(hl.data(), list, hl.size() * sizeof(uint2), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess)
+          break;
+        std::sort(hl.begin(), hl.end(), [](const uint2 &x, const uint2 &y) { return x.x != y.x ? x.x < y.x : x.y < y.y; });
+        for (const uint2 &q : hl)
+          if (!used[q.x] && !used[q.y]) {
+            used[q.x] = used[q.y] = 1;
+            hp.push_back(q.x);
+            hp.push_back(q.y);
+          }
+        unsigned *const dp = reinterpret_cast<unsigned *>(list);
+        if (cudaMemcpyAsync(dp, hp.data(), hp.size() * 4, cudaMemcpyHostToDevice, s) != cudaSuccess ||
+            !rotate_pairs<CPLX>(mi, ni, G, sc.ldr, Gi, sc.ldi, V, (long long)ldV, Vi, (long long)(CPLX ? ldVi : ldV), dp,
+                                (int)(hp.size() / 2), tol64, cnt, s) ||
+            cudaStreamSynchronize(s) != cudaSuccess)
+          return VJ_ERR_CUDA;
+        continue;
+      }
+      // (the series below is to eighth order: |K|^9 / 9! stays below rounding)
+      if (!(f <= 0.06) || !(cmax <= 0.25 * before))
         break;
       before = cmax;
-      const int terms = (f < 1e-8) ? 1 : (f < 6e-6) ? 2 : (f < 1.8e-4) ? 3 : (f < 1.4e-3) ? 4 : (f < 5.7e-3) ? 5 : 6;
+      // orders of the series: |K|^(order + 1) / (order + 1)! below 5e-17
+      const int order = (f < 1e-8) ? 1 : (f < 6e-6) ? 2 : (f < 1.8e-4) ? 3 : (f < 1.4e-3) ? 4 : (f < 5.7e-3) ? 5 : (f < 0.015) ? 6 : (f < 0.03) ? 7 : 8;
       const long long np = (long long)(P * nn);
       const unsigned gl = (unsigned)((np + 255) / 256 < 4096 ? (np + 255) / 256 : 4096);
       const int nk = digits(f * f), ng = digits(8.0 * cmax), nv = digits(f);  // for the powers of K, G N, V N
+      // exp(K) - I = E + O with E = K^2 (1/2! + K^2 (1/4! + ...)), O = K + K (K^2 (1/3! + K^2 (1/5! + ...)))
+      static const double inv[9] = {1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720, 1.0 / 5040, 1.0 / 40320};
       Mat Ev{nullptr, nullptr};
-      bool ok = true;
-      if (terms >= 2) {
-        // K^2 (in H's place)
-        ok = cut_rows(K.re, K.im, n, n, ni, nullptr, oa) && cut_prod(K, nullptr, ob) && mult(oa, ob, H, 0, nk);
-        k_lincomb<<<gl, 256, 0, s>>>(np, 0.5, H.re, 0.0, E.re);
+      if (order >= 2) {
+        const Mat &P2 = H;  // K^2 takes the Gram matrix's place
+        if (!cut_rows(K.re, K.im, n, n, ni, nullptr, oa) || !cut_prod(K, nullptr, ob) || !mult(oa, ob, P2, 0, nk))
+          return VJ_ERR_CUDA;
         Ev = E;
+        const int te = order & ~1, to = (order - 1) | 1;  // the last even and odd orders
+        const bool powers = te >= 4 || to >= 5;
+        if (powers && !cut_rows(P2.re, P2.im, n, n, ni, nullptr, oa))
+          return VJ_ERR_CUDA;
+        // X := c_last K^2, then X := c K^2 + K^2 X down to the order of `first`
+        auto horner = [&](const Mat &X, int last, int first) {
+          k_lincomb<<<gl, 256, 0, s>>>(np, inv[last], P2.re, 0.0, X.re);
+          for (int k = last - 2; k >= first; k -= 2) {
+            if (!cut_prod(X, nullptr, ob) || !mult(oa, ob, Q, 0, nk))
+              return false;
+            k_lincomb<<<gl, 256, 0, s>>>(np, inv[k], P2.re, 0.0, X.re);
+            k_lincomb<<<gl, 256, 0, s>>>(np, 1.0, Q.re, 1.0, X.re);
+          }
+          return true;
+        };
+        if (!horner(E, te, 2) || (to >= 3 && !horner(S, to, 3)))
+          return VJ_ERR_CUDA;
+        if (to >= 3 && (!cut_rows(K.re, K.im, n, n, ni, nullptr, oa) || !cut_prod(S, nullptr, ob) ||
+                        !mult(oa, ob, K, 1, nk)))
+          return VJ_ERR_CUDA;
       }
-      if (ok && terms >= 3) {
-        // K^3; the odd part K + K^3 / 6 takes K's place
-        ok = cut_prod(H, nullptr, ob) && mult(oa, ob, P3, 0, nk);
-        k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 6.0, P3.re, 1.0, K.re);
-      }
-      if (ok && terms >= 4) {
-        ok = cut_rows(H.re, H.im, n, n, ni, nullptr, oa) && mult(oa, ob, Q, 0, nk);  // K^4
-        k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 24.0, Q.re, 1.0, E.re);
-      }
-      if (ok && terms >= 5) {
-        ok = cut_prod(P3, nullptr, ob) && mult(oa, ob, Q, 0, nk);  // K^5
-        k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 120.0, Q.re, 1.0, K.re);
-      }
-      if (ok && terms >= 6) {
-        ok = cut_rows(P3.re, P3.im, n, n, ni, nullptr, oa) && mult(oa, ob, Q, 0, nk);  // K^6
-        k_lincomb<<<gl, 256, 0, s>>>(np, 1.0 / 720.0, Q.re, 1.0, E.re);
-      }
-      if (!ok)
-        return VJ_ERR_CUDA;
       k_exp_parts<<<tiles, tblk, 0, s>>>(ni, K, Ev, ek, Q);
       if (!cut_rows(G, Gi, sc.ldr, sc.ldi, mi, ek, oa) || !cut_prod(K, nullptr, ob) || !mult_g(oa, ob, ek, 1, ng) ||
           !cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, nullptr, oa) || !cut_prod(Q, nullptr, ob) ||
@@ -1190,10 +1274,6 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
         return VJ_ERR_CUDA;
       ++sw64;
     }
-    unsigned herr = 0;
-    if (cudaMemcpyAsync(&herr, gerr, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaStreamSynchronize(s) != cudaSuccess || herr)
-      return VJ_ERR_CUDA;
     // A sweep whose rotated pairs all had |cos| <= 1e-11 leaves off-diagonal terms of the
     // order of their squares (times n / relative gap), far below the tolerance: its
     // confirming sweep is skipped, the reference's sweep below confirms.
@@ -1213,6 +1293,16 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
       if (mu <= 1e-11f)
         break;
     }
+    // (the sweeps' result is certified by its Gram matrix, too)
+    if (sweeps && sw64) {
+      if (!survey(8))
+        return VJ_ERR_CUDA;
+      certified = (!hst.over && asdbl(hst.cosbound) <= lim);
+    }
+    unsigned herr = 0;
+    if (cudaMemcpyAsync(&herr, gerr, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        cudaStreamSynchronize(s) != cudaSuccess || herr)
+      return VJ_ERR_CUDA;
     if (presweeps)
       presweeps[1] = sw64;
     // columns in descending order of their norms, the order the reference's sweeps keep
