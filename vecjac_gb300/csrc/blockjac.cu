@@ -29,10 +29,12 @@
 
 #include <cmath>
 #include <cstdint>
+#include <cstdlib>
 #include <cstring>
 #include <vector>
 
 #include "svd_core.cuh"
+#include "pjs.cuh"
 #include "tc.cuh"
 #include "vj_host.h"
 
@@ -106,9 +108,18 @@ __device__ __forceinline__ float *pair_col(const Cols &X, int I, int J, int c)
   return base + (long long)col * X.ld;
 }
 
-// block pair k of block step s of the round-robin ordering of nb blocks (I < J)
+// block pair k (I < J) of block step s of the round-robin ordering of nb blocks, or of step s -
+// MODULUS of their modulus ordering
+constexpr int MODULUS = 1 << 24;
 __device__ __forceinline__ void block_pair(int nb, int s, int k, int &I, int &J)
 {
+  if (s >= MODULUS) {
+    unsigned p, q;
+    pair_mod((unsigned)nb, (unsigned)(s - MODULUS), (unsigned)k, p, q);
+    I = (int)p;
+    J = (int)q;
+    return;
+  }
   const int N = nb - 1;
   int a, c;
   if (k == 0) {
@@ -994,7 +1005,10 @@ long long block_sweep(bool cplx, int m, int n, float *Gr, float *Gi, long long l
   const Cols G{Gr, cplx ? Gi : nullptr, ldg, p.b}, W{Wr, cplx ? Wi : nullptr, ldw, p.b};
   if (cudaMemsetAsync(stats, 0, 16, s) != cudaSuccess)
     return -1;
-  for (int step = 0; step < p.nb - 1; ++step) {
+  const char *eo = getenv("VJ_BLOCK_ORD");
+  const bool mod = !(eo && *eo == '0');
+  for (int st = 0; st < (mod ? p.nb : p.nb - 1); ++st) {
+    const int step = mod ? MODULUS + st : st;
     if (terms == 3)
       k_gram<3><<<p.npairs * p.ksplit, 128, GRAM_SMEM, s>>>(G, m, p.nb, step, p.ksplit, Spart, stats + 2);
     else

@@ -49,6 +49,11 @@ long long block_sweep(bool cplx, int m, int n, float *Gr, float *Gi, long long l
                       long long ldw, unsigned char *scratch, unsigned *stats, float tol, int inner, int terms,
                       cudaStream_t s, float *mu);
 
+// defined in colblk.cu: sweeps by small blocks of columns, a CTA per pair of blocks
+int col_blocks(bool cplx, long long m, long long n);
+long long col_block_sweep(bool cplx, int m, int n, float *Gr, float *Gi, float *Wr, float *Wi, float tol, unsigned *cnt,
+                          cudaStream_t s, float *mu);
+
 // defined in jsvd.cu
 template <typename T, bool CPLX>
 vj_fint svd_dev_entry(vj_fnat m, vj_fnat n, T *G, vj_fnat ldG, T *Gi, vj_fnat ldGi, T *V, vj_fnat ldV, T *Vi,
@@ -885,6 +890,8 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   const char *eb = getenv("VJ_BLOCK");
   const bool blk = !(eb && *eb == '0') && block_sweeps_apply(CPLX, m, n, m) &&
                    ((eb && *eb == '1') || n >= (CPLX ? 1024 : 2048));
+  const char *ec = getenv("VJ_COLBLK");
+  const int ncol = (!(ec && *ec == '0') && !blk) ? col_blocks(CPLX, m, n) : 0;
   const char *et = getenv("VJ_BLOCK_TERMS");
   const int terms = (et && atoi(et) == 3) ? 3 : 6;
   const char *ei = getenv("VJ_BLOCK_INNER");
@@ -1034,13 +1041,17 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     unsigned sw = 0;
     const float stop = 4.f * tol;
     const long long nbk = n / (CPLX ? 32 : 64), hw = CPLX ? 32 : 64;
-    const double every = blk ? (double)(nbk - 1) * (double)(nbk / 2) * inner * (double)(2 * hw - 1) * (double)hw
+    const long long cbn = ncol ? n / (ncol / 2) : 0;
+    const double every = ncol ? (double)cbn * (double)(cbn / 2) * (double)ncol * (double)(ncol / 2)
+                         : blk ? (double)(nbk - 1) * (double)(nbk / 2) * inner * (double)(2 * hw - 1) * (double)hw
                              : (double)stp * (double)(n / 2);
     for (; sw < maxsw; ++sw) {
       float mu = 0.f;
       const long long hc =
           blk ? block_sweep(CPLX, mi, ni, G32, CPLX ? G32 + mn : nullptr, m, W32, CPLX ? W32 + nn : nullptr, n, bscr,
                             cnt, tol, inner, terms, s, &mu)
+          : ncol ? col_block_sweep(CPLX, mi, ni, G32, CPLX ? G32 + mn : nullptr, W32, CPLX ? W32 + nn : nullptr, tol, cnt,
+                                   s, &mu)
               : presweep<float, CPLX>(mi, ni, G32, m, CPLX ? G32 + mn : nullptr, m, W32, n, CPLX ? W32 + nn : nullptr,
                                       n, js, stp, tol, cnt, s, &mu);
       if (hc < 0)

@@ -101,7 +101,7 @@ __device__ __forceinline__ void dot_acc(const FpOps<T> &o, T pd, T dn, T &s, T &
   sum_step(o, dn, s_, t_);
 }
 
-#ifdef __CUDA_ARCH__
+#ifdef __CUDACC__
 // Two FP32 values in one register pair and the packed operations on them (each half rounded
 // like the scalar operation): half the instructions of two recurrences that run in step.
 struct F32x2 {
