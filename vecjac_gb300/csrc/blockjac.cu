@@ -29,7 +29,6 @@
 
 #include <cmath>
 #include <cstdint>
-#include <cstdlib>
 #include <cstring>
 #include <vector>
 
@@ -579,8 +578,8 @@ __device__ __forceinline__ Rot pair_rot(float ha, float hb, float cr, float ci, 
 // ends the step.
 constexpr int EVD_THREADS = 256;
 template <bool CPLX>
-__global__ void __launch_bounds__(EVD_THREADS) k_pair_evd(const float *Sred, int sweeps, float tol, float4 *rlog,
-                                                          int *rranks, unsigned *stats)
+__global__ void __launch_bounds__(EVD_THREADS) k_pair_evd(const float *Sred, int sweeps, int cross, float tol,
+                                                          float4 *rlog, int *rranks, unsigned *stats)
 {
   using E = typename std::conditional<CPLX, float2, float>::type;
   constexpr int N = CPLX ? 64 : 128;  // order of H
@@ -605,7 +604,9 @@ __global__ void __launch_bounds__(EVD_THREADS) k_pair_evd(const float *Sred, int
     if (u < v)
       tri[u * P - u * (u + 1) / 2 + (v - u - 1)] = (unsigned short)((u << 8) | v);
   }
-  float4 *lg = rlog + (size_t)blockIdx.x * sweeps * (N - 1) * P;
+  // the steps of a sweep: every pair (round-robin), or only those between the two blocks
+  const int nsteps = cross ? P : N - 1;
+  float4 *lg = rlog + (size_t)blockIdx.x * sweeps * nsteps * P;
   // H from S; only the upper triangle of H is stored (an entry (i, j) with i > j is the
   // conjugate of the stored (j, i)), so that an update writes each entry once
   for (int q = tid; q < N * N; q += EVD_THREADS) {
@@ -645,7 +646,7 @@ __global__ void __launch_bounds__(EVD_THREADS) k_pair_evd(const float *Sred, int
   unsigned nrot = 0u;
   float mu = 0.f;
   for (int sw = 0; sw < sweeps; ++sw)
-    for (int stp = 0; stp < N - 1; ++stp) {
+    for (int stp = 0; stp < nsteps; ++stp) {
       // the step's pairs, their rotations and new diagonal blocks (warp 0; lane u: pairs
       // u, u + 32)
       if (warp == 0) {
@@ -653,7 +654,11 @@ __global__ void __launch_bounds__(EVD_THREADS) k_pair_evd(const float *Sred, int
         for (int h = 0; h < PL; ++h) {
           const int u = lane + 32 * h;
           int a, c;
-          if (u == 0) {
+          if (cross) {
+            a = u;
+            c = P + ((u + stp) & (P - 1));
+          }
+          else if (u == 0) {
             a = stp;
             c = N - 1;
           }
@@ -681,7 +686,7 @@ __global__ void __launch_bounds__(EVD_THREADS) k_pair_evd(const float *Sred, int
           const float4 rec =
               act ? make_float4(r.c, r.sr, r.si, __uint_as_float(tag)) : make_float4(1.f, 0.f, 0.f, __uint_as_float(tag));
           rot[u] = rec;
-          lg[(size_t)(sw * (N - 1) + stp) * P + u] = rec;
+          lg[(size_t)(sw * nsteps + stp) * P + u] = rec;
           if (act) {
             if constexpr (CPLX) {
               H[p * LD + p] = make_float2(r.d1, 0.f);
@@ -799,7 +804,7 @@ template <bool CPLX> static size_t br_smem()
   return (size_t)C::ROWS * C::LD * (CPLX ? 8 : 4) + (size_t)C::CHUNK * (C::N / 2) * 16 + (size_t)C::N * 4;
 }
 template <bool CPLX>
-__global__ void __launch_bounds__(BR_THREADS) k_build_r(const float4 *rlog, const int *rranks, int sweeps,
+__global__ void __launch_bounds__(BR_THREADS) k_build_r(const float4 *rlog, const int *rranks, int steps,
                                                         unsigned char *Rimg)
 {
   using E = typename std::conditional<CPLX, float2, float>::type;
@@ -812,7 +817,6 @@ __global__ void __launch_bounds__(BR_THREADS) k_build_r(const float4 *rlog, cons
   int *rank = reinterpret_cast<int *>(lg + CH * P);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int pair = blockIdx.x / BR_PARTS, r0 = (blockIdx.x % BR_PARTS) * ROWS;
-  const int steps = sweeps * (N - 1);
   const float4 *src = rlog + (size_t)pair * steps * P;
   for (int i = tid; i < N; i += BR_THREADS)
     rank[i] = rranks[(size_t)pair * N + i];
@@ -984,14 +988,19 @@ size_t block_sweep_scratch(bool cplx, long long m, long long n, int inner)
          rlog_records(cplx, p.npairs, inner) * 16 + (size_t)p.npairs * (cplx ? 64 : 128) * 4 + 256;
 }
 
-// One block sweep (nb - 1 block steps) on planar FP32 G (m x n) and W (n x n), both with
+// One block sweep on planar FP32 G (m x n) and W (n x n), both with
 // the given leading dimensions. scratch: block_sweep_scratch bytes; stats: 4 device words
 // (zeroed here; [0] rotations, [1] max scaled |h_pq| of a rotated pair as float bits, [2]
 // error flag). terms: 6 (FP32-accurate products) or 3. Returns rotations, or -1 (launch
-// failure or a kernel whose wait gave up).
+// failure or a kernel whose wait gave up). fast: the blocks in modulus order (nb block steps instead
+// of the round-robin's nb - 1, and about half as many sweeps: at 4096 x 2048 complex 7 + 4 instead
+// of 13 + 4), and, real data, after the first block step, which takes every block once, only the pairs between a
+// pair's two blocks in its eigenproblem: half of its Jacobi steps for about a fifth more sweeps
+// (4096 x 2048 real FP32 stages 133 -> 102 ms; complex 136 -> 148 ms, whose eigenproblem is half as
+// long).
 long long block_sweep(bool cplx, int m, int n, float *Gr, float *Gi, long long ldg, float *Wr, float *Wi,
                       long long ldw, unsigned char *scratch, unsigned *stats, float tol, int inner, int terms,
-                      cudaStream_t s, float *mu)
+                      bool fast, cudaStream_t s, float *mu)
 {
   using namespace bj;
   if (!attrs_set(cplx))
@@ -1005,22 +1014,21 @@ long long block_sweep(bool cplx, int m, int n, float *Gr, float *Gi, long long l
   const Cols G{Gr, cplx ? Gi : nullptr, ldg, p.b}, W{Wr, cplx ? Wi : nullptr, ldw, p.b};
   if (cudaMemsetAsync(stats, 0, 16, s) != cudaSuccess)
     return -1;
-  const char *eo = getenv("VJ_BLOCK_ORD");
-  const bool mod = !(eo && *eo == '0');
-  for (int st = 0; st < (mod ? p.nb : p.nb - 1); ++st) {
-    const int step = mod ? MODULUS + st : st;
+  for (int st = 0; st < (fast ? p.nb : p.nb - 1); ++st) {
+    const int step = fast ? MODULUS + st : st, cross = (fast && st && !cplx) ? 1 : 0;
+    const int jsteps = inner * (cross ? (cplx ? 32 : 64) : (cplx ? 63 : 127));
     if (terms == 3)
       k_gram<3><<<p.npairs * p.ksplit, 128, GRAM_SMEM, s>>>(G, m, p.nb, step, p.ksplit, Spart, stats + 2);
     else
       k_gram<6><<<p.npairs * p.ksplit, 128, GRAM_SMEM, s>>>(G, m, p.nb, step, p.ksplit, Spart, stats + 2);
     k_gram_reduce<<<p.npairs * 16, 256, 0, s>>>(Spart, p.ksplit, Sred);
     if (cplx) {
-      k_pair_evd<true><<<p.npairs, EVD_THREADS, evd_smem(true), s>>>(Sred, inner, tol, rlog, rranks, stats);
-      k_build_r<true><<<p.npairs * BR_PARTS, BR_THREADS, br_smem<true>(), s>>>(rlog, rranks, inner, Rimg);
+      k_pair_evd<true><<<p.npairs, EVD_THREADS, evd_smem(true), s>>>(Sred, inner, cross, tol, rlog, rranks, stats);
+      k_build_r<true><<<p.npairs * BR_PARTS, BR_THREADS, br_smem<true>(), s>>>(rlog, rranks, jsteps, Rimg);
     }
     else {
-      k_pair_evd<false><<<p.npairs, EVD_THREADS, evd_smem(false), s>>>(Sred, inner, tol, rlog, rranks, stats);
-      k_build_r<false><<<p.npairs * BR_PARTS, BR_THREADS, br_smem<false>(), s>>>(rlog, rranks, inner, Rimg);
+      k_pair_evd<false><<<p.npairs, EVD_THREADS, evd_smem(false), s>>>(Sred, inner, cross, tol, rlog, rranks, stats);
+      k_build_r<false><<<p.npairs * BR_PARTS, BR_THREADS, br_smem<false>(), s>>>(rlog, rranks, jsteps, Rimg);
     }
     if (terms == 3)
       k_apply<3><<<p.npairs * p.q, APPLY_THREADS, APPLY_SMEM, s>>>(G, m, W, n, p.nb, step, p.tg, p.tw, p.q, Rimg,
@@ -1156,7 +1164,7 @@ extern "C" vj_fint vj_block_sweep_dev(int cplx, vj_fnat m, vj_fnat n, float *Gr,
   }
   float mu_ = 0.f;
   const long long r = block_sweep(cplx != 0, (int)m, (int)n, Gr, Gi, (long long)ldG, Wr, Wi, (long long)ldW, scr,
-                                  stats, tol, inner, terms, (cudaStream_t)stream, &mu_);
+                                  stats, tol, inner, terms, false, (cudaStream_t)stream, &mu_);
   cudaFree(scr);
   cudaFree(stats);
   if (mu)

@@ -1,6 +1,6 @@
-// FP32 one-sided Jacobi sweeps by small blocks of columns, one CTA per pair of blocks: the FP32
-// stages of the mixed-precision SVD (mixed.cu) for matrices whose pair of blocks fits in a
-// CTA's shared memory.
+// FP32 one-sided Jacobi sweeps by small blocks of columns, a CTA or a small cluster per pair of
+// blocks: the FP32 stages of the mixed-precision SVD (mixed.cu) for matrices whose pair of blocks
+// fits in shared memory.
 //
 // A sweep of column pairs is n pivot steps of 2-4 us that are launch, load and reduction
 // latency (3.5 us per step at 1024 x 1024 real, 512 CTAs of one pair each). Here the n columns are
@@ -8,10 +8,13 @@
 // of blocks: it copies their 2b columns of G and of the rotation accumulator W into shared memory
 // (bulk copies; W's arrive during the eigenproblem), forms the 2b x 2b Gram matrix of G's (all
 // warps, rows over threads, a lane's partial sums of all entries in registers), runs one cyclic
-// two-sided Jacobi sweep on it, accumulating the rotation R, and writes G R and W R. A sweep is
+// two-sided Jacobi sweep (over the pairs between the blocks only, but for the first step) on it,
+// accumulating the rotation R, and writes G R and W R. A sweep is
 // n / b such steps (modulus ordering of the blocks and inside them, with the longer column first:
 // it needs half as many sweeps as the round-robin ordering), so the per-step latencies are paid
-// n / b instead of n times. FP32 Gram entries are as accurate relative to the column
+// n / b instead of n times. Where the pairs leave SMs idle, or their columns need more shared
+// memory, the CTAs of a cluster split the rows: each adds up the partial Gram sums of all of them
+// in the same order, solves the same eigenproblem and rotates its own rows. FP32 Gram entries are as accurate relative to the column
 // norms as the dot products of a column pair; the sweeps precondition the FP64 phases, which
 // decide the result.
 #include <cuda_runtime.h>
@@ -27,7 +30,7 @@ namespace vj {
 namespace cb {
 
 constexpr int NT = 256;
-constexpr size_t SMEM_MAX = 208 * 1024;
+constexpr size_t SMEM_MAX = 204 * 1024;
 
 struct Args {
   float *Gr, *Gi, *Wr, *Wi;  // leading dimensions m and n
@@ -69,15 +72,24 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
   constexpr int NH = NC * (NC + 1) / 2;                      // entries of the upper triangle
   constexpr int NA = CPLX ? NC + 2 * (NH - NC) : NH;         // real sums: diagonal, then pairs (re, im)
   extern __shared__ __align__(128) float X[];                // plane, column, m rows of G and n of W
-  __shared__ float part[NT / 32][NA];
+  __shared__ float part[NT / 32][NA], total[NA], gram[NA];
   __shared__ float Hr[2][NC][NC + 1], Hi[2][CPLX ? NC : 1][NC + 1];  // (this step's and the next's)
   __shared__ __align__(16) float Rr[NC][NC], Ri[CPLX ? NC : 1][NC];
+  __shared__ unsigned short ptab[NC][B];  // p | q << 8 of pair u of a step
   __shared__ unsigned long long bar[2];
   __shared__ unsigned s_rot, s_mu;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  const int m = a.m, n = a.n;
+  unsigned rank, cs;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(cs));
+  const int pairno = (int)(blockIdx.x / cs);
+  // this CTA's rows of G and of W, in groups of four
+  const int g0 = (int)((long long)(m >> 2) * rank / cs), g1 = (int)((long long)(m >> 2) * (rank + 1) / cs);
+  const int w0 = (int)((long long)(n >> 2) * rank / cs), w1 = (int)((long long)(n >> 2) * (rank + 1) / cs);
+  const int gq = g1 - g0, wq = w1 - w0, rows = 4 * (gq + wq);
   unsigned I, J;
-  pair_mod((unsigned)a.nb, (unsigned)a.step, blockIdx.x, I, J);
-  const int m = a.m, n = a.n, rows = m + n;
+  pair_mod((unsigned)a.nb, (unsigned)a.step, (unsigned)pairno, I, J);
   auto col = [&](int c) { return (c < B) ? (int)I * B + c : (int)J * B + (c - B); };
   auto xcol = [&](int pl, int c) { return X + (size_t)(pl * NC + c) * rows; };
   if (tid == 0) {
@@ -88,18 +100,30 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
   __syncthreads();
   pdl_enter();
   if (tid == 0) {
-    mbar_expect_tx(&bar[0], (unsigned)(NC * P * m * 4));
-    for (int c = 0; c < NC; ++c) {
-      tma_load_1d(xcol(0, c), a.Gr + (size_t)col(c) * m, (unsigned)(m * 4), &bar[0]);
+    mbar_expect_tx(&bar[0], (unsigned)(NC * P * gq * 16));
+    for (int c = 0; c < NC && gq; ++c) {
+      tma_load_1d(xcol(0, c), a.Gr + (size_t)col(c) * m + 4 * g0, (unsigned)(gq * 16), &bar[0]);
       if (CPLX)
-        tma_load_1d(xcol(1, c), a.Gi + (size_t)col(c) * m, (unsigned)(m * 4), &bar[0]);
+        tma_load_1d(xcol(1, c), a.Gi + (size_t)col(c) * m + 4 * g0, (unsigned)(gq * 16), &bar[0]);
     }
-    mbar_expect_tx(&bar[1], (unsigned)(NC * P * n * 4));
-    for (int c = 0; c < NC; ++c) {
-      tma_load_1d(xcol(0, c) + m, a.Wr + (size_t)col(c) * n, (unsigned)(n * 4), &bar[1]);
+    mbar_expect_tx(&bar[1], (unsigned)(NC * P * wq * 16));
+    for (int c = 0; c < NC && wq; ++c) {
+      tma_load_1d(xcol(0, c) + 4 * gq, a.Wr + (size_t)col(c) * n + 4 * w0, (unsigned)(wq * 16), &bar[1]);
       if (CPLX)
-        tma_load_1d(xcol(1, c) + m, a.Wi + (size_t)col(c) * n, (unsigned)(n * 4), &bar[1]);
+        tma_load_1d(xcol(1, c) + 4 * gq, a.Wi + (size_t)col(c) * n + 4 * w0, (unsigned)(wq * 16), &bar[1]);
     }
+  }
+  // every pair of the columns in the first step of a sweep (which takes every block once), the pairs
+  // between the two blocks in the others: half of the Jacobi steps, and no more sweeps
+  const int nst = a.step ? B : NC;
+  if (tid < NC * B) {
+    unsigned p, q;
+    pair_mod(NC, (unsigned)(tid / B), (unsigned)(tid % B), p, q);
+    if (nst == B) {
+      p = tid % B;
+      q = B + (tid % B + tid / B) % B;
+    }
+    ptab[tid / B][tid % B] = (unsigned short)(p | (q << 8));
   }
   bool ok = mbar_wait_bounded(&bar[0]);
   // ---- Gram matrix: rows over threads, four at a time ----
@@ -108,7 +132,7 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
 #pragma unroll
     for (int i = 0; i < NA; ++i)
       acc[i] = 0.0f;
-    for (int g = tid; g < (m >> 2); g += NT) {
+    for (int g = tid; g < gq; g += NT) {
       float4 xr[NC], xi[CPLX ? NC : 1];
 #pragma unroll
       for (int c = 0; c < NC; ++c) {
@@ -153,20 +177,52 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
     }
     warp_sums<NA>(acc, part[warp]);
   }
+  if (cs > 1) {
+    // every CTA's sums to every CTA; the same sums in the same order everywhere
+    __syncthreads();
+    for (int e = tid; e < NA; e += NT) {
+      float t = 0.0f;
+      for (int w = 0; w < NT / 32; ++w)
+        t += part[w][e];
+      total[e] = t;
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    for (int e = tid; e < NA; e += NT) {
+      float t = 0.0f;
+      for (unsigned r = 0; r < cs; ++r) {
+        unsigned addr;
+        float v;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"(smem_u32(&total[e])), "r"(r));
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+        t += v;
+      }
+      gram[e] = t;
+    }
+    // (no CTA leaves, or writes its sums again, before all have read them: waited for at the end)
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  }
+  else {
+    __syncthreads();
+    for (int e = tid; e < NA; e += NT) {
+      float t = 0.0f;
+      for (int w = 0; w < NT / 32; ++w)
+        t += part[w][e];
+      gram[e] = t;
+    }
+  }
+  auto leave = [&]() {
+    if (cs > 1)
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  };
   __syncthreads();
   for (int q = tid; q < NC * NC; q += NT) {
     const int i = q / NC, j = q % NC;
     if (i <= j) {
       const int u = i * NC - i * (i + 1) / 2 + (j - i - 1);  // pair (i, j) among the pairs
       const int e = (i == j) ? i : NC + (CPLX ? 2 : 1) * u;
-      float s = 0.0f, t = 0.0f;
-      for (int w = 0; w < NT / 32; ++w) {
-        s += part[w][e];
-        if (CPLX && i != j)
-          t += part[w][e + 1];
-      }
-      Hr[0][i][j] = Hr[0][j][i] = s;
+      Hr[0][i][j] = Hr[0][j][i] = gram[e];
       if (CPLX) {
+        const float t = (i != j) ? gram[e + 1] : 0.0f;
         Hi[0][CPLX ? i : 0][j] = t;
         Hi[0][CPLX ? j : 0][i] = -t;
       }
@@ -185,29 +241,32 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
     float cs, sr, si;  // cosine, sine times e^{i phi}
     bool go, sw;       // rotated; the second new column is the longer one and goes first
   };
-  float mu = 0.0f;
+  const float tol2 = a.tol * a.tol;
+  float mu2 = 0.0f;
   unsigned nrot = 0u;
-  for (int st = 0; st < NC; ++st) {
+  for (int st = 0; st < nst; ++st) {
     const int cur = st & 1;
-    // the rotation of pair (p, q): t^2 + 2 zeta t - 1 = 0, zeta = (b - a) / (2 |c|)
-    auto rotation = [&](int p, int q, float *cosine) {
+    // the rotation of pair (p, q): with d = b - a and w = sqrt(d^2 + 4 |c|^2), cs^2 = (1 + |d| / w) / 2
+    // and the sine times e^{i phi} sign(d) c / (w cs); two reciprocal roots, refined by a Newton
+    // step each, as the dependent operations of a step are all that counts here
+    auto rotation = [&](int p, int q, float *cos2) {
       const float ha = Hr[cur][p][p], hb = Hr[cur][q][q], cr = Hr[cur][p][q], ci = CPLX ? Hi[cur][CPLX ? p : 0][q] : 0.0f;
-      Rotation r{1.0f, 0.0f, 0.0f, false, false};
-      // (in terms of the cosine, so that short columns' squares do not underflow)
-      const float ra = rsqrtf(ha), rb = rsqrtf(hb), xr = cr * ra * rb, xi = CPLX ? ci * ra * rb : 0.0f;
+      // (c and d over sqrt(a b): squares of short columns' entries would leave the range)
+      const float ir = rsqrtf(ha) * rsqrtf(hb), xr = cr * ir, xi = ci * ir, d = (hb - ha) * ir;
       const float c2 = CPLX ? __fmaf_rn(xr, xr, xi * xi) : xr * xr;
-      if (ha > 0.0f && hb > 0.0f && c2 >= a.tol * a.tol) {
-        const float ic = rsqrtf(c2), zeta = 0.5f * (hb - ha) * ra * rb * ic, az = fabsf(zeta);
-        const float t = (az > 1e15f) ? __fdividef(0.5f, zeta)
-                                     : copysignf(__fdividef(1.0f, az + sqrtf(__fmaf_rn(az, az, 1.0f))), zeta);
-        const float d = __fmaf_rn(t, t, 1.0f), ac = c2 * ic * (ha * ra) * (hb * rb);
-        float cs = rsqrtf(d);
-        cs = __fmaf_rn(cs * 0.5f, __fmaf_rn(-d * cs, cs, 1.0f), cs);
-        const float sn = t * cs * ic;
-        r = Rotation{cs, sn * xr, CPLX ? sn * xi : 0.0f, true, hb + t * ac > ha - t * ac};
-        if (cosine)
-          *cosine = c2 * ic;
-      }
+      // (no branch: what a pair that is not rotated computes is dropped at the end)
+      const bool go = ha > 0.0f && hb > 0.0f && c2 >= tol2 && fabsf(d) < 1e18f;
+      const float w2 = __fmaf_rn(d, d, 4.0f * c2);
+      float iw = rsqrtf(w2);
+      iw = __fmaf_rn(0.5f * iw, __fmaf_rn(-w2 * iw, iw, 1.0f), iw);
+      const float u = __fmaf_rn(0.5f * fabsf(d), iw, 0.5f);
+      float iu = rsqrtf(u);
+      iu = __fmaf_rn(0.5f * iu, __fmaf_rn(-u * iu, iu, 1.0f), iu);
+      const float k = go ? copysignf(iw * iu, d) : 0.0f;
+      // (the new norms are a - t |c| and b + t |c| with t of d's sign: the longer stays the longer)
+      const Rotation r{go ? u * iu : 1.0f, go ? k * xr : 0.0f, (CPLX && go) ? k * xi : 0.0f, go, go && d >= 0.0f};
+      if (cos2)
+        *cos2 = go ? c2 : 0.0f;
       return r;
     };
     // (x, y) <- (cs x - conj(s) y, cs y + s x), exchanged when the second is the longer
@@ -228,20 +287,18 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
     };
     if (tid < B * B) {
       const int u = tid / B, v = tid % B;
-      unsigned pu, qu, pv, qv;
-      pair_mod(NC, (unsigned)st, (unsigned)u, pu, qu);
-      pair_mod(NC, (unsigned)st, (unsigned)v, pv, qv);
-      float cosine = 0.0f;
-      const Rotation rv = rotation((int)pv, (int)qv, (u == v) ? &cosine : nullptr);
-      Rotation ru = rotation((int)pu, (int)qu, nullptr);
-      if (u == v) {
-        nrot += rv.go ? 1u : 0u;
-        mu = fmaxf(mu, cosine);
-      }
+      const unsigned tu = ptab[st][u], tv = ptab[st][v], pu = tu & 255u, qu = tu >> 8, pv = tv & 255u, qv = tv >> 8;
       auto h = [&](unsigned i, unsigned j) {
         return make_float2(Hr[cur][i][j], CPLX ? Hi[cur][CPLX ? i : 0][j] : 0.0f);
       };
       float2 b00 = h(pu, pv), b01 = h(pu, qv), b10 = h(qu, pv), b11 = h(qu, qv);
+      float cosine = 0.0f;
+      const Rotation rv = rotation((int)pv, (int)qv, &cosine);
+      Rotation ru = rotation((int)pu, (int)qu, nullptr);
+      if (u == v) {
+        nrot += rv.go ? 1u : 0u;
+        mu2 = fmaxf(mu2, cosine);
+      }
       turn(rv, b00, b01);
       turn(rv, b10, b11);
       ru.si = -ru.si;  // rows: the conjugate
@@ -259,8 +316,7 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
     }
     else if (tid < B * B + NC * B) {
       const int w = tid - B * B, u = w % B, i = w / B;
-      unsigned p, q;
-      pair_mod(NC, (unsigned)st, (unsigned)u, p, q);
+      const unsigned t = ptab[st][u], p = t & 255u, q = t >> 8;
       const Rotation r = rotation((int)p, (int)q, nullptr);
       if (r.go) {
         float2 x = make_float2(Rr[i][p], CPLX ? Ri[CPLX ? i : 0][p] : 0.0f),
@@ -278,7 +334,7 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
   }
   if (nrot) {
     atomicAdd(&s_rot, nrot);
-    atomicMax(&s_mu, __float_as_uint(mu));
+    atomicMax(&s_mu, __float_as_uint(sqrtf(mu2)));
   }
   ok = mbar_wait_bounded(&bar[1]) && ok;
   if (!__syncthreads_and(ok)) {
@@ -287,17 +343,20 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
       atomicOr(a.cnt + 2, 1u);
     (void)mbar_wait_bounded(&bar[0]);
     (void)mbar_wait_bounded(&bar[1]);
+    leave();
     return;
   }
-  if (!s_rot)
+  if (!s_rot) {
+    leave();
     return;
-  if (tid == 0) {
+  }
+  if (tid == 0 && rank == 0) {
     atomicAdd(a.cnt, s_rot);
     atomicMax(a.cnt + 1, s_mu);
   }
   // ---- G R and W R: four rows per thread ----
-  for (int g = tid; g < (rows >> 2); g += NT) {
-    const bool isg = g < (m >> 2);
+  for (int g = tid; g < gq + wq; g += NT) {
+    const bool isg = g < gq;
     F32x2 o[CPLX ? 2 : 1][NC][2];
 #pragma unroll
     for (int pl = 0; pl < P; ++pl)
@@ -342,7 +401,7 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
       }
     }
     const size_t ld = isg ? (size_t)m : (size_t)n;
-    const int r4 = isg ? g : g - (m >> 2);
+    const int r4 = isg ? g0 + g : w0 + g - gq;
 #pragma unroll
     for (int pl = 0; pl < P; ++pl) {
       float *const base = isg ? (pl ? a.Gi : a.Gr) : (pl ? a.Wi : a.Wr);
@@ -355,38 +414,71 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
       }
     }
   }
+  leave();
 }
 
-static size_t smem(bool cplx, int nc, long long m, long long n) { return (size_t)nc * (cplx ? 2u : 1u) * (size_t)(m + n) * 4u; }
+// a CTA's share of the columns of a pair of blocks
+static size_t smem(bool cplx, int nc, int cs, long long m, long long n)
+{
+  return (size_t)nc * (cplx ? 2u : 1u) * 16u * (size_t)((m / 4 + cs - 1) / cs + (n / 4 + cs - 1) / cs);
+}
+
+struct Shape {
+  int nc, cs;  // columns per pair of blocks (0: not for this shape), CTAs per pair
+};
+// As wide blocks as shared memory allows a cluster; two CTAs per pair where that keeps all of a step's
+// on the GPU at once, or as many as shared memory asks for.
+static Shape shape(bool cplx, long long m, long long n)
+{
+  if ((m & 3) || (n & 3))
+    return Shape{0, 0};
+  const int sms = host::sm_count();
+  for (int nc = cplx ? 8 : 16; nc >= (cplx ? 4 : 8); nc >>= 1) {
+    if (n % nc)
+      continue;
+    // (more than two CTAs per pair only for room: the exchange of the sums costs what they save)
+    int cs = ((n / nc) * 2 <= sms) ? 2 : 1;
+    while (cs < 8 && smem(cplx, nc, cs, m, n) > SMEM_MAX)
+      cs *= 2;
+    if (smem(cplx, nc, cs, m, n) <= SMEM_MAX)
+      return Shape{nc, cs};
+  }
+  return Shape{0, 0};
+}
 
 }  // namespace cb
 
-// columns per block pair of the small-block sweeps for this shape, or 0 when they do not apply:
-// whole blocks, at least two of them, and a pair's columns within a CTA's shared memory
-int col_blocks(bool cplx, long long m, long long n)
-{
-  if ((m & 3) || (n & 3))
-    return 0;
-  for (int nc = cplx ? 8 : 16; nc >= (cplx ? 4 : 8); nc >>= 1)
-    if (n % nc == 0 && cb::smem(cplx, nc, m, n) <= cb::SMEM_MAX)
-      return nc;
-  return 0;
-}
+// columns per block pair of the small-block sweeps for this shape, or 0 when they do not apply
+int col_blocks(bool cplx, long long m, long long n) { return cb::shape(cplx, m, n).nc; }
 
 // one block sweep; the number of rotations (< 0: an error) and the largest |cos| of a rotated pair
 long long col_block_sweep(bool cplx, int m, int n, float *Gr, float *Gi, float *Wr, float *Wi, float tol, unsigned *cnt,
                           cudaStream_t s, float *mu)
 {
-  const int nc = col_blocks(cplx, m, n);
+  const cb::Shape sh = cb::shape(cplx, m, n);
+  const int nc = sh.nc;
   void (*const k)(cb::Args) = cplx ? (nc == 8 ? cb::k_col_blocks<true, 8> : cb::k_col_blocks<true, 4>)
                                    : (nc == 16 ? cb::k_col_blocks<false, 16> : cb::k_col_blocks<false, 8>);
-  const size_t sm = cb::smem(cplx, nc, m, n);
+  const size_t sm = cb::smem(cplx, nc ? nc : 4, sh.cs ? sh.cs : 1, m, n);
   if (!nc || cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm) != cudaSuccess ||
       cudaMemsetAsync(cnt, 0, 12, s) != cudaSuccess)
     return -1;
   cb::Args a{Gr, Gi, Wr, Wi, m, n, n / (nc / 2), 0, tol, cnt};
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  at[1].id = cudaLaunchAttributeClusterDimension;
+  at[1].val.clusterDim.x = (unsigned)sh.cs;
+  at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
+  cfg.gridDim = dim3((unsigned)(a.nb / 2 * sh.cs));
+  cfg.blockDim = dim3(cb::NT);
+  cfg.dynamicSmemBytes = sm;
+  cfg.stream = s;
   for (a.step = 0; a.step < a.nb; ++a.step)
-    if (host::launch_pdl(k, dim3((unsigned)(a.nb / 2)), dim3(cb::NT), sm, s, a) != cudaSuccess)
+    if (cudaLaunchKernelEx(&cfg, k, a) != cudaSuccess)
       return -1;
   unsigned hc[3] = {0u, 0u, 1u};
   if (cudaGetLastError() != cudaSuccess || cudaMemcpyAsync(hc, cnt, 12, cudaMemcpyDeviceToHost, s) != cudaSuccess ||

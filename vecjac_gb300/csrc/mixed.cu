@@ -47,7 +47,7 @@ bool block_sweeps_apply(bool cplx, long long m, long long n, long long ld);
 size_t block_sweep_scratch(bool cplx, long long m, long long n, int inner);
 long long block_sweep(bool cplx, int m, int n, float *Gr, float *Gi, long long ldg, float *Wr, float *Wi,
                       long long ldw, unsigned char *scratch, unsigned *stats, float tol, int inner, int terms,
-                      cudaStream_t s, float *mu);
+                      bool fast, cudaStream_t s, float *mu);
 
 // defined in colblk.cu: sweeps by small blocks of columns, a CTA per pair of blocks
 int col_blocks(bool cplx, long long m, long long n);
@@ -880,18 +880,18 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     return VJ_ERR_NO_GPU;
   const int P = CPLX ? 2 : 1;
   const size_t mn = (size_t)m * n, nn = (size_t)n * n;
-  // FP32 stages: block sweeps on the tensor cores where the shape has whole blocks and at
-  // least 16 block pairs per step (fewer pairs leave most SMs idle in the pair
-  // eigenproblems: at 1024 x 1024 real the column-pair sweeps take 109 ms against 176 ms,
-  // at 4096 x 2048 real the block sweeps 495 ms against 685 ms). VJ_BLOCK=0 in the
-  // environment selects the column-pair sweeps, VJ_BLOCK=1 the block sweeps wherever the
-  // shape allows; VJ_BLOCK_TERMS (6 or 3) the terms of the split products, VJ_BLOCK_INNER
-  // the inner Jacobi sweeps per block pair.
+  // FP32 stages: block sweeps on the tensor cores where the shape has whole blocks and at least 16
+  // block pairs per step; else sweeps by small blocks of columns in one or two CTAs (colblk.cu)
+  // where a pair of blocks fits in shared memory; else column-pair sweeps. Measured, FP32 stages: 1024
+  // x 1024 real 54 ms by column pairs, 16 by small blocks, 44 on the tensor cores; 2048 x 1024
+  // complex 50 by small blocks, 41 on the tensor cores; 4096 x 2048 real 115 and 102. VJ_BLOCK=0 in
+  // the environment selects the column-pair sweeps, VJ_BLOCK=1 the tensor-core block sweeps wherever
+  // the shape allows; VJ_BLOCK_TERMS (6 or 3) the terms of the split products, VJ_BLOCK_INNER the
+  // inner Jacobi sweeps per block pair.
   const char *eb = getenv("VJ_BLOCK");
   const bool blk = !(eb && *eb == '0') && block_sweeps_apply(CPLX, m, n, m) &&
                    ((eb && *eb == '1') || n >= (CPLX ? 1024 : 2048));
-  const char *ec = getenv("VJ_COLBLK");
-  const int ncol = (!(ec && *ec == '0') && !blk) ? col_blocks(CPLX, m, n) : 0;
+  const int ncol = (!(eb && *eb == '0') && !blk) ? col_blocks(CPLX, m, n) : 0;
   const char *et = getenv("VJ_BLOCK_TERMS");
   const int terms = (et && atoi(et) == 3) ? 3 : 6;
   const char *ei = getenv("VJ_BLOCK_INNER");
@@ -1032,24 +1032,24 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     // 2. FP32 sweeps until a sweep rotates nothing
     // (a sweep whose rotated pairs were all within 4x the tolerance ends the stage without
     // a confirming sweep: the stage is a preconditioner, the next one finishes the work;
-    // a stage that another one follows also ends once a sweep rotates fewer than half of
+    // a stage that another one follows also ends once a sweep rotates fewer than 0.7 of
     // all possible pairs: the first stage works on A rounded to FP32, where the directions
     // of singular values below FP32 resolution are noise that the next stage resolves
-    // properly, and its long tail of sweeps over them costs more than the next stage's
-    // extra sweeps -- at 4096 x 2048 complex, 31 + 16 FP32 sweeps in 2.58 s against
-    // 18 + 18 in 2.47 s)
+    // properly. At 0.5 the 1024 x 1024 real matrix takes one sweep more; at 0.9 and above the
+    // FP64 phase of matrices with sigma over 6 decades and more takes a refinement or, at 1,
+    // sweeps more.)
     unsigned sw = 0;
     const float stop = 4.f * tol;
     const long long nbk = n / (CPLX ? 32 : 64), hw = CPLX ? 32 : 64;
     const long long cbn = ncol ? n / (ncol / 2) : 0;
-    const double every = ncol ? (double)cbn * (double)(cbn / 2) * (double)ncol * (double)(ncol / 2)
-                         : blk ? (double)(nbk - 1) * (double)(nbk / 2) * inner * (double)(2 * hw - 1) * (double)hw
+    const double every = ncol ? (double)(cbn / 2) * (double)(ncol / 2) * ((double)ncol + (double)(cbn - 1) * (double)(ncol / 2))
+                         : blk ? (double)(nbk / 2) * inner * (double)hw * (CPLX ? (double)nbk * (double)(2 * hw - 1) : (double)(2 * hw - 1) + (double)(nbk - 1) * (double)hw)
                              : (double)stp * (double)(n / 2);
     for (; sw < maxsw; ++sw) {
       float mu = 0.f;
       const long long hc =
           blk ? block_sweep(CPLX, mi, ni, G32, CPLX ? G32 + mn : nullptr, m, W32, CPLX ? W32 + nn : nullptr, n, bscr,
-                            cnt, tol, inner, terms, s, &mu)
+                            cnt, tol, inner, terms, true, s, &mu)
           : ncol ? col_block_sweep(CPLX, mi, ni, G32, CPLX ? G32 + mn : nullptr, W32, CPLX ? W32 + nn : nullptr, tol, cnt,
                                    s, &mu)
               : presweep<float, CPLX>(mi, ni, G32, m, CPLX ? G32 + mn : nullptr, m, W32, n, CPLX ? W32 + nn : nullptr,
@@ -1061,7 +1061,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
                      (double)mu);
       if (!hc)
         break;
-      if (mu < stop || (stage + 1 < stages && 2.0 * (double)hc < every)) {
+      if (mu < stop || (stage + 1 < stages && (double)hc < 0.7 * every)) {
         ++sw;
         break;
       }
