@@ -172,6 +172,7 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
   __shared__ int s_col[P][2], s_n[P][2], s_live[P], s_trk[P];
   __shared__ int s_err;
   __shared__ unsigned long long bar;
+  __shared__ int s_trans[P];
   // before the previous step is waited for: the pivot table, which no step writes
   const unsigned *r = a.js + (size_t)st * (size_t)a.n;
   const long long n_2 = a.n >> 1;
@@ -240,6 +241,11 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
         atomicMin((long long *)&g->err, (long long)VJ_ERR_ARG);
       return;
     }
+  }
+  if (STAGE && (d.gres || d.ovf)) {
+    // the rescaled columns are read by the copies below (another proxy)
+    asm volatile("fence.proxy.async;" ::: "memory");
+    __syncthreads();
   }
   if (d.vres)
     for (int j = 0; j < np; ++j) {
@@ -339,8 +345,18 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
       }
     }
   };
-  produce(0, tid, 256);
-  __syncthreads();
+  // the first chunk by seven warps, beside what the last one finds out about the pairs from their
+  // norms; it joins the barrier after the first chunk's recurrences
+  if (warp == 7) {
+    if (lane < np) {
+      const PairState<T> &s = ps[lane];
+      pre[lane] = pair_pre(s.ep, s.fp, s.eq, s.fq, a.gst);
+    }
+  }
+  else {
+    produce(0, tid, 224);
+    asm volatile("bar.sync 1, 224;" ::: "memory");
+  }
   T cs = 0, ct = 0;  // this lane's recurrence
   const int gl = warp * 32 + lane;
   const int nchunks = (mi + D::RC - 1) / D::RC;
@@ -378,10 +394,6 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
         sum_step(ops, v[0], cs, ct);
     }
     else {
-      if (ck == 0 && warp == 7 && lane < np) {
-        const PairState<T> &s = ps[lane];
-        pre[lane] = pair_pre(s.ep, s.fp, s.eq, s.fq, a.gst);
-      }
       if (ck + 1 < nchunks && pt >= 0)
         produce(ck + 1, pt, D::NPT);
     }
@@ -396,45 +408,59 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
   }
   __syncthreads();
   tphase(2);
-  // ---- 3. convergence, 2x2, classification: one quad of warp 0 per pair ----
-  if (warp == 0) {
+  // ---- 3. convergence, 2x2, classification: one quad of warp 0 per pair; complex data: the modulus
+  // of the cosine and the test by warp 1 beside the 2x2, which is computed for every pair ----
+  {
     const int q4 = lane & 3, base = lane & ~3;
     const int j = min(lane >> 2, np - 1);
     const bool own = (q4 == 0) && (lane >> 2) < np;
     PairState<T> &s = ps[j];
     const T ep = s.ep, fp_ = s.fp, eq = s.eq, fq = s.fq;
-    // nu = S(s_pd) + (S(t_pd) + (S(s_dn) + S(t_dn))), divided by fx fy
-    const T de = fq * fp_;
-    const T(*ds)[2] = dsum + j * D::NCH + ((CPLX && (q4 & 1)) ? 2 : 0);
-    const T z = F::div(ds[0][0] + (ds[0][1] + (ds[1][0] + ds[1][1])), de);
-    T zr = __shfl_sync(0xffffffffu, z, base), zi = CPLX ? __shfl_sync(0xffffffffu, z, base + 1) : (T)0;
-    if (!s_live[j]) {
-      zr = 0;
-      zi = 0;
-    }
     long long code = 0;
-    if (CPLX) {
-      if (!visfinite(zr))
-        code = a.e_dot;
-      if (!visfinite(zi))
-        code = (a.e_doti < code) ? a.e_doti : code;
-    }
-    else if (!visfinite(zr))
-      code = a.e_dot;
-    const T ab = CPLX ? vhypot(zr, zi) : vabs(zr);
-    const bool trans = (code == 0) && (a.tol <= ab);
-    T cc = 1, at = 0, sat = 0;
+    bool trans = false;
+    T zr = 0, zi = 0, cc = 1, at = 0, sat = 0;
     unsigned perm = 0u;
     const PairPre<T> pp = pre[j];
-    if (__any_sync(0xffffffffu, trans)) {
-      // (a pair that is not transformed passes ones and is ignored)
-      const T w11 = trans ? pp.w11 : (T)1, w22 = trans ? pp.w22 : (T)1, w21r = trans ? scalef(zr, pp.dd) : (T)1;
-      if constexpr (CPLX)
-        perm = cjac2_quad<T>(w11, w22, w21r, trans ? scalef(zi, pp.dd) : (T)1, q4, base, cc, at, sat);
-      else
-        perm = rjac2_quad<T>(w11, w22, w21r, q4, base, cc, at);
+    if (warp == 0 || (CPLX && warp == 1)) {
+      // nu = S(s_pd) + (S(t_pd) + (S(s_dn) + S(t_dn))), divided by fx fy
+      const T de = fq * fp_;
+      const T(*ds)[2] = dsum + j * D::NCH + ((CPLX && (q4 & 1)) ? 2 : 0);
+      const T z = F::div(ds[0][0] + (ds[0][1] + (ds[1][0] + ds[1][1])), de);
+      zr = __shfl_sync(0xffffffffu, z, base);
+      zi = CPLX ? __shfl_sync(0xffffffffu, z, base + 1) : (T)0;
+      if (!s_live[j]) {
+        zr = 0;
+        zi = 0;
+      }
+      if (CPLX) {
+        if (!visfinite(zr))
+          code = a.e_dot;
+        if (!visfinite(zi))
+          code = (a.e_doti < code) ? a.e_doti : code;
+      }
+      else if (!visfinite(zr))
+        code = a.e_dot;
+      if (!CPLX || warp == 1) {
+        const T ab = CPLX ? vhypot(zr, zi) : vabs(zr);
+        trans = (code == 0) && (a.tol <= ab);
+        if (CPLX && own)
+          s_trans[j] = trans ? 1 : 0;
+      }
+      if (CPLX ? (warp == 0) : __any_sync(0xffffffffu, trans)) {
+        // (a pair that is not transformed passes ones and is ignored)
+        const bool in = CPLX ? (s_live[j] && code == 0) : trans;
+        const T w11 = in ? pp.w11 : (T)1, w22 = in ? pp.w22 : (T)1, w21r = in ? scalef(zr, pp.dd) : (T)1;
+        if constexpr (CPLX)
+          perm = cjac2_quad<T>(w11, w22, w21r, in ? scalef(zi, pp.dd) : (T)1, q4, base, cc, at, sat);
+        else
+          perm = rjac2_quad<T>(w11, w22, w21r, q4, base, cc, at);
+      }
     }
-    if (own) {
+    if (CPLX) {
+      __syncthreads();
+      trans = s_trans[j] != 0;
+    }
+    if (warp == 0 && own) {
       s.a21r = zr;
       s.a21i = zi;
       s.skip = 0;
