@@ -9,6 +9,7 @@
 // strides over the arrays, so every byte of HBM is touched exactly once.
 #include <cfenv>
 #include <cstdlib>
+#include <cstring>
 #include <cuda_runtime.h>
 
 #include "jac2.cuh"
@@ -181,6 +182,41 @@ static vj_fint bjac2_host(vj_fint n, int internal, const T *a11, const T *a22, c
     if (r < 0)
       return r;
     return (cudaStreamSynchronize(st[0]) == cudaSuccess) ? 1 : VJ_ERR_CUDA;
+  }
+  // Few problems into pageable outputs: one launch that writes into page-locked memory, from
+  // which this thread copies to the caller's arrays. A copy by the engine into pageable memory
+  // costs 8 us of this thread's time for each of the five or six arrays whatever its size; this
+  // thread's copies move about 14 GB/s. Measured, with fresh inputs, engine / here: FP64 16
+  // problems 82 / 39 us, 4096 (128 KiB of outputs) 95 / 55, 16384 (512 KiB) 107 / 86, 65536
+  // (2 MiB) 122 / 208; FP32 complex 16384 (320 KiB) 108 / 76, 65536 (1.3 MiB) 122 / 148.
+  if (!internal && host::pageable_access() && !(eo && *eo == 'c') && al16(a11) && al16(a22) && al16(a21r) &&
+      al16(a21i)) {
+    constexpr int nout = CPLX ? 5 : 4;
+    T *const hout[5] = {c, cat, CPLX ? sat : l1, CPLX ? l1 : l2, CPLX ? l2 : nullptr};
+    const size_t bytes = (size_t)nn * sizeof(T), per = (bytes + 15u) & ~(size_t)15u;
+    const size_t pb = (size_t)(nn / LANES) * sizeof(unsigned);
+    bool plain = (nn > 0) && (nn <= (long long)host::SMALL_OUT) && (nout * bytes <= host::SMALL_OUT) &&
+                 host::host_written(p);
+    for (int k = 0; plain && k < nout; ++k)
+      plain = host::host_written(hout[k]);
+    char *const base = plain ? host::small_out() : nullptr;
+    cudaStream_t st[2];
+    if (base && host::streams2(st)) {
+      T *out[5];
+      for (int k = 0; k < nout; ++k)
+        out[k] = reinterpret_cast<T *>(base + k * per);
+      unsigned *const op = reinterpret_cast<unsigned *>(base + nout * per);
+      const vj_fint r = bjac2_dev<T, CPLX>(n, 0, a11, a22, a21r, a21i, out[0], out[1], CPLX ? out[2] : nullptr,
+                                           CPLX ? out[3] : out[2], CPLX ? out[4] : out[3], op, st[0]);
+      if (r < 0)
+        return r;
+      if (cudaStreamSynchronize(st[0]) != cudaSuccess)
+        return VJ_ERR_CUDA;
+      for (int k = 0; k < nout; ++k)
+        memcpy(hout[k], out[k], bytes);
+      memcpy(p, op, pb);
+      return 1;
+    }
   }
   if (!internal && host::pageable_access() && al16(a11) && al16(a22) && al16(a21r) && al16(a21i)) {
     const long long chunk = host::bjac2_chunk(nn, sizeof(T), CPLX, LANES);

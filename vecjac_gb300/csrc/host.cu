@@ -53,6 +53,18 @@ bool host_pinned(const void *p)
   return at.type == cudaMemoryTypeHost;
 }
 
+bool host_written(const void *p)
+{
+  if (!p)
+    return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type != cudaMemoryTypeDevice;
+}
+
 bool pageable_access()
 {
   static int vs[MAX_DEVICES] = {};  // 0 unknown, 1 yes, 2 no
@@ -110,6 +122,19 @@ void *batch_plan(size_t bytes)
   if (!q[dev].reserve((size_t)BATCH_SLOTS * bytes))
     return nullptr;
   return q[dev].ptr + (size_t)(next[dev]++ % BATCH_SLOTS) * bytes;
+}
+
+char *small_out()
+{
+  static char *buf[MAX_DEVICES] = {};
+  char *&b = buf[device_slot()];
+  // (a permutation word for every 8 or 16 problems, each array to 16 bytes)
+  if (!b && cudaHostAlloc(reinterpret_cast<void **>(&b), SMALL_OUT + (SMALL_OUT >> 5) + 256, cudaHostAllocPortable) !=
+                cudaSuccess) {
+    cudaGetLastError();
+    b = nullptr;
+  }
+  return b;
 }
 
 Staging &staging2()

@@ -40,6 +40,8 @@ int sm_count();
 bool pageable_access();
 // p (NULL counts as true) is page-locked host memory (cudaHostAlloc / cudaHostRegister)
 bool host_pinned(const void *p);
+// p is memory that this thread may write (not NULL, not device memory)
+bool host_written(const void *p);
 
 // device memory reused across host-API calls; grows on demand, never shrinks
 struct Staging {
@@ -51,6 +53,11 @@ Staging &staging();
 Staging &staging2();
 // scratch of the mixed-precision SVD (its inner SVD calls use staging2)
 Staging &staging3();
+
+// page-locked host memory for the outputs of one small 2x2 call (SMALL_OUT bytes of arrays and
+// their permutation words), allocated on first use, one per device, under host_call_lock
+constexpr size_t SMALL_OUT = (size_t)512 << 10;
+char *small_out();
 
 // device memory for one launch of the batched SVD (always the same size): its work queues and
 // what its CTAs need to know of the batch (allocated on first use)
