@@ -154,6 +154,15 @@ __device__ unsigned cjac2_quad(T a1, T a2, T ar, T ai, int r, int base, T &c, T 
   return bit;
 }
 
+// the norm from its scaled sum of squares: warp_nrm2's value
+template <typename T> __device__ __forceinline__ T finish_nrm_unit(T acc, typename fp<T>::U mx)
+{
+  const T a = fp<T>::val(mx);
+  if (!visfinite(a))
+    return visnan(a) ? fp<T>::qnan() : a;
+  return (mx == 0) ? (T)0 : scale2(fp<T>::sqrt_(acc), ilogb_(a));
+}
+
 template <typename T, bool CPLX, bool STAGE, int P>
 __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int last)
 {
@@ -168,11 +177,12 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
   __shared__ T dsum[D::NG][2];
   __shared__ U cmx[P][NC];           // largest |.| of the changed columns' planes
   __shared__ U vmx;
-  __shared__ T cnrm[2 * P][CPLX ? 2 : 1];
   __shared__ int s_col[P][2], s_n[P][2], s_live[P], s_trk[P];
   __shared__ int s_err;
   __shared__ unsigned long long bar;
   __shared__ int s_trans[P];
+  __shared__ T cnrm[2 * P][CPLX ? 2 : 1];
+  constexpr bool LATE_V = sizeof(T) == 4;  // V is rotated beside the norms (where it is not tracked)
   // before the previous step is waited for: the pivot table, which no step writes
   const unsigned *r = a.js + (size_t)st * (size_t)a.n;
   const long long n_2 = a.n >> 1;
@@ -500,9 +510,9 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
       T *Gip = CPLX ? (a.Gi + p * a.ldGi) : nullptr, *Giq = CPLX ? (a.Gi + q * a.ldGi) : nullptr;
       T *Vip = CPLX ? (a.Vi + p * a.ldVi) : nullptr, *Viq = CPLX ? (a.Vi + q * a.ldVi) : nullptr;
       const bool trk = pair_apply<T, CPLX, STAGE, (P == 4) ? 8 : 4>(
-          ps[j], a.m, a.n, a.G + p * a.ldG, a.G + q * a.ldG, Gip, Giq, a.V + p * a.ldV, a.V + q * a.ldV, Vip, Viq,
-          rcol(j, 0), rcol(j, 1), CPLX ? rcol(j, 2) : nullptr, CPLX ? rcol(j, 3) : nullptr, a.eS + p, a.eS + q,
-          a.fS + p, a.fS + q, ltid, TPP, a.trackv != 0, mx, mV);
+          ps[j], a.m, (LATE_V && !a.trackv) ? 0 : a.n, a.G + p * a.ldG, a.G + q * a.ldG, Gip, Giq, a.V + p * a.ldV,
+          a.V + q * a.ldV, Vip, Viq, rcol(j, 0), rcol(j, 1), CPLX ? rcol(j, 2) : nullptr, CPLX ? rcol(j, 3) : nullptr,
+          a.eS + p, a.eS + q, a.fS + p, a.fS + q, ltid, TPP, a.trackv != 0, mx, mV);
       if (ltid == 0)
         s_trk[j] = trk ? 1 : 0;
     }
@@ -521,7 +531,8 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
   }
   __syncthreads();
   tphase(4);
-  if (tid == 0) {
+  // the changed columns' largest |.| for the next step's decisions
+  auto post_max = [&]() {
     U bg = 0;
     for (int j = 0; j < np; ++j)
 #pragma unroll
@@ -539,38 +550,113 @@ __global__ void __launch_bounds__(256) k_step(SvdArgs<T> a, int st, int g3, int 
       if (bv)
         atomicMax(&nxt.nMV, (unsigned long long)bv);
     }
-  }
-  // ---- 5. norms of the changed columns for the next step: one warp per column and plane ----
-  // (not after the last step of the last allowed sweep: the reference returns there with
-  // the norms of those columns not yet recomputed)
-  if (last)
-    return;
-  auto changed = [&](int j, int c) {
-    const int code = ps[j].code;
-    return !ps[j].skip && (code == 2 || code == -2 || (c && (code == 3 || code == -3)));
   };
-  constexpr int NPL = CPLX ? 2 : 1;
-  for (int u = warp; u < 2 * np * NPL; u += 8) {
-    const int pl = u % NPL, j = u / (2 * NPL), c = (u / NPL) & 1;
-    if (changed(j, c)) {
-      const T *x = rcol(j, 2 * pl + c);
-      const T nv = s_trk[j] ? warp_nrm2_scaled<T>(x, a.m, (unsigned long long)cmx[j][2 * pl + c]) : warp_nrm2<T>(x, a.m);
-      if (lane == 0)
-        cnrm[2 * j + c][pl] = nv;
+  // ---- 5. norms of the changed columns for the next step (not after the last step of the last
+  // allowed sweep: the reference returns there with the norms of those columns not yet recomputed) ----
+  if constexpr (LATE_V) {
+    // FP32: by the first warps, two sums of squares at once on each (a pair's columns, or the planes
+    // of a complex column), which are latency; the other warps rotate V beside them (656 x 608: 2.8k
+    // and 3.3k clocks of rotations and norms become 2.2k and 2.0k). In FP64 V's operations would
+    // queue before those of the norms in the sub-partitions' FP64 units (1024 x 1024: 23.6k clocks
+    // in place of 8.2k), so there V is rotated with G. (Nor a step later, beside the dot products,
+    // which that slows from 47.4k to 52.4k.)
+    if (tid == 255)
+      post_max();
+    constexpr int NI = CPLX ? 2 * P : P, NWN = (NI < 4) ? NI : 4;
+    if (warp >= NWN || last) {
+      if (!a.trackv) {
+        // (the pairs in turn, a stretch of rows to each warp that shares one)
+        const int w = last ? warp : warp - NWN, nw = last ? 8 : 8 - NWN;
+        const int share = (nw + np - 1) / np, per = (((int)a.n + share - 1) / share + 31) & ~31;
+        for (int u = w; u < np * share; u += nw) {
+          const int j = u % np, r0 = (u / np) * per, rows = min(per, (int)a.n - r0);
+          const long long p = colp(j) * a.ldV + r0, q = colq(j) * a.ldV + r0;
+          const long long pi = colp(j) * a.ldVi + r0, qi = colq(j) * a.ldVi + r0;
+          if (rows > 0)
+            v_apply<T, CPLX, (P == 4) ? 8 : 4>(ps[j], rows, a.V + p, a.V + q, CPLX ? a.Vi + pi : nullptr,
+                                               CPLX ? a.Vi + qi : nullptr, lane, 32);
+        }
+      }
     }
+    else
+      for (int u = warp; u < (CPLX ? 2 * np : np); u += NWN) {
+        const int j = CPLX ? u >> 1 : u, code = ps[j].code;
+        const bool rot = (code == 2 || code == -2), gs = (code == 3 || code == -3);
+        if (ps[j].skip || !(rot || (gs && (!CPLX || (u & 1)))))
+          continue;
+        const int c0 = CPLX ? (u & 1) : 0, c1 = CPLX ? c0 + 2 : 1;
+        const T *x = rcol(j, c0), *y = rcol(j, c1);
+        U mx = cmx[j][c0], my = cmx[j][c1];
+        if (!s_trk[j]) {
+          mx = my = 0;
+          for (int i = lane; i < mi; i += 32) {
+            amax(mx, x[i]);
+            amax(my, y[i]);
+          }
+          mx = warp_max_bits(mx);
+          my = warp_max_bits(my);
+        }
+        T ax, ay;
+        pair_sumsq<T>(mi, x, y, mx, my, ax, ay);
+        ay = __shfl_sync(0xffffffffu, ay, 0);
+        // a norm on lane 0 and one on lane 1
+        T nv = finish_nrm_unit<T>(lane ? ay : ax, lane ? my : mx);
+        if (CPLX)
+          nv = vhypot(nv, __shfl_sync(0xffffffffu, nv, 1));
+        const int c = CPLX ? c0 : lane;
+        if (lane < (CPLX ? 1 : 2) && (rot || c)) {
+          T e, f;
+          ef_split(nv, e, f);
+          a.eS[s_col[j][c]] = e;
+          a.fS[s_col[j][c]] = f;
+          if (!(nv <= svdc<T>::RMAX))
+            atomicOr(&nxt.ovf, 1);
+        }
+      }
   }
-  __syncthreads();
-  if (tid < 2 * np && changed(tid >> 1, tid & 1)) {
-    const int j = tid >> 1, c = tid & 1;
-    T nv = cnrm[tid][0];
-    if (CPLX)
-      nv = vhypot(nv, cnrm[tid][CPLX ? 1 : 0]);
-    T e, f;
-    ef_split(nv, e, f);
-    a.eS[s_col[j][c]] = e;
-    a.fS[s_col[j][c]] = f;
-    if (!(nv <= svdc<T>::RMAX))
-      atomicOr(&nxt.ovf, 1);
+  else {
+    // FP64: a warp per column and plane, the largest magnitudes of rotated columns first
+    constexpr int NPL = CPLX ? 2 : 1;
+    auto changed = [&](int j, int c) {
+      const int code = ps[j].code;
+      return !ps[j].skip && (code == 2 || code == -2 || (c && (code == 3 || code == -3)));
+    };
+    for (int u = warp; u < 2 * np * NPL; u += 8) {
+      const int pl = u % NPL, j = u / (2 * NPL), c = (u / NPL) & 1;
+      if (changed(j, c)) {
+        const T *x = rcol(j, 2 * pl + c);
+        U mx = cmx[j][2 * pl + c];
+        if (!s_trk[j]) {
+          mx = 0;
+#pragma unroll 8
+          for (int i = lane; i < mi; i += 32)
+            amax(mx, x[i]);
+          mx = warp_max_bits(mx);
+          if (lane == 0)
+            cmx[j][2 * pl + c] = mx;
+        }
+        if (!last) {
+          const T nv = warp_nrm2_scaled<T>(x, a.m, (unsigned long long)mx);
+          if (lane == 0)
+            cnrm[2 * j + c][pl] = nv;
+        }
+      }
+    }
+    __syncthreads();
+    if (tid == 255)
+      post_max();
+    if (!last && tid < 2 * np && changed(tid >> 1, tid & 1)) {
+      const int j = tid >> 1, c = tid & 1;
+      T nv = cnrm[tid][0];
+      if (CPLX)
+        nv = vhypot(nv, cnrm[tid][CPLX ? 1 : 0]);
+      T e, f;
+      ef_split(nv, e, f);
+      a.eS[s_col[j][c]] = e;
+      a.fS[s_col[j][c]] = f;
+      if (!(nv <= svdc<T>::RMAX))
+        atomicOr(&nxt.ovf, 1);
+    }
   }
   tphase(5);
 }

@@ -539,9 +539,9 @@ __device__ __forceinline__ void rot_cplx(int rows, const T *rxr, const T *rxi, c
 // rp/rq[/rpi/rqi], which is a staged copy when STG, written to both; the columns themselves
 // otherwise) and of V. mx collects this thread's max |.| of the rows that the transformed
 // columns p and q of G receive (their imaginary planes in mx[2], mx[3]) and mV, with trackv,
-// that of V. Returns whether mx holds the maxima of the changed columns: false for a
-// rotation by nothing or by a plain exchange, whose columns count as changed without being
-// tracked. UR: rows per thread in flight (rot_real; half of it for complex columns).
+// that of V. Returns whether mx holds the maxima of the changed columns: false for an FP64
+// rotation, and for a rotation by nothing or by a plain exchange, whose columns count as changed
+// without being tracked. UR: rows per thread in flight (rot_real; half of it for complex columns).
 template <typename T, bool CPLX, bool STG, int UR>
 __device__ bool pair_apply(const PairState<T> &s, long long m, long long nv, T *Gp, T *Gq, T *Gip, T *Giq, T *Vp,
                            T *Vq, T *Vip, T *Viq, T *rp, T *rq, T *rpi, T *rqi, T *eSp, T *eSq, T *fSp, T *fSq,
@@ -661,14 +661,18 @@ __device__ bool pair_apply(const PairState<T> &s, long long m, long long nv, T *
       }
       return false;
     }
+    // FP64 rotations do not collect the largest |.|: a result of the FP64 unit that goes on to the
+    // integer pipe costs more (1024 x 1024: 17.1k clocks for G's columns instead of 11.1k) than
+    // another pass over the columns (0.8k).
+    constexpr bool TRK = sizeof(T) == 4;
     U v0 = 0, v1 = 0;
     if (real_rot) {
-      rot_real<T, STG, UR>((int)m, rp, rq, Gp, Gq, rp, rq, at, c, perm, ltid, TPP, true, mx[0], mx[1]);
+      rot_real<T, STG, UR>((int)m, rp, rq, Gp, Gq, rp, rq, at, c, perm, ltid, TPP, TRK, mx[0], mx[1]);
       rot_real<T, false, UR>((int)nv, Vp, Vq, Vp, Vq, nullptr, nullptr, at, c, perm, ltid, TPP, trackv, v0, v1);
       if (trackv)
         mV = (v0 > v1) ? v0 : v1;
       if (CPLX) {
-        rot_real<T, STG, UR>((int)m, rpi, rqi, Gip, Giq, rpi, rqi, at, c, perm, ltid, TPP, true, mx[CPLX ? 2 : 0],
+        rot_real<T, STG, UR>((int)m, rpi, rqi, Gip, Giq, rpi, rqi, at, c, perm, ltid, TPP, TRK, mx[CPLX ? 2 : 0],
                                   mx[CPLX ? 3 : 1]);
         rot_real<T, false, UR>((int)nv, Vip, Viq, Vip, Viq, nullptr, nullptr, at, c, perm, ltid, TPP, trackv, v0, v1);
         if (trackv) {
@@ -680,7 +684,7 @@ __device__ bool pair_apply(const PairState<T> &s, long long m, long long nv, T *
     else if constexpr (CPLX) {
       U v4[4] = {0, 0, 0, 0};
       rot_cplx<T, STG, UR / 2>((int)m, rp, rpi, rq, rqi, Gp, Gip, Gq, Giq, rp, rpi, rq, rqi, at, sat, c, perm, ltid,
-                                TPP, true, mx);
+                                TPP, TRK, mx);
       rot_cplx<T, false, UR / 2>((int)nv, Vp, Vip, Vq, Viq, Vp, Vip, Vq, Viq, nullptr, nullptr, nullptr, nullptr,
                                     at, sat, c, perm, ltid, TPP, trackv, v4);
       if (trackv) {
@@ -689,8 +693,38 @@ __device__ bool pair_apply(const PairState<T> &s, long long m, long long nv, T *
           mV = (v4[k] > mV) ? v4[k] : mV;
       }
     }
+    return TRK;
   }
   return true;
+}
+
+// What pair_apply does to V's columns, apart from it: rows rows from Vp, Vq (imaginary parts Vip,
+// Viq) on, by ltid of TPP threads
+template <typename T, bool CPLX, int UR>
+__device__ __forceinline__ void v_apply(const PairState<T> &s, int rows, T *Vp, T *Vq, T *Vip, T *Viq, int ltid, int TPP)
+{
+  const int code = s.code;
+  if (s.skip || code == 1 || code == 3)
+    return;
+  const bool rot = (code == 2 || code == -2), perm = (code == -2);
+  const bool real_rot = !CPLX || s.sat == (T)0;
+  if (rot && !(real_rot && s.cat == (T)0)) {
+    typename fp<T>::U m[4] = {0, 0, 0, 0};
+    if (real_rot) {
+      rot_real<T, false, UR>(rows, Vp, Vq, Vp, Vq, nullptr, nullptr, s.cat, s.c, perm, ltid, TPP, false, m[0], m[1]);
+      if (CPLX)
+        rot_real<T, false, UR>(rows, Vip, Viq, Vip, Viq, nullptr, nullptr, s.cat, s.c, perm, ltid, TPP, false, m[2],
+                               m[3]);
+    }
+    else if constexpr (CPLX)
+      rot_cplx<T, false, UR / 2>(rows, Vp, Vip, Vq, Viq, Vp, Vip, Vq, Viq, nullptr, nullptr, nullptr, nullptr, s.cat,
+                                 s.sat, s.c, perm, ltid, TPP, false, m);
+  }
+  else if (!rot || (s.c == (T)1 && perm)) {
+    swap_cols(Vp, Vq, rows, ltid, TPP);
+    if (CPLX)
+      swap_cols(Vip, Viq, rows, ltid, TPP);
+  }
 }
 
 }  // namespace vj

@@ -102,4 +102,69 @@ template <typename T> __device__ T warp_nrm2(const T *x, long long m)
   return warp_nrm2_scaled(x, m, warp_max_u64((unsigned long long)mx));
 }
 
+// The sums of squares of two columns, each scaled by 2^-k with k the exponent of its largest
+// magnitude (mx, my: that magnitude's bits; zero or not finite: the sum is not used), in the
+// project's norm order (svd_norm.cuh) for one warp, on its lane 0.
+template <typename T>
+__device__ void pair_sumsq(int m, const T *x, const T *y, typename fp<T>::U mx, typename fp<T>::U my, T &ax, T &ay)
+{
+  using F = fp<T>;
+  const int lane = (int)(threadIdx.x & 31u);
+  const T vx = F::val(mx), vy = F::val(my);
+  const int kx = (mx && visfinite(vx)) ? -ilogb_(vx) : 0, ky = (my && visfinite(vy)) ? -ilogb_(vy) : 0;
+  ax = ay = (T)0;
+  if (sizeof(T) == 4 && kx >= 1 - F::BIAS && kx <= F::BIAS && ky >= 1 - F::BIAS && ky <= F::BIAS) {
+    // (the product by a normal power of two is scale2's value)
+    const T px = pow2<T>(kx), py = pow2<T>(ky);
+#pragma unroll 4
+    for (int i = lane; i < m; i += 32) {
+      const T a = x[i] * px, b = y[i] * py;
+      ax = F::fma_(a, a, ax);
+      ay = F::fma_(b, b, ay);
+    }
+  }
+  else {
+    // four rows of a lane at a time, rows past the end as zeros (which add nothing)
+    auto scaled = [](T v, int k, bool &fast) {
+      const int e = (int)((F::bits(v) & ~F::SIGN) >> F::MB);
+      if ((F::bits(v) & ~F::SIGN) != 0)
+        fast = fast && (e > 0) && (e + k > 0) && (e + k <= F::EMAXB);
+      return (e == 0) ? (T)0 : F::val(F::bits(v) + ((typename F::U)(long long)k << F::MB));
+    };
+    for (int i = lane; i < m; i += 128) {
+      T a[4], b[4], sa[4], sb[4];
+      bool fast = true;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool in = i + 32 * u < m;
+        a[u] = in ? x[i + 32 * u] : (T)0;
+        b[u] = in ? y[i + 32 * u] : (T)0;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        sa[u] = scaled(a[u], kx, fast);
+        sb[u] = scaled(b[u], ky, fast);
+      }
+      if (!fast) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          sa[u] = scale2(a[u], kx);
+          sb[u] = scale2(b[u], ky);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (u == 0 || i + 32 * u < m) {
+          ax = F::fma_(sa[u], sa[u], ax);
+          ay = F::fma_(sb[u], sb[u], ay);
+        }
+    }
+  }
+#pragma unroll
+  for (int w = 16; w >= 1; w >>= 1) {
+    ax = ax + __shfl_down_sync(0xffffffffu, ax, w);
+    ay = ay + __shfl_down_sync(0xffffffffu, ay, w);
+  }
+}
+
 }  // namespace vj
