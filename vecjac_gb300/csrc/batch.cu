@@ -23,6 +23,17 @@ namespace vj {
 constexpr int BATCH_CS = 4;
 constexpr double BATCH_SHARE = 1.0;
 
+// Unless the caller sets the number of CTAs per SM, the batch is done by two launches: the large
+// matrices and the wide ones, whose cost is more than BATCH_WIDE of a CTA's share of the batch, by
+// two CTAs of 128 registers per SM, and the others by four CTAs of 64 registers, which start as the
+// first launch's end. A matrix is done sooner by one of two CTAs than of four, which counts at the
+// end of the batch; many small ones are done sooner by four, whose waits for memory and for the few
+// threads of a 2x2 overlap. 4000 FP32 matrices of up to 256 rows: 141 ms (two CTAs 141, four 154),
+// 1500 FP64 ones of up to 128 rows: 105 ms (105, 115), 4000 FP64 16 x 16: 16.8 ms (22.3, 17.2),
+// 4000 FP32 64 x 32: 10.1 ms (11.8, 10.6). With a smaller BATCH_WIDE, 2000 FP64 64 x 64 take 154
+// instead of 141 ms, with a larger one the uneven batches 151 and 119 ms (at 0.6).
+constexpr double BATCH_WIDE = 0.15;
+
 // a matrix's work, up to its number of sweeps
 __device__ __forceinline__ double batch_cost(long long m, long long n)
 {
@@ -36,7 +47,7 @@ template <typename T>
 __global__ void __launch_bounds__(1024) k_plan(BatchArgs<T> a, int slots, int warps, double share)
 {
   __shared__ double sum[32];
-  __shared__ unsigned end;
+  __shared__ unsigned end, endw;
   const int tid = threadIdx.x;
   double c = 0;
   for (long long i = tid; i < a.count; i += blockDim.x)
@@ -46,7 +57,7 @@ __global__ void __launch_bounds__(1024) k_plan(BatchArgs<T> a, int slots, int wa
   if ((tid & 31) == 0)
     sum[tid >> 5] = c;
   if (tid == 0)
-    end = 0u;
+    end = endw = 0u;
   __syncthreads();
   c = 0;
   for (int w = 0; w < 32; ++w)
@@ -57,15 +68,20 @@ __global__ void __launch_bounds__(1024) k_plan(BatchArgs<T> a, int slots, int wa
     const int b = a.order ? a.order[i] : (int)i;
     if (batch_cost(a.m[b], a.n[b]) > limit)
       atomicMax(&end, (unsigned)(i + 1));
+    if (batch_cost(a.m[b], a.n[b]) > BATCH_WIDE * c / slots)
+      atomicMax(&endw, (unsigned)(i + 1));
   }
-  if (tid < 256)
-    a.plan->on_sm[tid] = 0u;
+  if (tid < 512)
+    a.plan->on_sm[tid >> 8][tid & 255] = 0u;
   __syncthreads();
   if (tid == 0) {
     a.plan->next_large = 0u;
+    a.plan->next_wide = 0u;
     a.plan->next = 0u;
     a.plan->end_large = end;
+    a.plan->end_wide = endw;
     a.plan->limit = limit;
+    a.plan->wide = BATCH_WIDE * c / slots;
   }
 }
 
@@ -81,7 +97,8 @@ __device__ __noinline__ void svd_matrix(const BatchArgs<T> &a, BatchShared<T> &s
 
 // MINB: the register bound for MINB resident CTAs of 256 threads per SM (more, smaller
 // CTAs when the caller launches fewer threads per CTA). The best bound depends on the
-// batch (the autotuner of vecjac_gb300/batch.py searches it with the CTA size).
+// batch (the autotuner of vecjac_gb300/batch.py searches it with the CTA size); a.part says which
+// of the batch's matrices the launch does.
 template <typename T, int MINB>
 __global__ void __launch_bounds__(256, MINB) k_batch(BatchArgs<T> a)
 {
@@ -91,9 +108,11 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchArgs<T> a)
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
   BatchPlan *const plan = a.plan;
-  const double limit = plan->limit;
+  const double limit = plan->limit, widec = plan->wide;
   const unsigned end = plan->end_large;
   auto large = [&](int b) { return batch_cost(a.m[b], a.n[b]) > limit; };
+  if (a.part == 1)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // the large matrices, by whole clusters
   if (end && size > 1u) {
     const Team tm{(int)rank, (int)size};
@@ -126,25 +145,28 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchArgs<T> a)
   // the others, by single CTAs: the r-th CTA of an SM takes part when there are more than r
   // matrices per SM, so that few matrices spread over the SMs (108 FP64 matrices of up to 35
   // rows: 9.2 ms when the two CTAs of an SM may both take one, 7.1 ms apart)
-  const bool split = end && size > 1u;
+  const bool split = end && (size > 1u || a.part == 2);
   if (threadIdx.x == 0) {
     unsigned sm;
     asm("mov.u32 %0, %%smid;" : "=r"(sm));
-    s_b[1] = (long long)atomicAdd(&plan->on_sm[sm & 255u], 1u);
+    s_b[1] = (long long)atomicAdd(&plan->on_sm[a.part == 2][sm & 255u], 1u);
   }
   __syncthreads();
-  if (s_b[1] * (long long)a.sms >= a.count)
-    return;
+  unsigned *const head = (a.part == 1) ? &plan->next_wide : &plan->next;
+  const long long stop = (s_b[1] * (long long)a.sms >= a.count) ? 0
+                         : (a.part == 1)                        ? (long long)plan->end_wide
+                                                                : a.count;
   for (;;) {
     __syncthreads();
     if (threadIdx.x == 0) {
       long long got = -1;
       for (;;) {
-        const long long i = (long long)atomicAdd(&plan->next, 1u);
-        if (i >= a.count)
+        const long long i = stop ? (long long)atomicAdd(head, 1u) : 0;
+        if (i >= stop)
           break;
         const int b = a.order ? a.order[i] : (int)i;
-        if (!split || i >= (long long)end || !large(b)) {
+        const bool mine = a.part == 0 || (batch_cost(a.m[b], a.n[b]) > widec) == (a.part == 1);
+        if (mine && !(split && i < (long long)end && large(b))) {
           got = b;
           break;
         }
@@ -154,13 +176,12 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchArgs<T> a)
     __syncthreads();
     const long long b = s_b[0];
     if (b < 0)
-      return;
+      break;
     svd_matrix<T>(a, sh, (int)b, Team{0, 1}, &sh);
   }
+  if (a.part == 2)  // (the launch ends when the first part has, too)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-
-// default register bound: FP32 4 CTAs of 256 threads per SM, FP64 2
-template <typename T> constexpr int batch_occ_default() { return sizeof(T) == 4 ? 4 : 2; }
 
 template <typename T>
 static vj_fint batch_dev(vj_fint count, const long long *m, const long long *n, T *G, const long long *offG, T *V,
@@ -175,8 +196,9 @@ static vj_fint batch_dev(vj_fint count, const long long *m, const long long *n, 
     return VJ_ERR_NO_GPU;
   if (block != 64 && block != 128 && block != 256)
     block = 128;
-  if (occ < 2 || occ > 6)
-    occ = batch_occ_default<T>();
+  const bool parts = (occ < 2 || occ > 6);
+  if (parts)
+    occ = 2;
   cudaStream_t s = (cudaStream_t)stream;
   BatchPlan *plan = static_cast<BatchPlan *>(host::batch_plan(sizeof(BatchPlan)));
   if (!plan)
@@ -188,6 +210,7 @@ static vj_fint batch_dev(vj_fint count, const long long *m, const long long *n, 
   a.strategy = (int)strategy;
   a.swp = swp;
   a.sms = host::sm_count();
+  a.part = parts ? 1 : 0;
   void (*k)(BatchArgs<T>) = (occ == 2)   ? k_batch<T, 2>
                             : (occ == 3) ? k_batch<T, 3>
                             : (occ == 4) ? k_batch<T, 4>
@@ -214,6 +237,20 @@ static vj_fint batch_dev(vj_fint count, const long long *m, const long long *n, 
   cfg.gridDim = dim3((unsigned)(((long long)clusters < count ? (long long)clusters : (long long)count) * BATCH_CS));
   if (cudaLaunchKernelEx(&cfg, k, a) != cudaSuccess)
     return VJ_ERR_CUDA;
+  if (parts) {
+    // the others: these CTAs start as the first launch's end
+    a.part = 2;
+    void (*const k2)(BatchArgs<T>) = k_batch<T, 4>;
+    int per = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k2, block, 0) != cudaSuccess || per < 1) {
+      cudaGetLastError();
+      per = 1;
+    }
+    const long long most = (long long)per * a.sms;
+    if (host::launch_pdl(k2, dim3((unsigned)(most < count ? most : (long long)count)), dim3((unsigned)block), 0, s, a) !=
+        cudaSuccess)
+      return VJ_ERR_CUDA;
+  }
   return (cudaGetLastError() == cudaSuccess) ? 0 : VJ_ERR_CUDA;
 }
 

@@ -21,10 +21,11 @@ constexpr int BATCH_MAXN = 512;
 
 // what the steps of one launch share about the batch (batch.cu, k_plan)
 struct BatchPlan {
-  unsigned next_large, next;  // work-queue heads: matrices for whole clusters, for single CTAs
-  unsigned end_large;         // one past the last large matrix in the caller's order
-  double limit;               // a matrix of a larger cost (batch_cost) is large
-  unsigned on_sm[256];        // CTAs of each SM that have come to take single matrices
+  // work-queue heads: matrices for whole clusters, wide ones and the others for single CTAs
+  unsigned next_large, next_wide, next;
+  unsigned end_large, end_wide;  // one past the last large, wide matrix in the caller's order
+  double limit, wide;            // a matrix of a larger cost (batch_cost) is large, wide
+  unsigned on_sm[2][256];        // CTAs of each SM that have come to take single matrices, by launch
 };
 
 template <typename T> struct BatchArgs {
@@ -36,7 +37,8 @@ template <typename T> struct BatchArgs {
   BatchPlan *plan;
   int strategy;
   unsigned swp;
-  int sms;  // SMs of the device
+  int sms;   // SMs of the device
+  int part;  // 0 all matrices, 1 large and wide ones, 2 the others
 };
 
 // what a step leaves for the next (three slots in turn: read, written, being cleared)
@@ -153,6 +155,19 @@ __device__ void team_scale(T *A, long long rows, long long cols, int e, int gw, 
 }
 
 #ifdef __CUDA_ARCH__
+// pair_sumsq for columns whose scale factors are not normal
+__device__ __noinline__ void pair_sumsq_rare(int m, const float *x, const float *y, unsigned mx, unsigned my, float &ax,
+                                             float &ay)
+{
+  pair_sumsq<float>(m, x, y, mx, my, ax, ay);
+}
+// the largest of m, |x| and |y|, a NaN if one is one
+__device__ __forceinline__ float max_nan(float m, float x, float y)
+{
+  float r;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(m), "f"(x), "f"(y));
+  return r;
+}
 // the larger of m and |x|, a NaN if either is one
 __device__ __forceinline__ float max_nan(float m, float x)
 {
@@ -160,7 +175,99 @@ __device__ __forceinline__ float max_nan(float m, float x)
   asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(m), "f"(fabsf(x)));
   return r;
 }
-// rot_real (svd_core.cuh) for FP32 columns at 8-byte boundaries and one warp: two rows per
+// A pair of FP32 columns of up to 32 K rows in registers: rotated (rot_real of svd_core.cuh),
+// written back, and the new columns' largest magnitudes and sums of squares (pair_sumsq, the same
+// values in the same order) from the registers, so that a rotation waits for memory once: for the
+// loads of G's and V's columns together. Rows of a lane are 32 apart, as the sums take them, and
+// two of them share a packed operation.
+template <int K> struct ColsF32 {
+  float u[K], w[K];
+  __device__ __forceinline__ void load(int rows, const float *x, const float *y)
+  {
+    const int lane = (int)(threadIdx.x & 31u);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const bool in = lane + 32 * k < rows;
+      u[k] = in ? x[lane + 32 * k] : 0.0f;
+      w[k] = in ? y[lane + 32 * k] : 0.0f;
+    }
+  }
+  __device__ __forceinline__ void rotate(float at, float c)
+  {
+    const F32x2 t = f2_make(at, at), tn = f2_make(-at, -at), cc = f2_make(c, c);
+    const bool cone = (c == 1.0f);
+#pragma unroll
+    for (int k = 0; k < K; k += 2) {
+      const F32x2 x = f2_make(u[k], u[k + 1]), y = f2_make(w[k], w[k + 1]);
+      F32x2 a = f2_fma(y, t, x), b = f2_fma(x, tn, y);
+      if (!cone) {
+        a = f2_mul(a, cc);
+        b = f2_mul(b, cc);
+      }
+      f2_get(a, u[k], u[k + 1]);
+      f2_get(b, w[k], w[k + 1]);
+    }
+  }
+  __device__ __forceinline__ void store(int rows, float *x, float *y) const
+  {
+    const int lane = (int)(threadIdx.x & 31u);
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+      if (lane + 32 * k < rows) {
+        x[lane + 32 * k] = u[k];
+        y[lane + 32 * k] = w[k];
+      }
+  }
+};
+template <int K>
+__device__ __forceinline__ void rot_sum_f32(int m, int n, float *x, float *y, float *vx, float *vy, float at, float c,
+                                            bool perm, unsigned (&mx)[2], float &ax, float &ay)
+{
+  ColsF32<K> g, v;
+  g.load(m, x, y);
+  v.load(n, vx, vy);
+  g.rotate(at, c);
+  g.store(m, perm ? y : x, perm ? x : y);
+  v.rotate(at, c);
+  v.store(n, perm ? vy : vx, perm ? vx : vy);
+  float mu = 0.0f, mw = 0.0f;
+#pragma unroll
+  for (int k = 0; k < K; k += 2) {
+    mu = max_nan(mu, g.u[k], g.u[k + 1]);
+    mw = max_nan(mw, g.w[k], g.w[k + 1]);
+  }
+  const unsigned bu = warp_max_bits(fp<float>::bits(mu)), bw = warp_max_bits(fp<float>::bits(mw));
+  mu = fp<float>::val(bu);
+  mw = fp<float>::val(bw);
+  const int ku = (bu && visfinite(mu)) ? -ilogb_(mu) : 0, kw = (bw && visfinite(mw)) ? -ilogb_(mw) : 0;
+  constexpr int B = fp<float>::BIAS;
+  mx[0] = perm ? bw : bu;
+  mx[1] = perm ? bu : bw;
+  if (ku >= 1 - B && ku <= B && kw >= 1 - B && kw <= B) {
+    const F32x2 pu = f2_make(pow2<float>(ku), pow2<float>(ku)), pw = f2_make(pow2<float>(kw), pow2<float>(kw));
+    float su = 0.0f, sw = 0.0f;
+#pragma unroll
+    for (int k = 0; k < K; k += 2) {
+      float a0, a1, b0, b1;
+      f2_get(f2_mul(f2_make(g.u[k], g.u[k + 1]), pu), a0, a1);
+      f2_get(f2_mul(f2_make(g.w[k], g.w[k + 1]), pw), b0, b1);
+      su = __fmaf_rn(a1, a1, __fmaf_rn(a0, a0, su));
+      sw = __fmaf_rn(b1, b1, __fmaf_rn(b0, b0, sw));
+    }
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+      su = su + __shfl_down_sync(0xffffffffu, su, o);
+      sw = sw + __shfl_down_sync(0xffffffffu, sw, o);
+    }
+    ax = perm ? sw : su;
+    ay = perm ? su : sw;
+  }
+  else {
+    __syncwarp();
+    pair_sumsq_rare(m, x, y, mx[0], mx[1], ax, ay);
+  }
+}
+// rot_real (svd_core.cuh) for longer FP32 columns at 8-byte boundaries and one warp: two rows per
 // load and packed FMAs; m is a multiple of 16. UR loads of two rows in flight.
 struct RotF32 {
   F32x2 t, tn, c;
@@ -292,6 +399,15 @@ template <typename T> __device__ __noinline__ bool put_norm(T acc, typename fp<T
   *eS = e;
   *fS = f;
   return !(d <= svdc<T>::RMAX);
+}
+
+// an FP64 dot product (its registers apart: 1500 matrices of up to 128 rows 109.5 -> 105.1 ms; FP32
+// ones are faster with theirs shared)
+__device__ __noinline__ double far_nu(int m, const double *x, const double *y, double ex, double ey, bool live)
+{
+  double zr, zi;
+  pair_nu<double, false>(m, x, nullptr, y, nullptr, ex, ey, live, zr, zi);
+  return zr;
 }
 
 // the whole SVD of one matrix by this team; returns the sweep count or an error code
@@ -449,7 +565,10 @@ __device__ long long svd_one(const BatchArgs<T> &a, BatchShared<T> &sh, long lon
         const T ep = eS[p], eq = eS[q];
         const bool live = (eq >= -svdc<T>::RMAX) && (ep >= -svdc<T>::RMAX);
         T zr, zi;
-        pair_nu<T, false>(m, col(q), nullptr, col(p), nullptr, live ? eq : (T)0, live ? ep : (T)0, live, zr, zi);
+        if constexpr (sizeof(T) == 8)
+          zr = far_nu(m, col(q), col(p), live ? eq : (T)0, live ? ep : (T)0, live);
+        else
+          pair_nu<T, false>(m, col(q), nullptr, col(p), nullptr, live ? eq : (T)0, live ? ep : (T)0, live, zr, zi);
         if (lane % L == 0)
           sh.z[lp] = live ? zr : (T)0;
       }
@@ -490,13 +609,21 @@ __device__ long long svd_one(const BatchArgs<T> &a, BatchShared<T> &sh, long lon
         T *Gp = col(p), *Gq = col(q), *Vp = V + p * n, *Vq = V + q * n;
         const T at = sh.z[lp], cc = sh.c[lp];
         U mx[2] = {0, 0};
-        bool trk = true;
+        bool trk = true, have = false;  // have: the sums of squares, too
+        T ax = (T)0, ay = (T)0;
         if ((code == 2 || code == -2) && at != (T)0) {
           U d0, d1;
           bool done = false;
 #ifdef __CUDA_ARCH__
           if constexpr (sizeof(T) == 4)
-            if (al8) {
+            if (m <= 256) {
+              if (m <= 128)
+                rot_sum_f32<4>(m, n, Gp, Gq, Vp, Vq, at, cc, code == -2, mx, ax, ay);
+              else
+                rot_sum_f32<8>(m, n, Gp, Gq, Vp, Vq, at, cc, code == -2, mx, ax, ay);
+              have = done = true;
+            }
+            else if (al8) {
               rot_f32<true>(m, Gp, Gq, at, cc, code == -2, mx[0], mx[1]);
               rot_f32<false>(n, Vp, Vq, at, cc, code == -2, d0, d1);
               done = true;
@@ -524,17 +651,19 @@ __device__ long long svd_one(const BatchArgs<T> &a, BatchShared<T> &sh, long lon
         }
         if (code == -1)
           continue;
-        warp_sync();  // the columns as written by the other lanes
-        if (!trk)
-          cols_max<T>(m, Gp, Gq, mx);
-        mx[0] = warp_max_bits(mx[0]);
-        mx[1] = warp_max_bits(mx[1]);
+        if (!have) {
+          warp_sync();  // the columns as written by the other lanes
+          if (!trk)
+            cols_max<T>(m, Gp, Gq, mx);
+          mx[0] = warp_max_bits(mx[0]);
+          mx[1] = warp_max_bits(mx[1]);
+        }
         mG = (mx[0] > mG) ? mx[0] : mG;
         mG = (mx[1] > mG) ? mx[1] : mG;
         if (last)
           continue;
-        T ax, ay;
-        pair_sumsq<T>(m, Gp, Gq, mx[0], mx[1], ax, ay);
+        if (!have)
+          pair_sumsq<T>(m, Gp, Gq, mx[0], mx[1], ax, ay);
         if (lane == 0) {
           sh.acc[lp][0] = ax;
           sh.acc[lp][1] = ay;
