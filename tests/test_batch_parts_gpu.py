@@ -63,3 +63,22 @@ def test_parts_agree(kind, order):
     torch.cuda.synchronize()
     for x, y in zip(got, (b.info, b.eS, b.fS, b.G, b.V)):
         assert torch.equal(x, y)
+
+
+def test_parts_in_a_graph():
+    import torch
+    from vecjac_gb300 import batch as B
+    from vecjac_gb300 import build
+    build.build()
+    rng = np.random.default_rng(4)
+    mats = [rng.standard_normal(s).astype(np.float32) for s in [(128, 96)] * 3 + [(32, 32)] * 500]
+    b = B.Batch(mats, "s")
+    b.run(4, block=128)
+    torch.cuda.synchronize()
+    want = [t.clone() for t in (b.info, b.eS, b.fS, b.G, b.V)]
+    g = B.capture(b, 4, block=128)
+    for _ in range(3):
+        g.replay()
+    torch.cuda.synchronize()
+    for x, y in zip(want, (b.info, b.eS, b.fS, b.G, b.V)):
+        assert torch.equal(x, y)

@@ -27,8 +27,8 @@ _BLOCK = {}
 
 def _tuned_block(A, strategy, swp):
     """Launch configuration of the batched kernel for this matrix shape and precision: the
-    CTA size (64, 128, 256 threads) at the default register bound, then the register bound
-    (resident 256-thread CTAs per SM) at the best size, each timed on up to 2432 of the
+    CTA size (64, 128, 256 threads) in the default two launches, then one launch with each
+    register bound (resident 256-thread CTAs per SM) at the best size, each timed on up to 2432 of the
     matrices (after one warm-up); the fastest (block, occupancy) is kept for the process."""
     import torch
     key = (tuple(A.shape[1:]), A.dtype, strategy)
@@ -45,12 +45,10 @@ def _tuned_block(A, strategy, swp):
             torch.cuda.synchronize()
             return e0.elapsed_time(e1)
 
-        d = 4 if A.dtype == torch.float32 else 2
-        times = {(blk, d): timed(blk, d) for blk in (64, 128, 256)}
-        best_blk = min((64, 128, 256), key=lambda b: times[(b, d)])
-        for occ in ((3, 4, 5) if A.dtype == torch.float32 else (2, 3, 4)):
-            if (best_blk, occ) not in times:
-                times[(best_blk, occ)] = timed(best_blk, occ)
+        times = {(blk, 0): timed(blk, 0) for blk in (64, 128, 256)}
+        best_blk = min((64, 128, 256), key=lambda b: times[(b, 0)])
+        for occ in (2, 3, 4):
+            times[(best_blk, occ)] = timed(best_blk, occ)
         _BLOCK[key] = min(times, key=times.get)
     return _BLOCK[key]
 

@@ -64,7 +64,7 @@ class Batch:
     def run(self, strategy=4, swp=999, block=128, stream=None, reset=True, occupancy=0):
         """Enqueue the batch (asynchronous). reset=True first restores G from the packed input.
         block: threads per CTA (64, 128, 256); occupancy: the kernel's register bound in
-        resident 256-thread CTAs per SM (2..6, 0 = the library's default)."""
+        resident 256-thread CTAs per SM (2..6 in one launch, 0 = two launches, csrc/batch.cu)."""
         if reset:
             self.G.copy_(self.G0)
         f = getattr(api.lib(), "vj_%svjsvd_batch_tuned_dev" % self.kind)
@@ -107,7 +107,7 @@ def autotune(batch, strategy=4, blocks=(64, 128, 256), occupancies=None, sample=
     per (precision, coarse size histogram)."""
     import torch
     if occupancies is None:
-        occupancies = (3, 4, 5) if batch.kind == "s" else (2, 3, 4)
+        occupancies = (2, 3, 4, 5) if batch.kind == "s" else (2, 3, 4)
     key = (batch.kind, tuple(np.histogram(batch.n, bins=[0, 32, 64, 128, 256, 513])[0] > 0), tuple(blocks),
            tuple(occupancies))
     if key in _TUNED:
