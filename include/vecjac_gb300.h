@@ -130,17 +130,19 @@ vj_fint vj_cvjsvd_dev(vj_fnat m, vj_fnat n, float *Gr, vj_fnat ldGr, float *Gi, 
 
 /* Mixed-precision SVD (FP64 data, result to FP64 accuracy): `stages` rounds (0: 2) of FP32
  * one-sided Jacobi sweeps on the current G rounded to FP32 (block sweeps on the tensor
- * cores where n allows, vj_block_sweep_dev), each followed by an FP64 Cholesky QR of the
- * accumulated rotation W (columns in ascending order of norm) and the FP64 products
- * G := G Q, V := V Q; FP64 sweeps with plain dot products on G and V to half the
- * reference's tolerance; then the FP64 finishing sweeps of dvjsvd_/zvjsvd_ with V preset
+ * cores where n allows, vj_block_sweep_dev, else sweeps by small blocks of columns or by
+ * pairs), each followed by an FP64 orthonormalisation of the accumulated rotation W
+ * (columns in ascending order of norm) and the FP64 products G := G W, V := V W; FP64
+ * refinements G := G exp(K), V := V exp(K) from the Gram matrix of G's columns to half the
+ * reference's tolerance (sweeps with plain dot products where those do not get there); then the FP64 finishing sweeps of dvjsvd_/zvjsvd_ with V preset
  * (the reference's iwork[0] != 0 mode, src/dvjsvd.c:88-96, src/zvjsvd.c:100-110), whose
  * first sweep is checked for every pair at once first and skipped when it would change
  * nothing. Shape rules and return values are dvjsvd_'s/zvjsvd_'s (the finishing phase's
  * sweep count or its error); presweeps (optional, 2 entries) receives the number of FP32
- * sweeps and of plain-dot FP64 sweeps. js/stp is the pivot table of every phase; swp caps
- * each phase (presweep phases at most 60). All arrays on the device. Links cuBLAS and
- * cuSOLVER for the FP64 GEMMs and the Cholesky factorisation. */
+ * sweeps and of FP64 refinements and plain-dot sweeps. js/stp is the pivot table of the
+ * phases by pairs; swp caps each phase (presweep phases at most 60). All arrays on the
+ * device. The FP64 products are exact digit products on the tensor cores; no library is
+ * called. */
 vj_fint vj_dvjsvd_mixed_dev(vj_fnat m, vj_fnat n, double *G, vj_fnat ldG, double *V, vj_fnat ldV, double *eS,
                             double *fS, const unsigned *js, unsigned stp, unsigned swp, unsigned stages,
                             unsigned *presweeps, void *stream);
@@ -199,8 +201,8 @@ vj_fint vj_dsvd_adjoint_batch_dev(vj_fint count, vj_fnat m, vj_fnat n, vj_fnat k
                                   const double *V, const double *dS, const double *dU, const double *dV, double *dA,
                                   double gap, void *stream);
 
-/* Batched SVD of `count` independent real matrices in one persistent launch (FP64 d,
- * FP32 s), each with the result dvjsvd_/svjsvd_ give for it (V := I, pivot strategy 2 or 4
+/* Batched SVD of `count` independent real matrices in two persistent launches (FP64 d,
+ * FP32 s; csrc/batch.cu), each with the result dvjsvd_/svjsvd_ give for it (V := I, pivot strategy 2 or 4
  * generated on the fly, sweep cap swp). All arrays are on the device: matrix b is
  * m[b] x n[b] (the reference's rules: m >= n, m % 8 / % 16, (n/2) % 8 / % 16, n <= 512),
  * column-major with leading dimension m[b] at G + offG[b]; V at V + offV[b] (n x n,
@@ -217,9 +219,9 @@ vj_fint vj_svjsvd_batch_dev(vj_fint count, const long long *m, const long long *
                             float *V, const long long *offV, float *eS, float *fS, const long long *offS,
                             const int *order, long strategy, unsigned swp, long long *info, int block, void *stream);
 /* The same with the kernel's register bound chosen: `occupancy` resident CTAs of 256
- * threads per SM (2 to 6; fewer registers per thread, more CTAs, some spills above 4 for
- * FP32 and 3 for FP64; 0 = the default, 4 for FP32 and 2 for FP64). The package's
- * autotuner searches (block, occupancy) per batch. */
+ * threads per SM in one launch (2 to 6; fewer registers per thread, more CTAs, more
+ * spills; 0 = the two launches of the form above: 2 for the matrices that finish last, 4
+ * for the others). The package's autotuner searches (block, occupancy) per batch. */
 vj_fint vj_dvjsvd_batch_tuned_dev(vj_fint count, const long long *m, const long long *n, double *G,
                                   const long long *offG, double *V, const long long *offV, double *eS, double *fS,
                                   const long long *offS, const int *order, long strategy, unsigned swp,

@@ -1,4 +1,4 @@
-"""Batched SVD of many uneven real matrices in one persistent launch, with an autotuner
+"""Batched SVD of many uneven real matrices in a call of one or two persistent launches, with an autotuner
 for the launch configuration (CTA size and the kernel's register bound, i.e. resident
 CTAs per SM) and CUDA-graph capture of the launch.
 
@@ -16,7 +16,7 @@ import numpy as np
 from . import api
 
 _TUNED = {}
-# the library's default register bound (resident 256-thread CTAs per SM) per precision
+# the register bound (resident 256-thread CTAs per SM) at which the autotuner times the CTA sizes
 DEFAULT_OCC = {"s": 4, "d": 2}
 
 

@@ -1,10 +1,10 @@
-// Batched one-sided Jacobi SVD: thousands of independent matrices of uneven size in one
-// persistent launch (real FP64 and FP32; every matrix with dvjsvd_'s / svjsvd_'s result).
+// Batched one-sided Jacobi SVD: thousands of independent matrices of uneven size in one call
+// of one or two persistent launches (real FP64 and FP32; every matrix with dvjsvd_'s / svjsvd_'s
+// result).
 //
 // A matrix is worked on by one CTA, or, when it is so large that its CTA would finish after
 // the rest of the batch, by a cluster of BATCH_CS CTAs (svd_one's team, batch_core.cuh). Each
-// team runs the reference driver on its matrix (src/dvjsvd.c:78-638) with one barrier per
-// pivot step. Matrices are handed out by atomic work queues in the order the caller gives
+// team runs the reference driver on its matrix (src/dvjsvd.c:78-638). Matrices are handed out by atomic work queues in the order the caller gives
 // (largest first balances the tail); a matrix stops at its own convergence (its own sweep
 // count, its own info entry), so uneven convergence does not hold the batch back. Pivot pairs
 // are computed on the fly from the strategy's closed form (pjs.cuh), so no tables are stored.

@@ -4,8 +4,9 @@
 // The n columns of the FP32 matrix G (m x n, split real/imaginary planes) and of the
 // rotation accumulator W (n x n) are cut into blocks of b columns (b = 64 real, 32
 // complex, so that a block pair is 128 real columns: [G_I G_J], or [Re G_I Re G_J Im G_I
-// Im G_J]). A block sweep visits every pair of blocks once in the round-robin order, n/b/2
-// independent pairs per block step, and for each pair
+// Im G_J]). A block sweep visits every pair of blocks once, n/b/2 independent pairs per block step, in
+// the modulus order with the longer columns first for the mixed SVD (half the sweeps of the round-robin
+// order, which the separate entry points keep), and for each pair
 //   1. k_gram:  S = X^T X, the real Gram matrix of the pair's 128 real columns X (128 x 128,
 //      K = m, split over several CTAs), on the tensor cores (its symmetry halves the cross
 //      terms of the split products), and k_gram_reduce: the sum over the K splits;

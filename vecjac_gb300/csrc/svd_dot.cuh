@@ -1,7 +1,8 @@
 // The SVD's scaled compensated dot products in the reference's lane order (src/ddpscl.c,
 // src/zdpscl.c): the per-precision constants, 2Sum, the lanes' halving-tree sum, the
-// 8/16-lane form (pair_dot: the FP32 step and the batched kernel) and the FP64 form with
-// one accumulator chain per warp (chain_dot: the FP64 step). Device code that needs only
+// 8/16-lane form (pair_nu: the batched kernel; pair_dot: its quotient) and the FP64 form with
+// one accumulator chain per warp (chain_dot: the check of a whole sweep's pairs; the step kernel,
+// jsvd.cu, splits products and chains between warps itself). Device code that needs only
 // vj_fp.cuh, threadIdx.x and __shfl_down_sync, so that a host harness can run it lane by
 // lane.
 #pragma once

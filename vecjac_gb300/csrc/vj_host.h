@@ -32,7 +32,7 @@ struct NearestRounding {
 // true when a CUDA device is usable (checked once; the current device is used)
 bool gpu_ready();
 // Library state is kept per device (the current device of each call): SM count, staging
-// buffers, streams, the batch queue, the cuBLAS / cuSOLVER handles of the mixed SVD.
+// buffers, streams, the batch queues.
 constexpr int MAX_DEVICES = 64;
 int device_slot();
 int sm_count();
@@ -97,7 +97,7 @@ bool trace_enabled();
 void trace_phases(const unsigned long long *cycles, int count);
 
 // phase times (ms) of the last mixed-precision SVD, its number of FP32 launches and whether
-// its FP32 stages ran as block sweeps on the tensor cores (1) or column-pair sweeps (0)
+// its FP32 stages ran as block sweeps on the tensor cores (1) or by small blocks or pairs (0)
 void mixed_phases_set(double fp32, double gemm, double fp64, double fin, double fp32_steps, double block);
 
 // elements per chunk of a host-pointer 2x2 call (a multiple of `lanes`)
