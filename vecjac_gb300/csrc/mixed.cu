@@ -1184,6 +1184,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     unsigned sw64 = 0;
     bool sweeps = true;
     double before = 1e300;
+    constexpr unsigned MAXIT = 20;  // Gram matrices at most
     constexpr unsigned CAP = 8192;  // pairs of nearly equal norms that are rotated one by one
     uint2 *const list = reinterpret_cast<uint2 *>(d2);  // (free between the products)
     double *const rows = vec;
@@ -1202,16 +1203,16 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
       k_rowmax<<<1, 1024, 0, s>>>(ni, rows, st);
       return read_stats();
     };
-    for (unsigned it = 0; it < 12u && swp; ++it) {
+    for (unsigned it = 0; it < MAXIT && swp; ++it) {
       oz::Operand oa, ob;
       // (5 digits give the first cosines, of the order of FP32 rounding, to about 1e-11)
       const int nd = it ? 8 : 5;
       if (!survey(nd))
         return VJ_ERR_CUDA;
-      const double cmax = asdbl(hst.cosmax), f = std::min(std::sqrt(hst.f2), asdbl(hst.rowmax) + 1e-7 * (double)n);
+      const double cmax = asdbl(hst.cosmax), norm = std::min(std::sqrt(hst.f2), asdbl(hst.rowmax) + 1e-7 * (double)n);
       if (trace)
         std::fprintf(stderr, "mixed SVD refinement %u: %u pairs above the tolerance, max |cos| %.3e, |K| <= %.2e, %u left "
-                     "out, %.1f ms since the phase began\n", it, hst.over, cmax, f, hst.skipped,
+                     "out, %.1f ms since the phase began\n", it, hst.over, cmax, norm, hst.skipped,
                      std::chrono::duration<double, std::milli>(now() - t0).count());
       if (nd == 8 && !hst.over && cmax <= tol64) {
         sweeps = false;
@@ -1224,7 +1225,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
         std::vector<uint2> hl(hst.skipped < CAP ? hst.skipped : CAP);
         std::vector<unsigned> hp;
         std::vector<char> used((size_t)n, 0);
-        if (hst.skipped > (unsigned)(n / 2) || hst.skipped > CAP || it == 11u ||
+        if (hst.skipped > (unsigned)(n / 2) || hst.skipped > CAP || it + 1u == MAXIT ||
             cudaMemcpyAsync(hl.data(), list, hl.size() * sizeof(uint2), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaStreamSynchronize(s) != cudaSuccess)
           break;
@@ -1243,10 +1244,19 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
           return VJ_ERR_CUDA;
         continue;
       }
-      // (the series below is to eighth order: |K|^9 / 9! stays below rounding)
-      if (!(f <= 0.06) || !(cmax <= 0.25 * before))
+      if (!(norm <= 0.48) || !(cmax <= 0.25 * before))
         break;
       before = cmax;
+      // The series below is to eighth order (|K|^9 / 9! stays below rounding up to 0.06); the
+      // rotation by a larger K is that by K / 2^r, 2^r times. (4096 x 2048 complex with sigma down to
+      // 1e-8, whose FP32 stages leave |K| = 0.2: 194 ms instead of 1016 with the sweeps)
+      int reps = 1;
+      while (norm > 0.06 * reps)
+        reps *= 2;
+      const double f = norm / reps;
+      if (reps > 1)
+        k_lincomb<<<(unsigned)std::min<size_t>((P * nn + 255) / 256, 4096), 256, 0, s>>>((long long)(P * nn), 1.0 / reps,
+                                                                                      K.re, 0.0, K.re);
       // orders of the series: |K|^(order + 1) / (order + 1)! below 5e-17
       const int order = (f < 1e-8) ? 1 : (f < 6e-6) ? 2 : (f < 1.8e-4) ? 3 : (f < 1.4e-3) ? 4 : (f < 5.7e-3) ? 5 : (f < 0.015) ? 6 : (f < 0.03) ? 7 : 8;
       const long long np = (long long)(P * nn);
@@ -1282,10 +1292,17 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
           return VJ_ERR_CUDA;
       }
       k_exp_parts<<<tiles, tblk, 0, s>>>(ni, K, Ev, ek, Q);
-      if (!cut_rows(G, Gi, sc.ldr, sc.ldi, mi, ek, oa) || !cut_prod(K, nullptr, ob) || !mult_g(oa, ob, ek, 1, ng) ||
-          !cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, nullptr, oa) || !cut_prod(Q, nullptr, ob) ||
-          !mult_v(oa, ob, 1, nv))
+      if (!cut_prod(K, nullptr, ob))
         return VJ_ERR_CUDA;
+      for (int r = 0; r < reps; ++r)
+        if (!cut_rows(G, Gi, sc.ldr, sc.ldi, mi, ek, oa) || !mult_g(oa, ob, ek, 1, ng))
+          return VJ_ERR_CUDA;
+      if (!cut_prod(Q, nullptr, ob))
+        return VJ_ERR_CUDA;
+      for (int r = 0; r < reps; ++r)
+        if (!cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, nullptr, oa) ||
+            !mult_v(oa, ob, 1, nv))
+          return VJ_ERR_CUDA;
       ++sw64;
     }
     // A sweep whose rotated pairs all had |cos| <= 1e-11 leaves off-diagonal terms of the
