@@ -163,9 +163,9 @@ def vjsvd_dev(kind, m, n, G, ldG, V, ldV, eS, fS, js, stp, swp=999, preset=False
 def vjsvd_mixed_dev(kind, m, n, G, ldG, V, ldV, eS, fS, js, stp, swp=999, Gi=None, ldGi=None, Vi=None, ldVi=None,
                     stream=None, stages=0):
     """Mixed-precision device SVD of FP64 data (kind "d" or "z"): `stages` (0: 2) rounds of
-    FP32 sweeps with FP64 re-orthogonalisation, plain-dot FP64 sweeps, then the reference's
-    FP64 sweeps with V preset. Returns (finishing sweeps or error code, FP32 sweeps,
-    plain-dot FP64 sweeps)."""
+    FP32 sweeps with FP64 re-orthogonalisation, FP64 refinements (or plain-dot sweeps), then the
+    reference's FP64 sweeps with V preset. Returns (finishing sweeps or error code, FP32 sweeps,
+    FP64 refinements and plain-dot sweeps)."""
     if kind not in "dz":
         raise ValueError("the mixed-precision SVD takes FP64 data (kind d or z)")
     L = lib()
