@@ -623,6 +623,7 @@ struct PairStats {
   unsigned long long cosmax, cosbound;  // largest |cos| and largest upper bound of one (bits of doubles)
   double f2;                            // squared Frobenius norm of the rotation generator
   unsigned long long rowmax;            // its largest row sum (bits of a double)
+  unsigned long long genmax, factmax;   // its largest entry in scaled form; that of the factor of G (bits)
   unsigned over, skipped;               // pairs above the tolerance; of those, not in the generator
   unsigned listed;                      // the latter again, as they are listed
 };
@@ -689,14 +690,15 @@ __global__ void __launch_bounds__(256) k_neg_upper(int n, Mat H, Mat M, PairStat
 // The generator K of the rotation exp(K) that makes the columns of G orthogonal to first order,
 // from the lower triangle of the Gram matrix H of the columns times 2^-e_j: K_ij = h_ij / (h_jj -
 // h_ii) in the columns' true lengths, stored as K~_ij = 2^(e_i - e_j) K_ij (the factor of column i
-// of length about 1 in column j of length about 1: never much larger than the cosine, however the
-// lengths differ). Pairs with |cos| below `tol` / 4 are left alone; pairs with |K_ij| > 2^-6 (nearly
+// of length about 1 in column j of length about 1: a few times the cosine at most where the lengths
+// differ, the cosine over the squared lengths' relative difference, up to 2^-6, where they nearly
+// agree; st->genmax: the largest of them). Pairs with |cos| below `tol` / 4 are left alone; pairs with |K_ij| > 2^-6 (nearly
 // equal lengths) too: they are counted, and the first `cap` of them go to list. rows: the row sums of
 // |K_ij|. hb: bound of the error of a Gram entry.
 __global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, Mat Kt, double tol, double hb,
                                                    PairStats *st, double *rows, uint2 *list, unsigned cap)
 {
-  double cm = 0, cb = 0, f2 = 0;
+  double cm = 0, cb = 0, f2 = 0, km = 0;
   unsigned over = 0, skipped = 0;
   lower_tiles(
       n,
@@ -721,6 +723,7 @@ __global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, M
               if (k <= 0.015625 * fabs(di)) {
                 kij = make_double2(hr / di, him / di);
                 kji = make_double2(-hr / dj, him / dj);
+                km = fmax(km, a / fmin(fabs(di), fabs(dj)));
                 const double q = k / fabs(di);
                 f2 += 2.0 * q * q;
                 if (q > 1e-7) {  // (n smaller ones add at most 1e-7 n to a row sum)
@@ -750,6 +753,7 @@ __global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, M
   for (int o = 16; o >= 1; o >>= 1) {
     cm = fmax(cm, __shfl_xor_sync(0xffffffffu, cm, o));
     cb = fmax(cb, __shfl_xor_sync(0xffffffffu, cb, o));
+    km = fmax(km, __shfl_xor_sync(0xffffffffu, km, o));
     f2 += __shfl_xor_sync(0xffffffffu, f2, o);
     over += __shfl_xor_sync(0xffffffffu, over, o);
     skipped += __shfl_xor_sync(0xffffffffu, skipped, o);
@@ -757,6 +761,7 @@ __global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, M
   if (threadIdx.x == 0 && blockIdx.y <= blockIdx.x) {
     stat_max(&st->cosmax, cm);
     stat_max(&st->cosbound, cb);
+    stat_max(&st->genmax, km);
     if (f2 > 0)
       atomicAdd(&st->f2, f2);
     if (over)
@@ -788,10 +793,16 @@ __global__ void k_lincomb(long long n, double a, const double *x, double b, doub
 // From the odd and even parts O~, E~ of exp(K) - I in scaled form (E may be empty): O~ := O~ + E~ (for
 // the columns of G), and N = exp(K) - I in true form (for V), whose two entries of a pair both
 // come from the scaled entry that is divided by the ratio of the lengths, by the parts' symmetry
-// (O^H = -O, E^H = E): the other one would be multiplied by it, errors included.
-__global__ void __launch_bounds__(256) k_exp_parts(int n, Mat O, Mat E, const int *e, Mat N)
+// (O^H = -O, E^H = E): the other one would be multiplied by it, errors included. The largest |entry| of
+// the new O~ into st->factmax.
+__global__ void __launch_bounds__(256) k_exp_parts(int n, Mat O, Mat E, const int *e, Mat N, PairStats *st)
 {
   __shared__ double2 so[32][33], se[32][33];
+  double mx = 0;
+  auto large = [&](const double2 &v) {
+    const double a = fmax(fabs(v.x), fabs(v.y));
+    mx = (v.x == v.x && v.y == v.y) ? fmax(mx, a) : 1e300;  // (a NaN must not pass for a small value)
+  };
   const int bi = blockIdx.x, bj = blockIdx.y;
   if (bj > bi)
     return;
@@ -814,12 +825,14 @@ __global__ void __launch_bounds__(256) k_exp_parts(int n, Mat O, Mat E, const in
       const size_t o = (size_t)j * n + i;
       const double2 a = get(O, o), b = get(E, o);
       double2 x = make_double2(a.x + b.x, a.y + b.y), y = make_double2(0, 0);
+      large(x);
       O.re[o] = x.x;
       if (O.im)
         O.im[o] = x.y;
       if (i != j) {
         const double2 c = so[k][threadIdx.x], f = se[k][threadIdx.x];
         so[k][threadIdx.x] = make_double2(c.x + f.x, c.y + f.y);
+        large(so[k][threadIdx.x]);
         const int d = max(-2000, min(2000, e[j] - e[i]));
         if (d <= 0) {
           y = make_double2(scalbn(b.x - a.x, d), scalbn(a.y - b.y, d));  // (j, i) from (i, j)
@@ -849,6 +862,10 @@ __global__ void __launch_bounds__(256) k_exp_parts(int n, Mat O, Mat E, const in
       }
     }
   }
+  for (int o = 16; o >= 1; o >>= 1)
+    mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  if (threadIdx.x == 0)
+    stat_max(&st->factmax, mx);
 }
 
 static bool copy2d(double *dst, long long ldd, const double *src, long long lds, long long rows, long long cols,
@@ -1261,7 +1278,10 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
       const int order = (f < 1e-8) ? 1 : (f < 6e-6) ? 2 : (f < 1.8e-4) ? 3 : (f < 1.4e-3) ? 4 : (f < 5.7e-3) ? 5 : (f < 0.015) ? 6 : (f < 0.03) ? 7 : 8;
       const long long np = (long long)(P * nn);
       const unsigned gl = (unsigned)((np + 255) / 256 < 4096 ? (np + 255) / 256 : 4096);
-      const int nk = digits(f * f), ng = digits(8.0 * cmax), nv = digits(f);  // for the powers of K, G N, V N
+      // digits for the powers of K and for V N; for G N by the largest entry of its factor, which may be
+      // any number of times the largest cosine (pairs of nearly equal lengths), below
+      const double x = std::max(f, asdbl(hst.genmax) / reps);
+      const int nk = digits(x * x), nv = digits(f);
       // exp(K) - I = E + O with E = K^2 (1/2! + K^2 (1/4! + ...)), O = K + K (K^2 (1/3! + K^2 (1/5! + ...)))
       static const double inv[9] = {1.0, 1.0, 1.0 / 2, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720, 1.0 / 5040, 1.0 / 40320};
       Mat Ev{nullptr, nullptr};
@@ -1291,9 +1311,10 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
                         !mult(oa, ob, K, 1, nk)))
           return VJ_ERR_CUDA;
       }
-      k_exp_parts<<<tiles, tblk, 0, s>>>(ni, K, Ev, ek, Q);
-      if (!cut_prod(K, nullptr, ob))
+      k_exp_parts<<<tiles, tblk, 0, s>>>(ni, K, Ev, ek, Q, st);
+      if (!read_stats() || !cut_prod(K, nullptr, ob))
         return VJ_ERR_CUDA;
+      const int ng = digits(8.0 * asdbl(hst.factmax));
       for (int r = 0; r < reps; ++r)
         if (!cut_rows(G, Gi, sc.ldr, sc.ldi, mi, ek, oa) || !mult_g(oa, ob, ek, 1, ng))
           return VJ_ERR_CUDA;
