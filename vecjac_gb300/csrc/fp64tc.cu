@@ -10,9 +10,9 @@
 // s + t < nd share an FP32 accumulator in TMEM: its integers stay below 2^24 for 128 elements
 // of K (at most 8 pairs of products up to 2^14), so every sum is exact; then the accumulators
 // are read out into 64-bit integers, which hold the sums of up to 2^22 elements of K exactly, and the two halves of the weights are joined and rounded once at the end. What is
-// left out, the pairs of weight nd and above and the digits past the last, is below 2^-50.8
-// (nd = 7) or 2^-59.6 (nd = 8) of K times the two rows' scales (each at most four times its
-// row's largest entry).
+// left out, the pairs of weight nd and above and the digits past the last, is below 2^-54.9 (nd = 7) or
+// 2^-62.8 (nd = 8; OMITTED8 of gram_bound.cuh) of K times the two rows' scales (the powers of two by
+// which they are divided, at most four times their largest entries).
 //
 // k_gemm: a CTA forms a 128 x 64 tile of C: eight accumulators of 64 columns fill the 512 columns
 // of TMEM. Two operand stages of KB = 32 (up to 96 KiB each) come by bulk copies; one thread

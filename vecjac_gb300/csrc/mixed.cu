@@ -38,6 +38,7 @@
 #include <cuda_runtime.h>
 
 #include "fp64tc.cuh"
+#include "gram_bound.cuh"
 #include "presweep.cuh"
 #include "svd_core.cuh"
 #include "vj_fp.cuh"
@@ -694,7 +695,7 @@ __global__ void __launch_bounds__(256) k_neg_upper(int n, Mat H, Mat M, PairStat
 // differ, the cosine over the squared lengths' relative difference, up to 2^-6, where they nearly
 // agree; st->genmax: the largest of them). Pairs with |cos| below `tol` / 4 are left alone; pairs with |K_ij| > 2^-6 (nearly
 // equal lengths) too: they are counted, and the first `cap` of them go to list. rows: the row sums of
-// |K_ij|. hb: bound of the error of a Gram entry.
+// |K_ij|. hb: bound of the error of each real sum in a Gram entry (1e300: none, no certificate).
 __global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, Mat Kt, double tol, double hb,
                                                    PairStats *st, double *rows, uint2 *list, unsigned cap)
 {
@@ -709,10 +710,10 @@ __global__ void __launch_bounds__(256) k_generator(int n, Mat H, const int *e, M
           const double hr = H.re[o], him = H.im ? H.im[o] : 0.0;
           const double hi = H.re[(size_t)i * n + i], hj = H.re[(size_t)j * n + j];
           if (hi > 0 && hj > 0) {
-            const double a = H.im ? hypot(hr, him) : fabs(hr), s = rsqrt(hi) * rsqrt(hj);
-            const double c = a * s;
+            const double a = H.im ? hypot(hr, him) : fabs(hr), ri = rsqrt(hi), rj = rsqrt(hj);
+            const double c = a * (ri * rj);
             cm = (c <= 2.0) ? fmax(cm, c) : 2.0;  // (a NaN counts as large)
-            cb = (c <= 2.0) ? fmax(cb, (a * (1.0 + 1e-14) + hb) * s * (1.0 + 1e-14)) : 2.0;
+            cb = (c <= 2.0) ? fmax(cb, oz::cosine_bound(a, ri, rj, hb, H.im != nullptr)) : 2.0;
             over += (c > tol) ? 1u : 0u;
             if (c > 0.25 * tol) {
               // d = e_j - e_i: denominators h_jj 4^d - h_ii and h_jj - h_ii 4^-d
@@ -1191,7 +1192,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   //    Pairs of nearly equal norms, whose rotation is not small, are rotated one by one before;
   //    whatever that and a refinement cannot improve goes to the sweeps, which run until no pair
   //    is left.
-  bool certified = false;
+  bool certified = false;  // every cosine is below the finishing check's limit (k_generator's bound)
   if (total32) {
     const double u = 1.1102230246251565e-16;
     const double tol64 = 0.5 * std::sqrt((double)m) * u;
@@ -1209,8 +1210,8 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     // the Gram matrix with nd digits, the generator and what it finds; columns' exponents in ek
     auto survey = [&](int nd) {
       oz::Operand oa;
-      // digit pairs left out of the Gram entries: with 8 digits below 2^-62.8 per element of K
-      const double hb = (nd == 8) ? (double)((long long)P * m) * 1.25e-19 : 1e300;
+      // what the 8 digits leave out of a real sum over the P m elements of K
+      const double hb = (nd == 8) ? (double)((long long)P * m) * oz::OMITTED8 : 1e300;
       if (!cut_cols(G, Gi, sc.ldr, sc.ldi, mi, oa) || !gram(oa, H, 0, nd) ||
           cudaMemcpyAsync(ek, e1, (size_t)n * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
           cudaMemsetAsync(st, 0, sizeof(PairStats), s) != cudaSuccess ||
@@ -1408,7 +1409,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   host::mixed_phases_set(ms32, msgemm, ms64, msfin, steps32, blk ? 1.0 : 0.0);
   if (trace)
     std::fprintf(stderr, "mixed SVD phases (ms): FP32 sweeps %.1f, orthonormalisation + products %.1f, FP64 refinement + sort %.1f, "
-                 "finishing %.1f\n", ms32, msgemm, ms64, msfin);
+                 "finishing %.1f, certified %d\n", ms32, msgemm, ms64, msfin, certified ? 1 : 0);
   return r;
 }
 
