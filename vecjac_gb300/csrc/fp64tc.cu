@@ -9,7 +9,7 @@
 // Algorithms 59, 2012; on tensor cores D. Mukunoki et al., ISC 2020). The pairs of one weight w =
 // s + t < nd share an FP32 accumulator in TMEM: its integers stay below 2^24 for 128 elements
 // of K (at most 8 pairs of products up to 2^14), so every sum is exact; then the accumulators
-// are read out into 64-bit integers, which hold the sums of up to 2^22 elements of K exactly, and the two halves of the weights are joined and rounded once at the end. What is
+// are read out into 64-bit integers, which hold the sums of up to MAX_K elements of K exactly, and the two halves of the weights are joined and rounded once at the end. What is
 // left out, the pairs of weight nd and above and the digits past the last, is below 2^-54.9 (nd = 7) or
 // 2^-62.8 (nd = 8; OMITTED8 of gram_bound.cuh) of K times the two rows' scales (the powers of two by
 // which they are divided, at most four times their largest entries).
@@ -192,7 +192,7 @@ __device__ __forceinline__ double scaled(double x, int n) { return scalbn(x, n);
 // ND: digits used, a template so that the issue of the MMAs is straight-line code with constant
 // descriptor offsets (computed in loops, the issuing thread took three times the MMAs' own time)
 template <int ND>
-__global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Result C, int kb0, int nkb, unsigned *err)
+__global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Result C, int nkb, unsigned *err)
 {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *const smem = smem_raw + ((1024u - (tc::saddr(smem_raw) & 1023u)) & 1023u);
@@ -204,7 +204,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
   const int half = cb / (B.np / ROWB), j0 = cb * ROWB - half * B.np;
   if (j0 >= C.cols || rb * 128 >= C.rows || (C.lower && rb * 128 + 127 < j0))
     return;
-  const int nkb_all = A.kp / KB * A.parts;
   if (tid == 0) {
     tc::mbar_init1(&full[0]);
     tc::mbar_init1(&full[1]);
@@ -222,9 +221,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
   tc::fence_after();
   const uint32_t tmem = tslot;
   const long long blk = (long long)DIGITS * PLANE;  // bytes between K blocks
-  const unsigned char *const a0 = A.d + ((long long)(2 * rb) * nkb_all + kb0) * blk,
-                            *const a1 = a0 + (long long)nkb_all * blk,
-                            *const b0 = B.d + ((long long)cb * nkb_all + kb0) * blk;
+  const unsigned char *const a0 = A.d + (long long)(2 * rb) * nkb * blk, *const a1 = a0 + (long long)nkb * blk,
+                            *const b0 = B.d + (long long)cb * nkb * blk;
   auto load = [&](int kb) {
     const int st = kb & 1;
     const uint32_t s0 = tc::saddr(smem) + st * STAGE;
@@ -365,7 +363,7 @@ cudaError_t row_exponents(const Source &s, int *e, cudaStream_t st)
   return cudaGetLastError();
 }
 
-cudaError_t split(const Source &s, const Operand &o, cudaStream_t st)
+cudaError_t split_exponents(const Source &s, const Operand &o, cudaStream_t st)
 {
   if (s.mode == ROWS) {
     k_fill_int<<<(s.rows + 255) / 256, 256, 0, st>>>(o.e, s.rows, NOEXP);
@@ -375,13 +373,24 @@ cudaError_t split(const Source &s, const Operand &o, cudaStream_t st)
   else
     k_expo_cols<<<(s.rows + 7) / 8, 256, 0, st>>>(s, o.e);
   k_expo_final<<<(o.np + 255) / 256, 256, 0, st>>>(o.e, s.rows, o.np, o.halves);
+  return cudaGetLastError();
+}
+
+cudaError_t split_digits(const Source &s, const Operand &o, cudaStream_t st)
+{
   k_digits<<<dim3((unsigned)(o.kp / KB * o.parts), (unsigned)(o.np / ROWB * o.halves)), 256, 0, st>>>(s, o);
   return cudaGetLastError();
 }
 
+cudaError_t split(const Source &s, const Operand &o, cudaStream_t st)
+{
+  const cudaError_t e = split_exponents(s, o, st);
+  return (e != cudaSuccess) ? e : split_digits(s, o, st);
+}
+
 cudaError_t gemm(const Operand &A, const Operand &B, const Result &C, int nd, unsigned *err, cudaStream_t st)
 {
-  void (*const k)(Operand, Operand, Result, int, int, unsigned *) = (nd <= 3)   ? k_gemm<3>
+  void (*const k)(Operand, Operand, Result, int, unsigned *) = (nd <= 3)   ? k_gemm<3>
                                                                     : (nd == 4) ? k_gemm<4>
                                                                     : (nd == 5) ? k_gemm<5>
                                                                     : (nd == 6) ? k_gemm<6>
@@ -391,13 +400,10 @@ cudaError_t gemm(const Operand &A, const Operand &B, const Result &C, int nd, un
   if (e != cudaSuccess)
     return e;
   const dim3 grid((unsigned)(B.np / ROWB * B.halves), (unsigned)((C.rows + 127) / 128));
-  // panels of K whose sums the 64-bit integers hold (2^22 elements), added up in FP64
-  const int nkb = A.kp / KB * A.parts, most = (1 << 22) / KB;
-  Result c = C;
-  for (int kb = 0; kb < nkb; kb += most) {
-    k<<<grid, THREADS, SMEM, st>>>(A, B, c, kb, nkb - kb < most ? nkb - kb : most, err);
-    c.add = 1;
-  }
+  const long long nkb = (long long)(A.kp / KB) * A.parts;
+  if (nkb > MAX_K / KB)
+    return cudaErrorInvalidValue;
+  k<<<grid, THREADS, SMEM, st>>>(A, B, C, (int)nkb, err);
   return cudaGetLastError();
 }
 

@@ -46,8 +46,14 @@ struct Operand {
 Operand shape(const Source &s, bool cplx);
 // exponents of the source's columns (COLS; 0 for a zero column), rows entries
 cudaError_t row_exponents(const Source &s, int *e, cudaStream_t st);
-// row exponents and digits of a source
+// row exponents and digits of a source: both, or apart, where the digits are those of a part of the K
+// over which the exponents were taken (e of o; its K does not matter to the exponents)
 cudaError_t split(const Source &s, const Operand &o, cudaStream_t st);
+cudaError_t split_exponents(const Source &s, const Operand &o, cudaStream_t st);
+cudaError_t split_digits(const Source &s, const Operand &o, cudaStream_t st);
+// most rows of operands of rows, and most elements of K over all parts, that the launches and the
+// 64-bit sums take at once
+constexpr long long MAX_ROWS = 1ll << 21, MAX_K = 1ll << 22;
 
 // Where a product goes: column j of half 0 to re, of half 1 to im. Scaled: times the rows'
 // powers of two and 2^ej[j] (ej may be null). add: added to what is there. lower: only the
@@ -59,7 +65,7 @@ struct Result {
   const int *ej;
   int scaled, add, lower;
 };
-// C (+)= A B^T over the operands' K (A one half), with digits 0..nd-1 of each (3 <= nd <= 8); err is set
+// C (+)= A B^T over the operands' K (A one half, K up to MAX_K), with digits 0..nd-1 of each (3 <= nd <= 8); err is set
 // nonzero when a wait inside the kernel gave up
 cudaError_t gemm(const Operand &A, const Operand &B, const Result &C, int nd, unsigned *err, cudaStream_t st);
 

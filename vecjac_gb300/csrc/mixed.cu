@@ -919,19 +919,38 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   const int inner = (ei && atoi(ei) >= 1 && atoi(ei) <= 8) ? atoi(ei) : 1;
   const size_t blkb = blk ? ((block_sweep_scratch(CPLX, m, n, inner) + 255) & ~(size_t)255) : 0;
   // scratch: the FP32 copy of G and W (P m n and P n n floats); five P n n matrices of doubles; two
-  // digit operands of the FP64 products (fp64tc.cuh), the first as large as G's columns or rows
-  // take, the second as an n x n matrix takes, with their exponents; counters; the block sweeps'
-  // own. The columns' gather before the finishing sweeps goes through the digits' room.
+  // digit operands of the FP64 products (fp64tc.cuh), the first as large as the columns or rows
+  // of a panel of G's rows take, the second as an n x n matrix takes, with their exponents; counters;
+  // the block sweeps' own. The columns' gather before the finishing sweeps goes through the digits'
+  // room. Panels: the digits of all of G's columns take 16 (real) or 64 bytes per element, and
+  // operands have at most oz::MAX_ROWS rows, so more digits than that gather takes and 2 GiB are cut
+  // and multiplied a panel of rows at a time (whole up to 11,000 x 11,000 real, and 4,194,304 x 16 in
+  // four).
   const int ni = (int)n, mi = (int)m;
-  oz::Source sc{G, Gi, (long long)ldG, (long long)(CPLX ? ldGi : ldG), ni, mi, nullptr, 0, oz::COLS};
-  oz::Source sr{G, Gi, (long long)ldG, (long long)(CPLX ? ldGi : ldG), mi, ni, nullptr, 0, oz::ROWS};
-  const oz::Operand oc = oz::shape(sc, CPLX), orw = oz::shape(sr, CPLX);
+  const oz::Source sc{G, Gi, (long long)ldG, (long long)(CPLX ? ldGi : ldG), ni, mi, nullptr, 0, oz::COLS};
+  const long long row_digits = oz::pad(n, 128) * P * P * 2 * oz::DIGITS;  // bytes per row of G's columns
+  long long pr = (long long)(std::max(mn * 8, (size_t)1 << 31) / (size_t)row_digits);
+  pr = std::min(pr, oz::MAX_ROWS);
+  const int panel = (int)((pr >= m) ? m : std::max(pr / 128 * 128, 128ll));
+  auto panel_rows = [&](int r0) { return mi - r0 < panel ? mi - r0 : panel; };
+  // the rows of G from r0 on, as columns (against which K runs along the rows) or rows of an operand
+  auto g_cols = [&](int r0) {
+    oz::Source p = sc;
+    p.re = G + r0;
+    p.im = CPLX ? Gi + r0 : nullptr;
+    p.len = panel_rows(r0);
+    return p;
+  };
+  auto g_rows = [&](int r0, const int *x) {
+    return oz::Source{G + r0, CPLX ? Gi + r0 : nullptr, sc.ldr, sc.ldi, panel_rows(r0), ni, x, -1, oz::ROWS};
+  };
+  const oz::Operand oc = oz::shape(g_cols(0), CPLX), orw = oz::shape(g_rows(0, nullptr), CPLX);
   const oz::Operand on = oz::shape(oz::Source{G, Gi, 0, 0, ni, ni, nullptr, 0, oz::PROD}, CPLX);
   auto up = [](size_t x) { return (x + 1023) & ~(size_t)1023; };
   const size_t f32b = up(P * (mn + nn) * 4), f64b = up(5 * P * nn * 8);
   const size_t d1b = up(std::max({(size_t)oc.bytes(), (size_t)orw.bytes(), (size_t)on.bytes(), mn * 8}));
   const size_t d2b = up(std::max((size_t)on.bytes(), nn * 8));
-  const size_t e1b = up((size_t)(2 * std::max(oc.np, orw.np)) * 4), e2b = up((size_t)(2 * on.np) * 4);
+  const size_t e1b = up((size_t)2 * std::max({oc.np, orw.np, on.np}) * 4), e2b = up((size_t)(2 * on.np) * 4);
   const size_t ekb = up((size_t)n * 4), vecb = up((size_t)n * 16);
   host::Staging &stg = host::staging3();
   if (!stg.reserve(f32b + f64b + d1b + d2b + e1b + e2b + ekb + vecb + 1024 + blkb))
@@ -962,28 +981,27 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   const dim3 tiles((unsigned)((n + 31) / 32), (unsigned)((n + 31) / 32)), tblk(32, 8);
   if (cudaMemsetAsync(gerr, 0, 4, s) != cudaSuccess)
     return VJ_ERR_CUDA;
-  // X's columns (for X^H X), rows (for X Y) or an n x n matrix as the right factor, cut into digits
+  // the columns (for X^H X) or rows (for X Y) of an n x n X, or X as the right factor, cut into digits
   auto cut = [&](const oz::Source &src, unsigned char *d, int *e, oz::Operand &o) {
     o = oz::shape(src, CPLX);
     o.d = d;
     o.e = e;
     return oz::split(src, o, s) == cudaSuccess;
   };
-  auto cut_cols = [&](const double *re, const double *im, long long ldr, long long ldi, int rows, oz::Operand &o) {
-    return cut(oz::Source{re, im, ldr, ldi, ni, rows, nullptr, 0, oz::COLS}, d1, e1, o);
+  auto cut_cols = [&](const double *re, const double *im, long long ldr, long long ldi, oz::Operand &o) {
+    return cut(oz::Source{re, im, ldr, ldi, ni, ni, nullptr, 0, oz::COLS}, d1, e1, o);
   };
-  auto cut_rows = [&](const double *re, const double *im, long long ldr, long long ldi, int rows, const int *x,
-                      oz::Operand &o) {
-    return cut(oz::Source{re, im, ldr, ldi, rows, ni, x, -1, oz::ROWS}, d1, e1, o);
+  auto cut_rows = [&](const double *re, const double *im, long long ldr, long long ldi, const int *x, oz::Operand &o) {
+    return cut(oz::Source{re, im, ldr, ldi, ni, ni, x, -1, oz::ROWS}, d1, e1, o);
   };
   auto cut_prod = [&](const Mat &X, const int *x, oz::Operand &o) {
     return cut(oz::Source{X.re, X.im, n, n, ni, ni, x, 1, oz::PROD}, d2, e2, o);
   };
   // H's lower triangle = X^H X of columns cut into o
-  auto gram = [&](const oz::Operand &o, const Mat &H, int scaled, int nd) {
+  auto gram = [&](const oz::Operand &o, const Mat &H, int nd) {
     oz::Operand a = o;
     a.halves = 1;
-    return oz::gemm(a, o, oz::Result{H.re, H.im, n, n, ni, ni, nullptr, scaled, 0, 1}, nd, gerr, s) == cudaSuccess;
+    return oz::gemm(a, o, oz::Result{H.re, H.im, n, n, ni, ni, nullptr, 1, 0, 1}, nd, gerr, s) == cudaSuccess;
   };
   // X (+)= A B for an n x n X
   auto mult = [&](const oz::Operand &A, const oz::Operand &B, const Mat &X, int add, int nd) {
@@ -994,8 +1012,35 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     return oz::gemm(A, B, oz::Result{V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, ni, nullptr, 1, add, 0},
                     nd, gerr, s) == cudaSuccess;
   };
-  auto mult_g = [&](const oz::Operand &A, const oz::Operand &B, const int *ej, int add, int nd) {
-    return oz::gemm(A, B, oz::Result{G, Gi, sc.ldr, sc.ldi, mi, ni, ej, 1, add, 0}, nd, gerr, s) == cudaSuccess;
+  // G's rows enter with their columns' 2^-x
+  auto mult_g = [&](const int *x, const oz::Operand &B, const int *ej, int add, int nd) {
+    for (int r0 = 0; r0 < mi; r0 += panel) {
+      oz::Operand A;
+      if (!cut(g_rows(r0, x), d1, e1, A) ||
+          oz::gemm(A, B, oz::Result{G + r0, CPLX ? Gi + r0 : nullptr, sc.ldr, sc.ldi, panel_rows(r0), ni, ej, 1, add, 0},
+                   nd, gerr, s) != cudaSuccess)
+        return false;
+    }
+    return true;
+  };
+  // H's lower triangle = G^H G, the columns divided by their powers of two (left in e1)
+  auto gram_g = [&](const Mat &H, int nd) {
+    oz::Operand o = oc;
+    o.e = e1;
+    if (oz::split_exponents(sc, o, s) != cudaSuccess)
+      return false;
+    for (int r0 = 0; r0 < mi; r0 += panel) {
+      const oz::Source p = g_cols(r0);
+      o = oz::shape(p, CPLX);
+      o.d = d1;
+      o.e = e1;
+      oz::Operand a = o;
+      a.halves = 1;
+      if (oz::split_digits(p, o, s) != cudaSuccess ||
+          oz::gemm(a, o, oz::Result{H.re, H.im, n, n, ni, ni, nullptr, 0, r0 ? 1 : 0, 1}, nd, gerr, s) != cudaSuccess)
+        return false;
+    }
+    return true;
   };
   // digits that a correction of relative size x needs: what nd digits leave out, about 2^(5 - 8 nd)
   // of a product of rows of length 1, stays below 2^-57
@@ -1135,7 +1180,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     // justify: 4 give E to 1e-9, 6 to 1e-13)
     int nd = 4;
     for (int round = 0;; ++round) {
-      if (!cut_cols(T.re, T.im, n, n, ni, oa) || !gram(oa, M[1], 1, nd) ||
+      if (!cut_cols(T.re, T.im, n, n, oa) || !gram(oa, M[1], nd) ||
           cudaMemsetAsync(st, 0, sizeof(PairStats), s) != cudaSuccess)
         return VJ_ERR_CUDA;
       k_neg_upper<<<tiles, tblk, 0, s>>>(ni, M[1], M[2], st);
@@ -1146,7 +1191,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
         std::fprintf(stderr, "mixed SVD stage %u: largest entry of W^H W - I %.2e\n", stage, emax);
       if (!(emax < 0.03) || round == 8)
         return VJ_ERR_CUDA;  // W was not near unitary
-      if (!cut_rows(T.re, T.im, n, n, ni, nullptr, oa) || !cut_prod(M[2], nullptr, ob) ||
+      if (!cut_rows(T.re, T.im, n, n, nullptr, oa) || !cut_prod(M[2], nullptr, ob) ||
           !mult(oa, ob, T, 1, digits(emax)))
         return VJ_ERR_CUDA;
       const double next = std::max(emax * emax * rn_, nd == 4 ? 1e-9 : nd == 6 ? 1e-13 : 0.0);
@@ -1161,11 +1206,10 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
       if (!copy2d(V, ldV, T.re, n, n, n, s) || (CPLX && !copy2d(Vi, ldVi, T.im, n, n, n, s)))
         return VJ_ERR_CUDA;
     }
-    else if (!cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, nullptr, oa) ||
+    else if (!cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), nullptr, oa) ||
              !cut_prod(T, nullptr, ob) || !mult_v(oa, ob, 0, 8))
       return VJ_ERR_CUDA;
-    if (oz::row_exponents(sc, ek, s) != cudaSuccess || !cut_rows(G, Gi, sc.ldr, sc.ldi, mi, ek, oa) ||
-        !cut_prod(T, ek, ob) || !mult_g(oa, ob, nullptr, 0, 8))
+    if (oz::row_exponents(sc, ek, s) != cudaSuccess || !cut_prod(T, ek, ob) || !mult_g(ek, ob, nullptr, 0, 8))
       return VJ_ERR_CUDA;
     {
       if (cudaStreamSynchronize(s) != cudaSuccess)
@@ -1202,6 +1246,8 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     unsigned sw64 = 0;
     bool sweeps = true;
     double before = 1e300;
+    // (the entries of a Gram matrix of several panels are rounded sums of the panels')
+    const double pan = (panel < mi) ? 4.0 * u * (double)((mi + panel - 1) / panel) : 0.0;
     constexpr unsigned MAXIT = 20;  // Gram matrices at most
     constexpr unsigned CAP = 8192;  // pairs of nearly equal norms that are rotated one by one
     uint2 *const list = reinterpret_cast<uint2 *>(d2);  // (free between the products)
@@ -1209,11 +1255,9 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     const Mat &H = M[0], &K = M[1], &S = M[2], &Q = M[3], &E = M[4];
     // the Gram matrix with nd digits, the generator and what it finds; columns' exponents in ek
     auto survey = [&](int nd) {
-      oz::Operand oa;
       // what the 8 digits leave out of a real sum over the P m elements of K
       const double hb = (nd == 8) ? (double)((long long)P * m) * oz::OMITTED8 : 1e300;
-      if (!cut_cols(G, Gi, sc.ldr, sc.ldi, mi, oa) || !gram(oa, H, 0, nd) ||
-          cudaMemcpyAsync(ek, e1, (size_t)n * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
+      if (!gram_g(H, nd) || cudaMemcpyAsync(ek, e1, (size_t)n * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess ||
           cudaMemsetAsync(st, 0, sizeof(PairStats), s) != cudaSuccess ||
           cudaMemsetAsync(rows, 0, (size_t)n * 8, s) != cudaSuccess)
         return false;
@@ -1234,7 +1278,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
                      std::chrono::duration<double, std::milli>(now() - t0).count());
       if (nd == 8 && !hst.over && cmax <= tol64) {
         sweeps = false;
-        certified = (asdbl(hst.cosbound) <= lim);
+        certified = (asdbl(hst.cosbound) + pan <= lim);
         break;
       }
       if (hst.skipped) {
@@ -1288,12 +1332,12 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
       Mat Ev{nullptr, nullptr};
       if (order >= 2) {
         const Mat &P2 = H;  // K^2 takes the Gram matrix's place
-        if (!cut_rows(K.re, K.im, n, n, ni, nullptr, oa) || !cut_prod(K, nullptr, ob) || !mult(oa, ob, P2, 0, nk))
+        if (!cut_rows(K.re, K.im, n, n, nullptr, oa) || !cut_prod(K, nullptr, ob) || !mult(oa, ob, P2, 0, nk))
           return VJ_ERR_CUDA;
         Ev = E;
         const int te = order & ~1, to = (order - 1) | 1;  // the last even and odd orders
         const bool powers = te >= 4 || to >= 5;
-        if (powers && !cut_rows(P2.re, P2.im, n, n, ni, nullptr, oa))
+        if (powers && !cut_rows(P2.re, P2.im, n, n, nullptr, oa))
           return VJ_ERR_CUDA;
         // X := c_last K^2, then X := c K^2 + K^2 X down to the order of `first`
         auto horner = [&](const Mat &X, int last, int first) {
@@ -1308,7 +1352,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
         };
         if (!horner(E, te, 2) || (to >= 3 && !horner(S, to, 3)))
           return VJ_ERR_CUDA;
-        if (to >= 3 && (!cut_rows(K.re, K.im, n, n, ni, nullptr, oa) || !cut_prod(S, nullptr, ob) ||
+        if (to >= 3 && (!cut_rows(K.re, K.im, n, n, nullptr, oa) || !cut_prod(S, nullptr, ob) ||
                         !mult(oa, ob, K, 1, nk)))
           return VJ_ERR_CUDA;
       }
@@ -1317,13 +1361,12 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
         return VJ_ERR_CUDA;
       const int ng = digits(8.0 * asdbl(hst.factmax));
       for (int r = 0; r < reps; ++r)
-        if (!cut_rows(G, Gi, sc.ldr, sc.ldi, mi, ek, oa) || !mult_g(oa, ob, ek, 1, ng))
+        if (!mult_g(ek, ob, ek, 1, ng))
           return VJ_ERR_CUDA;
       if (!cut_prod(Q, nullptr, ob))
         return VJ_ERR_CUDA;
       for (int r = 0; r < reps; ++r)
-        if (!cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, nullptr, oa) ||
-            !mult_v(oa, ob, 1, nv))
+        if (!cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), nullptr, oa) || !mult_v(oa, ob, 1, nv))
           return VJ_ERR_CUDA;
       ++sw64;
     }
@@ -1350,7 +1393,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     if (sweeps && sw64) {
       if (!survey(8))
         return VJ_ERR_CUDA;
-      certified = (!hst.over && asdbl(hst.cosbound) <= lim);
+      certified = (!hst.over && asdbl(hst.cosbound) + pan <= lim);
     }
     unsigned herr = 0;
     if (cudaMemcpyAsync(&herr, gerr, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
