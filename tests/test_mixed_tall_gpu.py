@@ -39,3 +39,10 @@ def run(kind, m, n, seed=1):
 @pytest.mark.parametrize("kind", ["d", "z"])
 def test_more_rows_than_a_grid(kind):
     run(kind, 65535 * 64 + 72, 16)
+
+
+@pytest.mark.parametrize("kind", ["d", "z"])
+@pytest.mark.parametrize("m,n", [(1000, 16), (1032, 16), (2056, 96), (5000, 80), (33336, 64), (40008, 144)])
+def test_split_k(kind, m, n):
+    """K split over CTAs: from one slice to many, the last of them shorter than the others."""
+    run(kind, m, n)

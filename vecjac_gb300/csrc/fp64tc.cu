@@ -17,9 +17,12 @@
 // k_gemm: a CTA forms a 128 x 64 tile of C: eight accumulators of 64 columns fill the 512 columns
 // of TMEM. Two operand stages of KB = 32 (up to 96 KiB each) come by bulk copies; one thread
 // issues copies and MMAs; all eight warps read out. The operands' blocks come from L2 (84 KiB
-// per 56 MMAs of 128 x 64 x 16 with nd = 7), which bounds it.
+// per 56 MMAs of 128 x 64 x 16 with nd = 7), which bounds it. Where the tiles are fewer than half of the
+// SMs and K is long (the Gram matrix of a tall matrix: one tile up to n = 64), several CTAs take a
+// stretch of K each and leave their integers, which k_gemm_sum adds up: still exact, so the same bits.
 #include "fp64tc.cuh"
 
+#include <algorithm>
 #include <cstdint>
 
 #include "tc.cuh"
@@ -189,10 +192,33 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, unsigne
 // 2^n x for a normal or zero x and any n (exact while the result is normal)
 __device__ __forceinline__ double scaled(double x, int n) { return scalbn(x, n); }
 
+// entry (r, j) of C's half from its sums of weights 0-3 and 4-7
+__device__ __forceinline__ void put_entry(const Operand &A, const Operand &B, const Result &C, int half, int r, int j,
+                                          int er, long long hi, long long lo)
+{
+  double *const out = half ? C.im : C.re;
+  const long long ld = half ? C.ldi : C.ldr;
+  // (hi 2^32 + lo) 2^-72
+  double v = fma((double)hi, 4294967296.0, (double)lo);
+  v = scaled(v, -72 + (C.scaled ? er + B.e[half * B.np + j] + (C.ej ? C.ej[j] : 0) : 0));
+  double *const to = out + (long long)j * ld + r;
+  *to = C.add ? *to + v : v;
+}
+
+// column tiles per half of C
+__host__ __device__ inline int col_tiles(const Result &C) { return (C.cols + ROWB - 1) / ROWB; }
+
+// where the sums of slice blockIdx.z of tile (cb, rb) begin: 64 columns of 128 rows
+__device__ __forceinline__ size_t part_tile(int cb, int rb)
+{
+  return (((size_t)blockIdx.z * gridDim.y + rb) * gridDim.x + cb) * (size_t)(128 * ROWB);
+}
+
 // ND: digits used, a template so that the issue of the MMAs is straight-line code with constant
 // descriptor offsets (computed in loops, the issuing thread took three times the MMAs' own time)
 template <int ND>
-__global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Result C, int nkb, unsigned *err)
+__global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Result C, int nkb_all, longlong2 *part,
+                                                       unsigned *err)
 {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char *const smem = smem_raw + ((1024u - (tc::saddr(smem_raw) & 1023u)) & 1023u);
@@ -201,8 +227,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
   __shared__ int s_fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int cb = blockIdx.x, rb = blockIdx.y;  // 64 columns, 128 rows
-  const int half = cb / (B.np / ROWB), j0 = cb * ROWB - half * B.np;
-  if (j0 >= C.cols || rb * 128 >= C.rows || (C.lower && rb * 128 + 127 < j0))
+  const int half = cb / col_tiles(C), j0 = (cb - half * col_tiles(C)) * ROWB;
+  if (C.lower && rb * 128 + 127 < j0)
     return;
   if (tid == 0) {
     tc::mbar_init1(&full[0]);
@@ -220,9 +246,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
   __syncthreads();
   tc::fence_after();
   const uint32_t tmem = tslot;
+  // this CTA's stretch of K
+  const int per = (nkb_all + (int)gridDim.z - 1) / (int)gridDim.z, kb0 = (int)blockIdx.z * per,
+            nkb = min(per, nkb_all - kb0);
   const long long blk = (long long)DIGITS * PLANE;  // bytes between K blocks
-  const unsigned char *const a0 = A.d + (long long)(2 * rb) * nkb * blk, *const a1 = a0 + (long long)nkb * blk,
-                            *const b0 = B.d + (long long)cb * nkb * blk;
+  const unsigned char *const a0 = A.d + ((long long)(2 * rb) * nkb_all + kb0) * blk,
+                            *const a1 = a0 + (long long)nkb_all * blk,
+                            *const b0 = B.d + ((long long)((half * B.np + j0) / ROWB) * nkb_all + kb0) * blk;
   auto load = [&](int kb) {
     const int st = kb & 1;
     const uint32_t s0 = tc::saddr(smem) + st * STAGE;
@@ -317,22 +347,21 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
     }
     (void)tc::mbar_wait(&ready, 0u, WAIT_CYCLES);
   }
+  else if (gridDim.z > 1) {
+    longlong2 *const to = part + part_tile(blockIdx.x, blockIdx.y) + (warp >> 2) * 32 * 128 + (warp & 3) * 32 + lane;
+#pragma unroll
+    for (int c = 0; c < 32; ++c)
+      to[c * 128] = make_longlong2(hi[c], lo[c]);
+  }
   else {
     const int r = rb * 128 + (warp & 3) * 32 + lane;
     if (r < C.rows) {
-      double *const out = half ? C.im : C.re;
-      const long long ld = half ? C.ldi : C.ldr;
       const int er = C.scaled ? A.e[r] : 0;
 #pragma unroll
       for (int c = 0; c < 32; ++c) {
         const int j = j0 + (warp >> 2) * 32 + c;
-        if (j < C.cols) {
-          // (hi 2^32 + lo) 2^-72
-          double v = fma((double)hi[c], 4294967296.0, (double)lo[c]);
-          v = scaled(v, -72 + (C.scaled ? er + B.e[half * B.np + j] + (C.ej ? C.ej[j] : 0) : 0));
-          double *const to = out + (long long)j * ld + r;
-          *to = C.add ? *to + v : v;
-        }
+        if (j < C.cols)
+          put_entry(A, B, C, half, r, j, er, hi[c], lo[c]);
       }
     }
   }
@@ -342,6 +371,29 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
   __syncwarp();
   if (warp == 0)
     tc::tmem_dealloc(tmem, 512);
+}
+
+// C from the slices' sums: a CTA per tile, a thread per row and column
+__global__ void __launch_bounds__(256) k_gemm_sum(Operand A, Operand B, Result C, int slices, const longlong2 *part)
+{
+  const int cb = blockIdx.x, rb = blockIdx.y;
+  const int half = cb / col_tiles(C), j0 = (cb - half * col_tiles(C)) * ROWB;
+  if (C.lower && rb * 128 + 127 < j0)
+    return;
+  const size_t slice = (size_t)gridDim.x * gridDim.y * (size_t)(128 * ROWB);
+  for (int q = threadIdx.x; q < 128 * ROWB; q += 256) {
+    const int r = rb * 128 + (q & 127), j = j0 + (q >> 7);
+    if (r >= C.rows || j >= C.cols)
+      continue;
+    long long hi = 0, lo = 0;
+    const longlong2 *p = part + part_tile(cb, rb) + q;
+#pragma unroll 4
+    for (int z = 0; z < slices; ++z, p += slice) {
+      hi += p->x;
+      lo += p->y;
+    }
+    put_entry(A, B, C, half, r, j, C.scaled ? A.e[r] : 0, hi, lo);
+  }
 }
 
 Operand shape(const Source &s, bool cplx)
@@ -388,22 +440,38 @@ cudaError_t split(const Source &s, const Operand &o, cudaStream_t st)
   return (e != cudaSuccess) ? e : split_digits(s, o, st);
 }
 
-cudaError_t gemm(const Operand &A, const Operand &B, const Result &C, int nd, unsigned *err, cudaStream_t st)
+// K blocks of a slice at least
+constexpr long long MIN_SLICE = 16;
+
+// (slices x tiles <= SMs)
+size_t part_bytes() { return (size_t)host::sm_count() * 128 * ROWB * sizeof(longlong2); }
+
+cudaError_t gemm(const Operand &A, const Operand &B, const Result &C, int nd, unsigned *err, unsigned char *part,
+                 cudaStream_t st)
 {
-  void (*const k)(Operand, Operand, Result, int, unsigned *) = (nd <= 3)   ? k_gemm<3>
-                                                                    : (nd == 4) ? k_gemm<4>
-                                                                    : (nd == 5) ? k_gemm<5>
-                                                                    : (nd == 6) ? k_gemm<6>
-                                                                    : (nd == 7) ? k_gemm<7>
-                                                                                : k_gemm<8>;
+  void (*const k)(Operand, Operand, Result, int, longlong2 *, unsigned *) = (nd <= 3)   ? k_gemm<3>
+                                                                           : (nd == 4) ? k_gemm<4>
+                                                                           : (nd == 5) ? k_gemm<5>
+                                                                           : (nd == 6) ? k_gemm<6>
+                                                                           : (nd == 7) ? k_gemm<7>
+                                                                                       : k_gemm<8>;
   const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM);
   if (e != cudaSuccess)
     return e;
-  const dim3 grid((unsigned)(B.np / ROWB * B.halves), (unsigned)((C.rows + 127) / 128));
   const long long nkb = (long long)(A.kp / KB) * A.parts;
   if (nkb > MAX_K / KB)
     return cudaErrorInvalidValue;
-  k<<<grid, THREADS, SMEM, st>>>(A, B, C, (int)nkb, err);
+  // (with lower, the tiles above the diagonal return at once)
+  dim3 grid((unsigned)(col_tiles(C) * B.halves), (unsigned)((C.rows + 127) / 128));
+  const long long tiles = (long long)grid.x * grid.y;
+  long long slices = std::min((long long)host::sm_count() / tiles, nkb / MIN_SLICE);
+  if (slices > 1)  // (none of them empty)
+    slices = (nkb + (nkb + slices - 1) / slices - 1) / ((nkb + slices - 1) / slices);
+  grid.z = (unsigned)std::max(slices, 1ll);
+  longlong2 *const sums = reinterpret_cast<longlong2 *>(part);
+  k<<<grid, THREADS, SMEM, st>>>(A, B, C, (int)nkb, sums, err);
+  if (grid.z > 1)
+    k_gemm_sum<<<dim3(grid.x, grid.y), 256, 0, st>>>(A, B, C, (int)grid.z, sums);
   return cudaGetLastError();
 }
 

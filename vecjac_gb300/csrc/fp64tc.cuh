@@ -66,8 +66,11 @@ struct Result {
   int scaled, add, lower;
 };
 // C (+)= A B^T over the operands' K (A one half, K up to MAX_K), with digits 0..nd-1 of each (3 <= nd <= 8); err is set
-// nonzero when a wait inside the kernel gave up
-cudaError_t gemm(const Operand &A, const Operand &B, const Result &C, int nd, unsigned *err, cudaStream_t st);
+// nonzero when a wait inside the kernel gave up. part: part_bytes() of scratch for products whose K is
+// split over CTAs (the same bits as unsplit).
+size_t part_bytes();
+cudaError_t gemm(const Operand &A, const Operand &B, const Result &C, int nd, unsigned *err, unsigned char *part,
+                 cudaStream_t st);
 
 }  // namespace oz
 }  // namespace vj

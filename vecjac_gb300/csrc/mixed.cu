@@ -951,9 +951,9 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   const size_t d1b = up(std::max({(size_t)oc.bytes(), (size_t)orw.bytes(), (size_t)on.bytes(), mn * 8}));
   const size_t d2b = up(std::max((size_t)on.bytes(), nn * 8));
   const size_t e1b = up((size_t)2 * std::max({oc.np, orw.np, on.np}) * 4), e2b = up((size_t)(2 * on.np) * 4);
-  const size_t ekb = up((size_t)n * 4), vecb = up((size_t)n * 16);
+  const size_t ekb = up((size_t)n * 4), vecb = up((size_t)n * 16), partb = up(oz::part_bytes());
   host::Staging &stg = host::staging3();
-  if (!stg.reserve(f32b + f64b + d1b + d2b + e1b + e2b + ekb + vecb + 1024 + blkb))
+  if (!stg.reserve(f32b + f64b + d1b + d2b + e1b + e2b + ekb + vecb + partb + 1024 + blkb))
     return VJ_ERR_NOMEM;
   unsigned char *at = reinterpret_cast<unsigned char *>(stg.ptr);
   auto take = [&](size_t bytes) {
@@ -968,6 +968,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   int *e1 = reinterpret_cast<int *>(take(e1b)), *e2 = reinterpret_cast<int *>(take(e2b));
   int *ek = reinterpret_cast<int *>(take(ekb));  // exponents of G's columns
   double *vec = reinterpret_cast<double *>(take(vecb));
+  unsigned char *const part = take(partb);  // the sums of products whose K is split over CTAs
   unsigned char *cells = take(1024);
   unsigned char *bscr = at;
   unsigned long long *cell = reinterpret_cast<unsigned long long *>(cells);
@@ -1001,16 +1002,16 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   auto gram = [&](const oz::Operand &o, const Mat &H, int nd) {
     oz::Operand a = o;
     a.halves = 1;
-    return oz::gemm(a, o, oz::Result{H.re, H.im, n, n, ni, ni, nullptr, 1, 0, 1}, nd, gerr, s) == cudaSuccess;
+    return oz::gemm(a, o, oz::Result{H.re, H.im, n, n, ni, ni, nullptr, 1, 0, 1}, nd, gerr, part, s) == cudaSuccess;
   };
   // X (+)= A B for an n x n X
   auto mult = [&](const oz::Operand &A, const oz::Operand &B, const Mat &X, int add, int nd) {
-    return oz::gemm(A, B, oz::Result{X.re, X.im, n, n, ni, ni, nullptr, 1, add, 0}, nd, gerr, s) == cudaSuccess;
+    return oz::gemm(A, B, oz::Result{X.re, X.im, n, n, ni, ni, nullptr, 1, add, 0}, nd, gerr, part, s) == cudaSuccess;
   };
   // V (+)= A B, G (+)= A B (G's columns times 2^ej)
   auto mult_v = [&](const oz::Operand &A, const oz::Operand &B, int add, int nd) {
     return oz::gemm(A, B, oz::Result{V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), ni, ni, nullptr, 1, add, 0},
-                    nd, gerr, s) == cudaSuccess;
+                    nd, gerr, part, s) == cudaSuccess;
   };
   // G's rows enter with their columns' 2^-x
   auto mult_g = [&](const int *x, const oz::Operand &B, const int *ej, int add, int nd) {
@@ -1018,7 +1019,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
       oz::Operand A;
       if (!cut(g_rows(r0, x), d1, e1, A) ||
           oz::gemm(A, B, oz::Result{G + r0, CPLX ? Gi + r0 : nullptr, sc.ldr, sc.ldi, panel_rows(r0), ni, ej, 1, add, 0},
-                   nd, gerr, s) != cudaSuccess)
+                   nd, gerr, part, s) != cudaSuccess)
         return false;
     }
     return true;
@@ -1037,7 +1038,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
       oz::Operand a = o;
       a.halves = 1;
       if (oz::split_digits(p, o, s) != cudaSuccess ||
-          oz::gemm(a, o, oz::Result{H.re, H.im, n, n, ni, ni, nullptr, 0, r0 ? 1 : 0, 1}, nd, gerr, s) != cudaSuccess)
+          oz::gemm(a, o, oz::Result{H.re, H.im, n, n, ni, ni, nullptr, 0, r0 ? 1 : 0, 1}, nd, gerr, part, s) != cudaSuccess)
         return false;
     }
     return true;
