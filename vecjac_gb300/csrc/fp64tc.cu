@@ -68,14 +68,23 @@ __global__ void k_fill_int(int *x, int n, int v)
     x[i] = v;
 }
 
-// largest exponents of the operand's rows. COLS, PROD: a warp per row
-__global__ void __launch_bounds__(256) k_expo_cols(Source s, int *e)
+// e: the power of two by which row r is scaled (magnitudes below 1/2) from its largest exponent, for
+// every half of np rows
+__device__ __forceinline__ void put_exponent(int *e, int r, int np, int halves, int m)
+{
+  const int v = (m == NOEXP) ? 0 : m + 2;
+  for (int h = 0; h < halves; ++h)
+    e[h * np + r] = v;
+}
+
+// the operand's row exponents. COLS, PROD: a warp per row
+__global__ void __launch_bounds__(256) k_expo_cols(Source s, int *e, int np, int halves)
 {
   const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (r >= s.rows)
+  if (r >= np)
     return;
   int m = NOEXP;
-  for (int k = lane; k < s.len; k += 32) {
+  for (int k = lane; k < s.len && r < s.rows; k += 32) {
     const int a = s.ek ? s.esign * s.ek[k] : 0;
     int x = expo(s.re[(long long)r * s.ldr + k]);
     m = max(m, x == NOEXP ? x : x + a);
@@ -86,15 +95,20 @@ __global__ void __launch_bounds__(256) k_expo_cols(Source s, int *e)
   }
   m = __reduce_max_sync(0xffffffffu, m);
   if (lane == 0)
-    e[r] = m;
+    put_exponent(e, r, np, halves, m);
 }
-// ROWS: threads along the rows, blockIdx.y along K
-__global__ void __launch_bounds__(256) k_expo_rows(Source s, int *e)
+// ROWS: threads along the rows, blockIdx.y along K; several of them collect the largest exponents, for
+// k_expo_final
+__global__ void __launch_bounds__(256) k_expo_rows(Source s, int *e, int np)
 {
   const int r = blockIdx.x * 256 + threadIdx.x;
-  if (r >= s.rows)
+  if (r >= s.rows) {
+    if (gridDim.y == 1 && r < np)
+      e[r] = 0;
     return;
+  }
   int m = NOEXP;
+#pragma unroll 8
   for (int k = blockIdx.y; k < s.len; k += gridDim.y) {
     const int a = s.ek ? s.esign * s.ek[k] : 0;
     int x = expo(s.re[(long long)k * s.ldr + r]);
@@ -104,17 +118,15 @@ __global__ void __launch_bounds__(256) k_expo_rows(Source s, int *e)
       m = max(m, x == NOEXP ? x : x + a);
     }
   }
-  atomicMax(e + r, m);
+  if (gridDim.y == 1)
+    put_exponent(e, r, np, 1, m);
+  else
+    atomicMax(e + r, m);
 }
-// e: the power of two by which a row is scaled (magnitudes below 1/2), for every half
-__global__ void k_expo_final(int *e, int rows, int np, int halves)
+__global__ void k_expo_final(int *e, int rows, int np)
 {
-  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < np; r += gridDim.x * blockDim.x) {
-    const int m = (r < rows) ? e[r] : NOEXP;
-    const int v = (m == NOEXP) ? 0 : m + 2;
-    for (int h = 0; h < halves; ++h)
-      e[h * np + r] = v;
-  }
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < np; r += gridDim.x * blockDim.x)
+    put_exponent(e, r, np, 1, (r < rows) ? e[r] : NOEXP);
 }
 
 // x 2^-64 2^... as a 64-bit integer: round(x 2^(64 - e)), |x| < 2^(e - 1)
@@ -410,21 +422,21 @@ Operand shape(const Source &s, bool cplx)
 
 cudaError_t row_exponents(const Source &s, int *e, cudaStream_t st)
 {
-  k_expo_cols<<<(s.rows + 7) / 8, 256, 0, st>>>(s, e);
-  k_expo_final<<<(s.rows + 255) / 256, 256, 0, st>>>(e, s.rows, s.rows, 1);
+  k_expo_cols<<<(s.rows + 7) / 8, 256, 0, st>>>(s, e, s.rows, 1);
   return cudaGetLastError();
 }
 
 cudaError_t split_exponents(const Source &s, const Operand &o, cudaStream_t st)
 {
-  if (s.mode == ROWS) {
+  if (s.mode != ROWS)
+    k_expo_cols<<<(o.np + 7) / 8, 256, 0, st>>>(s, o.e, o.np, o.halves);
+  else if (s.len <= 32)  // (a thread goes along all of K: no largest exponents to collect)
+    k_expo_rows<<<(o.np + 255) / 256, 256, 0, st>>>(s, o.e, o.np);
+  else {
     k_fill_int<<<(s.rows + 255) / 256, 256, 0, st>>>(o.e, s.rows, NOEXP);
-    const int gy = s.len < 32 ? s.len : 32;
-    k_expo_rows<<<dim3((unsigned)((s.rows + 255) / 256), (unsigned)gy), 256, 0, st>>>(s, o.e);
+    k_expo_rows<<<dim3((unsigned)((s.rows + 255) / 256), 32u), 256, 0, st>>>(s, o.e, o.np);
+    k_expo_final<<<(o.np + 255) / 256, 256, 0, st>>>(o.e, s.rows, o.np);
   }
-  else
-    k_expo_cols<<<(s.rows + 7) / 8, 256, 0, st>>>(s, o.e);
-  k_expo_final<<<(o.np + 255) / 256, 256, 0, st>>>(o.e, s.rows, o.np, o.halves);
   return cudaGetLastError();
 }
 
@@ -440,8 +452,8 @@ cudaError_t split(const Source &s, const Operand &o, cudaStream_t st)
   return (e != cudaSuccess) ? e : split_digits(s, o, st);
 }
 
-// K blocks of a slice at least
-constexpr long long MIN_SLICE = 16;
+// K blocks of a slice at least (1000 x 16 real 1.57 ms with 4, 1.68 with 16; 512 x 512 real 9.3 and 9.7)
+constexpr long long MIN_SLICE = 4;
 
 // (slices x tiles <= SMs)
 size_t part_bytes() { return (size_t)host::sm_count() * 128 * ROWB * sizeof(longlong2); }
