@@ -960,30 +960,38 @@ static inline bool is_al(const void *p)
 template <typename T, bool CPLX> struct StepPairs {
   static constexpr int MAX = (CPLX && sizeof(T) == 4) ? 2 : 4;
 };
-// the step kernel for about P pairs per CTA and m rows (columns staged in shared memory when
+// the step kernel for at most P pairs per CTA and m rows (columns staged in shared memory when
 // they and the product buffers fit in 192 KiB), with its dynamic shared memory allowed
 template <typename T> struct StepLaunch {
   void (*k)(SvdArgs<T>, int, int, int);
   size_t smem;
   int pairs;  // per CTA
 };
+constexpr size_t STEP_SMEM = 192 * 1024;
 template <typename T, bool CPLX, int P> static size_t step_smem(long long m)
 {
   return StepDims<T, CPLX, P>::buf_bytes() + (size_t)m * sizeof(T) * (CPLX ? 4u : 2u) * P;
 }
+template <typename T, bool CPLX, int P> static StepLaunch<T> step_of(long long m)
+{
+  if (step_smem<T, CPLX, P>(m) <= STEP_SMEM)
+    return {k_step<T, CPLX, true, P>, step_smem<T, CPLX, P>(m), P};
+  if constexpr (sizeof(T) == 4 && P > 1)
+    return step_of<T, CPLX, 1>(m);
+  else
+    return {k_step<T, CPLX, false, P>, StepDims<T, CPLX, P>::buf_bytes(), P};
+}
+// Where the columns of P pairs do not fit, FP32 takes one pair per CTA, which fits up to 22,528 rows
+// (real; 10,240 complex) and pays beyond it, too, where the columns are read from L2 (a step, milliseconds per
+// n of them, with the most pairs and with one: 6144 x 704 real 102, 15.7; 30000 x 1024 1129, 384;
+// 9600 x 640 complex 142, 76). FP64 keeps the P that the number of pairs asks for: its recurrences and
+// rotations share the FP64 unit's instructions between pairs (4096 x 1024 real 139 with four pairs, 234
+// with two or one, 16000 x 64, 32 pairs, 34 with four and 26 with one).
 template <typename T, bool CPLX> static StepLaunch<T> step_launch(long long m, int P)
 {
-  constexpr int PMAX = StepPairs<T, CPLX>::MAX;
-  constexpr size_t LIM = 192 * 1024;
-  StepLaunch<T> r;
-  if (P == 1 && step_smem<T, CPLX, 1>(m) <= LIM)
-    r = {k_step<T, CPLX, true, 1>, step_smem<T, CPLX, 1>(m), 1};
-  else if (P <= 2 && step_smem<T, CPLX, 2>(m) <= LIM)
-    r = {k_step<T, CPLX, true, 2>, step_smem<T, CPLX, 2>(m), 2};
-  else if (step_smem<T, CPLX, PMAX>(m) <= LIM)
-    r = {k_step<T, CPLX, true, PMAX>, step_smem<T, CPLX, PMAX>(m), PMAX};
-  else
-    r = {k_step<T, CPLX, false, PMAX>, StepDims<T, CPLX, PMAX>::buf_bytes(), PMAX};
+  StepLaunch<T> r = (P == 1)   ? step_of<T, CPLX, 1>(m)
+                    : (P == 2) ? step_of<T, CPLX, 2>(m)
+                               : step_of<T, CPLX, StepPairs<T, CPLX>::MAX>(m);
   if (r.smem > 40 * 1024 &&
       cudaFuncSetAttribute(r.k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r.smem) != cudaSuccess)
     r.k = nullptr;
