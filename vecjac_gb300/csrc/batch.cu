@@ -1,11 +1,11 @@
 // Batched one-sided Jacobi SVD: thousands of independent matrices of uneven size in one call
-// of one or two persistent launches (real FP64 and FP32; every matrix with dvjsvd_'s / svjsvd_'s
+// of persistent launches (real FP64 and FP32; every matrix with dvjsvd_'s / svjsvd_'s
 // result).
 //
 // A matrix is worked on by one CTA, or, when it is so large that its CTA would finish after
-// the rest of the batch, by a cluster of BATCH_CS CTAs (svd_one's team, batch_core.cuh). Each
-// team runs the reference driver on its matrix (src/dvjsvd.c:78-638). Matrices are handed out by atomic work queues in the order the caller gives
-// (largest first balances the tail); a matrix stops at its own convergence (its own sweep
+// the rest of the batch and clusters do them sooner (k_plan), by a cluster of BATCH_CS CTAs (svd_one's
+// team, batch_core.cuh). Each team runs the reference driver on its matrix (src/dvjsvd.c:78-638). Matrices
+// are handed out by atomic work queues in the order the caller gives (largest first balances the tail); a matrix stops at its own convergence (its own sweep
 // count, its own info entry), so uneven convergence does not hold the batch back. Pivot pairs
 // are computed on the fly from the strategy's closed form (pjs.cuh), so no tables are stored.
 // Matrix sizes: m >= n, n <= 512, and the reference's divisibility rules (the host wrapper
@@ -16,19 +16,29 @@
 
 namespace vj {
 
-// CTAs per cluster, and the cost of a large matrix in shares of a CTA (k_plan): 300 FP32
-// matrices of up to 512 rows take 717 ms by single CTAs and 171 ms in clusters of 4 (119 ms in
-// clusters of 8), 1500 FP64 ones of up to 128 rows 129, 117 and 145 ms, and from half a share
-// 128 ms in clusters of 4: a cluster larger than its matrix leaves CTAs idle.
+// CTAs per cluster: 300 FP32 matrices of up to 512 rows take 717 ms by single CTAs and 171 ms in clusters
+// of 4 (119 ms in clusters of 8), 1500 FP64 ones of up to 128 rows 129, 117 and 145 ms: a cluster
+// larger than its matrix leaves CTAs idle.
 constexpr int BATCH_CS = 4;
-constexpr double BATCH_SHARE = 1.0;
 
-// Unless the caller sets the number of CTAs per SM, the batch is done by two launches: the large
+// What a matrix gains from a cluster over a CTA, by the groups of pairs per warp of a CTA: measured
+// alone on the GPU, FP64 1.5, 2.0, 3.0 and 3.6 times at 1, 2, 4 and 8 groups per warp (128 x 64 to 512 x
+// 256 by 256 and 128 threads), FP32 1.2, 1.5, 1.9, 2.4 and 3.0 at 1 to 16 (more where single CTAs'
+// matrices would not fit in L2 together: 152 of 512 x 256 106 ms by clusters, 155 by CTAs).
+template <typename T> __device__ __forceinline__ double team_gain(long long n, int warps)
+{
+  const float r = fmaxf((float)n / (float)(2 * (32 / svdc<T>::LANES) * warps), 0.25f);
+  const float g = (sizeof(T) == 8) ? 1.5f * sqrtf(r) : 1.25f * exp2f(0.42f * log2f(r));
+  return (double)fminf(fmaxf(g, 1.05f), (sizeof(T) == 8) ? 3.7f : 3.2f);
+}
+
+// Unless the caller sets the number of CTAs per SM, the batch is done in two parts: the large
 // matrices and the wide ones, whose cost is more than BATCH_WIDE of a CTA's share of the batch, by
 // two CTAs of 128 registers per SM, and the others by four CTAs of 64 registers, which start as the
 // first launch's end. A matrix is done sooner by one of two CTAs than of four, which counts at the
 // end of the batch; many small ones are done sooner by four, whose waits for memory and for the few
-// threads of a 2x2 overlap. 4000 FP32 matrices of up to 256 rows: 141 ms (two CTAs 141, four 154),
+// threads of a 2x2 overlap. (The first part has a second launch, of the CTAs that its clusters leave room
+// for, batch_dev.) 4000 FP32 matrices of up to 256 rows: 141 ms (two CTAs 141, four 154),
 // 1500 FP64 ones of up to 128 rows: 105 ms (105, 115), 4000 FP64 16 x 16: 16.8 ms (22.3, 17.2),
 // 4000 FP32 64 x 32: 10.1 ms (11.8, 10.6). With a smaller BATCH_WIDE, 2000 FP64 64 x 64 take 154
 // instead of 141 ms, with a larger one the uneven batches 151 and 119 ms (at 0.6).
@@ -40,30 +50,84 @@ __device__ __forceinline__ double batch_cost(long long m, long long n)
   return (n > 0 && m > 0) ? (double)n * (double)n * (double)(m + n) : 0.0;
 }
 
-// The queues' heads and the size from which a matrix is large: its cost above `share` times
-// what each of `slots` CTAs would have of the whole batch's, and enough groups of pairs for
-// more than the `warps` warps of one CTA. One CTA of 1024 threads.
+// The queues' heads and the sizes from which a matrix is large (done by a cluster) and wide, for `teams`
+// clusters, `slots` CTAs of `warps` warps in all. Large is what costs more than a CTA slot would have of
+// the batch and has enough groups of pairs for more than the warps of one CTA, or nothing, where
+// single CTAs would be done sooner: the times of both are estimated in units of a matrix's cost on an SM
+// of its own, from the clusters' matrices in rounds (the last, partly filled one at 0.8), all work at
+// the rates of clusters and of single CTAs (two on an SM take 1.45 times as long as one: an SM's rate
+// grows with the root of their number; half of the longest matrix where they queue), and the longest single matrix
+// after the clusters that it waits for. Equal matrices, one per SM, went through the clusters in three
+// rounds before: 152 FP64 128 x 64 42 ms, 22 by single CTAs, 152 FP32 304 x 32 3.9 and 1.5; uneven ones
+// keep their clusters (300 FP64 of up to 128 rows 45 ms, 135 without). One CTA of 1024 threads.
 template <typename T>
-__global__ void __launch_bounds__(1024) k_plan(BatchArgs<T> a, int slots, int warps, double share)
+__global__ void __launch_bounds__(1024) k_plan(BatchArgs<T> a, int teams, int slots, int warps)
 {
-  __shared__ double sum[32];
+  // sums: cost of all, number and time of the large ones, cost of the others; maxima: cost of all, time of
+  // the large ones, cost of the others; minimum: time of the large ones
+  enum { ALL, NUM, TIME, OTHERS, MOST, TMOST, OMOST, TLEAST, NV };
+  __shared__ double sh[NV][32];
   __shared__ unsigned end, endw;
   const int tid = threadIdx.x;
-  double c = 0;
-  for (long long i = tid; i < a.count; i += blockDim.x)
-    c += batch_cost(a.m[i], a.n[i]);
-  for (int o = 16; o >= 1; o >>= 1)
-    c += __shfl_xor_sync(0xffffffffu, c, o);
-  if ((tid & 31) == 0)
-    sum[tid >> 5] = c;
+  double v[NV] = {0, 0, 0, 0, 0, 0, 0, 1e300};
+  // the values of `mask` over all threads, to every one of them
+  auto reduce = [&](unsigned mask) {
+    auto warp = [&](int k) {
+      for (int o = 16; o >= 1; o >>= 1) {
+        const double w = __shfl_xor_sync(0xffffffffu, v[k], o);
+        v[k] = (k < MOST) ? v[k] + w : (k < TLEAST) ? fmax(v[k], w) : fmin(v[k], w);
+      }
+    };
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      if (mask >> k & 1u) {
+        warp(k);
+        if ((tid & 31) == 0)
+          sh[k][tid >> 5] = v[k];
+      }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NV; ++k)
+      if (mask >> k & 1u) {
+        v[k] = sh[k][tid & 31];
+        warp(k);
+      }
+  };
+  for (long long i = tid; i < a.count; i += blockDim.x) {
+    const double w = batch_cost(a.m[i], a.n[i]);
+    v[ALL] += w;
+    v[MOST] = fmax(v[MOST], w);
+  }
   if (tid == 0)
     end = endw = 0u;
-  __syncthreads();
-  c = 0;
-  for (int w = 0; w < 32; ++w)
-    c += sum[w];
+  reduce(1u << ALL | 1u << MOST);
+  const double c = v[ALL];
   const double nmin = 2.0 * (32 / svdc<T>::LANES) * warps;  // columns that one CTA's warps take at once
-  const double limit = fmax(share * c / slots, 2.0 * nmin * nmin * nmin);
+  double limit = fmax(c / slots, 2.0 * nmin * nmin * nmin);
+  if (v[MOST] > limit) {
+    for (long long i = tid; i < a.count; i += blockDim.x) {
+      const double w = batch_cost(a.m[i], a.n[i]);
+      if (w > limit) {
+        const double t = w / team_gain<T>(a.n[i], warps);
+        v[NUM] += 1;
+        v[TIME] += t;
+        v[TMOST] = fmax(v[TMOST], t);
+        v[TLEAST] = fmin(v[TLEAST], t);
+      }
+      else {
+        v[OTHERS] += w;
+        v[OMOST] = fmax(v[OMOST], w);
+      }
+    }
+    reduce(1u << NUM | 1u << TIME | 1u << OTHERS | 1u << TMOST | 1u << OMOST | 1u << TLEAST);
+    const double rate = sqrt((double)a.sms * (double)slots), t = v[TIME] / teams;
+    const double rounds = fmax(v[TMOST], t + ((v[NUM] > teams) ? 0.8 * v[TLEAST] : 0.0));
+    const double with = fmax(fmax(rounds, t + v[OTHERS] / rate + (((double)a.count - v[NUM] > slots) ? 0.5 * v[OMOST] : 0.0)),
+                             ((v[NUM] >= teams) ? t : 0.0) + v[OMOST]);
+    const double without = fmax(v[MOST], c / rate + ((a.count > slots) ? 0.5 * v[MOST] : 0.0));
+    if (without <= with)
+      limit = 1e300;
+  }
   for (long long i = tid; i < a.count; i += blockDim.x) {
     const int b = a.order ? a.order[i] : (int)i;
     if (batch_cost(a.m[b], a.n[b]) > limit)
@@ -111,7 +175,7 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchArgs<T> a)
   const double limit = plan->limit, widec = plan->wide;
   const unsigned end = plan->end_large;
   auto large = [&](int b) { return batch_cost(a.m[b], a.n[b]) > limit; };
-  if (a.part == 1)
+  if (a.part != 2)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // the large matrices, by whole clusters
   if (end && size > 1u) {
@@ -145,7 +209,7 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchArgs<T> a)
   // the others, by single CTAs: the r-th CTA of an SM takes part when there are more than r
   // matrices per SM, so that few matrices spread over the SMs (108 FP64 matrices of up to 35
   // rows: 9.2 ms when the two CTAs of an SM may both take one, 7.1 ms apart)
-  const bool split = end && (size > 1u || a.part == 2);
+  const bool split = end && (size > 1u || a.part == 2 || a.fill);
   if (threadIdx.x == 0) {
     unsigned sm;
     asm("mov.u32 %0, %%smid;" : "=r"(sm));
@@ -179,7 +243,8 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchArgs<T> a)
       break;
     svd_matrix<T>(a, sh, (int)b, Team{0, 1}, &sh);
   }
-  if (a.part == 2)  // (the launch ends when the first part has, too)
+  // (the launch ends when the one before has, too; one CTA waits for it, the others make room)
+  if ((a.part == 2 || a.fill) && blockIdx.x == 0)
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
@@ -211,6 +276,7 @@ static vj_fint batch_dev(vj_fint count, const long long *m, const long long *n, 
   a.swp = swp;
   a.sms = host::sm_count();
   a.part = parts ? 1 : 0;
+  a.fill = 0;
   void (*k)(BatchArgs<T>) = (occ == 2)   ? k_batch<T, 2>
                             : (occ == 3) ? k_batch<T, 3>
                             : (occ == 4) ? k_batch<T, 4>
@@ -232,16 +298,32 @@ static vj_fint batch_dev(vj_fint count, const long long *m, const long long *n, 
     clusters = 1;
   }
   const int slots = clusters * BATCH_CS;
-  k_plan<T><<<1, 1024, 0, s>>>(a, slots, block / 32, BATCH_SHARE);
+  k_plan<T><<<1, 1024, 0, s>>>(a, clusters, slots, block / 32);
   // a cluster per matrix at most: every matrix may be large
   cfg.gridDim = dim3((unsigned)(((long long)clusters < count ? (long long)clusters : (long long)count) * BATCH_CS));
   if (cudaLaunchKernelEx(&cfg, k, a) != cudaSuccess)
     return VJ_ERR_CUDA;
+  // The SMs that no cluster fits on (their number in a processing cluster is not always a multiple of
+  // four) get single CTAs, in a launch that starts beside the first: 152 equal matrices otherwise find
+  // 148 SMs and take two rounds (FP64 128 x 64: 42 ms).
+  int per = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, block, 0) != cudaSuccess) {
+    cudaGetLastError();
+    per = 0;
+  }
+  const long long room = (long long)per * a.sms - slots;
+  if (room > 0 && count > clusters) {
+    a.fill = 1;
+    if (host::launch_pdl(k, dim3((unsigned)(room < count ? room : (long long)count)), dim3((unsigned)block), 0, s, a) !=
+        cudaSuccess)
+      return VJ_ERR_CUDA;
+    a.fill = 0;
+  }
   if (parts) {
     // the others: these CTAs start as the first launch's end
     a.part = 2;
     void (*const k2)(BatchArgs<T>) = k_batch<T, 4>;
-    int per = 0;
+    per = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k2, block, 0) != cudaSuccess || per < 1) {
       cudaGetLastError();
       per = 1;

@@ -39,6 +39,7 @@ template <typename T> struct BatchArgs {
   unsigned swp;
   int sms;   // SMs of the device
   int part;  // 0 all matrices, 1 large and wide ones, 2 the others
+  int fill;  // the launch of the CTAs that the clusters leave room for
 };
 
 // what a step leaves for the next (three slots in turn: read, written, being cleared)
