@@ -1244,8 +1244,9 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     const double tol64 = 0.5 * std::sqrt((double)m) * u;
     // the finishing check's limit (jsvd.cu, k_certify)
     const double lim = 0.9 * std::sqrt((double)m) * u - 16.0 * u;
-    const unsigned maxsw64 = swp < 20u ? swp : 20u;
-    unsigned sw64 = 0;
+    // swp caps the phase: what changes G and V, refinements, rotations of single pairs and sweeps, each
+    // pass over the pairs counted (20 sweeps at most)
+    unsigned sw64 = 0, passes = 0;
     bool sweeps = true;
     double before = 1e300;
     // (the entries of a Gram matrix of several panels are rounded sums of the panels')
@@ -1283,6 +1284,8 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
         certified = (asdbl(hst.cosbound) + pan <= lim);
         break;
       }
+      if (passes >= swp)
+        break;
       if (hst.skipped) {
         // pairs of nearly equal norms: rotate disjoint ones of them by their angles and look again
         // (many of them are clusters, where the sweeps do better)
@@ -1306,6 +1309,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
                                 (int)(hp.size() / 2), tol64, cnt, s) ||
             cudaStreamSynchronize(s) != cudaSuccess)
           return VJ_ERR_CUDA;
+        ++passes;
         continue;
       }
       if (!(norm <= 0.48) || !(cmax <= 0.25 * before))
@@ -1381,7 +1385,9 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
         if (!cut_rows(V, Vi, (long long)ldV, (long long)(CPLX ? ldVi : ldV), nullptr, oa) || !mult_v(oa, ob, 1, nv))
           return VJ_ERR_CUDA;
       ++sw64;
+      ++passes;
     }
+    const unsigned maxsw64 = std::min(swp - std::min(passes, swp), 20u);
     // A sweep whose rotated pairs all had |cos| <= 1e-11 leaves off-diagonal terms of the
     // order of their squares (times n / relative gap), far below the tolerance: its
     // confirming sweep is skipped, the reference's sweep below confirms.
