@@ -967,7 +967,7 @@ def bench_batch(args, vj, dist, rank, world, kind):
     from vecjac_gb300 import batch as B
     mats = gen_uneven(args.batch_count, 77 + rank, kind)
     b = B.Batch(mats, kind)
-    blk, occ = B.autotune(b, args.pivot)
+    blk, occ = B.autotune(b, args.pivot, occupancies=B.OCCUPANCIES[kind])
     g = B.capture(b, args.pivot, block=blk, occupancy=occ)
     for _ in range(max(0, args.warmup - 1)):
         g.replay()
@@ -1009,14 +1009,16 @@ def bench_batch(args, vj, dist, rank, world, kind):
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": round(ms, 2), "higher_is_better": True,
             "scaling": "weak", "vs_baseline": None, "dtype": "f64" if kind == "d" else "f32",
             "data": "synthetic (m~U[16,512], n~U[8,m], Q1 diag(sigma) Q2^T, sigma=10^U(-4,0))",
-            "config": {"workload": "%d matrices in one persistent launch (CUDA graph), pivot id %d, block %d, "
-                       "register bound for %d CTAs of 256 threads per SM (autotuned)"
+            "config": {"workload": "%d matrices in one call (CUDA graph), pivot id %d, block %d, "
+                       "register bound for %d CTAs of 256 threads per SM (0: two parts), autotuned"
                        % (len(mats), args.pivot, blk, occ), "errors": int((info < 0).sum()),
                        "mean_sweeps": float(info[info >= 0].mean())},
             "flops_per_s": flops / (ms * 1e-3),
             "one_launch_per_matrix_s_estimate": round(per_launch, 2),
             "speedup_vs_per_matrix_launches": round(per_launch / (ms * 1e-3), 2),
-            "clocks": clk.summary(), "gpu_launches": 2 * args.steps}
+            "clocks": clk.summary(),
+            # (the plan, the clusters, the CTAs that they leave room for, and the default's second part)
+            "gpu_launches": (4 if occ == 0 else 3) * args.steps}
     out["roofline"] = svd_roofline(out["flops_per_s"], kind == "d",
                                    "k_batch<%s>" % ("double" if kind == "d" else "float"))
     if rank == 0 and args.cpu_baseline:

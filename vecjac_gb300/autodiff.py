@@ -16,6 +16,7 @@ import ctypes as C
 import numpy as np
 
 from . import api
+from .batch import count_bucket
 
 
 def _p(t):
@@ -26,12 +27,13 @@ _BLOCK = {}
 
 
 def _tuned_block(A, strategy, swp):
-    """Launch configuration of the batched kernel for this matrix shape and precision: the
-    CTA size (64, 128, 256 threads) in the default two launches, then one launch with each
+    """Launch configuration of the batched kernel for this matrix shape, precision and number of
+    matrices per SM (to a power of two): the CTA size (64, 128, 256 threads) in the default two
+    parts, then one launch with each
     register bound (resident 256-thread CTAs per SM) at the best size, each timed on up to 2432 of the
     matrices (after one warm-up); the fastest (block, occupancy) is kept for the process."""
     import torch
-    key = (tuple(A.shape[1:]), A.dtype, strategy)
+    key = (tuple(A.shape[1:]), A.dtype, strategy, count_bucket(A.shape[0]))
     if key not in _BLOCK:
         sub = A[: min(A.shape[0], 2432)]
 

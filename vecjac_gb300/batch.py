@@ -1,4 +1,4 @@
-"""Batched SVD of many uneven real matrices in a call of one or two persistent launches, with an autotuner
+"""Batched SVD of many uneven real matrices in one call of persistent launches, with an autotuner
 for the launch configuration (CTA size and the kernel's register bound, i.e. resident
 CTAs per SM) and CUDA-graph capture of the launch.
 
@@ -16,8 +16,19 @@ import numpy as np
 from . import api
 
 _TUNED = {}
-# the register bound (resident 256-thread CTAs per SM) at which the autotuner times the CTA sizes
+# the register bound (resident 256-thread CTAs per SM) at which the autotuner times the CTA sizes,
+# unless the library's default (0) is among the bounds asked for
 DEFAULT_OCC = {"s": 4, "d": 2}
+# what svd_batch has timed: the library's default (the parts of csrc/batch.cu), then one launch each
+OCCUPANCIES = {"s": (0, 2, 3, 4, 5), "d": (0, 2, 3, 4)}
+
+
+def count_bucket(count):
+    """The matrices per SM to the nearest power of two (1/8 to 16): the best launch configuration
+    depends on it, as a single wave of matrices wants few large CTAs and a queue of them many."""
+    import torch
+    sms = torch.cuda.get_device_properties(torch.cuda.current_device()).multi_processor_count
+    return int(min(4, max(-3, round(np.log2(max(count, 1) / sms)))))
 
 
 def padded_shape(m, n, kind):
@@ -64,7 +75,7 @@ class Batch:
     def run(self, strategy=4, swp=999, block=128, stream=None, reset=True, occupancy=0):
         """Enqueue the batch (asynchronous). reset=True first restores G from the packed input.
         block: threads per CTA (64, 128, 256); occupancy: the kernel's register bound in
-        resident 256-thread CTAs per SM (2..6 in one launch, 0 = two launches, csrc/batch.cu)."""
+        resident 256-thread CTAs per SM (2..6 in one launch, 0 = in two parts, csrc/batch.cu)."""
         if reset:
             self.G.copy_(self.G0)
         f = getattr(api.lib(), "vj_%svjsvd_batch_tuned_dev" % self.kind)
@@ -101,15 +112,16 @@ def autotune(batch, strategy=4, blocks=(64, 128, 256), occupancies=None, sample=
     """Pick the launch configuration for this batch's size mix: the CTA size (threads per
     matrix) and the kernel's register bound (resident CTAs per SM), by timing candidates
     on a random sample of the batch's matrices (CUDA events, after one warm-up): first the
-    CTA sizes at the default bound, then the bounds at the best CTA size. The sample is
+    CTA sizes at the library's default (0, if among the occupancies) or at DEFAULT_OCC, then
+    the occupancies at the best CTA size. The sample is
     large enough to fill the GPU several times (2432 matrices by default), so that it
     measures throughput rather than its largest matrix. Returns (block, occupancy); cached
-    per (precision, coarse size histogram)."""
+    per (precision, coarse size histogram, matrices per SM)."""
     import torch
     if occupancies is None:
         occupancies = (2, 3, 4, 5) if batch.kind == "s" else (2, 3, 4)
     key = (batch.kind, tuple(np.histogram(batch.n, bins=[0, 32, 64, 128, 256, 513])[0] > 0), tuple(blocks),
-           tuple(occupancies))
+           tuple(occupancies), count_bucket(batch.count))
     if key in _TUNED:
         return _TUNED[key]
     rng = np.random.default_rng(0)
@@ -133,7 +145,7 @@ def autotune(batch, strategy=4, blocks=(64, 128, 256), occupancies=None, sample=
         torch.cuda.synchronize()
         return e0.elapsed_time(e1)
 
-    d = DEFAULT_OCC[batch.kind]
+    d = 0 if 0 in occupancies else DEFAULT_OCC[batch.kind]
     times = {}
     for blk in blocks:
         times[(blk, d)] = timed(blk, d)
@@ -162,10 +174,10 @@ def capture(batch, strategy=4, swp=999, block=128, occupancy=0):
 
 
 def svd_batch(mats, kind="d", strategy=4, swp=999, block=None):
-    """SVD of every matrix in `mats` (real numpy arrays of any m >= n <= 512) in one launch."""
+    """SVD of every matrix in `mats` (real numpy arrays of any m >= n <= 512) in one call."""
     import torch
     b = Batch(mats, kind)
-    blk, occ = (block, 0) if block else autotune(b, strategy)
+    blk, occ = (block, 0) if block else autotune(b, strategy, occupancies=OCCUPANCIES[kind])
     b.run(strategy, swp, blk, occupancy=occ)
     torch.cuda.synchronize()
     return b.results()
