@@ -248,33 +248,13 @@ __global__ void __launch_bounds__(256, MINB) k_batch(BatchArgs<T> a)
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-template <typename T>
-static vj_fint batch_dev(vj_fint count, const long long *m, const long long *n, T *G, const long long *offG, T *V,
-                         const long long *offV, T *eS, T *fS, const long long *offS, const int *order,
-                         long strategy, unsigned swp, long long *info, int block, int occ, void *stream)
+// the call's launches (occ 0: the default's parts)
+template <typename T> static vj_fint batch_launch(BatchArgs<T> a, int block, int occ, cudaStream_t s)
 {
-  if (count < 0 || (strategy != 2l && strategy != 4l))
-    return VJ_ERR_ARG;
-  if (!count)
-    return 0;
-  if (!host::gpu_ready())
-    return VJ_ERR_NO_GPU;
-  if (block != 64 && block != 128 && block != 256)
-    block = 128;
-  const bool parts = (occ < 2 || occ > 6);
+  const long long count = a.count;
+  const bool parts = !occ;
   if (parts)
     occ = 2;
-  cudaStream_t s = (cudaStream_t)stream;
-  BatchPlan *plan = static_cast<BatchPlan *>(host::batch_plan(sizeof(BatchPlan)));
-  if (!plan)
-    return VJ_ERR_NOMEM;
-  BatchArgs<T> a;
-  a.count = count;
-  a.m = m; a.n = n; a.offG = offG; a.offV = offV; a.offS = offS; a.order = order;
-  a.G = G; a.V = V; a.eS = eS; a.fS = fS; a.info = info; a.plan = plan;
-  a.strategy = (int)strategy;
-  a.swp = swp;
-  a.sms = host::sm_count();
   a.part = parts ? 1 : 0;
   a.fill = 0;
   void (*k)(BatchArgs<T>) = (occ == 2)   ? k_batch<T, 2>
@@ -334,6 +314,35 @@ static vj_fint batch_dev(vj_fint count, const long long *m, const long long *n, 
       return VJ_ERR_CUDA;
   }
   return (cudaGetLastError() == cudaSuccess) ? 0 : VJ_ERR_CUDA;
+}
+
+template <typename T>
+static vj_fint batch_dev(vj_fint count, const long long *m, const long long *n, T *G, const long long *offG, T *V,
+                         const long long *offV, T *eS, T *fS, const long long *offS, const int *order,
+                         long strategy, unsigned swp, long long *info, int block, int occ, void *stream)
+{
+  if (count < 0 || (strategy != 2l && strategy != 4l))
+    return VJ_ERR_ARG;
+  if (!count)
+    return 0;
+  if (!host::gpu_ready())
+    return VJ_ERR_NO_GPU;
+  if (block != 64 && block != 128 && block != 256)
+    block = 128;
+  cudaStream_t s = (cudaStream_t)stream;
+  host::BatchPlanSlot slot;
+  if (!host::batch_plan_take(sizeof(BatchPlan), s, slot))
+    return VJ_ERR_NOMEM;
+  BatchArgs<T> a;
+  a.count = count;
+  a.m = m; a.n = n; a.offG = offG; a.offV = offV; a.offS = offS; a.order = order;
+  a.G = G; a.V = V; a.eS = eS; a.fS = fS; a.info = info;
+  a.plan = reinterpret_cast<BatchPlan *>(slot.ptr);
+  a.strategy = (int)strategy;
+  a.swp = swp;
+  a.sms = host::sm_count();
+  const vj_fint r = batch_launch<T>(a, block, (occ < 2 || occ > 6) ? 0 : occ, s);
+  return (!host::batch_plan_done(slot, s) && !r) ? VJ_ERR_CUDA : r;
 }
 
 }  // namespace vj

@@ -2,6 +2,7 @@
 #include <cstring>
 #include <mutex>
 
+#include "plan_slots.h"
 #include "vj_host.h"
 
 namespace vj {
@@ -108,20 +109,117 @@ Staging &staging()
   return s[device_slot()];
 }
 
-void *batch_plan(size_t bytes)
+namespace {
+// one per device and never destroyed (a graph may outlive the library's statics)
+struct Plans {
+  static constexpr int EAGER = 256, CHUNK = 64;
+  std::mutex mu;
+  char *eager = nullptr;
+  cudaEvent_t event[EAGER] = {};
+  EagerSlots slots{EAGER};
+  GraphSlots graph;
+  std::vector<char *> chunks;  // CHUNK slots of captured launches each
+};
+struct PlanOwner {  // a captured launch's slot, released with its graph
+  Plans *plans;
+  int slot;
+};
+Plans &plans()
 {
-  // a slot per launch, in turn: launches on several streams or threads do not share one
-  // unless BATCH_SLOTS later ones have been made while the first is still running
-  constexpr unsigned BATCH_SLOTS = 1024;
+  static Plans *const p = new Plans[MAX_DEVICES];
+  return p[device_slot()];
+}
+void CUDART_CB plan_release(void *v)
+{
+  PlanOwner *const o = static_cast<PlanOwner *>(v);
+  {
+    std::lock_guard<std::mutex> lk(o->plans->mu);
+    o->plans->graph.give_back(o->slot);
+  }
+  delete o;
+}
+}  // namespace
+
+bool batch_plan_take(size_t bytes, cudaStream_t s, BatchPlanSlot &p)
+{
   bytes = (bytes + 255) & ~(size_t)255;
-  static std::mutex mu;
-  static Staging q[MAX_DEVICES];
-  static unsigned next[MAX_DEVICES] = {};
-  const int dev = device_slot();
-  std::lock_guard<std::mutex> lk(mu);
-  if (!q[dev].reserve((size_t)BATCH_SLOTS * bytes))
-    return nullptr;
-  return q[dev].ptr + (size_t)(next[dev]++ % BATCH_SLOTS) * bytes;
+  Plans &q = plans();
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  cudaGraph_t g = nullptr;
+  if (cudaStreamGetCaptureInfo(s, &cap, nullptr, &g, nullptr, nullptr, nullptr) != cudaSuccess) {
+    cudaGetLastError();  // (the legacy stream while another thread captures: not captured itself)
+    cap = cudaStreamCaptureStatusNone;
+  }
+  std::lock_guard<std::mutex> lk(q.mu);
+  if (cap == cudaStreamCaptureStatusActive) {
+    int slot = q.graph.take();
+    if (slot < 0) {
+      char *c = nullptr;
+      // (an allocation is no part of the capture)
+      cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&c), Plans::CHUNK * bytes);
+      cudaThreadExchangeStreamCaptureMode(&mode);
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+      }
+      q.chunks.push_back(c);
+      q.graph.grow(Plans::CHUNK);
+      slot = q.graph.take();
+    }
+    PlanOwner *const o = new PlanOwner{&q, slot};
+    cudaUserObject_t obj;
+    if (cudaUserObjectCreate(&obj, o, plan_release, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+      cudaGetLastError();
+      q.graph.give_back(slot);
+      delete o;
+      return false;
+    }
+    if (cudaGraphRetainUserObject(g, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+      cudaGetLastError();
+      return false;  // (the slot is lost, not shared)
+    }
+    p.ptr = q.chunks[(size_t)(slot / Plans::CHUNK)] + (size_t)(slot % Plans::CHUNK) * bytes;
+    p.slot = -1;
+    return true;
+  }
+  if (!q.eager) {
+    if (cudaMalloc(reinterpret_cast<void **>(&q.eager), Plans::EAGER * bytes) != cudaSuccess) {
+      cudaGetLastError();
+      q.eager = nullptr;
+      return false;
+    }
+  }
+  const int slot = q.slots.take();
+  if (slot < 0)
+    return false;
+  cudaEvent_t &ev = q.event[slot];
+  if ((!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) ||
+      (q.slots.used[(size_t)slot] && cudaStreamWaitEvent(s, ev, 0) != cudaSuccess)) {
+    cudaGetLastError();
+    q.slots.held[(size_t)slot] = 0;
+    return false;
+  }
+  p.ptr = q.eager + (size_t)slot * bytes;
+  p.slot = slot;
+  return true;
+}
+
+bool batch_plan_done(const BatchPlanSlot &p, cudaStream_t s)
+{
+  if (p.slot < 0)
+    return true;
+  Plans &q = plans();
+  std::lock_guard<std::mutex> lk(q.mu);
+  const bool ok = cudaEventRecord(q.event[p.slot], s) == cudaSuccess;
+  if (!ok) {
+    cudaGetLastError();
+    if (cudaStreamSynchronize(s) != cudaSuccess)
+      return false;  // (the slot stays held)
+  }
+  q.slots.done(p.slot);
+  return ok;
 }
 
 char *small_out()

@@ -59,9 +59,17 @@ Staging &staging3();
 constexpr size_t SMALL_OUT = (size_t)512 << 10;
 char *small_out();
 
-// device memory for one launch of the batched SVD (always the same size): its work queues and
-// what its CTAs need to know of the batch (allocated on first use)
-void *batch_plan(size_t bytes);
+// Device memory for one call of the batched SVD (always the same size): its work queues and
+// what its CTAs need to know of the batch. take before the call's launches, done after them, on
+// the same stream. No two calls that may run at the same time share it: a call enqueued to
+// run has a slot that waits for the call before on it, a captured one a slot of the graph's own,
+// given back when the graph and its instances are gone.
+struct BatchPlanSlot {
+  char *ptr = nullptr;
+  int slot = -1;  // >= 0: an event is to be recorded
+};
+bool batch_plan_take(size_t bytes, cudaStream_t s, BatchPlanSlot &p);
+bool batch_plan_done(const BatchPlanSlot &p, cudaStream_t s);
 
 // two non-blocking streams owned by the library
 bool streams2(cudaStream_t s[2]);
