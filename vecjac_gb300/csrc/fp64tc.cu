@@ -292,9 +292,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
     }
   }
   bool ok = true;
+  uint32_t phase = 0;  // of `ready` that the last group entered ends
   const int groups = (nkb + GROUP - 1) / GROUP;
   for (int g = 0; g < groups; ++g) {
     const int k1 = min(nkb, (g + 1) * GROUP);
+    phase = (uint32_t)(g & 1);
     if (tid == 0) {
       for (int kb = g * GROUP; kb < k1 && ok; ++kb) {
         const int st = kb & 1;
@@ -328,7 +330,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
         s_fail = 1;
       tc::commit(&ready);
     }
-    const bool w = tc::mbar_wait(&ready, (uint32_t)(g & 1), WAIT_CYCLES);
+    const bool w = tc::mbar_wait(&ready, phase, WAIT_CYCLES);
     if (__syncthreads_or(!w || (tid == 0 && s_fail))) {
       ok = false;
       break;
@@ -357,7 +359,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_gemm(Operand A, Operand B, Resul
       for (int kb = (loaded >= 2) ? loaded - 2 : 0; kb < loaded; ++kb)
         (void)tc::mbar_wait(&full[kb & 1], (uint32_t)((kb >> 1) & 1), WAIT_CYCLES);
     }
-    (void)tc::mbar_wait(&ready, 0u, WAIT_CYCLES);
+    (void)tc::mbar_wait(&ready, phase, WAIT_CYCLES);
   }
   else if (gridDim.z > 1) {
     longlong2 *const to = part + part_tile(blockIdx.x, blockIdx.y) + (warp >> 2) * 32 * 128 + (warp & 3) * 32 + lane;
