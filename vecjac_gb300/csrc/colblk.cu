@@ -125,7 +125,8 @@ template <bool CPLX, int NC> __global__ void __launch_bounds__(NT, 1) k_col_bloc
     }
     ptab[tid / B][tid % B] = (unsigned short)(p | (q << 8));
   }
-  bool ok = mbar_wait_bounded(&bar[0]);
+  // (one answer per warp: its lanes go into the shuffles of the sums together, or none does)
+  bool ok = __all_sync(0xffffffffu, mbar_wait_bounded(&bar[0]));
   // ---- Gram matrix: rows over threads, four at a time ----
   if (ok) {
     float acc[NA];
