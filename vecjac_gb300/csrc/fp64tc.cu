@@ -56,7 +56,7 @@ __device__ __forceinline__ double element(const Source &s, int h, int r, int p, 
 {
   if (s.mode == ROWS)
     return p ? s.im[(long long)k * s.ldi + r] : s.re[(long long)k * s.ldr + r];
-  const bool im = (s.mode == COLS) ? (h != p) : (h != p);
+  const bool im = h != p;
   const double v = im ? s.im[(long long)r * s.ldi + k] : s.re[(long long)r * s.ldr + k];
   const bool neg = (s.mode == COLS) ? (h && p) : (!h && p);
   return neg ? -v : v;

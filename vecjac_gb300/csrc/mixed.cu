@@ -71,12 +71,6 @@ __global__ void k_to_f32(const double *A, long long ld, long long rows, long lon
       B[j * rows + i] = __double2float_rn(scale2(A[j * ld + i], e));
 }
 
-__global__ void k_to_f64(const float *A, long long n, double *B)
-{
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    B[i] = (double)A[i];
-}
-
 template <typename T> __global__ void k_eye_p(T *V, long long ld, long long n, int diag)
 {
   for (long long j = blockIdx.y; j < n; j += gridDim.y)

@@ -48,14 +48,6 @@ template <typename T> struct SvdArgs {
   long long e_dot, e_doti, e_appg, e_appv;
 };
 
-template <typename T> __device__ __forceinline__ unsigned long long tbits(T x)
-{
-  return (unsigned long long)fp<T>::bits(x);
-}
-
-// |x| bits, NaN above inf, so that an integer max flags NaNs as "not finite"
-
-
 // ---- TMA (cp.async.bulk) staging of a column pair into shared memory ----
 __device__ __forceinline__ unsigned smem_u32(const void *p)
 {
@@ -131,24 +123,7 @@ template <typename T> __device__ __forceinline__ T vhypot(T x, T y)
   return z * M_;
 }
 
-// norm of column c (real, or complex with planes) by one warp; writes eS/fS; returns d.
-// xr/xi point to the column (in global or in shared memory).
-template <typename T, bool CPLX> __device__ T col_norm_at(const SvdArgs<T> &a, long long c, const T *xr, const T *xi)
-{
-  T d = warp_nrm2(xr, a.m);
-  if (CPLX) {
-    const T di = warp_nrm2(xi, a.m);
-    d = vhypot(d, di);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    T e, f;
-    ef_split(d, e, f);
-    a.eS[c] = e;
-    a.fS[c] = f;
-  }
-  return d;
-}
-
+// norm of column c (real, or complex with planes) by one warp; writes eS/fS; returns d
 template <typename T, bool CPLX> __device__ T col_norm(const SvdArgs<T> &a, long long c)
 {
   T d = warp_nrm2(a.G + c * a.ldG, a.m);
