@@ -1367,7 +1367,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
           return VJ_ERR_CUDA;
         fact = asdbl(hst.factmax);
       }
-      const int ng = digits(8.0 * fact);
+      const int ng = digits(std::max(8.0 * cmax, fact));
       if (!cut_prod(K, nullptr, ob))
         return VJ_ERR_CUDA;
       for (int r = 0; r < reps; ++r)
