@@ -180,10 +180,10 @@ vj_fint vj_block_sweep_dev(int cplx, vj_fnat m, vj_fnat n, float *Gr, float *Gi,
                            vj_fnat ldW, float tol, int inner, int terms, float *mu, void *stream);
 
 /* Phase times of the calling thread's last vj_?vjsvd_mixed_dev call, in milliseconds:
- * out[0] FP32 sweeps, out[1] orthonormalisation of W and the GEMMs, out[2] plain-dot FP64 sweeps
- * and the column sort, out[3] the reference's finishing sweeps; out[4] the number of FP32
+ * out[0] FP32 sweeps, out[1] orthonormalisation of W and the products, out[2] FP64 refinements and
+ * plain-dot sweeps and the column sort, out[3] the reference's finishing sweeps; out[4] the number of FP32
  * kernel launches; out[5] 1 when the FP32 stages ran as block sweeps on the tensor cores,
- * 0 for column-pair sweeps. */
+ * 0 for sweeps by small blocks of columns or by pairs. */
 vj_fint vj_last_mixed_phases(double out[6]);
 
 /* Adjoint of the thin SVD A = U diag(S) V^T (m >= n, V square), batched over `count`
@@ -201,7 +201,7 @@ vj_fint vj_dsvd_adjoint_batch_dev(vj_fint count, vj_fnat m, vj_fnat n, vj_fnat k
                                   const double *V, const double *dS, const double *dU, const double *dV, double *dA,
                                   double gap, void *stream);
 
-/* Batched SVD of `count` independent real matrices in two persistent launches (FP64 d,
+/* Batched SVD of `count` independent real matrices by persistent launches (FP64 d,
  * FP32 s; csrc/batch.cu), each with the result dvjsvd_/svjsvd_ give for it (V := I, pivot strategy 2 or 4
  * generated on the fly, sweep cap swp). All arrays are on the device: matrix b is
  * m[b] x n[b] (the reference's rules: m >= n, m % 8 / % 16, (n/2) % 8 / % 16, n <= 512),
@@ -220,7 +220,7 @@ vj_fint vj_svjsvd_batch_dev(vj_fint count, const long long *m, const long long *
                             const int *order, long strategy, unsigned swp, long long *info, int block, void *stream);
 /* The same with the kernel's register bound chosen: `occupancy` resident CTAs of 256
  * threads per SM in one launch (2 to 6; fewer registers per thread, more CTAs, more
- * spills; 0 = the two launches of the form above: 2 for the matrices that finish last, 4
+ * spills; 0 = the two parts of the form above: 2 for the matrices that finish last, 4
  * for the others). The package's autotuner searches (block, occupancy) per batch. */
 vj_fint vj_dvjsvd_batch_tuned_dev(vj_fint count, const long long *m, const long long *n, double *G,
                                   const long long *offG, double *V, const long long *offV, double *eS, double *fS,

@@ -1,6 +1,6 @@
 """Differentiable batched SVD: torch.autograd.Function over the C ABI (ctypes).
 
-Forward: `vj_?vjsvd_batch_dev` (one persistent launch for the whole batch of same-shape
+Forward: `vj_?vjsvd_batch_dev` (one call for the whole batch of same-shape
 matrices; FP32 svjsvd_ / FP64 dvjsvd_ per matrix), then singular values sorted in
 descending order and every (u_j, v_j) pair sign-fixed so that the largest-magnitude entry
 of v_j is positive (a locally constant choice, so finite differences see the same branch).
@@ -56,7 +56,7 @@ def _tuned_block(A, strategy, swp):
 
 
 def svd_batch_dev(A, strategy=4, swp=999, block=None):
-    """SVD of every matrix of A (B, m, n) CUDA tensor (float32 or float64) in one launch
+    """SVD of every matrix of A (B, m, n) CUDA tensor (float32 or float64) in one call
     (block: threads per CTA, or (threads, register bound in resident 256-thread CTAs per
     SM); None = autotuned per shape). Returns (S (B, n), U (B, m, n), V (B, n, n),
     sweeps (B,)) unsorted, as the kernel leaves them."""

@@ -19,7 +19,7 @@ namespace vj {
 
 constexpr int BATCH_MAXN = 512;
 
-// what the steps of one launch share about the batch (batch.cu, k_plan)
+// what the launches of one call share about the batch (batch.cu, k_plan)
 struct BatchPlan {
   // work-queue heads: matrices for whole clusters, wide ones and the others for single CTAs
   unsigned next_large, next_wide, next;

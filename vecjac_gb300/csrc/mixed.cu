@@ -26,7 +26,7 @@
 // once (by the last Gram matrix, whose error is bounded, or by jsvd.cu's k_certify and k_confirm)
 // and skipped when it would transform nothing.
 // Measured, before (FP64 products by a library, FP64 sweeps, column-pair FP32 sweeps) and now:
-// 1024 x 1024 real 139 and 20.5 ms, 4096 x 2048 complex 1517 and 257 ms.
+// 1024 x 1024 real 139 and 20.4 ms, 4096 x 2048 complex 1517 and 251 to 260 ms (by machine).
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>

@@ -233,8 +233,8 @@ template <> struct FpOps<double> {
   double one, mzero, half;
   static __device__ __forceinline__ FpOps make()
   {
-    // (gridDim.z is 1 in every launch, which the assembler cannot know: it folds known
-    // constants back into the two-operand forms)
+    // (gridDim.z is 1 in every launch of a kernel that uses this, which the assembler cannot know: it folds
+    // known constants back into the two-operand forms)
     const int z = (int)gridDim.z - 1;
     FpOps o;
     o.one = __hiloint2double(0x3ff00000 + z, z);
