@@ -554,8 +554,17 @@ __device__ __forceinline__ Rot pair_rot(float ha, float hb, float cr, float ci, 
   const float cs = rsqrt_nr(fmaf(t, t, 1.f));
   const float sn = t * cs;
   r.c = cs;
-  r.sr = sn * (cr / ac);
-  r.si = sn * (ci / ac);
+  if (am < 1e-30f) {
+    // (|c| itself may be subnormal, where it has few bits left: the direction from quotients by the
+    // larger part, so that the rotation stays one)
+    const float u = cr / am, v = ci / am, s = rsqrt_nr(fmaf(u, u, v * v));
+    r.sr = sn * (u * s);
+    r.si = sn * (v * s);
+  }
+  else {
+    r.sr = sn * (cr / ac);
+    r.si = sn * (ci / ac);
+  }
   r.d1 = fmaf(-t, ac, ha);
   r.d2 = fmaf(t, ac, hb);
   r.go = 1;

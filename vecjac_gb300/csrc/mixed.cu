@@ -1058,6 +1058,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   const float tol = fmaxf(0.5f * sqrtf((float)m), 8.f) * 5.9604645e-8f;
   const unsigned maxsw = swp < 60u ? swp : 60u;
   unsigned total32 = 0;
+  bool dropped = false;  // a stage's W was not near unitary
   // the wall-clock time of each phase is kept for vj_last_mixed_phases (every phase ends
   // with a stream synchronisation, so host time is device time here); with VJ_TRACE=1 it
   // also goes to stderr
@@ -1185,8 +1186,10 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
       const double emax = asdbl(hst.cosmax), rn_ = std::sqrt((double)n);
       if (trace)
         std::fprintf(stderr, "mixed SVD stage %u: largest entry of W^H W - I %.2e\n", stage, emax);
-      if (!(emax < 0.03) || round == 8)
-        return VJ_ERR_CUDA;  // W was not near unitary
+      // (G and V are as the stages before left them: the FP64 phase takes it from there)
+      dropped = !(emax < 0.03) || round == 8;
+      if (dropped)
+        break;
       if (!cut_rows(T.re, T.im, n, n, nullptr, oa) || !cut_prod(M[2], nullptr, ob) ||
           !mult(oa, ob, T, 1, digits(emax)))
         return VJ_ERR_CUDA;
@@ -1194,6 +1197,10 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
       if (nd == 8 && next < 2e-17)
         break;
       nd = (next * next * rn_ < 2e-17) ? 8 : 6;
+    }
+    if (dropped) {
+      total32 -= sw;
+      break;
     }
     // 4. V <- V W (V_0 = I, so the first stage that rotates sets V = W), G <- G W; G's columns
     //    enter the product with their lengths' powers of two moved to the rows of W, so that the
@@ -1218,7 +1225,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   if (presweeps)
     presweeps[0] = total32;
   if (!total32) {
-    // nothing was rotated (zero matrix or columns already orthogonal): V := I
+    // nothing was rotated (zero matrix, columns already orthogonal, or a first stage dropped): V := I
     k_eye_p<double><<<grid2(n, n), 256, 0, s>>>(V, (long long)ldV, n, 1);
     if (CPLX)
       k_eye_p<double><<<grid2(n, n), 256, 0, s>>>(Vi, (long long)ldVi, n, 0);
@@ -1233,7 +1240,7 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
   //    whatever that and a refinement cannot improve goes to the sweeps, which run until no pair
   //    is left.
   bool certified = false;  // every cosine is below the finishing check's limit (k_generator's bound)
-  if (total32) {
+  if (total32 || dropped) {
     const double u = 1.1102230246251565e-16;
     const double tol64 = 0.5 * std::sqrt((double)m) * u;
     // the finishing check's limit (jsvd.cu, k_certify)
