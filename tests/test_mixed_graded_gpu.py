@@ -42,3 +42,17 @@ def test_graded(kind, m, n, cols, rows):
     assert np.max(np.abs(U.conj().T @ U - np.eye(n))) <= 32 * n * EPS
     assert np.max(np.abs(V.conj().T @ V - np.eye(n))) <= 32 * n * EPS
     assert np.max(np.abs(A @ V - U * s)) <= 32 * n * EPS * s.max()
+
+
+@pytest.mark.parametrize("kind", ["d", "z"])
+@pytest.mark.parametrize("m,n,cols", [(128, 64, 4), (160, 96, 12), (520, 272, 12), (1032, 1024, 12), (520, 272, 30)])
+def test_columns_to_their_own_length(kind, m, n, cols):
+    """A v_j - u_j sigma_j within 32 n eps sigma_j, for every j: a short column's v_j needs its small
+    entries, where A's columns are long, to their own accuracy. (The terms of A v_j are of the order of
+    sigma_j, so that the products here add less than n eps sigma_j.)"""
+    A = matrix(kind, m, n, cols, 0, seed=2)
+    r, U, V, s = mixed(kind, A)
+    assert r >= 0, r
+    assert np.max(np.linalg.norm(A @ V - U * s, axis=0) / s) <= 32 * n * EPS
+    assert np.max(np.abs(U.conj().T @ U - np.eye(n))) <= 32 * n * EPS
+    assert np.max(np.abs(V.conj().T @ V - np.eye(n))) <= 32 * n * EPS
