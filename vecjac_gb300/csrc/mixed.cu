@@ -1215,12 +1215,12 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     //    own entries couples large columns of G into small ones, which no orthonormalisation of
     //    W undoes; the descending order measured worse.)
     const Mat &T = M[0];
+    std::vector<int> hp((size_t)n), he;  // (read by copies that the first round's read_stats waits for)
     {
       double *nrm = vec;
       int *perm = reinterpret_cast<int *>(vec + n);
       k_colnorm2_f32<CPLX><<<(unsigned)n, 256, 0, s>>>(mi, G32, CPLX ? G32 + mn : nullptr, nrm);
       std::vector<double> hn((size_t)n);
-      std::vector<int> hp((size_t)n);
       if (cudaMemcpyAsync(hn.data(), nrm, (size_t)n * 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
           cudaStreamSynchronize(s) != cudaSuccess)
         return VJ_ERR_CUDA;
@@ -1232,7 +1232,6 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
       k_widen_cols<<<grid2(n, n), 256, 0, s>>>(ni, W32, perm, T.re);
       if (CPLX)
         k_widen_cols<<<grid2(n, n), 256, 0, s>>>(ni, W32 + nn, perm, T.im);
-      std::vector<int> he;
       if (graded) {
         // the lengths of the columns that W makes (FP32 has no shorter ones than 2^-149)
         he.resize((size_t)n);
@@ -1243,9 +1242,6 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
         if (cudaMemcpyAsync(ek, he.data(), (size_t)n * 4, cudaMemcpyHostToDevice, s) != cudaSuccess)
           return VJ_ERR_CUDA;
       }
-      // (the copies read the host vectors: wait for them)
-      if (cudaStreamSynchronize(s) != cudaSuccess)
-        return VJ_ERR_CUDA;
     }
     oz::Operand oa, ob;
     // (the Gram matrices before the last need no more digits than their own second-order terms
@@ -1280,13 +1276,15 @@ static vj_fint mixed_dev(vj_fnat m_, vj_fnat n_, double *G, vj_fnat ldG, double 
     // 4. V <- V W (V_0 = I, so the first stage that rotates sets V = W), G <- G W; G's columns
     //    enter the product with their lengths' powers of two moved to the rows of W, so that the
     //    digits resolve every column of the result to its own length
+    if (oz::row_exponents(sc, ek, s) != cudaSuccess)
+      return VJ_ERR_CUDA;
     if (total32 == sw) {
       if (!copy2d(V, ldV, T.re, n, n, n, s) || (CPLX && !copy2d(Vi, ldVi, T.im, n, n, n, s)))
         return VJ_ERR_CUDA;
     }
-    else if (oz::row_exponents(sc, ek, s) != cudaSuccess || !cut_prod(T, nullptr, ob) || !mult_cols(sv, T, ob, M[3], M[4], 0, 8))
+    else if (!cut_prod(T, nullptr, ob) || !mult_cols(sv, T, ob, M[3], M[4], 0, 8))
       return VJ_ERR_CUDA;
-    if (oz::row_exponents(sc, ek, s) != cudaSuccess || !cut_prod(T, ek, ob) || !mult_g(ek, ob, nullptr, 0, 8))
+    if (!cut_prod(T, ek, ob) || !mult_g(ek, ob, nullptr, 0, 8))
       return VJ_ERR_CUDA;
     {
       if (cudaStreamSynchronize(s) != cudaSuccess)
